@@ -12,6 +12,7 @@ from ctypes import c_char_p, c_int, c_int64, c_size_t, c_void_p
 
 _PKG = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_PKG, "libnanoquant_b200.so")
+EXT_PATH = os.path.join(_PKG, "_nq_torch.so")
 
 NQ_F16, NQ_BF16 = 0, 1
 NQ_LSB_FIRST, NQ_HALF2 = 0, 1
@@ -98,6 +99,24 @@ def lib() -> ctypes.CDLL:
             fn.restype, fn.argtypes = res, args
         _lib = L
     return _lib
+
+
+_ext = None
+
+
+def ext():
+    """The C++ host path between torch and the library (``csrc/nq_torch.cpp``): argument handling and launch of a
+    call in one native function.  Raises ``ImportError`` when it has not been built."""
+    global _ext
+    if _ext is None:
+        if not os.path.exists(EXT_PATH):
+            raise ImportError(f"{EXT_PATH} not found. Build it with `python -m nanoquant_b200.build`.")
+        import torch  # noqa: F401  the libraries the extension links against
+        from . import _nq_torch
+        from . import ops
+        ops.connect_host_path(_nq_torch)
+        _ext = _nq_torch
+    return _ext
 
 
 def check(status: int, what: str) -> None:

@@ -1,0 +1,497 @@
+// Host path between PyTorch and the C ABI: what happens on the CPU for one call of a quantised linear.
+//
+// A decode call runs 5 to 10 us on the GPU.  The same argument handling in Python (dispatcher to a Python
+// implementation, attribute reads, ctypes) took 30 to 36 us a call and was what an eager decode step ran at; here it
+// is one C++ function per call: type and shape checks, one output allocation, one C ABI call.
+//
+// Two ways in:
+//   * the CUDA implementations of torch.ops.binary_kernels.* (schemas: nanoquant_b200/ops.py), for operands in the
+//     kernels' tile layout; operands in the reference's layouts go to the Python implementation, which converts them
+//     once and keeps the result on the tensor;
+//   * plain functions for this package's own modules (no dispatcher).  They return None whenever a call is not the
+//     plain case (other types, tensor subclasses, dispatch modes, odd dimensions); the caller then takes the general route.
+#include <Python.h>
+
+#include <ATen/core/Tensor.h>
+#include <ATen/ops/as_strided.h>
+#include <ATen/ops/empty.h>
+#include <c10/core/impl/TorchDispatchModeTLS.h>
+#include <c10/cuda/CUDAFunctions.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/python_variable.h>
+#include <torch/csrc/utils/object_ptr.h>
+#include <torch/csrc/utils/pybind.h>
+#include <torch/library.h>
+
+#include <mutex>
+#include <optional>
+
+#include "nanoquant_b200.h"
+
+namespace {
+
+using at::Tensor;
+using OptTensor = std::optional<Tensor>;
+
+constexpr int kMaxLinears = 4;
+constexpr int kMaxDevices = 64;
+
+// ---------------------------------------------------------------------------------------------------------------
+// Python callbacks, set once by nanoquant_b200.ops
+// ---------------------------------------------------------------------------------------------------------------
+PyObject* g_raise_status = nullptr;    // (status, what): raises
+PyObject* g_grow_scratch = nullptr;    // (device index, bytes): makes the scratch hold that many bytes, or raises
+PyObject* g_dyn_general = nullptr;     // Python implementations of the operators (reference operand layouts)
+PyObject* g_marlin_general = nullptr;
+
+// Calls a Python function with the GIL held and throws its exception.
+PyObject* call_python(PyObject* fn, PyObject* args) {
+    TORCH_CHECK(fn != nullptr, "nanoquant_b200: the host extension has not been initialised");
+    PyObject* r = PyObject_CallObject(fn, args);
+    Py_DECREF(args);
+    if (!r) {
+        python_error err;
+        err.persist();
+        throw std::move(err);
+    }
+    return r;
+}
+
+[[noreturn]] void fail(int status, const char* what) {
+    pybind11::gil_scoped_acquire gil;
+    Py_XDECREF(call_python(g_raise_status, Py_BuildValue("(is)", status, what)));
+    TORCH_CHECK(false, what, ": nq_status ", status);
+}
+
+// ---------------------------------------------------------------------------------------------------------------
+// scratch: one buffer per device (owned by nanoquant_b200.ops, which keeps it alive), a thread may override it
+// ---------------------------------------------------------------------------------------------------------------
+struct Scratch {
+    void* ptr = nullptr;
+    size_t bytes = 0;
+};
+Scratch g_scratch[kMaxDevices];
+std::mutex g_scratch_mutex;            // pointer and size change together
+thread_local Scratch t_override;
+
+Scratch scratch_of(int dev) {
+    if (t_override.ptr) return t_override;
+    std::lock_guard<std::mutex> lock(g_scratch_mutex);
+    return g_scratch[dev];
+}
+
+void grow_scratch(int dev, size_t bytes) {
+    pybind11::gil_scoped_acquire gil;
+    Py_DECREF(call_python(g_grow_scratch, Py_BuildValue("(in)", dev, (Py_ssize_t)bytes)));
+}
+
+// ---------------------------------------------------------------------------------------------------------------
+// launches
+// ---------------------------------------------------------------------------------------------------------------
+// Makes `dev` current for the C ABI call if it is not (a query and nothing else in the usual case).
+struct OnDevice {
+    explicit OnDevice(int dev) {
+        if (c10::cuda::current_device() != dev) guard.emplace(dev);
+    }
+    std::optional<c10::cuda::CUDAGuard> guard;
+};
+
+int dtype_id(at::ScalarType t) { return t == at::kHalf ? NQ_F16 : NQ_BF16; }
+bool is_16bit(at::ScalarType t) { return t == at::kHalf || t == at::kBFloat16; }
+
+// Up to four linears at T tokens: the decode kernel for few tokens and for sizes the tensor-core path does not
+// take (columns or ranks that are no multiple of 8), the tensor-core path for the rest.
+void launch(nq_linear_desc* d, int n, int64_t T, int dtype, int dev) {
+    static const int gemv_max = nq_gemv_max_tokens();
+    bool gemv = T <= gemv_max;
+    if (!gemv && n == 1 && (d->N % 8 != 0 || d->R % 8 != 0)) gemv = true;
+    OnDevice on(dev);
+    const nq_stream_t stream = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)dev).stream();
+    const auto fwd = gemv ? nq_gemv_group_fwd : nq_gemm_group_fwd;
+    Scratch s = scratch_of(dev);
+    int st = s.ptr ? fwd(d, n, (int)T, dtype, s.ptr, s.bytes, stream) : (int)NQ_ERR_SCRATCH;
+    if (st == NQ_ERR_SCRATCH) {   // nothing has been launched: the scratch is checked first
+        grow_scratch(dev, gemv ? nq_gemv_group_scratch_bytes(d, n, (int)T) : nq_gemm_group_scratch_bytes(d, n, (int)T));
+        s = scratch_of(dev);
+        st = fwd(d, n, (int)T, dtype, s.ptr, s.bytes, stream);
+    }
+    if (st < 0) fail(st, gemv ? "nq_gemv_group_fwd" : "nq_gemm_group_fwd");
+}
+
+// A linear's operands.  `rank` comes from the caller: the tile layout pads it.
+struct Linear {
+    const Tensor *s_in, *v, *s_mid, *u, *s_out, *bias;
+    int64_t rank;
+};
+
+void describe(nq_linear_desc& d, const Linear& l, const void* x, int64_t N, int64_t ldx, void* y, int64_t ldy) {
+    d = nq_linear_desc{};
+    d.x = x;
+    d.s_in = l.s_in->const_data_ptr();
+    d.v_tiles = l.v->const_data_ptr();
+    d.s_mid = l.s_mid ? l.s_mid->const_data_ptr() : nullptr;
+    d.u_tiles = l.u->const_data_ptr();
+    d.s_out = l.s_out->const_data_ptr();
+    d.y = y;
+    d.N = (int)N;
+    d.R = (int)l.rank;
+    d.M = (int)l.s_out->size(0);
+    d.ldx = ldx;
+    d.ldy = ldy;
+    d.bias = l.bias ? l.bias->const_data_ptr() : nullptr;
+}
+
+Tensor new_output(at::IntArrayRef shape, const Tensor& like) {
+    return at::empty(shape, like.options().requires_grad(false));
+}
+
+// y[..., M] for a contiguous x[..., N]
+Tensor linear(const Tensor& x, const Linear& l) {
+    const int64_t N = x.size(-1), T = N ? x.numel() / N : 0, M = l.s_out->size(0);
+    c10::SmallVector<int64_t, 4> shape(x.sizes().begin(), x.sizes().end());
+    shape.back() = M;
+    Tensor y = new_output(shape, x);
+    if (T == 0) return y;
+    nq_linear_desc d;
+    describe(d, l, x.const_data_ptr(), N, N, y.mutable_data_ptr(), M);
+    launch(&d, 1, T, dtype_id(x.scalar_type()), x.get_device());
+    return y;
+}
+
+// ---------------------------------------------------------------------------------------------------------------
+// operators
+// ---------------------------------------------------------------------------------------------------------------
+void check_operand(const Tensor& t, const char* name, at::ScalarType dtype, const char* dtype_name) {
+    TORCH_CHECK(t.is_cuda(), name, " must be a CUDA tensor");
+    TORCH_CHECK(t.is_contiguous(), name, " must be contiguous");
+    TORCH_CHECK(t.scalar_type() == dtype, name, " must be ", dtype_name, " tensor");
+}
+
+// The reference dispatches its tuning arguments through compile-time lists and raises ValueError on a miss
+// (cuda/meta_utils.h:14-38, cuda/gemv_kernel.cu:351-354); the kernels here have no such knobs.
+void check_sweep(const char* name, int64_t v, std::initializer_list<int64_t> choices) {
+    for (int64_t c : choices)
+        if (c == v) return;
+    std::string list;
+    for (int64_t c : choices) list += (list.empty() ? "" : ", ") + std::to_string(c);
+    TORCH_CHECK_VALUE(false, name, " should be one of [", list, "], but ", v, " was given");
+}
+
+PyObject* wrap(const OptTensor& t) {
+    if (!t) Py_RETURN_NONE;
+    return THPVariable_Wrap(*t);
+}
+Tensor unwrap_result(PyObject* r) {
+    Tensor y = THPVariable_Unpack(r);
+    Py_DECREF(r);
+    return y;
+}
+
+Tensor nanoquant_dyn_forward(const Tensor& x, const Tensor& scale_g, const Tensor& Ubits, const OptTensor& scale_l,
+                             const Tensor& Vbits, const Tensor& scale_h, int64_t th1, int64_t th2, int64_t rpw1,
+                             int64_t rpw2, int64_t acc1, int64_t acc2, int64_t pipe1, int64_t pipe2) {
+    if (Ubits.dim() != 3 || Vbits.dim() != 3 || !scale_l) {   // operands to convert, or a rank to look up
+        pybind11::gil_scoped_acquire gil;
+        return unwrap_result(call_python(g_dyn_general, Py_BuildValue(
+            "(NNNNNNLLLLLLLL)", THPVariable_Wrap(x), THPVariable_Wrap(scale_g), THPVariable_Wrap(Ubits), wrap(scale_l),
+            THPVariable_Wrap(Vbits), THPVariable_Wrap(scale_h), (long long)th1, (long long)th2, (long long)rpw1,
+            (long long)rpw2, (long long)acc1, (long long)acc2, (long long)pipe1, (long long)pipe2)));
+    }
+    const at::ScalarType dt = x.scalar_type();   // checks in the order of the reference (cuda/gemv_kernel.cu:317-338)
+    TORCH_CHECK(is_16bit(dt), "Support only Half or BFloat16");
+    const char* name = dt == at::kHalf ? "float16" : "bfloat16";
+    check_operand(x, "x", dt, name);
+    check_operand(scale_g, "scale_g", dt, name);
+    check_operand(scale_h, "scale_h", dt, name);
+    check_operand(Ubits, "Ubits", at::kInt, "int32");
+    check_operand(Vbits, "Vbits", at::kInt, "int32");
+    check_operand(*scale_l, "(*scale_l)", dt, name);
+    TORCH_CHECK(scale_g.size(0) == x.size(-1), "scale_g size mismatch");
+    check_sweep("n_th1", th1, {64, 128, 256});
+    check_sweep("n_rpw1", rpw1, {1, 2, 4, 8});
+    check_sweep("n_acc1", acc1, {1, 2});
+    check_sweep("n_pipe1", pipe1, {1, 2, 4, 8, 16});
+    check_sweep("n_th2", th2, {64, 128, 256});
+    check_sweep("n_rpw2", rpw2, {1, 2, 4, 8});
+    check_sweep("n_acc2", acc2, {1, 2});
+    check_sweep("n_pipe2", pipe2, {1, 2, 4, 8, 16});
+    return linear(x, Linear{&scale_g, &Ubits, &*scale_l, &Vbits, &scale_h, nullptr, scale_l->size(0)});
+}
+
+// `weight_u` is the FIRST stage (module V), `weight_v` the second (reference cuda/gemm.cpp:112-122)
+Tensor marlin_nanoquant_forward(const Tensor& x, const Tensor& weight_u, const Tensor& weight_v, const OptTensor& scale_g,
+                                const OptTensor& scale_l, const OptTensor& scale_h, const Tensor& workspace) {
+    if (weight_u.dim() == 3 && scale_g && scale_l && scale_h && is_16bit(x.scalar_type()) && x.dim() == 2)
+        return linear(x.is_contiguous() ? x : x.contiguous(),
+                      Linear{&*scale_g, &weight_u, &*scale_l, &weight_v, &*scale_h, nullptr, scale_l->size(0)});
+    pybind11::gil_scoped_acquire gil;
+    return unwrap_result(call_python(g_marlin_general, Py_BuildValue(
+        "(NNNNNNN)", THPVariable_Wrap(x), THPVariable_Wrap(weight_u), THPVariable_Wrap(weight_v), wrap(scale_g),
+        wrap(scale_l), wrap(scale_h), THPVariable_Wrap(workspace))));
+}
+
+TORCH_LIBRARY_IMPL(binary_kernels, CUDA, m) {
+    m.impl("nanoquant_dyn_forward", nanoquant_dyn_forward);
+    m.impl("marlin_nanoquant_forward", marlin_nanoquant_forward);
+}
+
+// ---------------------------------------------------------------------------------------------------------------
+// plain functions
+// ---------------------------------------------------------------------------------------------------------------
+// A tensor argument without anything that would have to go through the dispatcher.
+const Tensor* plain(PyObject* o) {
+    if (!THPVariable_Check(o)) return nullptr;
+    const Tensor& t = THPVariable_Unpack(o);
+    return t.is_cuda() && t.layout() == at::kStrided ? &t : nullptr;
+}
+bool exact_plain(PyObject* o) { return THPVariable_CheckExact(o) && !c10::impl::dispatch_mode_enabled(); }
+
+// (s_in, v_tiles, s_mid | None, u_tiles, s_out, rank, bias | None) from `a[0..6]`; false: not the plain case.
+bool parse_linear(PyObject* const* a, at::ScalarType dt, int64_t N, Linear& l) {
+    auto vec = [&](PyObject* o, int64_t n) -> const Tensor* {
+        const Tensor* t = plain(o);
+        return t && t->scalar_type() == dt && t->dim() == 1 && (n < 0 || t->size(0) == n) && t->is_contiguous() ? t : nullptr;
+    };
+    auto tiles = [&](PyObject* o) -> const Tensor* {
+        const Tensor* t = plain(o);
+        return t && t->scalar_type() == at::kInt && t->dim() == 3 && t->is_contiguous() ? t : nullptr;
+    };
+    l.rank = PyLong_AsLongLong(a[5]);
+    if (l.rank <= 0) { PyErr_Clear(); return false; }
+    l.s_in = vec(a[0], N);
+    l.v = tiles(a[1]);
+    l.s_mid = a[2] == Py_None ? nullptr : vec(a[2], l.rank);
+    l.u = tiles(a[3]);
+    l.s_out = vec(a[4], -1);
+    if (!l.s_in || !l.v || !l.u || !l.s_out || (a[2] != Py_None && !l.s_mid)) return false;
+    const int64_t M = l.s_out->size(0);
+    l.bias = a[6] == Py_None ? nullptr : vec(a[6], M);
+    if (a[6] != Py_None && !l.bias) return false;
+    // the tiles are what the descriptor's sizes say: 16 rows x 256 columns each
+    return l.v->size(0) == (l.rank + 15) / 16 && l.v->size(1) == (N + 255) / 256 && l.u->size(0) == (M + 15) / 16 &&
+           l.u->size(1) == (l.rank + 255) / 256;
+}
+
+// linear_forward(x, s_in, v_tiles, s_mid, u_tiles, s_out, rank, bias) -> y or None
+PyObject* py_linear_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    TORCH_CHECK(n == 8, "linear_forward takes 8 arguments");
+    if (!exact_plain(a[0])) Py_RETURN_NONE;
+    const Tensor* x = plain(a[0]);
+    Linear l;
+    if (!x || !is_16bit(x->scalar_type()) || (x->dim() != 2 && x->dim() != 3) || !x->is_contiguous() ||
+        !parse_linear(a + 1, x->scalar_type(), x->size(-1), l))
+        Py_RETURN_NONE;
+    Tensor y;
+    {
+        pybind11::gil_scoped_release no_gil;
+        y = linear(*x, l);
+    }
+    return THPVariable_Wrap(y);
+    END_HANDLE_TH_ERRORS
+}
+
+// group_forward(x | [x...], [(s_in, v_tiles, s_mid, u_tiles, s_out, rank, bias)...], residuals | None) -> [y...] or None.
+// The outputs lie side by side in one [T, sum(M)] buffer.
+PyObject* py_group_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    TORCH_CHECK(n == 3, "group_forward takes 3 arguments");
+    if (!PyList_CheckExact(a[1])) Py_RETURN_NONE;
+    const Py_ssize_t count = PyList_GET_SIZE(a[1]);
+    const bool many = PyList_CheckExact(a[0]), res = a[2] != Py_None;
+    if (count < 1 || count > kMaxLinears || (many && PyList_GET_SIZE(a[0]) != count) ||
+        (res && (!PyList_CheckExact(a[2]) || PyList_GET_SIZE(a[2]) != count)))
+        Py_RETURN_NONE;
+    nq_linear_desc d[kMaxLinears];
+    Linear l[kMaxLinears];
+    const Tensor* x[kMaxLinears];
+    int64_t width = 0;
+    for (Py_ssize_t i = 0; i < count; ++i) {
+        PyObject* xo = many ? PyList_GET_ITEM(a[0], i) : a[0];
+        if (!exact_plain(xo)) Py_RETURN_NONE;
+        x[i] = plain(xo);
+        PyObject* t = PyList_GET_ITEM(a[1], i);
+        if (!x[i] || !is_16bit(x[i]->scalar_type()) || x[i]->scalar_type() != x[0]->scalar_type() || x[i]->dim() < 2 ||
+            !x[i]->is_contiguous() || !PyTuple_CheckExact(t) || PyTuple_GET_SIZE(t) != 7 ||
+            !parse_linear(&PyTuple_GET_ITEM(t, 0), x[0]->scalar_type(), x[i]->size(-1), l[i]) ||
+            x[i]->sizes().slice(0, x[i]->dim() - 1) != x[0]->sizes().slice(0, x[0]->dim() - 1))
+            Py_RETURN_NONE;
+        width += l[i].s_out->size(0);
+    }
+    const int64_t T = x[0]->size(-1) ? x[0]->numel() / x[0]->size(-1) : 0;
+    if (T == 0) Py_RETURN_NONE;
+    const Tensor* r[kMaxLinears] = {};
+    for (Py_ssize_t i = 0; res && i < count; ++i) {
+        PyObject* ro = PyList_GET_ITEM(a[2], i);
+        if (ro == Py_None) continue;
+        r[i] = exact_plain(ro) ? plain(ro) : nullptr;
+        const int64_t M = l[i].s_out->size(0);
+        if (!r[i] || r[i]->scalar_type() != x[0]->scalar_type() || !r[i]->is_contiguous() || r[i]->size(-1) != M || r[i]->numel() != T * M)
+            Py_RETURN_NONE;
+    }
+    Tensor out = new_output({T, width}, *x[0]);
+    char* base = static_cast<char*>(out.mutable_data_ptr());
+    int64_t col = 0;
+    for (Py_ssize_t i = 0; i < count; ++i) {
+        const int64_t N = x[i]->size(-1), M = l[i].s_out->size(0);
+        describe(d[i], l[i], x[i]->const_data_ptr(), N, N, base + 2 * col, width);
+        if (r[i]) {
+            d[i].residual = r[i]->const_data_ptr();
+            d[i].ldr = M;
+        }
+        col += M;
+    }
+    {
+        pybind11::gil_scoped_release no_gil;
+        launch(d, (int)count, T, dtype_id(out.scalar_type()), out.get_device());
+    }
+    THPObjectPtr list(PyList_New(count));
+    if (!list) return nullptr;
+    col = 0;
+    for (Py_ssize_t i = 0; i < count; ++i) {
+        // [..., M] column view with the leading dimensions of x: tokens are `width` elements apart
+        c10::SmallVector<int64_t, 4> shape(x[0]->sizes().begin(), x[0]->sizes().end());
+        c10::SmallVector<int64_t, 4> strides(shape.size());
+        shape.back() = l[i].s_out->size(0);
+        strides.back() = 1;
+        int64_t step = width;
+        for (int k = (int)shape.size() - 2; k >= 0; --k) {
+            strides[k] = step;
+            step *= shape[k];
+        }
+        PyObject* y = THPVariable_Wrap(out.as_strided(shape, strides, col));
+        if (!y) return nullptr;
+        PyList_SET_ITEM(list.get(), i, y);
+        col += shape.back();
+    }
+    return list.release();
+    END_HANDLE_TH_ERRORS
+}
+
+// dense_gemv_forward(x, weight, bias | None) -> y or None
+PyObject* py_dense_gemv_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    TORCH_CHECK(n == 3, "dense_gemv_forward takes 3 arguments");
+    if (!exact_plain(a[0])) Py_RETURN_NONE;
+    const Tensor *x = plain(a[0]), *w = plain(a[1]), *b = a[2] == Py_None ? nullptr : plain(a[2]);
+    if (!x || !w || (a[2] != Py_None && !b) || !is_16bit(x->scalar_type()) || w->scalar_type() != x->scalar_type() ||
+        w->dim() != 2 || w->stride(1) != 1 || !x->is_contiguous() || x->dim() < 1 || x->size(-1) != w->size(1) || x->numel() == 0)
+        Py_RETURN_NONE;
+    const int64_t V = w->size(0), N = w->size(1), T = x->numel() / N;
+    if (b && (b->scalar_type() != x->scalar_type() || !b->is_contiguous() || b->numel() != V)) Py_RETURN_NONE;
+    c10::SmallVector<int64_t, 4> shape(x->sizes().begin(), x->sizes().end());
+    shape.back() = V;
+    Tensor y = new_output(shape, *x);
+    const int dev = x->get_device();
+    OnDevice on(dev);
+    const int st = nq_dense_gemv_fwd(x->const_data_ptr(), w->const_data_ptr(), b ? b->const_data_ptr() : nullptr,
+                                     y.mutable_data_ptr(), (int)T, (int)N, (int)V, w->stride(0), V, dtype_id(x->scalar_type()),
+                                     c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)dev).stream());
+    if (st < 0) fail(st, "nq_dense_gemv_fwd");
+    return THPVariable_Wrap(y);
+    END_HANDLE_TH_ERRORS
+}
+
+// repack(op, src, rows, cols, order) -> out or None: the pack / layout kernels on a contiguous CUDA tensor
+//   0 pack_rows, 1 unpack_rows, 2 rows_to_tiles, 3 tiles_to_rows, 4 pack_marlin (rows = out features)
+PyObject* py_repack(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    TORCH_CHECK(n == 5, "repack takes 5 arguments");
+    const Tensor* src = plain(a[1]);
+    const long op = PyLong_AsLong(a[0]), order = PyLong_AsLong(a[4]);
+    const int64_t rows = PyLong_AsLongLong(a[2]), cols = PyLong_AsLongLong(a[3]);
+    if (PyErr_Occurred()) return nullptr;
+    const bool dense = op == 0 || op == 4;
+    if (!src || !src->is_contiguous() || src->scalar_type() != (dense ? at::kChar : at::kInt)) Py_RETURN_NONE;
+    const int64_t words = (cols + 31) / 32, row_groups = (rows + 15) / 16, chunks = (cols + 255) / 256;
+    Tensor out;
+    const auto ints = src->options().dtype(at::kInt);
+    if (op == 0) out = at::empty({rows, words}, ints);
+    else if (op == 1) out = at::empty({rows, cols}, src->options().dtype(at::kChar));
+    else if (op == 2) out = at::empty({row_groups, chunks, 128}, ints);
+    else if (op == 3) out = at::empty({rows, words}, ints);
+    else if (op == 4) out = at::empty({cols / 16, rows / 2}, ints);
+    else Py_RETURN_NONE;
+    const int dev = src->get_device();
+    OnDevice on(dev);
+    const nq_stream_t stream = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)dev).stream();
+    const void* in = src->const_data_ptr();
+    void* o = out.mutable_data_ptr();
+    static const char* const kNames[5] = {"nq_pack_rows", "nq_unpack_rows", "nq_rows_to_tiles", "nq_tiles_to_rows", "nq_pack_marlin"};
+    const int st = op == 0   ? nq_pack_rows(static_cast<const int8_t*>(in), static_cast<int32_t*>(o), rows, cols, (int)order, stream)
+                   : op == 1 ? nq_unpack_rows(static_cast<const int32_t*>(in), static_cast<int8_t*>(o), rows, cols, (int)order, stream)
+                   : op == 2 ? nq_rows_to_tiles(static_cast<const int32_t*>(in), o, rows, cols, (int)order, stream)
+                   : op == 3 ? nq_tiles_to_rows(in, static_cast<int32_t*>(o), rows, cols, (int)order, stream)
+                             : nq_pack_marlin(static_cast<const int8_t*>(in), static_cast<int32_t*>(o), rows, cols, stream);
+    if (st < 0) fail(st, kNames[op]);
+    return THPVariable_Wrap(out);
+    END_HANDLE_TH_ERRORS
+}
+
+// permute_scale(s, kind, inverse) -> permuted copy or None
+PyObject* py_permute_scale(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    TORCH_CHECK(n == 3, "permute_scale takes 3 arguments");
+    const Tensor* s = plain(a[0]);
+    if (!s || !s->is_contiguous() || s->element_size() != 2) Py_RETURN_NONE;
+    const int kind = (int)PyLong_AsLong(a[1]), inverse = (int)PyLong_AsLong(a[2]);
+    if (PyErr_Occurred()) return nullptr;
+    Tensor out = new_output({s->numel()}, *s);
+    const int dev = s->get_device();
+    OnDevice on(dev);
+    const int st = nq_permute_scale16(s->const_data_ptr(), out.mutable_data_ptr(), s->numel(), kind, inverse,
+                                      c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)dev).stream());
+    if (st < 0) fail(st, "nq_permute_scale16");
+    return THPVariable_Wrap(out);
+    END_HANDLE_TH_ERRORS
+}
+
+// set_scratch(device, address, bytes); set_thread_scratch(address, bytes), address 0: none
+PyObject* py_set_scratch(PyObject*, PyObject* args) {
+    int dev;
+    unsigned long long ptr, bytes;
+    if (!PyArg_ParseTuple(args, "iKK", &dev, &ptr, &bytes)) return nullptr;
+    if (dev < 0 || dev >= kMaxDevices) {
+        PyErr_SetString(PyExc_ValueError, "device index out of range");
+        return nullptr;
+    }
+    std::lock_guard<std::mutex> lock(g_scratch_mutex);
+    g_scratch[dev] = Scratch{reinterpret_cast<void*>(ptr), (size_t)bytes};
+    Py_RETURN_NONE;
+}
+PyObject* py_set_thread_scratch(PyObject*, PyObject* args) {
+    unsigned long long ptr, bytes;
+    if (!PyArg_ParseTuple(args, "KK", &ptr, &bytes)) return nullptr;
+    t_override = Scratch{reinterpret_cast<void*>(ptr), (size_t)bytes};
+    Py_RETURN_NONE;
+}
+// set_callbacks(raise_status, grow_scratch, dyn_general, marlin_general)
+PyObject* py_set_callbacks(PyObject*, PyObject* args) {
+    PyObject* f[4];
+    if (!PyArg_ParseTuple(args, "OOOO", &f[0], &f[1], &f[2], &f[3])) return nullptr;
+    PyObject** slot[4] = {&g_raise_status, &g_grow_scratch, &g_dyn_general, &g_marlin_general};
+    for (int i = 0; i < 4; ++i) {
+        Py_INCREF(f[i]);
+        Py_XDECREF(*slot[i]);
+        *slot[i] = f[i];
+    }
+    Py_RETURN_NONE;
+}
+
+PyMethodDef kMethods[] = {
+    {"linear_forward", (PyCFunction)(void*)py_linear_forward, METH_FASTCALL, nullptr},
+    {"group_forward", (PyCFunction)(void*)py_group_forward, METH_FASTCALL, nullptr},
+    {"dense_gemv_forward", (PyCFunction)(void*)py_dense_gemv_forward, METH_FASTCALL, nullptr},
+    {"repack", (PyCFunction)(void*)py_repack, METH_FASTCALL, nullptr},
+    {"permute_scale", (PyCFunction)(void*)py_permute_scale, METH_FASTCALL, nullptr},
+    {"set_scratch", py_set_scratch, METH_VARARGS, nullptr},
+    {"set_thread_scratch", py_set_thread_scratch, METH_VARARGS, nullptr},
+    {"set_callbacks", py_set_callbacks, METH_VARARGS, nullptr},
+    {nullptr, nullptr, 0, nullptr}};
+PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_nq_torch", nullptr, -1, kMethods, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__nq_torch() { return PyModule_Create(&kModule); }

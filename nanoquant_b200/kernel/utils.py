@@ -33,6 +33,22 @@ def _to_cuda(t: torch.Tensor) -> torch.Tensor:
     return t.contiguous().cuda()
 
 
+def _int32(t: torch.Tensor) -> torch.Tensor:
+    return t if t.dtype == torch.int32 else t.to(torch.int32)
+
+
+_PACK_ROWS, _UNPACK_ROWS, _ROWS_TO_TILES, _TILES_TO_ROWS, _PACK_MARLIN = range(5)   # operations of `repack`
+
+
+def _repack(op: int, src: torch.Tensor, rows: int, cols: int, order: int = 0) -> torch.Tensor:
+    """One pack / layout kernel on `src` (staged to the GPU if it is not there), result on `src`'s device."""
+    ext = _lib.ext()
+    out = ext.repack(op, src, rows, cols, order)
+    if out is None:   # not a plain contiguous CUDA tensor
+        out = ext.repack(op, _to_cuda(src.detach()), rows, cols, order).to(src.device)
+    return out
+
+
 def _check_method(method: str) -> int:
     if method not in _lib.ORDER_ID:
         raise ValueError(f"Unsupported method: '{method}'. Supported methods are 'lsb_first', 'half2'.")
@@ -64,12 +80,7 @@ def pack_binary_gemv(tensor: torch.Tensor, method: str = "lsb_first") -> torch.T
         raise TypeError("Input tensor must be int8.")
     order = _check_method(method)
     rows, cols = tensor.shape
-    src = _to_cuda(tensor)
-    out = torch.empty((rows, (cols + 31) // 32), dtype=torch.int32, device=src.device)
-    with torch.cuda.device(src.device):
-        _lib.check(_lib.lib().nq_pack_rows(src.data_ptr(), out.data_ptr(), rows, cols, order,
-                                           _stream(src.device)), "nq_pack_rows")
-    return out.to(tensor.device)
+    return _repack(_PACK_ROWS, tensor, rows, cols, order)
 
 
 def unpack_binary_gemv(packed_tensor: torch.Tensor, original_shape: Tuple[int, int],
@@ -85,12 +96,7 @@ def unpack_binary_gemv(packed_tensor: torch.Tensor, original_shape: Tuple[int, i
         raise ValueError(
             f"Unsupported packed tensor shape. Expected ({rows}, {words}), got {packed_tensor.shape}.")
     order = _check_method(method)
-    src = _to_cuda(packed_tensor.to(torch.int32))
-    out = torch.empty((rows, cols), dtype=torch.int8, device=src.device)
-    with torch.cuda.device(src.device):
-        _lib.check(_lib.lib().nq_unpack_rows(src.data_ptr(), out.data_ptr(), rows, cols, order,
-                                             _stream(src.device)), "nq_unpack_rows")
-    return out.to(packed_tensor.device)
+    return _repack(_UNPACK_ROWS, _int32(packed_tensor), rows, cols, order)
 
 
 def reorder_packed(packed: torch.Tensor, method_in: str, method_out: str) -> torch.Tensor:
@@ -111,12 +117,10 @@ def _permute_scale(s: torch.Tensor, kind: int, inverse: bool = False) -> torch.T
         raise RuntimeError(f"scale of {s.numel()} elements is not a multiple of {group}")
     if s.element_size() != 2:
         raise TypeError("scale vectors must be fp16 or bf16 (the dtypes the kernels compute in)")
-    src = _to_cuda(s.reshape(-1))
-    out = torch.empty_like(src)
-    with torch.cuda.device(src.device):
-        _lib.check(_lib.lib().nq_permute_scale16(src.data_ptr(), out.data_ptr(), src.numel(), kind,
-                                                 int(inverse), _stream(src.device)), "nq_permute_scale16")
-    return out.to(s.device)
+    out = _lib.ext().permute_scale(s, kind, int(inverse))
+    if out is None:   # not a plain contiguous CUDA tensor
+        out = _lib.ext().permute_scale(_to_cuda(s.detach().reshape(-1)), kind, int(inverse)).to(s.device)
+    return out
 
 
 def pack_binary_marlin(weight: torch.Tensor, scale_in: torch.Tensor, scale_out: torch.Tensor):
@@ -126,15 +130,11 @@ def pack_binary_marlin(weight: torch.Tensor, scale_in: torch.Tensor, scale_out: 
     if out_f % 64 or in_f % 16:
         raise RuntimeError(f"shape '[{out_f // 64}, 4, 2, 8, {in_f // 16}, 2, 4, 2]' is invalid for input of size "
                            f"{out_f * in_f}")
-    src = _to_cuda(weight.to(torch.int8))
-    B = torch.empty((in_f // 16, out_f // 2), dtype=torch.int32, device=src.device)
-    with torch.cuda.device(src.device):
-        _lib.check(_lib.lib().nq_pack_marlin(src.data_ptr(), B.data_ptr(), out_f, in_f,
-                                             _stream(src.device)), "nq_pack_marlin")
+    B = _repack(_PACK_MARLIN, weight if weight.dtype == torch.int8 else weight.to(torch.int8), out_f, in_f)
     s_in = _permute_scale(scale_in, 0)
     s_out = _permute_scale(scale_out, 1)
     workspace_size = s_out.numel() // 128 * MARLIN_MIN_MAX_PAR
-    return B.to(weight.device), s_in, s_out, workspace_size
+    return B, s_in, s_out, workspace_size
 
 
 def pack_binary_marlin_fused(V_sign: torch.Tensor, U_sign: torch.Tensor, scale_g: torch.Tensor,
@@ -172,11 +172,8 @@ def pack_tiles(packed: torch.Tensor, shape: Tuple[int, int], method: str = "lsb_
     rows, cols = int(shape[0]), int(shape[1])
     if tuple(packed.shape) != (rows, (cols + 31) // 32):
         raise ValueError(f"packed tensor of shape {tuple(packed.shape)} does not hold a {rows}x{cols} matrix")
-    src = _to_cuda(packed.to(torch.int32))
-    out = torch.empty(tiles_shape(rows, cols), dtype=torch.int32, device=src.device)
-    with torch.cuda.device(src.device):
-        _lib.check(_lib.lib().nq_rows_to_tiles(src.data_ptr(), out.data_ptr(), rows, cols, _check_method(method),
-                                               _stream(src.device)), "nq_rows_to_tiles")
+    packed = _int32(packed if packed.is_cuda else _to_cuda(packed))
+    out = _repack(_ROWS_TO_TILES, packed, rows, cols, _check_method(method))
     out._nq_rows, out._nq_cols = rows, cols   # exact shape: the tiles pad rows to 16 and columns to 256
     return out
 
@@ -186,12 +183,7 @@ def unpack_tiles(tiles: torch.Tensor, shape: Tuple[int, int], method: str = "lsb
     rows, cols = int(shape[0]), int(shape[1])
     if tuple(tiles.shape) != tiles_shape(rows, cols):
         raise ValueError(f"tile tensor of shape {tuple(tiles.shape)} does not hold a {rows}x{cols} matrix")
-    src = _to_cuda(tiles)
-    out = torch.empty((rows, (cols + 31) // 32), dtype=torch.int32, device=src.device)
-    with torch.cuda.device(src.device):
-        _lib.check(_lib.lib().nq_tiles_to_rows(src.data_ptr(), out.data_ptr(), rows, cols, _check_method(method),
-                                               _stream(src.device)), "nq_tiles_to_rows")
-    return out
+    return _repack(_TILES_TO_ROWS, tiles if tiles.is_cuda else _to_cuda(tiles), rows, cols, _check_method(method))
 
 
 # reference aliases (kernel/utils.py:503-507)

@@ -12,7 +12,7 @@ from typing import List, Optional, Sequence
 
 import torch
 
-from .. import ops
+from .. import _lib, ops
 from .linear import NanoQuantLinear
 
 
@@ -32,7 +32,7 @@ class LinearGroup:
         # scratch for this group at decode batches and at up to 64 tokens, reserved now: a forward (or a stream
         # capture) then only reads the buffer's address
         shapes = [(m.in_features, m.rank, m.out_features) for m in self.modules]
-        device = self.modules[0].scale_post.device
+        device = self.modules[0].V_int8.device
         ops.reserve_scratch(device, max(ops.group_scratch_bytes(shapes, T) for T in (4, 24, 64)))
 
     @staticmethod
@@ -45,6 +45,13 @@ class LinearGroup:
                  out: Optional[torch.Tensor] = None) -> List[torch.Tensor]:
         """`x`: one ``[..., N]`` tensor for all linears, or one per linear.  Returns one ``[..., M_i]`` tensor per
         linear (column views of one buffer)."""
+        if out is None and not torch.compiler.is_compiling():
+            layers = [m.launch_operands() for m in self.modules]
+            if None not in layers:
+                ys = _lib.ext().group_forward(list(x) if isinstance(x, (list, tuple)) else x, layers,
+                                              None if residuals is None else list(residuals))
+                if ys is not None:
+                    return ys
         xs = list(x) if isinstance(x, (list, tuple)) else [x] * len(self.modules)
         lead = xs[0].shape[:-1]
         xs2 = []

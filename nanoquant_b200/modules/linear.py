@@ -13,6 +13,7 @@ from __future__ import annotations
 import torch
 import torch.nn as nn
 
+from .. import _lib
 from ..kernel.utils import binary_packer, get_kernel_function, pack_tiles
 
 # tuning arguments the reference passes to its GEMV (modules/linear.py:176-185); validated, then unused
@@ -61,6 +62,13 @@ class NanoQuantLinear(nn.Module):
         if not getattr(self, "do_kernel_inference", False):
             raise RuntimeError("NanoQuantLinear: call _prepare_kernel() first; this package implements the "
                                "CUDA kernel inference path only (no dense PyTorch forward)")
+        if not torch.compiler.is_compiling():
+            # One native call from here to the launch: on 16-bit contiguous CUDA activations this forward would spend
+            # four times the kernel's run time on dispatch otherwise.  None: not such a call, take the general route.
+            layer = self.launch_operands()
+            y = None if layer is None else _lib.ext().linear_forward(x, *layer)
+            if y is not None:
+                return y
         orig_dtype = x.dtype
         if x.dtype != self.dtype:
             x = x.to(self.dtype)
@@ -94,6 +102,19 @@ class NanoQuantLinear(nn.Module):
         if original_shape is not None:
             y = y.view(original_shape[0], original_shape[1], -1)
         return y.to(orig_dtype) if y.dtype != orig_dtype else y
+
+    def launch_operands(self):
+        """``(s_in, v_tiles, s_mid, u_tiles, s_out, rank, bias)`` as the launch takes them, read from the module's own
+        dictionaries (an attribute read of a registered parameter goes through ``nn.Module.__getattr__``, 0.4 us each);
+        None before ``_prepare_kernel`` or when a bias still has another type than the activations."""
+        d = self.__dict__
+        p = d["_parameters"]
+        bias = p.get("bias")
+        if bias is not None and bias.dtype is not d["dtype"]:
+            return None
+        if d["kernel_type"] == "gemv":
+            return (p["scale_pre"], d["V_int8"], p.get("scale_mid"), d["U_int8"], p["scale_post"], d["rank"], bias)
+        return (p["s1"], d["V_int8"], p["s2"], d["U_int8"], p["s3"], d["rank"], bias)
 
     # ------------------------------------------------------------ kernel set-up
     def _squeeze_scales(self, dtype):

@@ -7,6 +7,11 @@ ABI with ``data_ptr()`` and the current stream, fake (Meta) implementations
 give shapes for tracing (``pybind.cpp:11-31``, ``cuda/gemm.cpp:100-134``).
 Nothing here computes on the CPU.
 
+A call with operands in the tile layout runs in C++ from the dispatcher to the
+launch (``csrc/nq_torch.cpp``); the Python implementations below serve operands
+in the reference's layouts, which are converted and cached here, and every
+unusual call of the plain functions.
+
 Operand layouts accepted by ``nanoquant_dyn_forward``:
 
 * 2-D int32 ``[rows, cols/32]`` in ``half2`` bit order — what the reference's
@@ -69,7 +74,17 @@ def reserve_scratch(device: torch.device, nbytes: int) -> torch.Tensor:
             _retired.append(buf)   # a CUDA graph captured earlier may still point at the smaller buffer: keep it alive
         buf = torch.zeros(max(int(nbytes), _SCRATCH_MIN), dtype=torch.uint8, device=torch.device("cuda", idx))
         _scratch[idx] = buf
+        _lib.ext().set_scratch(idx, buf.data_ptr(), buf.numel())
     return buf
+
+
+def connect_host_path(ext) -> None:
+    """Give the C++ host path (``csrc/nq_torch.cpp``) what it calls back for: errors, scratch growth and the Python
+    implementations of the operators."""
+    ext.set_callbacks(_lib.check, lambda idx, nbytes: scratch_for(torch.device("cuda", idx), nbytes),
+                      _nanoquant_dyn_forward_cuda, _marlin_nanoquant_forward_cuda)
+    for idx, buf in _scratch.items():
+        ext.set_scratch(idx, buf.data_ptr(), buf.numel())
 
 
 def set_precise_intermediate(on: bool) -> bool:
@@ -108,11 +123,16 @@ def private_scratch(buf: torch.Tensor):
     """Run the enclosed launches of this thread on `buf` (uint8, zeroed once by the caller, 16-byte aligned)
     instead of the device's shared scratch: for concurrent streams."""
     prev = getattr(_override, "buf", None)
-    _override.buf = buf
+    _set_override(buf)
     try:
         yield buf
     finally:
-        _override.buf = prev
+        _set_override(prev)
+
+
+def _set_override(buf: Optional[torch.Tensor]) -> None:
+    _override.buf = buf
+    _lib.ext().set_thread_scratch(*((0, 0) if buf is None else (buf.data_ptr(), buf.numel())))
 
 
 def _dtype_id(t: torch.Tensor) -> int:
@@ -174,6 +194,9 @@ def dense_gemv_forward(x: torch.Tensor, weight: torch.Tensor, bias: Optional[tor
     For the layers the reference leaves as ``nn.Linear`` (``lm_head``, ``utils/load_utils.py:322``): ``weight``
     ``[V, N]`` fp16/bf16 with a unit inner stride, ``x`` ``[..., N]`` with at most ``nq_dense_gemv_max_tokens()``
     rows in total; more rows raise (a batched GEMM is the right tool there)."""
+    y = _lib.ext().dense_gemv_forward(x, weight, bias)
+    if y is not None:
+        return y
     _check_cuda_cont(x, "x", weight.dtype, str(weight.dtype))
     if weight.dim() != 2 or weight.stride(1) != 1 or not weight.is_cuda:
         raise RuntimeError("weight must be a CUDA [V, N] matrix with a unit inner stride")
@@ -443,7 +466,6 @@ def define_ops() -> None:
         "int num_thread_stage1=128, int num_thread_stage2=128, int num_row_per_warp_stage1=2, "
         "int num_row_per_warp_stage2=2, int num_acc_stage1=4, int num_acc_stage2=4, "
         "int num_pipeline_stage1=2, int num_pipeline_stage2=2) -> Tensor")
-    torch.library.impl("binary_kernels::nanoquant_dyn_forward", "CUDA")(_nanoquant_dyn_forward_cuda)
     torch.library.register_fake("binary_kernels::nanoquant_dyn_forward")(_nanoquant_dyn_forward_fake)
     torch.library.define(
         "binary_kernels::marlin_onebit_forward",
@@ -454,6 +476,10 @@ def define_ops() -> None:
         "binary_kernels::marlin_nanoquant_forward",
         "(Tensor x, Tensor weight_u, Tensor weight_v, Tensor? scale_g, Tensor? scale_l, Tensor? scale_h, "
         "Tensor(a!) workspace) -> Tensor")
-    torch.library.impl("binary_kernels::marlin_nanoquant_forward", "CUDA")(_marlin_nanoquant_forward_cuda)
     torch.library.register_fake("binary_kernels::marlin_nanoquant_forward")(_marlin_nanoquant_forward_fake)
+    # the CUDA implementations of the other two operators; without the built extension (schemas and tracing only) a
+    # call on CUDA tensors fails in the dispatcher
+    import os
+    if os.path.exists(_lib.EXT_PATH):
+        _lib.ext()
     _DEFINED = True

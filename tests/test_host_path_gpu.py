@@ -1,0 +1,58 @@
+"""The native host path of the modules against the general route, which serves every call it does not take."""
+import pytest
+import torch
+
+from oracle import nanoquant_oracle as oc
+from tests.util import exact_np
+
+pytestmark = pytest.mark.gpu
+
+
+def _module(N, R, M, dtype, kernel, bias, seed):
+    from nanoquant_b200.modules.linear import NanoQuantLinear
+    d = oc.synth_linear(N, R, M, 1, seed=seed)
+    t = lambda a: torch.from_numpy(a)
+    m = NanoQuantLinear(N, M, R)
+    if bias:
+        m.bias = torch.nn.Parameter(torch.linspace(-1, 1, M).to(dtype).cuda(), requires_grad=False)
+    s = lambda k: t(d[k]).float().to(dtype)
+    m.load_packed(t(oc.pack_rows(d["V"], "lsb_first")), (R, N), t(oc.pack_rows(d["U"], "lsb_first")), (M, R), s("s_pre"),
+                  s("s_post"), s("s_mid"), dtype=dtype, kernel_type=kernel)
+    return m, d
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("kernel,bias", [("gemv", False), ("gemv", True), ("gemm", False), ("gemm", True)])
+@pytest.mark.parametrize("lead", [(1,), (3, 1), (2, 17)])
+def test_module_call_equals_the_general_route(dtype, kernel, bias, lead):
+    from nanoquant_b200 import _lib, ops
+    m, d = _module(256, 96, 200, dtype, kernel, bias, seed=5)
+    x = torch.randn(*lead, 256, device="cuda").to(dtype)
+    ops_of = m.launch_operands()
+    assert _lib.ext().linear_forward(x, *ops_of) is not None          # the native path takes this call
+    want = ops.linear_forward(x.reshape(-1, 256), *ops_of[:6], bias=ops_of[6]).view(*lead, 200)
+    assert torch.equal(m(x), want)
+    # calls it leaves alone: other dtype, a strided input, a residual of another type
+    assert _lib.ext().linear_forward(x.float(), *ops_of) is None
+    assert torch.equal(m(x.float()).to(dtype), want)
+    wide = torch.zeros(*lead, 512, device="cuda", dtype=dtype)
+    wide[..., ::2] = x
+    assert torch.equal(m(wide[..., ::2]), want)
+    y64 = oc.forward_fp64(exact_np(x.reshape(-1, 256)), d["V"], d["U"], *[exact_np(t) for t in (ops_of[0], ops_of[2], ops_of[4])],
+                          **({"bias": exact_np(ops_of[6])} if bias else {}))
+    assert oc.rel_err(exact_np(want.reshape(-1, 200)), y64) <= 2e-3 + 2.0 ** -8
+
+
+@pytest.mark.parametrize("T", [1, 4, 5, 33])
+def test_group_call_equals_the_general_route(T):
+    from nanoquant_b200 import ops
+    from nanoquant_b200.modules.group import LinearGroup
+    mods = [_module(256, 96, M, torch.bfloat16, "gemv", M == 64, seed=M)[0] for M in (200, 64)]
+    x = torch.randn(T, 256, device="cuda").to(torch.bfloat16)
+    res = [torch.randn(T, 200, device="cuda").to(torch.bfloat16), None]
+    lay = [m.launch_operands() for m in mods]
+    for r in (None, res):
+        want = ops.group_forward([x, x], [a[:6] for a in lay], T, torch.bfloat16, x.device, [a[6] for a in lay], r)
+        got = LinearGroup(mods)(x.view(T, 1, 256), residuals=r)
+        assert [tuple(y.shape) for y in got] == [(T, 1, 200), (T, 1, 64)]
+        assert all(torch.equal(a.reshape(T, -1), b) for a, b in zip(got, want))
