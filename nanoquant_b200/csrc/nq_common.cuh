@@ -43,7 +43,8 @@ int sm_count();
 // store; a consumer CTA of the same launch loads the pairs it needs and repeats the load until every tag
 // equals the tag of this launch.  The first poll after the last producer store has landed already returns
 // the data, which takes an arrive / poll / reload sequence (three memory round trips) and any device-wide
-// barrier off the critical path.  Consumers spin on other CTAs, so the launch must be cooperative.
+// barrier off the critical path.  Consumers spin on other CTAs, so either every CTA of the launch is known to be
+// resident, or a consumer that polls in vain computes what is missing itself.
 //
 // The tag is the launch count of the scratch buffer, read from a 64-bit arrival counter in its header:
 // every launch advances it by exactly kTagSpan (the first CTA adds kTagSpan - (CTAs - 1), every other CTA
@@ -63,28 +64,30 @@ struct TagCtx {
     unsigned limit;      // polls a wait of this thread may still spend; 0 after an expiry (sticky: one missing
                          // producer costs every thread one limit, not one limit per element it waits for)
     unsigned* status;    // device status word (header word 2)
-    unsigned begun;      // tag and status have been read
 };
-// Reads the launch tag and the status word of the scratch header.  Issue it AFTER the first data loads of the
-// kernel: its results are first needed when a tag is compared or stored, so the round trips overlap.  A status
+// The launch counter and the status word of the scratch header as they are read: issue the read with the first data
+// loads of the kernel and finish it where a tag is first compared or stored, so that the round trips overlap.  A status
 // left by an earlier expiry on this scratch disables spinning altogether (the data of such a launch is void anyway).
-__device__ __forceinline__ void tag_begin(TagCtx& tc, unsigned* header, unsigned limit) {
-    unsigned long long c;
-    unsigned st;
-    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(c) : "l"(header) : "memory");
-    asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(st) : "l"(header + 2) : "memory");
-    tc.tag = 0x7FF00000u | ((unsigned)(c / kTagSpan) & 0xFFFFFu);
-    tc.limit = st ? 0u : limit;
+struct TagRaw {
+    unsigned long long counter;
+    unsigned status;
+};
+__device__ __forceinline__ void tag_read(TagRaw& r, const unsigned* header) {
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(r.counter) : "l"(header) : "memory");
+    asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(r.status) : "l"(header + 2) : "memory");
+}
+__device__ __forceinline__ void tag_finish(TagCtx& tc, const TagRaw& r, unsigned* header, unsigned limit) {
+    tc.tag = 0x7FF00000u | ((unsigned)(r.counter / kTagSpan) & 0xFFFFFu);
+    tc.limit = r.status ? 0u : limit;
     tc.status = header + 2;
-    tc.begun = 1u;
 }
 __device__ __forceinline__ void tag_wait_expired(TagCtx& tc) {
     atomicExch(tc.status, (unsigned)(-NQ_ERR_TIMEOUT));
     tc.limit = 0u;
 }
-// This CTA's arrival at the counter.  Issued by one thread, once per launch, after a CTA barrier that every
-// thread passes behind its own tag_begin() read: the arrival that completes the span would otherwise show
-// the next launch's tag to a thread of the same CTA that reads late.
+// This CTA's arrival at the counter.  Issued by one thread, once per launch, after a CTA barrier that every thread
+// passes behind the first USE of its tag (a load that has only been issued may still be on its way): the arrival that
+// completes the span would otherwise show the next launch's tag to a thread of the same CTA that reads late.
 __device__ __forceinline__ void launch_arrive(unsigned long long* counter, bool first_cta, unsigned n_ctas) {
     const unsigned long long w = first_cta ? (unsigned long long)(kTagSpan - (n_ctas - 1)) : 1ull;
     asm volatile("red.relaxed.gpu.global.add.u64 [%0], %1;" ::"l"(counter), "l"(w) : "memory");
@@ -94,6 +97,39 @@ __device__ __forceinline__ void launch_arrive(unsigned long long* counter, bool 
 __device__ __forceinline__ void store_tagged(void* base, long long i, float val, unsigned tag) {
     const unsigned long long w = ((unsigned long long)tag << 32) | (unsigned long long)__float_as_uint(val);
     asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(static_cast<unsigned long long*>(base) + i), "l"(w) : "memory");
+}
+
+// ---------------------------------------------------------------------------
+// mbarriers and bulk copies
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+
+__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
+}
+__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+// One bounded attempt: the hardware suspends the thread until the phase completes or the
+// time hint (ns) runs out, so a waiting warp does not compete for issue slots.
+__device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity), "r"(2000u)
+        : "memory");
+    return ok != 0;
+}
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                 ::"r"(dst), "l"(src), "r"(bytes), "r"(bar)
+                 : "memory");
 }
 
 // ---------------------------------------------------------------------------

@@ -1,10 +1,10 @@
-// Decode GEMV for the binary low-rank linear, one launch per group of linears.
+// Decode kernel for the binary low-rank linear, one launch per group of linears.
 //
 //   y = s_out * (U . (s_mid * (V . (s_in * x))))          T <= 4 tokens per launch
 //
-// The kernel is bound by the HBM stream of the packed factors and, for the layer
-// sizes of 8B-class decoders, by latency; both call for as few instructions per
-// weight and per phase as possible.
+// For 8B-class layers the launch is a chain of dependent latencies (dependency on the previous kernel, input load,
+// main loop, hand-over of the rank-R intermediate between CTAs, main loop, output), not a bandwidth problem: the
+// packed factors of a launch are a few MB.  The design keeps every step of that chain short.
 //
 //  * The packed sign bits are the A operand of an integer tensor-core MMA
 //    (mma.sync m16n8k32 s8*s8->s32) WITHOUT unpacking: in the tile layout (see
@@ -12,106 +12,104 @@
 //    {0, 2^j} ({0, -128} for j = 7), so one LOP3 prepares four weights and the eight
 //    masks j = 0..7 consume a whole 32-bit word.  Columns [32j, 32j+32) of a
 //    256-column chunk form the "class" j.
-//  * The input vector of a phase (s_in*x, or the rank-R intermediate t) is turned,
-//    once per CTA, into 17-bit fixed point X with a per-token scale.  A column of
-//    class j is stored as X * 2^(7-j) (negated for j = 7), split into three signed
-//    bytes.  The product of the A value 2^j and that operand is 2^7 * X for every
-//    class, so all eight masks accumulate into ONE accumulator per output row and
-//    byte term.  The three byte terms of a token are three of the N = 8 MMA columns.
-//  * sum(+-X) = sum(X) - 2 * sum_{bit=1}(X).  All accumulation is exact int32 /
-//    int64, so the result does not depend on the order in which warps add up.
-//
-// A SIMT sign-flip-add inner loop issues ~1.5 instructions per weight and tops out
-// near one third of the HBM rate on this part, which is why the integer MMA is
-// used as a wide dot-product unit here.
+//  * The input of a phase (s_in*x, or the rank-R intermediate t) becomes fixed point with one scale per token and
+//    CHUNK: a warp takes a (token, chunk) unit, its maximum is one warp reduction, and no CTA-wide maximum (a barrier
+//    and a second pass) stands between the load and the conversion.  A column of class j is stored as
+//    Z = round(p * inv * 2^(7-j)) (negated for j = 7), at most 23 bits, split into three signed bytes.  2^j * Z is
+//    128 * p * inv for every class, so all eight masks accumulate into ONE accumulator per output row and byte
+//    term.  The three byte terms of a token are three of the N = 8 MMA columns.
+//  * sum(+-p) = sum(p) - 2 * sum_{bit=1}(p): exact int32 per (row, chunk).  These sums go through shared memory and
+//    are added in fp32 in an order that depends on nothing but the number of chunks: a linear's result is the same
+//    bits alone, in a launch group and however its rows are dealt to CTAs and warps.
+//  * The 16 warps of a CTA split its rows x chunks into `wk` chunk slices x `wr` row slices; a warp keeps the B
+//    fragments of a chunk in registers for all its rows.
+//  * Two CTA barriers per phase: quantised input complete, partial sums complete.
 //
 // Phases: phase 1 computes t[T,R] (fp32, in scratch), phase 2 computes y.  Several
 // linears that share the two phases (q/k/v, gate/up) are processed in one launch.
 // There is no device-wide barrier between the phases: every element of t is stored
 // together with a tag of the launch and phase 2 polls the elements it needs until
-// they carry this launch's tag (see tag_begin / load8_tagged); the poll is bounded:
-// on expiry a status word is set and the thread goes on.  The weight stream of the
-// next job is started before that wait, so it overlaps with HBM traffic.  The kernel
-// is launched cooperative (all CTAs resident: consumers spin on other CTAs' data) and
-// with programmatic stream serialization: everything that does not depend on the
-// previous kernel (descriptor copy, first weight loads, an L2 prefetch of the input
-// scales) runs before griddepcontrol.wait.
+// they carry this launch's tag (nq_common.cuh).  A CTA that polls in vain computes the missing rows itself, so no wait
+// depends on CTAs that are not running (help_phase1); beyond that the poll is bounded: on expiry a status word is set and
+// the thread goes on.  The launch has programmatic stream serialization: the weight loads of both phases are started
+// before griddepcontrol.wait.
 //
-// For 8B-class layers the kernel is a chain of dependent latencies (memory round
-// trips, CTA barriers, the hand-over of t between the phases), not a bandwidth problem; the code
-// between the main loops is therefore kept short and free of divisions.
+// Measured against the first versions of this kernel (cooperative launch, one scale per token, partial sums added with
+// shared-memory atomics, weights by cp.async per warp): Qwen3-8B decode, eight layers in a graph, one token 291 -> 250 us,
+// four tokens 534 -> 430 us; launched eagerly a call took 10.6 us, of which the cooperative attribute 3.
+//
+// A SIMT sign-flip-add inner loop issues ~1.5 instructions per weight and tops out
+// near one third of the HBM rate on this part, which is why the integer MMA is
+// used as a wide dot-product unit here.
 //
 // replaces: src/nanoquant/kernel/cuda/gemv_kernel.cu:43-301 of the reference
 // (two kernels per linear, fp16/bf16 accumulation, sign-flip adds).
+#include <cstddef>
 #include <cstring>
 
 #include "nq_common.cuh"
 
 namespace nq {
 
-#ifndef NQ_GEMV_THREADS
-#define NQ_GEMV_THREADS 512
-#endif
-#ifndef NQ_GEMV_STAGES
-#define NQ_GEMV_STAGES 4
-#endif
-#ifndef NQ_GEMV_MIN_CTAS
-#define NQ_GEMV_MIN_CTAS 1
-#endif
-constexpr int kGemvThreads = NQ_GEMV_THREADS;
+constexpr int kGemvThreads = 512;
 constexpr int kGemvWarps = kGemvThreads / 32;
 constexpr int kMaxJobs = 4;         // linears per launch
-constexpr int kMaxTok = 4;          // tokens per launch (3 byte terms each, 8 MMA columns per column group)
-constexpr int kQMax = 64000;        // |X| bound: X * 2^7 splits into three signed bytes
-constexpr int kMaxK = 32768;        // keeps sum(X) and every accumulator inside int32
-constexpr int kStages = NQ_GEMV_STAGES;          // 1 KB weight slots in flight per warp
-constexpr size_t kRedBytes = 384;   // per-warp maxima: kMaxTok * kGemvWarps floats (16-byte aligned rows)
-constexpr size_t kFixedBytes = 512;
-constexpr size_t kRingBytes = (size_t)kGemvWarps * kStages * 1024;
+constexpr int kMaxTok = 4;          // tokens per launch (3 byte terms each in two column groups of 8)
+constexpr int kMaxCtas = 256;
+constexpr float kQMax = 32500.f;    // |p * inv| bound: Z <= kQMax * 2^7 stays inside the magic-number conversion
+constexpr int kMaxK = 32768;
+constexpr int kMaxChunks = kMaxK / 256;
 constexpr size_t kHeaderBytes = 256;
-constexpr unsigned kPollBackoffNs = 200;   // pause between two polls of the tagged intermediate
+constexpr int kMaxSlots = 8;        // weight blocks in flight
+// shared memory: mbarriers; the launch's descriptors; {unit value, sum} per chunk and token; weight slots
+constexpr size_t kOffParams = 128, kOffMeta = 1280;
+constexpr size_t kFixedBytes = kOffMeta + (size_t)kMaxTok * kMaxChunks * 8;
+static_assert(8 * kMaxSlots <= kOffParams && kFixedBytes % 128 == 0, "shared memory map");
+constexpr size_t kPartBytes = 32 << 10;    // partial sums of a row block
+constexpr size_t kSlotBytes = 64 << 10;    // weights of a row block
+constexpr unsigned kWeightWaitLimit = 1u << 20;   // attempts of up to ~2 us each
+constexpr unsigned kPollBackoffNs = 100;   // pause between two polls of the tagged intermediate (20: equal, 300: slower)
+constexpr unsigned kHelpAfter = 256;       // polls (about 0.1 ms) before a CTA helps
 
-// KIND_T: the rank-R intermediate between the phases, one 8-byte {fp32 value, launch tag} pair per element
-enum : int { KIND_F16 = 0, KIND_BF16 = 1, KIND_T = 2 };
+enum : int { KIND_F16 = 0, KIND_BF16 = 1 };
 
-struct Job {
+// One linear's share of a phase, 128 bytes.
+struct alignas(16) Job {
     const uint4* tiles;   // [row_groups][chunks][32]
-    const void* in;       // [T, ld_in]  fp16/bf16 (phase 1) or fp32 (phase 2)
-    const void* pre;      // [K] scale in the I/O dtype, or nullptr
+    const void* in;       // [T, ld_in]  fp16/bf16 (phase 1) or tagged fp32 (phase 2)
+    const void* pre;      // [K] scale in the I/O dtype (phase 1)
     const void* post;     // [rows] scale in the I/O dtype, or nullptr
-    void* out;            // [T, ld_out] fp32 (phase 1) or fp16/bf16 (phase 2)
+    void* out;            // [T, ld_out] tagged fp32 (phase 1) or fp16/bf16 (phase 2)
     const void* bias;     // [rows] in the I/O dtype or nullptr (phase 2)
     const void* resid;    // [T, ld_res] in the I/O dtype or nullptr (phase 2)
     long long ld_in, ld_out, ld_res;
     int rows, K;
-    int chunks;           // ceil(K / 256)
-    int items;            // ceil(rows / 32)
-    int in_kind, out_kind;
-    int vec;              // rows of `in` / `pre` are 16-byte aligned and K % 8 == 0
     int cta0, ncta;       // CTAs [cta0, cta0 + ncta) work on this job
-    int t_q, t_r;         // row tiles per CTA of the range: t_q, one more for its first t_r CTAs
-    int post_vec;         // `post` is 16-byte aligned and rows % 8 == 0: staged in shared memory with 16-byte copies
+    int g_q, g_r;         // row groups (16 rows) per CTA of the range: g_q, one more for its first g_r CTAs
+    int chunks;           // ceil(K / 256)
+    int gb;               // row groups per block (a block's weights and partial sums are in shared memory together)
+    uint16_t wk, wr;      // chunk slices x row slices of a CTA's work, one warp each
+    int vec;              // phase 1: rows of `in` and `pre` are 16-byte aligned, K a multiple of 8
+    int wk_magic, wr_magic;   // ceil(2^16 / wk), ceil(2^16 / wr): exact quotients of what the slices divide
 };
+static_assert(sizeof(Job) == 128 && offsetof(Job, cta0) == 88, "cta0..g_r are read as two 8-byte words");
 
-struct Phase {
-    Job job[kMaxJobs];
-    int njobs;
-};
-
-struct GemvParams {
-    Phase phase[2];
-    unsigned* header;     // [0..1] 64-bit arrival counter (launch tags), [2] status
-    unsigned spin_limit;  // polls before a wait for the tagged intermediate gives up
+struct alignas(16) GemvParams {
+    Job job[2 * kMaxJobs];  // phase 1, phase 2
+    unsigned* header;       // [0..1] 64-bit arrival counter (launch tags), [2] status
+    unsigned spin_limit;    // polls before a wait for the tagged intermediate gives up
+    unsigned help_after;    // polls before a CTA computes missing rows of the intermediate itself
     int T;
-    int scale_kind;       // dtype of the scale vectors (KIND_F16 / KIND_BF16)
-    int xq_stride;        // bytes between the int8 vectors in shared memory
-    int max_items;        // row tiles a CTA may own per job
+    int slots, slot_bytes;  // weight blocks in shared memory
+    int xq_off, part_off;   // shared-memory offsets behind the weight slots
+    uint8_t cta_job[kMaxCtas];   // per CTA: job of phase 1 + 16 * job of phase 2 (kMaxJobs: none)
 };
+constexpr int kParamWords = (int)(offsetof(GemvParams, cta_job) + 15) / 16;   // all but the table, rounded up
+static_assert(kOffParams + 16 * kParamWords <= kOffMeta, "shared memory map");
 
-__device__ __forceinline__ float load_as_float(const void* p, long long i, int kind) {
-    if (kind == KIND_F16) return __half2float(static_cast<const __half*>(p)[i]);
-    if (kind == KIND_BF16) return __bfloat162float(static_cast<const __nv_bfloat16*>(p)[i]);
-    return 0.f;   // the tagged intermediate goes through load1_tagged / load8_tagged
+template <int KIND>
+__device__ __forceinline__ float to_float(uint16_t h) {
+    return KIND == KIND_F16 ? __half2float(__ushort_as_half(h)) : __uint_as_float((uint32_t)h << 16);
 }
 
 __device__ __forceinline__ void mma_s8(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
@@ -121,723 +119,578 @@ __device__ __forceinline__ void mma_s8(int (&d)[4], uint32_t a0, uint32_t a1, ui
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-// Eight tagged elements (64 bytes) as floats, polled until all eight carry this launch's tag.  Every element is
-// one 64-bit word {value, tag}: a 64-bit access is single-copy atomic, so a matching tag implies its value.
-__device__ __forceinline__ void load8_tagged(const void* base, long long i, float (&v)[8], TagCtx& tc) {
-    const unsigned long long* p = static_cast<const unsigned long long*>(base) + i;
-    unsigned long long e[8];
-    for (unsigned spins = 0;; ++spins) {
-#pragma unroll
-        for (int k = 0; k < 4; ++k)
-            asm volatile("ld.relaxed.gpu.global.v2.b64 {%0,%1}, [%2];"
-                         : "=l"(e[2 * k]), "=l"(e[2 * k + 1]) : "l"(p + 2 * k) : "memory");
-        bool ok = true;
-#pragma unroll
-        for (int k = 0; k < 8; ++k) ok = ok && (unsigned)(e[k] >> 32) == tc.tag;
-        if (ok) break;
-        if (spins >= tc.limit) { tag_wait_expired(tc); break; }
-        __nanosleep(kPollBackoffNs);   // failed polls of 148 CTAs load the L2 lines the producers are storing to
-    }
-#pragma unroll
-    for (int k = 0; k < 8; ++k) v[k] = __uint_as_float((unsigned)e[k]);
-}
-__device__ __forceinline__ float load1_tagged(const void* base, long long i, TagCtx& tc) {
-    const unsigned long long* p = static_cast<const unsigned long long*>(base) + i;
-    unsigned long long e;
-    for (unsigned spins = 0;; ++spins) {
-        asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(e) : "l"(p) : "memory");
-        if ((unsigned)(e >> 32) == tc.tag) break;
-        if (spins >= tc.limit) { tag_wait_expired(tc); break; }
-    }
-    return __uint_as_float((unsigned)e);
-}
+// ---------------------------------------------------------------------------
+// input -> fixed point
+// ---------------------------------------------------------------------------
+// Quantised input in shared memory: per chunk 3*T rows of 256 bytes, row 3*tok + term (term 0 = least significant byte).
+// Inside a row the byte of column 32j + 16h + 4q + b sits at unit u = 4*(j/2) + q (16 bytes each, u ^= 4 in odd
+// rows), offset 8*(j%2) + 4h + b: lane (g, q) fetches the B registers {k = 4q.., k = 16+4q..} of masks 2i, 2i+1 with
+// ONE 128-bit load, and the eight lanes of a load phase (two rows) touch all 32 banks.
+__device__ __forceinline__ uint32_t xq_unit(int row, int u) { return (uint32_t)(u ^ ((row & 1) << 2)) * 16u; }
 
-// Eight consecutive elements of a vector as floats (one or two 128-bit loads).
-template <int KIND>
-__device__ __forceinline__ void load8(const void* base, long long i, float (&v)[8], TagCtx& tc) {
-    if (KIND == KIND_T) {
-        load8_tagged(base, i, v, tc);
-    } else {
-        const uint4 u = *reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(base) + i);
-        const uint32_t w[4] = {u.x, u.y, u.z, u.w};
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            if (KIND == KIND_F16) {
-                const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[e]));
-                v[2 * e] = f.x; v[2 * e + 1] = f.y;
-            } else {  // bf16 -> fp32 is a 16-bit shift
-                v[2 * e] = __uint_as_float(w[e] << 16);
-                v[2 * e + 1] = __uint_as_float(w[e] & 0xFFFF0000u);
-            }
-        }
-    }
-}
-
-// The launch tag is read behind the first input loads of the kernel (see tag_begin).
-__device__ __forceinline__ void tag_ensure(TagCtx& tc) {
-    if (!tc.begun) tag_begin(tc, tc.status - 2, tc.limit);
-}
-
-
-// The same split in two: the raw 128-bit loads of a block (so that several blocks can be in flight before
-// the first conversion) and the conversion.
-template <int KIND>
-struct Raw8 { uint4 a, b; };   // b: second half of an fp32 block
-template <int KIND>
-__device__ __forceinline__ void load_raw(const void* base, long long i, Raw8<KIND>& r, TagCtx& tc) {
-    if (KIND == KIND_T) {   // tagged pairs are polled until valid; the block keeps the eight values
-        float v[8];
-        load8_tagged(base, i, v, tc);
-        r.a = make_uint4(__float_as_uint(v[0]), __float_as_uint(v[1]), __float_as_uint(v[2]), __float_as_uint(v[3]));
-        r.b = make_uint4(__float_as_uint(v[4]), __float_as_uint(v[5]), __float_as_uint(v[6]), __float_as_uint(v[7]));
-    } else {
-        r.a = *reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(base) + i);
-    }
-}
-template <int KIND>
-__device__ __forceinline__ void to_float8(const Raw8<KIND>& r, float (&v)[8]) {
-    if (KIND == KIND_T) {
-        v[0] = __uint_as_float(r.a.x); v[1] = __uint_as_float(r.a.y); v[2] = __uint_as_float(r.a.z); v[3] = __uint_as_float(r.a.w);
-        v[4] = __uint_as_float(r.b.x); v[5] = __uint_as_float(r.b.y); v[6] = __uint_as_float(r.b.z); v[7] = __uint_as_float(r.b.w);
-    } else {
-        const uint32_t w[4] = {r.a.x, r.a.y, r.a.z, r.a.w};
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            if (KIND == KIND_F16) {
-                const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[e]));
-                v[2 * e] = f.x; v[2 * e + 1] = f.y;
-            } else {
-                v[2 * e] = __uint_as_float(w[e] << 16);
-                v[2 * e + 1] = __uint_as_float(w[e] & 0xFFFF0000u);
-            }
-        }
-    }
-}
-
-// Class-shifted operand of column k: X * 2^(7-j), negated for j = 7, j = (k % 256) / 32.
-__device__ __forceinline__ int class_shift(int X, int j) { return (j == 7) ? -X : (X << (7 - j)); }
-
-// Byte offset of column k inside an int8 vector: chunk base + 32*j + 8*q + 4*h + b for
-// k % 256 = 32*j + 16*h + 4*q + b, so that lane (g, q) fetches the two B registers
-// {k = 4q.., k = 16+4q..} of mask j with one 64-bit load.
-__device__ __forceinline__ int xq_pos(int k) {
-    const int kin = k & 255;
-    return (k & ~255) + (kin & 0xE0) + 2 * (kin & 12) + ((kin & 16) >> 2) + (kin & 3);
-}
-
-// red[t * kGemvWarps + warp] holds the per-warp maxima of token t.  Every thread derives the fixed-point
-// scale of its token from them itself (a few broadcast reads), which saves a serial step and a CTA barrier.
-__device__ __forceinline__ float token_max(const float* red, int t) {
-    const float4* r = reinterpret_cast<const float4*>(red + t * kGemvWarps);
-    float m = 0.f;
-#pragma unroll
-    for (int i = 0; i < kGemvWarps / 4; ++i) {
-        const float4 v = r[i];
-        m = fmaxf(m, fmaxf(fmaxf(v.x, v.y), fmaxf(v.z, v.w)));
-    }
-    return m;
-}
-// Units per value (0 when the maximum is zero or not finite: everything quantises to zero); the thread
-// for which `writer` holds records the value of one unit for the epilogue.
-__device__ __forceinline__ float token_inv(const float* red, int t, bool writer, float* delta) {
-    const float m = token_max(red, t);
-    const bool good = (m > 0.f) && (m < 3.0e38f);
-    // A rounded reciprocal times kQMax instead of a division: every thread computes the same value,
-    // |p * inv| stays within kQMax (1 + 2^-22), and the unit differs from 1 / inv by a relative 2^-22 at most.
-    if (writer) delta[t] = good ? m * (1.0f / (float)kQMax) : 0.f;
-    return good ? (float)kQMax * __frcp_rn(m) : 0.f;
-}
-// Warp-wide maximum of non-negative floats / sum of ints with one reduction instruction each.
-__device__ __forceinline__ float warp_max_abs(float m) {
-    return __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(m)));
-}
-
-// Write eight class-shifted operands (columns k8..k8+7 of one token) as three byte vectors.
-__device__ __forceinline__ void store_terms(const uint32_t (&Y)[8], int8_t* r0, int stride, int k8) {
-    // Y = 65536*b2 + 256*b1 + b0 with signed bytes: b0 = byte 0 of Y, b1 = byte 1 of
-    // Y + 0x80, b2 = byte 2 of Y + 0x8080
-    const int pos = xq_pos(k8);
-#pragma unroll
-    for (int w = 0; w < 2; ++w) {
-        const uint32_t y0 = Y[4 * w], y1 = Y[4 * w + 1], y2 = Y[4 * w + 2], y3 = Y[4 * w + 3];
-        const uint32_t z0 = y0 + 0x80u, z1 = y1 + 0x80u, z2 = y2 + 0x80u, z3 = y3 + 0x80u;
-        const uint32_t u0 = y0 + 0x8080u, u1 = y1 + 0x8080u, u2 = y2 + 0x8080u, u3 = y3 + 0x8080u;
-        const uint32_t b0 = __byte_perm(__byte_perm(y0, y1, 0x0040), __byte_perm(y2, y3, 0x0040), 0x5410);
-        const uint32_t b1 = __byte_perm(__byte_perm(z0, z1, 0x0051), __byte_perm(z2, z3, 0x0051), 0x5410);
-        const uint32_t b2 = __byte_perm(__byte_perm(u0, u1, 0x0062), __byte_perm(u2, u3, 0x0062), 0x5410);
-        *reinterpret_cast<uint32_t*>(r0 + pos + 8 * w) = b0;
-        *reinterpret_cast<uint32_t*>(r0 + stride + pos + 8 * w) = b1;
-        *reinterpret_cast<uint32_t*>(r0 + 2 * stride + pos + 8 * w) = b2;
-    }
-}
-
-// Quantise the input vectors of a job into shared memory.
-//   xq: 3*T int8 vectors (row 3*tok + term, term 0 = least significant byte), `stride`
-//       bytes apart, columns in xq_pos() order; columns K..Kpad are zero.
-//   sumx[tok]: sum of the (unshifted) fixed-point values, delta[tok]: value of one unit.
-// The code is kept as small loops on purpose: it runs once per phase, where
-// instruction fetch and latency, not arithmetic, set the pace.
-//
-// Vector path: rows of `in` / `pre` 16-byte aligned, K % 8 == 0; eight columns per thread and step.
-template <int IN_KIND>
-__device__ __noinline__ void quantise_vec(const Job& jb, int T, int8_t* xq, int stride, float* red,
-                                          int* sumx, float* delta, TagCtx& tc) {
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int K = jb.K, Kpad = jb.chunks * 256;
-    constexpr bool kHasPre = (IN_KIND != KIND_T);
-    constexpr int kBatch = 4;                       // blocks whose loads are issued before the first use:
-    constexpr int kStep = kGemvThreads * 8;         // one memory round trip per batch instead of one per block
-    tag_ensure(tc);
-    // pass 1: per-token max |in * pre|
-#pragma unroll 1
-    for (int t = 0; t < T; ++t) {
-        float m = 0.f;
-#pragma unroll 1
-        for (int k0 = tid * 8; k0 < K; k0 += kStep * kBatch) {
-            Raw8<IN_KIND> x[kBatch], sc[kBatch];
-#pragma unroll
-            for (int u = 0; u < kBatch; ++u) {
-                const int k8 = k0 + u * kStep;
-                x[u].a = x[u].b = make_uint4(0u, 0u, 0u, 0u);     // a zero block does not move the maximum
-                sc[u].a = sc[u].b = make_uint4(0u, 0u, 0u, 0u);
-                if (k8 < K) {
-                    load_raw<IN_KIND>(jb.in, t * jb.ld_in + k8, x[u], tc);
-                    if (kHasPre) load_raw<IN_KIND>(jb.pre, k8, sc[u], tc);
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < kBatch; ++u) {
-                float v[8], s[8];
-                to_float8<IN_KIND>(x[u], v);
-                if (kHasPre) to_float8<IN_KIND>(sc[u], s);
-#pragma unroll
-                for (int e = 0; e < 8; ++e) m = fmaxf(m, fabsf(kHasPre ? v[e] * s[e] : v[e]));
-            }
-        }
-        m = warp_max_abs(m);
-        if (lane == 0) red[t * kGemvWarps + warp] = m;
-    }
-    if (tid < kMaxTok) sumx[tid] = 0;
-    asm volatile("" ::"r"(tc.tag));   // the tag is in this thread's hands before the CTA can arrive at the counter
-    __syncthreads();
-    // pass 2: |p * inv| <= kQMax + 2^-7 by construction (same products as in pass 1), no clamp needed
-#pragma unroll 1
-    for (int t = 0; t < T; ++t) {
-        const float inv = token_inv(red, t, tid == 0, delta);
-        int8_t* r0 = xq + (3 * t) * stride;
-        int acc = 0;
-#pragma unroll 1
-        for (int k0 = tid * 8; k0 < Kpad; k0 += kStep * kBatch) {
-            Raw8<IN_KIND> x[kBatch], sc[kBatch];
-#pragma unroll
-            for (int u = 0; u < kBatch; ++u) {
-                const int k8 = k0 + u * kStep;
-                x[u].a = x[u].b = make_uint4(0u, 0u, 0u, 0u);     // columns K..Kpad quantise to zero
-                sc[u].a = sc[u].b = make_uint4(0u, 0u, 0u, 0u);
-                if (k8 < K) {
-                    load_raw<IN_KIND>(jb.in, t * jb.ld_in + k8, x[u], tc);
-                    if (kHasPre) load_raw<IN_KIND>(jb.pre, k8, sc[u], tc);
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < kBatch; ++u) {
-                const int k8 = k0 + u * kStep;
-                if (k8 < Kpad) {
-                    const int j = (k8 >> 5) & 7;
-                    float v[8], s[8];
-                    to_float8<IN_KIND>(x[u], v);
-                    if (kHasPre) to_float8<IN_KIND>(sc[u], s);
-                    uint32_t Y[8];  // class-shifted operands
-#pragma unroll
-                    for (int e = 0; e < 8; ++e) {
-                        const int X = __float2int_rn((kHasPre ? v[e] * s[e] : v[e]) * inv);
-                        acc += X;
-                        Y[e] = (uint32_t)class_shift(X, j);
-                    }
-                    store_terms(Y, r0, stride, k8);
-                }
-            }
-        }
-        acc = __reduce_add_sync(0xffffffffu, acc);
-        if (lane == 0 && acc != 0) atomicAdd(&sumx[t], acc);
-    }
-    __syncthreads();
-}
-
-// Vector path for inputs with at most one 8-column block per thread (T * Kpad / 8 <= threads, e.g. one token of
-// 4096 columns): each value is loaded once and stays in registers between the max pass and the conversion, so
-// the phase pays a single memory round trip for its input.  Kpad / 8 is a multiple of 32: a warp serves one token.
-template <int IN_KIND>
-__device__ __noinline__ void quantise_one(const Job& jb, int T, int8_t* xq, int stride, float* red,
-                                          int* sumx, float* delta, TagCtx& tc) {
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int K = jb.K, nv8 = jb.chunks * 32;
-    constexpr bool kHasPre = (IN_KIND != KIND_T);
-    const int t = tid / nv8, k8 = (tid - t * nv8) * 8;
-    const bool active = t < T;
-    float p[8];
-#pragma unroll
-    for (int e = 0; e < 8; ++e) p[e] = 0.f;
-    if (!kHasPre) tag_ensure(tc);          // the tagged intermediate is compared with the tag as it is loaded
-    Raw8<IN_KIND> xr, sr;
-    xr.a = xr.b = sr.a = sr.b = make_uint4(0u, 0u, 0u, 0u);
-    if (active && k8 < K) {
-        load_raw<IN_KIND>(jb.in, t * jb.ld_in + k8, xr, tc);
-        if (kHasPre) load_raw<IN_KIND>(jb.pre, k8, sr, tc);
-    }
-    if (kHasPre) tag_ensure(tc);           // behind the input loads: the two round trips overlap
-    if (active && k8 < K) {
-        to_float8<IN_KIND>(xr, p);
-        if (kHasPre) {
-            float s[8];
-            to_float8<IN_KIND>(sr, s);
-#pragma unroll
-            for (int e = 0; e < 8; ++e) p[e] *= s[e];
-        }
-    }
+// One unit, token `tok` of a chunk: lane l holds the products of columns 8l..8l+7 of the chunk (zeros beyond K).
+// `xq_chunk`: the chunk's rows; `meta`: {unit value, sum} of the unit.
+__device__ __forceinline__ void quantise_unit(float (&p)[8], unsigned char* xq_chunk, int tok, int2* meta) {
+    const int lane = threadIdx.x & 31, j = lane >> 2;
     float m = 0.f;
 #pragma unroll
     for (int e = 0; e < 8; ++e) m = fmaxf(m, fabsf(p[e]));
-    m = warp_max_abs(m);
-    // per-warp maxima in the [token][warp] table: a warp contributes to its token only
-    if (lane < kMaxTok) red[lane * kGemvWarps + warp] = (active && lane == t) ? m : 0.f;
-    if (tid < kMaxTok) sumx[tid] = 0;
-    asm volatile("" ::"r"(tc.tag));   // the tag is in this thread's hands before the CTA can arrive at the counter
-    __syncthreads();
-    if (active) {
-        const float inv = token_inv(red, t, k8 == 0, delta);
-        const int j = (k8 >> 5) & 7;
-        uint32_t Y[8];
-        int acc = 0;
+    m = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(m)));
+    if (!(m > 1e-31f && m < 3.0e38f)) {   // zero (below 1e-31 the reciprocal would overflow) or not finite: zeros
+        m = 1.f;
 #pragma unroll
-        for (int e = 0; e < 8; ++e) {
-            const int X = __float2int_rn(p[e] * inv);
-            acc += X;
-            Y[e] = (uint32_t)class_shift(X, j);
-        }
-        store_terms(Y, xq + (3 * t) * stride, stride, k8);
-        acc = __reduce_add_sync(0xffffffffu, acc);
-        if (lane == 0 && acc != 0) atomicAdd(&sumx[t], acc);
+        for (int e = 0; e < 8; ++e) p[e] = 0.f;
     }
-    __syncthreads();
+    // times 2^(7-j), negative for j = 7 (the A operand of class 7 is -128)
+    const float inv_j = kQMax * __frcp_rn(m) * __uint_as_float(j == 7 ? 0xBF800000u : (uint32_t)(127 + 7 - j) << 23);
+    // 1.5 * 2^23 + v rounds v to an integer Z in the low mantissa bits (|v| < 2^22).  With 0x8080 added, bytes 0 and 1
+    // of the sum are the two low signed bytes of Z with their top bits flipped, and bits 16..22 are the high byte + 64.
+    uint32_t z[8], zsum = 0;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+        z[e] = __float_as_uint(fmaf(p[e], inv_j, 12582912.f + 32896.f));
+        zsum += z[e];
+    }
+    unsigned char* r0 = xq_chunk + tok * (3 * 256) + 8 * (j & 1) + 2 * (lane & 2);
+    const int row0 = 3 * tok, u0 = 4 * (j >> 1) + 2 * (lane & 1);
+#pragma unroll
+    for (int w = 0; w < 2; ++w) {
+        const uint32_t* y = z + 4 * w;
+        const uint32_t lo01 = __byte_perm(y[0], y[1], 0x5140), lo23 = __byte_perm(y[2], y[3], 0x5140);   // {b0, b0', b1, b1'}
+        const uint32_t hi01 = __byte_perm(y[0], y[1], 0x0062), hi23 = __byte_perm(y[2], y[3], 0x0062);   // {b2, b2'}
+        const uint32_t b0 = __byte_perm(lo01, lo23, 0x5410) ^ 0x80808080u;
+        const uint32_t b1 = __byte_perm(lo01, lo23, 0x7632) ^ 0x80808080u;
+        const uint32_t b2 = (__byte_perm(hi01, hi23, 0x5410) + 0x40404040u) ^ 0x80808080u;   // - 64
+        *reinterpret_cast<uint32_t*>(r0 + xq_unit(row0, u0 + w)) = b0;
+        *reinterpret_cast<uint32_t*>(r0 + 256 + xq_unit(row0 + 1, u0 + w)) = b1;
+        *reinterpret_cast<uint32_t*>(r0 + 512 + xq_unit(row0, u0 + w)) = b2;
+    }
+    int sum = (int)(zsum - 8u * (0x4B400000u + 0x8080u));    // |sum| * 2^j <= 2^25
+    sum = __reduce_add_sync(0xffffffffu, j == 7 ? sum * -128 : sum * (1 << j));
+    if (lane == 0) *meta = make_int2(__float_as_int(m * (1.0f / (128.f * kQMax))), sum);
 }
 
-// The same with NI (2 or 4) blocks per thread: item f = tid + i * threads covers token f / nv8, columns
-// (f % nv8) * 8.  All NI loads of a thread are in flight together (the tagged intermediate is polled item by
-// item, but its later items are valid by then), nothing is loaded twice, and several tokens cost one memory
-// round trip instead of one per token and pass.
-template <int IN_KIND, int NI>
-__device__ __noinline__ void quantise_few(const Job& jb, int T, int8_t* xq, int stride, float* red,
-                                          int* sumx, float* delta, TagCtx& tc) {
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int K = jb.K, nv8 = jb.chunks * 32, items = T * nv8;
-    constexpr bool kHasPre = (IN_KIND != KIND_T);
-    float p[NI][8];
-    int tt[NI], kk[NI];
-    Raw8<IN_KIND> x[NI], sc[NI];
-    if (!kHasPre) tag_ensure(tc);
+template <int KIND>
+__device__ __forceinline__ void to_float8(const uint4& r, float (&v)[8]) {
+    const uint32_t w[4] = {r.x, r.y, r.z, r.w};
 #pragma unroll
-    for (int i = 0; i < NI; ++i) {
-        const int f = tid + i * kGemvThreads;
-        const int t = f / nv8;
-        tt[i] = f < items ? t : -1;
-        kk[i] = (f - t * nv8) * 8;
-        x[i].a = x[i].b = make_uint4(0u, 0u, 0u, 0u);
-        sc[i].a = sc[i].b = make_uint4(0u, 0u, 0u, 0u);
-        if (tt[i] >= 0 && kk[i] < K) {
-            load_raw<IN_KIND>(jb.in, t * jb.ld_in + kk[i], x[i], tc);
-            if (kHasPre) load_raw<IN_KIND>(jb.pre, kk[i], sc[i], tc);
+    for (int e = 0; e < 4; ++e) {
+        if (KIND == KIND_F16) {
+            const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[e]));
+            v[2 * e] = f.x; v[2 * e + 1] = f.y;
+        } else {  // bf16 -> fp32 is a 16-bit shift
+            v[2 * e] = __uint_as_float(w[e] << 16);
+            v[2 * e + 1] = __uint_as_float(w[e] & 0xFFFF0000u);
         }
     }
-    if (kHasPre) tag_ensure(tc);           // behind the input loads: the two round trips overlap
-    float wm[kMaxTok];   // this warp's maximum per token (a warp's item belongs to one token)
+}
+
+// Chunks a warp quantises: c, c + step, ... of `chunks`, of each the tokens [t0, t1).  One warp per chunk; with more
+// than one token and no more than half as many chunks as warps, two warps share a chunk's tokens.
+struct Share {
+    int c, step, t0, t1;
+};
+__device__ __forceinline__ Share share_of(int chunks, int T) {
+    const int warp = threadIdx.x >> 5;
+    if (T == 1 || 2 * chunks > kGemvWarps) return Share{warp, kGemvWarps, 0, T};
+    const int half = (T + 1) >> 1;
+    return (warp & 1) ? Share{warp >> 1, kGemvWarps / 2, half, T} : Share{warp >> 1, kGemvWarps / 2, 0, half};
+}
+
+// Phase 1: s_in * x.  MT: most tokens of a share.  The loads of a chunk's tokens, and those of the next chunk, are in
+// flight together; the conversion is one body that the tokens are shifted through.
+template <int KIND, int MT>
+__device__ __forceinline__ void quantise_x(const Job& jb, int T, unsigned char* xq, int2* meta) {
+    const int lane8 = (threadIdx.x & 31) * 8, K = jb.K, chunks = jb.chunks;
+    const Share sh = share_of(chunks, T);
+    const uint16_t* in = static_cast<const uint16_t*>(jb.in) + sh.t0 * jb.ld_in + lane8;
+    const uint16_t* pre = static_cast<const uint16_t*>(jb.pre) + lane8;
+    const long long ld = jb.ld_in;
+    uint4 x[MT], s, xn[MT], sn;
+    auto load = [&](int c, uint4 (&xr)[MT], uint4& sr) {
+        sr = make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
-    for (int q = 0; q < kMaxTok; ++q) wm[q] = 0.f;
+        for (int t = 0; t < MT; ++t) xr[t] = make_uint4(0u, 0u, 0u, 0u);
+        if (c * 256 + lane8 < K) {
+            sr = *reinterpret_cast<const uint4*>(pre + c * 256);
 #pragma unroll
-    for (int i = 0; i < NI; ++i) {
-        float s[8], m = 0.f;
-        to_float8<IN_KIND>(x[i], p[i]);
-        if (kHasPre) {
-            to_float8<IN_KIND>(sc[i], s);
+            for (int t = 0; t < MT; ++t)
+                if (t < sh.t1 - sh.t0) xr[t] = *reinterpret_cast<const uint4*>(in + t * ld + c * 256);
+        }
+    };
+    load(sh.c, x, s);
+#pragma unroll 1
+    for (int c = sh.c; c < chunks; c += sh.step) {
+        load(c + sh.step, xn, sn);
+#pragma unroll 1
+        for (int t = sh.t0; t < sh.t1; ++t) {
+            float p[8], q[8];
+            to_float8<KIND>(x[0], p);
+            to_float8<KIND>(s, q);
 #pragma unroll
-            for (int e = 0; e < 8; ++e) p[i][e] *= s[e];
+            for (int e = 0; e < 8; ++e) p[e] *= q[e];
+            quantise_unit(p, xq + c * T * (3 * 256), t, meta + c * T + t);
+#pragma unroll
+            for (int k = 0; k + 1 < MT; ++k) x[k] = x[k + 1];
         }
 #pragma unroll
-        for (int e = 0; e < 8; ++e) m = fmaxf(m, fabsf(p[i][e]));
-        m = warp_max_abs(m);
-#pragma unroll
-        for (int q = 0; q < kMaxTok; ++q) wm[q] = tt[i] == q ? fmaxf(wm[q], m) : wm[q];
+        for (int k = 0; k < MT; ++k) x[k] = xn[k];
+        s = sn;
     }
-    if (lane < kMaxTok) {
-        float v = wm[0];
-#pragma unroll
-        for (int q = 1; q < kMaxTok; ++q) v = lane == q ? wm[q] : v;
-        red[lane * kGemvWarps + warp] = v;
-    }
-    if (tid < kMaxTok) sumx[tid] = 0;
-    asm volatile("" ::"r"(tc.tag));   // the tag is in this thread's hands before the CTA can arrive at the counter
-    __syncthreads();
-#pragma unroll
-    for (int i = 0; i < NI; ++i) {
-        if (tt[i] >= 0) {      // warp-uniform
-            const float inv = token_inv(red, tt[i], kk[i] == 0, delta);
-            const int j = (kk[i] >> 5) & 7;
-            uint32_t Y[8];
-            int acc = 0;
+}
+// The same for inputs of any alignment and size: element loads, lane by lane.
+template <int KIND>
+__device__ __noinline__ void quantise_x_any(const Job& jb, int T, unsigned char* xq, int2* meta) {
+    const int lane8 = (threadIdx.x & 31) * 8, K = jb.K, chunks = jb.chunks;
+    const uint16_t* pre = static_cast<const uint16_t*>(jb.pre);
+    const Share sh = share_of(chunks, T);
+#pragma unroll 1
+    for (int c = sh.c; c < chunks; c += sh.step) {
+#pragma unroll 1
+        for (int t = sh.t0; t < sh.t1; ++t) {
+            const uint16_t* in = static_cast<const uint16_t*>(jb.in) + t * jb.ld_in;
+            uint16_t x[8], s[8];
 #pragma unroll
             for (int e = 0; e < 8; ++e) {
-                const int X = __float2int_rn(p[i][e] * inv);
-                acc += X;
-                Y[e] = (uint32_t)class_shift(X, j);
+                const int k = c * 256 + lane8 + e;
+                x[e] = k < K ? in[k] : (uint16_t)0;
+                s[e] = k < K ? pre[k] : (uint16_t)0;
             }
-            store_terms(Y, xq + (3 * tt[i]) * stride, stride, kk[i]);
-            acc = __reduce_add_sync(0xffffffffu, acc);
-            if (lane == 0 && acc != 0) atomicAdd(&sumx[tt[i]], acc);
+            float p[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) p[e] = to_float<KIND>(x[e]) * to_float<KIND>(s[e]);
+            quantise_unit(p, xq + c * T * (3 * 256), t, meta + c * T + t);
         }
     }
-    __syncthreads();
 }
-
-// Scalar path for unaligned or ragged inputs (any K, any alignment).
-__device__ __noinline__ void quantise_scalar(const Job& jb, int T, int scale_kind, int8_t* xq, int stride,
-                                             float* red, int* sumx, float* delta, TagCtx& tc) {
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int K = jb.K, Kpad = jb.chunks * 256;
-    tag_ensure(tc);
+// Phase 2: the tagged intermediate, polled until every element of a share's chunk (MT tokens at most) carries this
+// launch's tag.  Every element is one 64-bit word {value, tag}: a 64-bit access is single-copy atomic, so a matching
+// tag implies its value.  Returns false (for the whole warp) after `help_after` polls in vain.
+template <int MT>
+__device__ __forceinline__ bool quantise_t(const Job& jb, int T, unsigned char* xq, int2* meta, TagCtx& tc, unsigned help_after) {
+    constexpr int B = MT > 2 ? 2 : MT;       // tokens whose loads are in flight together
+    const int lane8 = (threadIdx.x & 31) * 8, K = jb.K, chunks = jb.chunks;
+    const Share sh = share_of(chunks, T);
+    const unsigned long long* in = static_cast<const unsigned long long*>(jb.in) + lane8;
+    const int ld = (int)jb.ld_in;
 #pragma unroll 1
-    for (int t = 0; t < T; ++t) {
-        float m = 0.f;
-        for (int k = tid; k < K; k += kGemvThreads) {
-            const float s = jb.pre ? load_as_float(jb.pre, k, scale_kind) : 1.f;
-            m = fmaxf(m, fabsf((jb.in_kind == KIND_T ? load1_tagged(jb.in, t * jb.ld_in + k, tc) : load_as_float(jb.in, t * jb.ld_in + k, jb.in_kind)) * s));
-        }
-        m = warp_max_abs(m);
-        if (lane == 0) red[t * kGemvWarps + warp] = m;
-    }
-    if (tid < kMaxTok) sumx[tid] = 0;
-    asm volatile("" ::"r"(tc.tag));   // the tag is in this thread's hands before the CTA can arrive at the counter
-    __syncthreads();
+    for (int c = sh.c; c < chunks; c += sh.step) {
+        const int left = K - (c * 256 + lane8);      // elements of the row from here on; rows are padded to eight
 #pragma unroll 1
-    for (int t = 0; t < T; ++t) {
-        const float inv = token_inv(red, t, tid == 0, delta);
-        int acc = 0;
-        for (int k = tid; k < Kpad; k += kGemvThreads) {
-            int X = 0;
-            if (k < K) {
-                const float s = jb.pre ? load_as_float(jb.pre, k, scale_kind) : 1.f;
-                X = __float2int_rn((jb.in_kind == KIND_T ? load1_tagged(jb.in, t * jb.ld_in + k, tc) : load_as_float(jb.in, t * jb.ld_in + k, jb.in_kind)) * s * inv);
-            }
-            acc += X;
-            const int y = class_shift(X, (k >> 5) & 7);
-            const int pos = xq_pos(k);
-            xq[(3 * t) * stride + pos] = (int8_t)(y & 0xFF);
-            xq[(3 * t + 1) * stride + pos] = (int8_t)(((y + 0x80) >> 8) & 0xFF);
-            xq[(3 * t + 2) * stride + pos] = (int8_t)(((y + 0x8080) >> 16) & 0xFF);
-        }
-        acc = __reduce_add_sync(0xffffffffu, acc);
-        if (lane == 0 && acc != 0) atomicAdd(&sumx[t], acc);
-    }
-    __syncthreads();
-}
-
-__device__ __forceinline__ void quantise_input(const Job& jb, int T, int scale_kind, int8_t* xq, int stride,
-                                               float* red, int* sumx, float* delta, TagCtx& tc) {
-    if (!jb.vec) quantise_scalar(jb, T, scale_kind, xq, stride, red, sumx, delta, tc);
-    else if (T * jb.chunks * 32 <= kGemvThreads) {
-        if (jb.in_kind == KIND_T) quantise_one<KIND_T>(jb, T, xq, stride, red, sumx, delta, tc);
-        else if (jb.in_kind == KIND_F16) quantise_one<KIND_F16>(jb, T, xq, stride, red, sumx, delta, tc);
-        else quantise_one<KIND_BF16>(jb, T, xq, stride, red, sumx, delta, tc);
-    }
-    else if (T * jb.chunks * 32 <= 2 * kGemvThreads) {
-        if (jb.in_kind == KIND_T) quantise_few<KIND_T, 2>(jb, T, xq, stride, red, sumx, delta, tc);
-        else if (jb.in_kind == KIND_F16) quantise_few<KIND_F16, 2>(jb, T, xq, stride, red, sumx, delta, tc);
-        else quantise_few<KIND_BF16, 2>(jb, T, xq, stride, red, sumx, delta, tc);
-    }
-    else if (T > 1 && T * jb.chunks * 32 <= 4 * kGemvThreads) {   // one token of that width: quantise_vec measured faster
-        if (jb.in_kind == KIND_T) quantise_few<KIND_T, 4>(jb, T, xq, stride, red, sumx, delta, tc);
-        else if (jb.in_kind == KIND_F16) quantise_few<KIND_F16, 4>(jb, T, xq, stride, red, sumx, delta, tc);
-        else quantise_few<KIND_BF16, 4>(jb, T, xq, stride, red, sumx, delta, tc);
-    }
-    else if (jb.in_kind == KIND_T) quantise_vec<KIND_T>(jb, T, xq, stride, red, sumx, delta, tc);
-    else if (jb.in_kind == KIND_F16) quantise_vec<KIND_F16>(jb, T, xq, stride, red, sumx, delta, tc);
-    else quantise_vec<KIND_BF16>(jb, T, xq, stride, red, sumx, delta, tc);
-}
-
-__device__ __forceinline__ void cp_async16(void* smem_dst, const void* gmem_src) {
-    const unsigned d = (unsigned)__cvta_generic_to_shared(smem_dst);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(gmem_src) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-
-// Per-warp cursor over the (tile, chunk) pairs of one job: 1 KB of packed weights per
-// pair (two row groups x 256 columns), pairs tile-major, one contiguous range per warp.
-struct PairStream {
-    int my_items;   // row tiles (32 rows) of this CTA in the job
-    int first;      // the first of them (they are consecutive)
-    int my_pairs;   // pairs of this warp
-    int begin_il, begin_c;   // first pair of this warp: local tile index, chunk
-    int l_il, l_c, l_n;      // next pair to fetch
-    int slot;                // which half of the output-scale staging buffer this job uses
-};
-
-// Every job of a phase has a contiguous range of CTAs of its own, sized by the host in proportion to its
-// packed bytes, and a CTA of the range owns a contiguous run of the job's row tiles (32 rows).  A CTA therefore
-// prepares the input of exactly one job per phase: a CTA with rows of two jobs would quantise two inputs one
-// after the other, a tail of 1.6-2 us that every other CTA waits for in the next phase or launch.
-// Returns the CTA's tiles of `jb`: first tile, count.
-__device__ __forceinline__ int my_tiles(const Job& jb, int& first) {
-    const int b = (int)blockIdx.x - jb.cta0;
-    first = 0;
-    if (b < 0 || b >= jb.ncta) return 0;
-    first = b * jb.t_q + min(b, jb.t_r);
-    return jb.t_q + (b < jb.t_r ? 1 : 0);
-}
-
-// The constants of a job that the weight stream needs, held in registers: a read of the shared-memory
-// descriptor behind an `asm volatile` with a memory clobber would be re-issued in every iteration.
-struct StreamJob {
-    const uint4* tiles;
-    int row_groups, chunks;
-};
-__device__ __forceinline__ StreamJob stream_job(const Job& jb) {
-    StreamJob sj;
-    sj.tiles = jb.tiles;
-    sj.row_groups = (jb.rows + 15) >> 4;
-    sj.chunks = jb.chunks;
-    return sj;
-}
-
-__device__ __forceinline__ void stream_issue(PairStream& st, const StreamJob& sj, uint4* ring, int lane) {
-    if (st.l_n < st.my_pairs) {
-        const int rg = 2 * (st.first + st.l_il);
-        const int rgb = (rg + 1 < sj.row_groups) ? rg + 1 : rg;  // odd tail: re-read, result discarded
-        uint4* dst = ring + (st.l_n % kStages) * 64 + lane;
-        cp_async16(dst, sj.tiles + ((size_t)rg * sj.chunks + st.l_c) * 32 + lane);
-        cp_async16(dst + 32, sj.tiles + ((size_t)rgb * sj.chunks + st.l_c) * 32 + lane);
-        if (++st.l_c == sj.chunks) { st.l_c = 0; ++st.l_il; }
-        ++st.l_n;
-    }
-    cp_async_commit();  // always commit so that group counting stays uniform
-}
-
-// Set the cursor up and start the first weight loads of a job.  They do not depend on
-// the job's input vector, so this runs before the input is ready (for a phase-2 job:
-// before the wait for the tagged intermediate, which then overlaps with the loads).
-__device__ __forceinline__ void stream_begin(PairStream& st, const Job& jb, uint4* ring, int warp,
-                                             int lane, uint16_t* post_s, int max_items) {
-    st.my_items = my_tiles(jb, st.first);
-    const int npairs = st.my_items * jb.chunks;            // < 2^27: the products below fit 32 bits
-    const int p_begin = npairs * warp / kGemvWarps;
-    st.my_pairs = npairs * (warp + 1) / kGemvWarps - p_begin;
-    st.begin_il = 0;
-    st.begin_c = p_begin;
-    while (st.begin_c >= jb.chunks) { st.begin_c -= jb.chunks; ++st.begin_il; }   // at most my_items steps
-    st.l_il = st.begin_il; st.l_c = st.begin_c; st.l_n = 0;
-    st.slot ^= 1;
-    // The output scales of this CTA's rows are needed right after the main loop: copy them into shared
-    // memory now (part of this thread's first copy group, complete when the main loop has drained).
-    if (jb.post_vec) {
-        const int row0 = 32 * st.first;
-        const int nrows = min(32 * st.my_items, jb.rows - row0);
-        const int i = (int)threadIdx.x;
-        if (8 * i < nrows)
-            cp_async16(post_s + st.slot * (32 * max_items) + 8 * i,
-                       static_cast<const uint16_t*>(jb.post) + row0 + 8 * i);
-    }
-    const StreamJob sj = stream_job(jb);
-#pragma unroll
-    for (int d = 0; d < kStages - 1; ++d) stream_issue(st, sj, ring, lane);
-}
-
-__device__ __forceinline__ bool cta_has_items(const Job& jb) {
-    int f;
-    return my_tiles(jb, f) > 0;
-}
-
-// The whole launch for one CTA: the jobs of phase 1, then the jobs of phase 2 (which poll the
-// tagged intermediate).  CG = column groups of 8 MMA columns (3 columns per token).
-template <int CG>
-__device__ __forceinline__ bool run_all(const Phase* phases, const GemvParams& P, unsigned char* smem) {
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int g = lane >> 2, q = lane & 3;
-    constexpr int kCols = 8 * CG;
-    // shared memory carve-up
-    float* red = reinterpret_cast<float*>(smem);                          // [warps][4] + [4]
-    int* sumx = reinterpret_cast<int*>(smem + kRedBytes);                 // [4]
-    float* delta = reinterpret_cast<float*>(smem + kRedBytes + 16);       // [4]
-    uint4* ring = reinterpret_cast<uint4*>(smem + kFixedBytes) + warp * (kStages * 64);  // [stage][2][32]
-    int* s1 = reinterpret_cast<int*>(smem + kFixedBytes + kRingBytes);    // [max_items][32 rows][kCols]
-    int8_t* xq = reinterpret_cast<int8_t*>(smem + kFixedBytes + kRingBytes + (size_t)P.max_items * (128 * kCols));
-    // output scales of the current and the next job: [2][max_items][32] two-byte entries behind the int8 vectors
-    uint16_t* post_s = reinterpret_cast<uint16_t*>(xq + (size_t)3 * P.T * P.xq_stride);
-
-    const int njobs = phases[0].njobs;        // same count in both phases
-    auto job_of = [&](int s) -> const Job& { return phases[s >= njobs].job[s >= njobs ? s - njobs : s]; };
-    auto next_step = [&](int s) {             // first step >= s in which this CTA owns row tiles
-        while (s < 2 * njobs && !cta_has_items(job_of(s))) ++s;
-        return s;
-    };
-    PairStream st;
-    st.slot = 0;
-    int s = next_step(0);
-    if (s < 2 * njobs) {
-        const Job& j0 = job_of(s);
-        stream_begin(st, j0, ring, warp, lane, post_s, P.max_items);
-    }
-    // Programmatic dependent launch: everything above (descriptor copy, first weight loads) may overlap
-    // with the tail of the previous kernel in the stream; the activations and the scratch (shared with
-    // that kernel) are only touched after it has completed.  No-ops without the launch attribute.
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    // All CTAs of this cooperative grid are resident, so CTAs of the next kernel that start early cannot keep one
-    // of ours from being scheduled: let the next kernel begin its prologue wherever an SM frees up.
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    // tag of this launch for the intermediate's {value, tag} pairs (and this CTA's arrival, which nobody waits for)
-    TagCtx tc;
-    tc.tag = 0u; tc.limit = P.spin_limit; tc.status = P.header + 2; tc.begun = 0u;   // read behind the first input loads
-    bool arrived = false;
+        for (int t0 = sh.t0; t0 < sh.t1; t0 += B) {
+            float v[B][8];
 #pragma unroll 1
-    while (true) {
-        if (s >= 2 * njobs) break;
-        const Job& jb = job_of(s);
-        const int chunks = jb.chunks;
-        for (int i = tid; i < st.my_items * (32 * kCols); i += kGemvThreads) s1[i] = 0;
-        quantise_input(jb, P.T, P.scale_kind, xq, P.xq_stride, red, sumx, delta, tc);
-        if (!arrived) {   // behind the CTA barriers of the quantiser
-            if (tid == 0) launch_arrive(reinterpret_cast<unsigned long long*>(P.header), blockIdx.x == 0, gridDim.x);
-            arrived = true;
-        }
-
-        // MMA column n = 8*cg + g reads int8 vector n (= 3*tok + term); unused columns re-read a valid one
-        const int8_t* bbase[CG];
+            for (unsigned spins = 0;; ++spins) {
+                unsigned wrong = 0;
+                unsigned long long e[B][8];
 #pragma unroll
-        for (int cg = 0; cg < CG; ++cg) {
-            const int n = 8 * cg + g;
-            bbase[cg] = xq + (n < 3 * P.T ? n : 3 * P.T - 1) * P.xq_stride + 8 * q;
-        }
-        int accA[CG][4], accB[CG][4];
+                for (int i = 0; i < B; ++i)
+                    if (left > 0 && t0 + i < sh.t1) {
 #pragma unroll
-        for (int cg = 0; cg < CG; ++cg)
-#pragma unroll
-            for (int i = 0; i < 4; ++i) { accA[cg][i] = 0; accB[cg][i] = 0; }
-        int c_il = st.begin_il, c_c = st.begin_c;
-        const StreamJob sj = stream_job(jb);
-        const int my_pairs = st.my_pairs;
-#pragma unroll 1
-        for (int n = 0; n < my_pairs; ++n) {
-            stream_issue(st, sj, ring, lane);
-            cp_async_wait<kStages - 1>();
-            __syncwarp();
-            const uint4* slot = ring + (n % kStages) * 64 + lane;
-            const uint4 ta = slot[0], tb = slot[32];
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const uint32_t m = 0x01010101u << j;
-#pragma unroll
-                for (int cg = 0; cg < CG; ++cg) {
-                    const uint2 b = *reinterpret_cast<const uint2*>(bbase[cg] + c_c * 256 + 32 * j);
-                    mma_s8(accA[cg], ta.x & m, ta.y & m, ta.z & m, ta.w & m, b.x, b.y);
-                    mma_s8(accB[cg], tb.x & m, tb.y & m, tb.z & m, tb.w & m, b.x, b.y);
-                }
-            }
-            __syncwarp();  // every lane has read the slot before it is refilled
-            // when this warp leaves the row tile, fold its partial sums into shared memory:
-            // lane (g, q) holds rows g / g+8 of both row groups, columns 2q, 2q+1 of each column group
-            if (++c_c == chunks || n + 1 == my_pairs) {
-                int* dst = s1 + c_il * (32 * kCols);
-#pragma unroll
-                for (int cg = 0; cg < CG; ++cg) {
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        const int col = 8 * cg + 2 * q + (i & 1);
-                        const int ra = g + 8 * (i >> 1);
-                        if (accA[cg][i] != 0) atomicAdd(&dst[ra * kCols + col], accA[cg][i]);
-                        if (accB[cg][i] != 0) atomicAdd(&dst[(16 + ra) * kCols + col], accB[cg][i]);
-                        accA[cg][i] = 0;
-                        accB[cg][i] = 0;
-                    }
-                }
-                if (c_c == chunks) { c_c = 0; ++c_il; }
-            }
-        }
-        cp_async_wait<0>();
-        __syncthreads();
-        const int my_items = st.my_items;
-        const int first_tile_of_job = st.first;
-        const uint16_t* my_post = post_s + st.slot * (32 * P.max_items);
-        // finalise: thread -> (token slot, row slot); tokens beyond the slot count and rows beyond the 128 row
-        // slots are covered by the strides.  The three column sums of a token are the byte terms of
-        // 128 * sum_{bit=1}(X); result = sum(X) - 2 * sum_{bit=1}(X) = sum(X) - terms / 64 (terms is a multiple of 128).
-        for (int tok = tid >> 7; tok < P.T; tok += kGemvThreads >> 7) {
-            const long long sx = sumx[tok];
-            const float dl = delta[tok];
-            for (int idx = tid & 127; idx < my_items * 32; idx += 128) {
-                const int row = 32 * first_tile_of_job + idx;
-                if (row < jb.rows) {
-                    float extra = 0.f;       // bias and residual of this output (phase 2), fetched before the arithmetic
-                    if (jb.bias) extra = load_as_float(jb.bias, row, P.scale_kind);
-                    if (jb.resid) extra += load_as_float(jb.resid, tok * jb.ld_res + row, P.scale_kind);
-                    const int* c = s1 + idx * kCols + 3 * tok;
-                    const long long terms = (long long)c[2] * 65536 + (long long)c[1] * 256 + (long long)c[0];
-                    float val = (float)(sx - (terms >> 6)) * dl;
-                    if (jb.post) val *= jb.post_vec ? load_as_float(my_post, idx, P.scale_kind)
-                                                    : load_as_float(jb.post, row, P.scale_kind);
-                    if (jb.out_kind == KIND_T) {
-                        store_tagged(jb.out, tok * jb.ld_out + row, val, tc.tag);
-                    } else if (jb.out_kind == KIND_F16) {
-                        // bias and residual in fp32 behind the output scale; same saturation bounds as the reference epilogue
-                        val = fminf(fmaxf(val + extra, -64504.0f), 64504.0f);
-                        static_cast<__half*>(jb.out)[tok * jb.ld_out + row] = __float2half(val);
+                        for (int u = 0; u < 4; ++u)
+                            asm volatile("ld.relaxed.gpu.global.v2.b64 {%0,%1}, [%2];"
+                                         : "=l"(e[i][2 * u]), "=l"(e[i][2 * u + 1])
+                                         : "l"(in + (t0 + i) * ld + c * 256 + 2 * u) : "memory");
                     } else {
-                        val = fminf(fmaxf(val + extra, -3.3895313892515355e+38f), 3.3895313892515355e+38f);
-                        static_cast<__nv_bfloat16*>(jb.out)[tok * jb.ld_out + row] = __float2bfloat16(val);
+#pragma unroll
+                        for (int u = 0; u < 8; ++u) e[i][u] = (unsigned long long)tc.tag << 32;
                     }
+#pragma unroll
+                for (int i = 0; i < B; ++i)
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) {
+                        wrong |= (unsigned)(e[i][u] >> 32) ^ tc.tag;
+                        v[i][u] = __uint_as_float((unsigned)e[i][u]);
+                    }
+                if (left > 0 && left < 8) {          // the padding of a row is not written
+                    wrong = 0;
+#pragma unroll
+                    for (int i = 0; i < B; ++i)
+#pragma unroll
+                        for (int u = 0; u < 8; ++u) {
+                            if (u < left) wrong |= (unsigned)(e[i][u] >> 32) ^ tc.tag;
+                            else v[i][u] = 0.f;
+                        }
+                }
+                if (__all_sync(0xffffffffu, wrong == 0u)) break;
+                if (spins >= tc.limit) { tag_wait_expired(tc); break; }   // the same in every lane
+                if (spins >= help_after) return false;
+                __nanosleep(kPollBackoffNs);   // failed polls of 148 CTAs load the L2 lines the producers are storing to
+            }
+#pragma unroll 1
+            for (int t = t0; t < t0 + B && t < sh.t1; ++t) {
+                quantise_unit(v[0], xq + c * T * (3 * 256), t, meta + c * T + t);
+                if (B > 1) {
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) v[0][u] = v[B - 1][u];
                 }
             }
         }
-        // Start the next job's weight stream after this job's results are on their way (their stores then
-        // overlap the address arithmetic below) and before any barrier, whose wait the loads overlap.
-        const int s_next = next_step(s + 1);
-        if (s_next < 2 * njobs)
-            stream_begin(st, job_of(s_next), ring, warp, lane, post_s, P.max_items);
-        __syncthreads();  // xq / s1 are reused by the next job
-        s = s_next;
-    }
-    if (!arrived) {   // a CTA without row tiles in either phase still counts towards the launch
-        tag_ensure(tc);
-        asm volatile("" ::"r"(tc.tag));
-        __syncthreads();
-        if (tid == 0) launch_arrive(reinterpret_cast<unsigned long long*>(P.header), blockIdx.x == 0, gridDim.x);
     }
     return true;
 }
 
-template <int CG>
-__global__ void __launch_bounds__(kGemvThreads, NQ_GEMV_MIN_CTAS) gemv_group_kernel(const __grid_constant__ GemvParams P) {
-    extern __shared__ __align__(16) unsigned char smem[];
-    // The descriptors are read with runtime indices; one cooperative copy out of the
-    // parameter bank into shared memory replaces many serial constant-cache misses.
-    __shared__ __align__(16) Phase sphase[2];
-    {
-        const uint32_t* src = reinterpret_cast<const uint32_t*>(&P.phase[0]);
-        uint32_t* dst = reinterpret_cast<uint32_t*>(&sphase[0]);
-        for (int i = threadIdx.x; i < (int)(sizeof(Phase) * 2 / 4); i += kGemvThreads) dst[i] = src[i];
-        __syncthreads();
+// ---------------------------------------------------------------------------
+// main loop and output of a row block
+// ---------------------------------------------------------------------------
+// What a warp does in a phase: chunk slice [c0, c1) of row slice rw of wr.
+struct Slice {
+    int c0, c1, rw;
+};
+__device__ __forceinline__ Slice slice_of(const Job& jb) {
+    const int warp = threadIdx.x >> 5;
+    Slice s;
+    s.rw = (warp * jb.wk_magic) >> 16;
+    const int kc = (warp - s.rw * jb.wk) * jb.chunks;
+    s.c0 = (kc * jb.wk_magic) >> 16;
+    s.c1 = ((kc + jb.chunks) * jb.wk_magic) >> 16;
+    return s;
+}
+// Floats of a (chunk, token) in the partial sums: 8 mod 32 spreads the tokens over the banks.
+__device__ __forceinline__ int part_stride(const Job& jb) { return jb.gb * 16 + 8; }
+
+// Partial sums of `nb` row groups whose weights lie at `weights` (shared memory, or global for kShared = false):
+// part[chunk][token][row of the block].
+template <int CG, bool kShared>
+__device__ __forceinline__ void mma_block(const Job& jb, const Slice& sl, int nb, int T, const unsigned char* weights,
+                                          const unsigned char* xq, const int2* meta, float* part) {
+    const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
+    const int chunks = jb.chunks, tok_stride = part_stride(jb), slice = T * tok_stride;
+    // rows [r0, r1) of the block (a warp beyond the row slices has none)
+    const int r0 = (sl.rw * nb * jb.wr_magic) >> 16, r1 = sl.rw < jb.wr ? ((sl.rw + 1) * nb * jb.wr_magic) >> 16 : 0;
+    if (r0 >= r1) return;
+    // MMA columns (see above for the rows of xq): CG = 1: column g = term min(g%4, 2) of token g/4; CG = 2: column g
+    // of group 0 = term g%2 of token g/2, of group 1 = term 2 of token g/2.  Columns of tokens that do not exist re-read
+    // the last one.
+    int row_b[CG];
+    if (CG == 1) {
+        row_b[0] = 3 * min(g >> 2, T - 1) + min(g & 3, 2);
+    } else {
+        row_b[0] = 3 * min(g >> 1, T - 1) + (g & 1);
+        row_b[CG - 1] = 3 * min(g >> 1, T - 1) + 2;
     }
-    run_all<CG>(sphase, P, smem);
+    const int my_tok = CG == 1 ? q >> 1 : q;
+    float* my_part = part + my_tok * tok_stride + g + (CG == 1 ? 8 * (q & 1) : 0) + r0 * 16;
+#pragma unroll 1
+    for (int c = sl.c0; c < sl.c1; ++c) {
+        uint32_t b[CG][16];
+#pragma unroll
+        for (int cg = 0; cg < CG; ++cg) {
+            const unsigned char* src = xq + c * T * (3 * 256) + row_b[cg] * 256 + xq_unit(row_b[cg], q);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {   // unit 4 * i + q: the flipped bit (4) is bit 0 of i
+                const uint4 v = *reinterpret_cast<const uint4*>(src + ((row_b[cg] & 1) ? ((i ^ 1) - 1) * 64 : i * 64));
+                b[cg][4 * i] = v.x; b[cg][4 * i + 1] = v.y; b[cg][4 * i + 2] = v.z; b[cg][4 * i + 3] = v.w;
+            }
+        }
+        const int2 mt = meta[c * T + min(my_tok, T - 1)];
+        const float d = __int_as_float(mt.x);
+        const unsigned char* w = weights + (r0 * chunks + c) * 512 + lane * 16;
+        float* dst = my_part + c * slice;
+#pragma unroll 1
+        for (int r = r0; r < r1; ++r, w += chunks * 512, dst += 16) {
+            uint4 t;
+            if (kShared) t = *reinterpret_cast<const uint4*>(w);
+            else t = __ldg(reinterpret_cast<const uint4*>(w));
+            // two accumulator sets: the MMAs of a set depend on each other, and a warp of a small layer has one or
+            // two of these steps
+            int acc[2][CG][4];
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+#pragma unroll
+                for (int cg = 0; cg < CG; ++cg)
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) acc[h][cg][i] = 0;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const uint32_t m = 0x01010101u << j;
+#pragma unroll
+                for (int cg = 0; cg < CG; ++cg)
+                    mma_s8(acc[j & 1][cg], t.x & m, t.y & m, t.z & m, t.w & m, b[cg][2 * j], b[cg][2 * j + 1]);
+            }
+#pragma unroll
+            for (int cg = 0; cg < CG; ++cg)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) acc[0][cg][i] += acc[1][cg][i];
+            // sum(+-p) of the chunk = unit * (sum - 2 * S), S the sum over the set bits from its three byte
+            // terms: exact modulo 2^32, and the result is below 2^30
+            auto bits_sum = [](int t0, int t1, int t2) { return (uint32_t)t0 + ((uint32_t)t1 << 8) + ((uint32_t)t2 << 16); };
+            auto value = [&](uint32_t S) { return d * (float)(int)((uint32_t)mt.y - 2u * S); };
+            const int* a = acc[0][0];
+            if (CG == 1) {
+                // lanes 2t (terms 0, 1) and 2t+1 (term 2) of token t trade halves: each keeps one row
+                const uint32_t va = (q & 1) ? bits_sum(0, 0, a[0]) : bits_sum(a[0], a[1], 0);   // row g
+                const uint32_t vb = (q & 1) ? bits_sum(0, 0, a[2]) : bits_sum(a[2], a[3], 0);   // row g + 8
+                const uint32_t other = __shfl_xor_sync(0xffffffffu, (q & 1) ? va : vb, 1);
+                if (my_tok < T) dst[0] = value(((q & 1) ? vb : va) + other);
+            } else if (my_tok < T) {
+                const int* a2 = acc[0][CG - 1];
+                dst[0] = value(bits_sum(a[0], a[1], a2[0]));
+                dst[8] = value(bits_sum(a[2], a[3], a2[2]));
+            }
+        }
+    }
+}
+
+// Outputs of a block: adds the chunks, scales, stores.  Four neighbouring threads share an output (token-major, rows of
+// the block): thread i of them adds the chunks c = i mod 4 in order, then the four sums are added pairwise.
+struct RawOut {          // scale, bias, residual as loaded: conversions wait for the data, so they come where it is used
+    uint32_t post, bias, resid;
+};
+__device__ __forceinline__ uint32_t load_raw(const void* p, long long i) {   // (a plain 16-bit load is widened, that is waited for, at once)
+    uint16_t h;
+    asm volatile("ld.global.nc.u16 %0, [%1];" : "=h"(h) : "l"(static_cast<const uint16_t*>(p) + i));
+    return h;
+}
+__device__ __forceinline__ uint32_t load_raw_rw(const void* p, long long i) {   // (the residual may be the output buffer)
+    uint16_t h;
+    asm volatile("ld.global.u16 %0, [%1];" : "=h"(h) : "l"(static_cast<const uint16_t*>(p) + i) : "memory");
+    return h;
+}
+__device__ __forceinline__ void output_of(int o, int nb16, int T, int& tok, int& idx) {
+    tok = 0; idx = o;
+#pragma unroll
+    for (int t = 1; t < kMaxTok; ++t)
+        if (t < T && idx >= nb16) { idx -= nb16; ++tok; }
+}
+__device__ __forceinline__ void load_raw_out(RawOut& r, const Job& jb, int row0, int nb16, int T, int o) {
+    int tok, idx;
+    output_of(o, nb16, T, tok, idx);
+    const int row = row0 + idx;
+    if (o < T * nb16 && row < jb.rows) {
+        if (jb.post) r.post = load_raw(jb.post, row);
+        if (jb.bias) r.bias = load_raw(jb.bias, row);
+        if (jb.resid) r.resid = load_raw_rw(jb.resid, tok * jb.ld_res + row);
+    }
+}
+// kTagged: the intermediate (fp32 with the launch's tag), else the result.  `raw`: the operands of the first output.
+template <int KIND, bool kTagged>
+__device__ __forceinline__ void emit_block(const Job& jb, int row0, int nb, int T, const float* part, unsigned tag, RawOut raw) {
+    const int i = threadIdx.x & 3, nb16 = nb * 16;
+    const int chunks = jb.chunks, tok_stride = part_stride(jb), slice = T * tok_stride;
+#pragma unroll 1
+    for (int o = (int)threadIdx.x >> 2; (o & ~7) < T * nb16; o += kGemvThreads / 4) {   // whole warps: eight outputs each
+        int tok, idx;
+        output_of(o, nb16, T, tok, idx);
+        const int row = row0 + idx;
+        const bool live = o < T * nb16 && row < jb.rows;
+        if (o >= kGemvThreads / 4) load_raw_out(raw, jb, row0, nb16, T, o);
+        float v = 0.f;
+        if (live) {
+            const float* src = part + tok * tok_stride + idx + i * slice;
+#pragma unroll 4
+            for (int c = i; c < chunks; c += 4, src += 4 * slice) v += *src;
+        }
+        v += __shfl_xor_sync(0xffffffffu, v, 1);
+        v += __shfl_xor_sync(0xffffffffu, v, 2);
+        if (live && i == 0) {
+            if (jb.post) v *= to_float<KIND>((uint16_t)raw.post);
+            if (kTagged) {
+                store_tagged(jb.out, tok * jb.ld_out + row, v, tag);
+            } else {
+                // bias and residual in fp32 behind the output scale; same saturation bounds as the reference epilogue
+                if (jb.bias) v += to_float<KIND>((uint16_t)raw.bias);
+                if (jb.resid) v += to_float<KIND>((uint16_t)raw.resid);
+                constexpr float lim = KIND == KIND_F16 ? 64504.0f : 3.3895313892515355e+38f;
+                v = fminf(fmaxf(v, -lim), lim);
+                if (KIND == KIND_F16) static_cast<__half*>(jb.out)[tok * jb.ld_out + row] = __float2half(v);
+                else static_cast<__nv_bfloat16*>(jb.out)[tok * jb.ld_out + row] = __float2bfloat16(v);
+            }
+        }
+    }
+}
+
+// Phase 1 of a job for every CTA whose rows are not there yet: called by a CTA that has polled in vain for a while.  The
+// missing CTAs may not be running (other work holds their SMs), so a wait must not depend on them: this makes the
+// launch finish however few of its CTAs run at a time, without the cooperative attribute (which cost 0.5 us per launch in
+// a graph and 3 us in a stream).  A row computed twice is written with the same bits.
+template <int KIND, int CG>
+__device__ __noinline__ void help_phase1(const Job& jb, int T, unsigned char* xq, int2* meta, float* part, unsigned tag) {
+    const int tid = threadIdx.x;
+    const Slice sl = slice_of(jb);
+    bool have_input = false;
+    for (int k = 0; k < jb.ncta; ++k) {
+        const int b = (int)((blockIdx.x + k) % (unsigned)jb.ncta);       // every helper starts at another share
+        const int first = b * jb.g_q + min(b, jb.g_r), groups = jb.g_q + (b < jb.g_r ? 1 : 0);
+        bool there = true;
+        for (int e = tid; e < T * groups * 16; e += kGemvThreads) {
+            const int tok = e / (groups * 16), row = first * 16 + e - tok * groups * 16;
+            unsigned long long w = (unsigned long long)tag << 32;
+            if (row < jb.rows)
+                asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];"
+                             : "=l"(w) : "l"(static_cast<unsigned long long*>(jb.out) + tok * jb.ld_out + row) : "memory");
+            there = there && (unsigned)(w >> 32) == tag;
+        }
+        if (__syncthreads_and(there)) continue;
+        if (!have_input) {
+            quantise_x_any<KIND>(jb, T, xq, meta);
+            have_input = true;
+            __syncthreads();
+        }
+        for (int blk = 0; blk < groups; blk += jb.gb) {
+            const int nb = min(jb.gb, groups - blk), row0 = (first + blk) * 16;
+            mma_block<CG, false>(jb, sl, nb, T, reinterpret_cast<const unsigned char*>(jb.tiles + (size_t)(first + blk) * jb.chunks * 32),
+                                 xq, meta, part);
+            __syncthreads();
+            RawOut raw = {};
+            load_raw_out(raw, jb, row0, nb * 16, T, tid >> 2);
+            emit_block<KIND, true>(jb, row0, nb, T, part, tag, raw);
+            __syncthreads();
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------
+// the kernel
+// ---------------------------------------------------------------------------
+// CG: column groups of 8 MMA columns (1: up to two tokens, 2: up to four).
+//
+// The launch takes about 7 us; its 16 warps need 4 issue cycles of every scheduler, 2 ns, for each instruction of the
+// common path, and most of them wait for something short.  So the descriptors come into shared memory in one round trip,
+// quotients are precomputed, batches go through one copy of the code, nothing lives in local memory (a spilled
+// register is a cold line: 40 bytes of stack made the launch 10 % slower), and ONE thread moves the weights: a CTA's row
+// groups are contiguous in the tile layout, so a block of them is one bulk copy, and the blocks of both phases that fit
+// in shared memory (all of them, for 8B-class layers) are on their way before the dependency wait.
+template <int KIND, int CG>
+__global__ void __launch_bounds__(kGemvThreads, 1) gemv_group_kernel(const __grid_constant__ GemvParams Pc) {
+    extern __shared__ __align__(128) unsigned char smem[];
+    const int tid = threadIdx.x, lane = tid & 31;
+    const uint32_t bars = smem_u32(smem);                                  // weight slot s is full: bars + 8 s
+    // Nothing is read from the parameter bank but here, in one round trip for all of it: a first touch of a line there
+    // costs some 700 cycles, and scalars read where they were needed cost that several times over in every launch.
+    // Every warp reads its share with addresses that are the same in all lanes (different ones are served one by one).
+    const unsigned my_jobs = Pc.cta_job[blockIdx.x];
+    {
+        const int warp = tid >> 5;
+        uint4 w[(kParamWords + kGemvWarps - 1) / kGemvWarps];
+#pragma unroll
+        for (int i = 0; i * kGemvWarps < kParamWords; ++i)
+            w[i] = reinterpret_cast<const uint4*>(&Pc)[min(warp + i * kGemvWarps, kParamWords - 1)];
+        if (lane == 0) {
+#pragma unroll
+            for (int i = 0; i * kGemvWarps < kParamWords; ++i)
+                reinterpret_cast<uint4*>(smem + kOffParams)[min(warp + i * kGemvWarps, kParamWords - 1)] = w[i];
+        }
+    }
+    if (tid >= kGemvThreads - kMaxSlots) {
+        mbar_init(bars + 8 * (tid - (kGemvThreads - kMaxSlots)), 1);
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // initialised barriers -> the bulk copies
+    }
+    __syncthreads();
+    const GemvParams& P = *reinterpret_cast<const GemvParams*>(smem + kOffParams);
+    const Job* jobs = P.job;
+    int2* meta = reinterpret_cast<int2*>(smem + kOffMeta);                 // [chunk][token] {unit value, sum}
+    unsigned char* weights = smem + kFixedBytes;
+    const int T = P.T, slots = P.slots, slot_bytes = P.slot_bytes;
+    unsigned char* xq = smem + P.xq_off;
+    float* part = reinterpret_cast<float*>(smem + P.part_off);
+    unsigned* const header = P.header;
+    const unsigned help_after = P.help_after;
+    // This CTA's job in each phase and its row groups of it: every job has a contiguous range of CTAs of its own, so a
+    // CTA prepares the input of one job per phase.
+    int first[2], groups[2], ji[2];
+#pragma unroll
+    for (int ph = 0; ph < 2; ++ph) {
+        const int i = (int)(my_jobs >> (4 * ph)) & 15;
+        ji[ph] = ph * kMaxJobs + min(i, kMaxJobs - 1);
+        const Job& jb = jobs[ji[ph]];
+        const int2 range = *reinterpret_cast<const int2*>(&jb.cta0), share = *reinterpret_cast<const int2*>(&jb.g_q);
+        const int c = (int)blockIdx.x - range.x;
+        first[ph] = c * share.x + min(c, share.y);
+        groups[ph] = i == kMaxJobs ? 0 : share.x + (c < share.y ? 1 : 0);   // 0: no work in that phase
+    }
+    // weight blocks in the order they are used: phase, then row groups; block i goes to slot i % slots
+    int l_ph = 0, l_g = 0, l_slot = 0;       // next block to load (one thread's)
+    auto load_block = [&]() {
+        if (l_ph == 0 && l_g >= groups[0]) { l_ph = 1; l_g = 0; }
+        if (l_ph == 1 && l_g >= groups[1]) return;
+        const Job& jb = jobs[l_ph ? ji[1] : ji[0]];
+        const int nb = min(jb.gb, (l_ph ? groups[1] : groups[0]) - l_g);
+        const uint32_t bytes = (uint32_t)(nb * jb.chunks) * 512u, bar = bars + 8 * l_slot;
+        mbar_expect_tx(bar, bytes);
+        bulk_load(smem_u32(weights) + (uint32_t)(l_slot * slot_bytes),
+                  jb.tiles + (size_t)((l_ph ? first[1] : first[0]) + l_g) * jb.chunks * 32, bytes, bar);
+        l_g += nb;
+        l_slot = l_slot + 1 == slots ? 0 : l_slot + 1;
+    };
+    const bool loader = tid == kGemvThreads - kMaxSlots;
+    if (loader) {
+#pragma unroll 1
+        for (int s = 0; s < slots; ++s) load_block();
+    }
+    // Programmatic dependent launch: everything above may overlap with the tail of the previous kernel in the stream;
+    // activations and scratch (shared with that kernel) are only touched after it has completed.
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    // let the next kernel begin its prologue wherever an SM frees up
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    TagCtx tc;
+
+    int slot = 0;                            // of the next weight block, and its barrier's phase
+    uint32_t parity = 0;
+#pragma unroll 1
+    for (int ph = 0; ph < 2; ++ph) {
+        const int my_groups = ph ? groups[1] : groups[0], row0 = 16 * (ph ? first[1] : first[0]);
+        const Job& jb = jobs[ph ? ji[1] : ji[0]];
+        const Slice sl = slice_of(jb);
+        // Operands of this thread's first output: needed behind the loop, on their way from here.  (They and the tag are
+        // not carried around a loop: that would copy the registers, and the copy would wait for the loads.)
+        RawOut raw0 = {};
+        if (ph == 0) {
+            // tag of this launch: read by every thread, used behind the barrier (the round trip overlaps the input loads)
+            TagRaw tag_raw;
+            tag_read(tag_raw, header);
+            if (my_groups > 0) {
+                if (jb.vec) quantise_x<KIND, 2 * CG>(jb, T, xq, meta);
+                else quantise_x_any<KIND>(jb, T, xq, meta);
+                load_raw_out(raw0, jb, row0, min(jb.gb, my_groups) * 16, T, tid >> 2);
+            }
+            __syncthreads();   // quantised input complete
+            tag_finish(tc, tag_raw, header, P.spin_limit);
+        } else if (my_groups > 0) {
+            load_raw_out(raw0, jb, row0, min(jb.gb, my_groups) * 16, T, tid >> 2);
+            while (!__syncthreads_and(quantise_t<2 * CG>(jb, T, xq, meta, tc, help_after)))
+                help_phase1<KIND, CG>(jobs[ji[1] - kMaxJobs], T, xq, meta, part, tc.tag);
+        }
+#pragma unroll 1
+        for (int blk = 0; blk < my_groups; blk += jb.gb) {
+            const int nb = min(jb.gb, my_groups - blk);
+#pragma unroll 1
+            for (unsigned spins = 0; !mbar_try(bars + 8 * slot, parity); ++spins)
+                if (spins >= kWeightWaitLimit) { tag_wait_expired(tc); break; }
+            mma_block<CG, true>(jb, sl, nb, T, weights + slot * slot_bytes, xq, meta, part);
+            __syncthreads();   // partial sums complete, this block's weights have been read
+            if (++slot == slots) { slot = 0; parity ^= 1u; }
+            if (loader) load_block();
+            // every thread has compared or stored the tag, or never will
+            if (ph == 1 && blk == 0 && tid == 0) launch_arrive(reinterpret_cast<unsigned long long*>(header), blockIdx.x == 0, gridDim.x);
+            RawOut raw = raw0;
+            if (blk > 0) load_raw_out(raw, jb, row0 + blk * 16, nb * 16, T, tid >> 2);
+            if (ph == 0) emit_block<KIND, true>(jb, row0 + blk * 16, nb, T, part, tc.tag, raw);
+            else emit_block<KIND, false>(jb, row0 + blk * 16, nb, T, part, tc.tag, raw);
+            if (blk + jb.gb < my_groups) __syncthreads();   // the partial sums have been read
+        }
+    }
+    if (groups[1] == 0) {
+        __syncthreads();
+        if (tid == 0) launch_arrive(reinterpret_cast<unsigned long long*>(header), blockIdx.x == 0, gridDim.x);
+    }
 }
 
 static size_t round_up(size_t v, size_t m) { return (v + m - 1) / m * m; }
 
-// Opt-in shared memory limit for both instantiations, set once per device.
+static const void* gemv_kernel(int kind, int tokens) {
+    if (kind == KIND_F16) return tokens <= 2 ? (const void*)gemv_group_kernel<KIND_F16, 1> : (const void*)gemv_group_kernel<KIND_F16, 2>;
+    return tokens <= 2 ? (const void*)gemv_group_kernel<KIND_BF16, 1> : (const void*)gemv_group_kernel<KIND_BF16, 2>;
+}
+
+// Opt-in shared memory limit of every instantiation, set once per device.
 static int dynamic_smem_limit(int dev, int* out) {
     static int cached[64];
     if (cached[dev & 63] == 0) {
         int optin = 0, lim = 1 << 30;
         NQ_CUDA_TRY(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-        const void* fns[2] = {(const void*)gemv_group_kernel<1>, (const void*)gemv_group_kernel<2>};
-        for (const void* fn : fns) {
+        for (int i = 0; i < 4; ++i) {
+            const void* fn = gemv_kernel(i & 1 ? KIND_BF16 : KIND_F16, i & 2 ? kMaxTok : 1);
             cudaFuncAttributes fa;
             NQ_CUDA_TRY(cudaFuncGetAttributes(&fa, fn));
             const int v = optin - (int)fa.sharedSizeBytes;  // the opt-in limit covers static + dynamic
@@ -850,6 +703,51 @@ static int dynamic_smem_limit(int dev, int* out) {
     return NQ_OK;
 }
 
+// Deal `grid` CTAs to the jobs of a phase so that the largest per-CTA stream (row groups x chunks) is as small as
+// possible: shares in proportion to the work, the rest one by one to the job that is worst off.
+static void deal_ctas(int grid, int n, const int* groups, const int* chunks, int* ncta) {
+    long long total = 0;
+    for (int i = 0; i < n; ++i) total += (long long)groups[i] * chunks[i];
+    int used = 0;
+    for (int i = 0; i < n; ++i) {
+        long long share = (long long)groups[i] * chunks[i] * grid / total;
+        if (share > groups[i]) share = groups[i];
+        ncta[i] = share < 1 ? 1 : (int)share;
+        used += ncta[i];
+    }
+    while (used < grid) {
+        int best = -1;
+        long long best_cost = -1;
+        for (int i = 0; i < n; ++i) {
+            if (ncta[i] >= groups[i]) continue;      // one row group per CTA already
+            const long long cost = (long long)((groups[i] + ncta[i] - 1) / ncta[i]) * chunks[i];
+            if (cost > best_cost) { best_cost = cost; best = i; }
+        }
+        if (best < 0) break;
+        ++ncta[best];
+        ++used;
+    }
+    while (used > grid) {      // the minimum of one each may have gone over
+        int most = 0;
+        for (int i = 1; i < n; ++i) most = ncta[i] > ncta[most] ? i : most;
+        --ncta[most];
+        --used;
+    }
+}
+
+// Chunk slices x row slices of the 16 warps for `groups` row groups of `chunks` chunks.  A step (512 bytes of weights)
+// costs about twice as much as fetching the B fragments of a chunk once.
+static void split_warps(int groups, int chunks, Job& j) {
+    int best = 1 << 30;
+    for (int k = 1; k <= kGemvWarps && k <= chunks; ++k) {
+        int r = kGemvWarps / k;
+        if (r > groups) r = groups;
+        const int cost = ((chunks + k - 1) / k) * (2 * ((groups + r - 1) / r) + 1);
+        if (cost < best) { best = cost; j.wk = (uint16_t)k; j.wr = (uint16_t)r; }
+    }
+    j.wk_magic = (65536 + j.wk - 1) / j.wk;
+    j.wr_magic = (65536 + j.wr - 1) / j.wr;
+}
 
 // ---------------------------------------------------------------------------
 // GEMV without caller-provided scratch
@@ -879,6 +777,9 @@ static int static_scratch_ptr(void** out) {
     return NQ_OK;
 }
 
+// {fp32, tag} words of a linear's intermediate, rows padded to eight elements
+static size_t intermediate_bytes(int R) { return round_up((size_t)kMaxTok * (size_t)((R + 7) / 8 * 8) * sizeof(uint2), 256); }
+
 static unsigned g_spin_limit = kSpinLimit;   // polls before a wait for the tagged intermediate gives up
 
 }  // namespace nq
@@ -889,7 +790,7 @@ extern "C" {
 
 size_t nq_gemv_scratch_bytes(int T, int N, int R, int M) {
     if (T <= 0 || N <= 0 || R <= 0 || M <= 0) return 0;
-    return kHeaderBytes + round_up((size_t)kMaxTok * (size_t)R * sizeof(uint2), 256);
+    return kHeaderBytes + intermediate_bytes(R);
 }
 
 size_t nq_gemv_group_scratch_bytes(const nq_linear_desc* d, int n_linears, int T) {
@@ -897,7 +798,7 @@ size_t nq_gemv_group_scratch_bytes(const nq_linear_desc* d, int n_linears, int T
     size_t b = kHeaderBytes;
     for (int i = 0; i < n_linears; ++i) {
         if (d[i].R <= 0) return 0;
-        b += round_up((size_t)kMaxTok * (size_t)d[i].R * sizeof(uint2), 256);
+        b += intermediate_bytes(d[i].R);
     }
     return b;
 }
@@ -911,7 +812,9 @@ int nq_gemv_group_fwd(const nq_linear_desc* d, int n_linears, int T, int dtype, 
     if (!aligned16(scratch)) return NQ_ERR_ALIGN;
     if (scratch_bytes < nq_gemv_group_scratch_bytes(d, n_linears, T)) return NQ_ERR_SCRATCH;
 
-    int maxK = 0;
+    int max_chunks = 0;
+    int rg[2][kMaxJobs], ck[2][kMaxJobs];      // row groups and chunks of the two phases
+    size_t packed = 0;
     for (int i = 0; i < n_linears; ++i) {
         const nq_linear_desc& L = d[i];
         if (!L.x || !L.s_in || !L.v_tiles || !L.u_tiles || !L.s_out || !L.y) return NQ_ERR_NULL;
@@ -920,8 +823,10 @@ int nq_gemv_group_fwd(const nq_linear_desc* d, int n_linears, int T, int dtype, 
         if (L.residual && L.ldr < L.M) return NQ_ERR_SHAPE;
         if (L.N > kMaxK || L.R > kMaxK) return NQ_ERR_UNSUPPORTED;
         if (!aligned16(L.v_tiles) || !aligned16(L.u_tiles)) return NQ_ERR_ALIGN;
-        maxK = L.N > maxK ? L.N : maxK;
-        maxK = L.R > maxK ? L.R : maxK;
+        rg[0][i] = (L.R + 15) / 16; ck[0][i] = (L.N + 255) / 256;
+        rg[1][i] = (L.M + 15) / 16; ck[1][i] = (L.R + 255) / 256;
+        for (int ph = 0; ph < 2; ++ph) max_chunks = ck[ph][i] > max_chunks ? ck[ph][i] : max_chunks;
+        packed += (size_t)L.R * ((size_t)L.N + L.M) / 8;
     }
     int dev = 0, smem_limit = 0;
     NQ_CUDA_TRY(cudaGetDevice(&dev));
@@ -929,144 +834,134 @@ int nq_gemv_group_fwd(const nq_linear_desc* d, int n_linears, int T, int dtype, 
         const int st = dynamic_smem_limit(dev, &smem_limit);
         if (st != NQ_OK) return st;
     }
-    // Number of CTAs: the dependent chain of a launch (broadcast of the input, hand-over of the intermediate,
-    // barriers, completion) costs about 15 ns per participating CTA, the stream gains from every SM.  Small
-    // launches therefore run on fewer CTAs than there are SMs (measured optimum on 148 SMs: 80-96 CTAs up to
-    // 5 MB of packed factors, 128 around 10 MB, all of them from 20 MB), which also lets the next kernel's CTAs
-    // start their prologue on the idle SMs.
-    const int sms = sm_count();
-    size_t packed = 0;
-    for (int i = 0; i < n_linears; ++i) packed += (size_t)d[i].R * ((size_t)d[i].N + d[i].M) / 8;
-    int grid = packed < (size_t)(3 << 20) ? sms * 3 / 5 : packed < (size_t)(7 << 20) ? sms * 13 / 20
-               : packed < (size_t)(20 << 20) ? sms * 7 / 8 : sms;
-    if (grid < kMaxJobs) grid = sms;
-    int cta_n[2][kMaxJobs];
-    int max_items = 1;
-    for (int ph = 0; ph < 2; ++ph) {
-        // deal the CTAs to the jobs of the phase: every job gets a contiguous range, sized so that the longest
-        // per-CTA stream (row tiles x chunks) is as short as possible
-        int items[kMaxJobs], chunks[kMaxJobs];
-        for (int i = 0; i < n_linears; ++i) {
-            items[i] = ((ph ? d[i].M : d[i].R) + 31) / 32;
-            chunks[i] = ((ph ? d[i].R : d[i].N) + 255) / 256;
-            cta_n[ph][i] = 1;
-        }
-        for (int used = n_linears; used < grid; ++used) {
-            int best = -1;
-            long long best_cost = -1;
-            for (int i = 0; i < n_linears; ++i) {
-                if (cta_n[ph][i] >= items[i]) continue;      // one tile per CTA already
-                const long long cost = (long long)((items[i] + cta_n[ph][i] - 1) / cta_n[ph][i]) * chunks[i];
-                if (cost > best_cost) { best_cost = cost; best = i; }
-            }
-            if (best < 0) break;
-            ++cta_n[ph][best];
-        }
-        for (int i = 0; i < n_linears; ++i) {
-            const int most = (items[i] + cta_n[ph][i] - 1) / cta_n[ph][i];
-            max_items = most > max_items ? most : max_items;
-        }
-    }
-    const int kpad = (maxK + 255) / 256 * 256;
-    const int stride = kpad + 32;  // 32 mod 128: conflict-free 64-bit fragment loads
+    GemvParams P;
+    memset(&P, 0, sizeof(P));
+    P.header = static_cast<unsigned*>(scratch);
+    P.spin_limit = g_spin_limit;
+    P.help_after = g_spin_limit / 16 < kHelpAfter ? g_spin_limit / 16 : kHelpAfter;
 
-    // tokens are processed in groups that fit the MMA columns (3 per token) and shared memory
-    auto cg_for = [](int t) { return t <= 2 ? 1 : 2; };
-    auto smem_for = [&](int t) {
-        return kFixedBytes + kRingBytes + (size_t)max_items * (128 * 8 * cg_for(t)) + (size_t)3 * t * stride +
-               (size_t)max_items * 128;   // + output scales of two jobs
-    };
+    // One CTA per SM, fewer for launches with less than 3 MB of packed factors (the o projection of an 8B-class layer and
+    // everything smaller): their row groups do not divide any finer by 148, and every CTA fetches the whole input and polls
+    // the whole intermediate.  Measured on Qwen3-8B at one token: all SMs 255, 7/10 of them 250, half of them 267 us per
+    // eight layers; with 7/8 for up to 20 MB 254.
+    int grid = sm_count() < kMaxCtas ? sm_count() : kMaxCtas;
+    if (packed < ((size_t)3 << 20)) grid = grid * 7 / 10;
+    {   // no more CTAs than the larger phase has row groups
+        int g[2] = {0, 0};
+        for (int i = 0; i < n_linears; ++i) { g[0] += rg[0][i]; g[1] += rg[1][i]; }
+        const int most = g[0] > g[1] ? g[0] : g[1];
+        if (grid > most) grid = most;
+        if (grid < n_linears) grid = n_linears;
+    }
+    // tokens are processed in groups that fit the MMA columns (3 per token) and shared memory: the quantised input,
+    // one row group's weights and its partial sums at least
     int tg = T < kMaxTok ? T : kMaxTok;
-    while (tg > 1 && smem_for(tg) > (size_t)smem_limit) --tg;
-    if (smem_for(tg) > (size_t)smem_limit) return NQ_ERR_UNSUPPORTED;
+    auto fixed_bytes = [&](int t) { return kFixedBytes + (size_t)3 * t * max_chunks * 256; };
+    const size_t least = (size_t)max_chunks * 512, least_part = (size_t)max_chunks * (16 + 8) * 4;   // part: per token
+    while (tg > 1 && fixed_bytes(tg) + least + tg * least_part > (size_t)smem_limit) --tg;
+    if (fixed_bytes(tg) + least + tg * least_part > (size_t)smem_limit) return NQ_ERR_UNSUPPORTED;
+
+    int cta_n[2][kMaxJobs];
+    for (int ph = 0; ph < 2; ++ph) deal_ctas(grid, n_linears, rg[ph], ck[ph], cta_n[ph]);
 
     const size_t esz = 2;
     for (int t0 = 0; t0 < T; t0 += tg) {
         const int tn = (T - t0) < tg ? (T - t0) : tg;
-        GemvParams P;
-        memset(&P, 0, sizeof(P));
-        P.header = static_cast<unsigned*>(scratch);
-        P.spin_limit = g_spin_limit;
         P.T = tn;
-        P.scale_kind = dtype;
-        P.xq_stride = stride;
-        P.max_items = max_items;
-        P.phase[0].njobs = P.phase[1].njobs = n_linears;
+        memset(P.cta_job, kMaxJobs * 17, sizeof(P.cta_job));
+        // room for a block's partial sums and weights; a single row group is always allowed (see above)
+        const size_t room = smem_limit - fixed_bytes(tn);
+        const size_t slot_room = room / 2 < kSlotBytes ? room / 2 : kSlotBytes;
+        const size_t slot_most = slot_room > least ? slot_room : least;
+        const size_t part_room = room - slot_most < kPartBytes ? room - slot_most : kPartBytes;
+        size_t part_used = 0, slot_used = 0;
+        int most_blocks = 0;
         size_t off = kHeaderBytes;
-        int cta_a = 0, cta_b = 0;       // first CTA of the next job's range in the two phases
+        int cta[2] = {0, 0};            // first CTA of the next job's range in the two phases
         for (int i = 0; i < n_linears; ++i) {
             const nq_linear_desc& L = d[i];
             void* tbuf = static_cast<char*>(scratch) + off;   // {fp32, tag} pairs, 8 bytes per element
-            off += round_up((size_t)kMaxTok * (size_t)L.R * sizeof(uint2), 256);
-            Job& a = P.phase[0].job[i];
+            const int ld_t = (L.R + 7) / 8 * 8;               // rows of the intermediate start on 64-byte boundaries
+            off += intermediate_bytes(L.R);
+            Job& a = P.job[i];
             a.tiles = static_cast<const uint4*>(L.v_tiles);
             a.in = static_cast<const char*>(L.x) + (size_t)t0 * L.ldx * esz;
             a.pre = L.s_in;
             a.post = L.s_mid;
             a.out = tbuf;
             a.ld_in = L.ldx;
-            a.ld_out = L.R;
+            a.ld_out = ld_t;
             a.rows = L.R;
             a.K = L.N;
-            a.chunks = (L.N + 255) / 256;
-            a.items = (L.R + 31) / 32;
-            a.in_kind = dtype;
-            a.out_kind = KIND_T;
             a.vec = (L.N % 8 == 0) && (L.ldx % 8 == 0) && aligned16(a.in) && aligned16(L.s_in);
-            a.post_vec = L.s_mid && (L.R % 8 == 0) && aligned16(L.s_mid);
-            a.cta0 = cta_a;
-            a.ncta = cta_n[0][i];
-            a.t_q = a.items / a.ncta;
-            a.t_r = a.items % a.ncta;
-            cta_a += a.ncta;
-            Job& b = P.phase[1].job[i];
+            Job& b = P.job[kMaxJobs + i];
             b.tiles = static_cast<const uint4*>(L.u_tiles);
             b.in = tbuf;
-            b.pre = nullptr;
             b.post = L.s_out;
             b.out = static_cast<char*>(L.y) + (size_t)t0 * L.ldy * esz;
             b.bias = L.bias;
             b.resid = L.residual ? static_cast<const char*>(L.residual) + (size_t)t0 * L.ldr * esz : nullptr;
             b.ld_res = L.ldr;
-            b.ld_in = L.R;
+            b.ld_in = ld_t;
             b.ld_out = L.ldy;
             b.rows = L.M;
             b.K = L.R;
-            b.chunks = (L.R + 255) / 256;
-            b.items = (L.M + 31) / 32;
-            b.in_kind = KIND_T;
-            b.out_kind = dtype;
-            b.vec = (L.R % 8 == 0);  // the intermediate lives in the 256-byte aligned scratch
-            b.post_vec = (L.M % 8 == 0) && aligned16(L.s_out);
-            b.cta0 = cta_b;
-            b.ncta = cta_n[1][i];
-            b.t_q = b.items / b.ncta;
-            b.t_r = b.items % b.ncta;
-            cta_b += b.ncta;
+            for (int ph = 0; ph < 2; ++ph) {
+                Job& j = P.job[ph * kMaxJobs + i];
+                j.chunks = ck[ph][i];
+                j.cta0 = cta[ph];
+                j.ncta = cta_n[ph][i];
+                j.g_q = rg[ph][i] / j.ncta;
+                j.g_r = rg[ph][i] % j.ncta;
+                for (int c = 0; c < j.ncta; ++c) {
+                    uint8_t& m = P.cta_job[cta[ph] + c];
+                    m = (uint8_t)(ph ? (m & 0x0F) | (i << 4) : (m & 0xF0) | i);
+                }
+                cta[ph] += j.ncta;
+                // blocks of row groups whose weights and partial sums fit their space, as equal as possible
+                const int most = j.g_q + (j.g_r ? 1 : 0);
+                auto part_bytes = [&](int gb) { return (size_t)j.chunks * tn * (gb * 16 + 8) * 4; };
+                for (int blocks = 1;; ++blocks) {
+                    j.gb = (most + blocks - 1) / blocks;
+                    if (j.gb == 1 || (part_bytes(j.gb) <= part_room && (size_t)j.gb * j.chunks * 512 <= slot_room && j.gb <= 128)) break;
+                }
+                split_warps(j.gb, j.chunks, j);
+                const size_t part = part_bytes(j.gb), slot = (size_t)j.gb * j.chunks * 512;
+                part_used = part > part_used ? part : part_used;
+                slot_used = slot > slot_used ? slot : slot_used;
+                const int blocks = (most + j.gb - 1) / j.gb;
+                most_blocks = blocks > most_blocks ? blocks : most_blocks;
+            }
         }
+        int slots = 2 * most_blocks;      // no CTA has more blocks than that in its two phases
+        if (slots > kMaxSlots) slots = kMaxSlots;
+        while (slots > 1 && fixed_bytes(tn) + part_used + slots * slot_used > (size_t)smem_limit) --slots;
+        P.slots = slots;
+        P.slot_bytes = (int)slot_used;
+        P.xq_off = (int)(kFixedBytes + slots * slot_used);
+        P.part_off = P.xq_off + 3 * tn * max_chunks * 256;
+        const size_t smem_bytes = P.part_off + part_used;
+        if (smem_bytes > (size_t)smem_limit) return NQ_ERR_UNSUPPORTED;
         void* args[] = {&P};
-        const void* fn = cg_for(tn) == 1 ? (const void*)gemv_group_kernel<1> : (const void*)gemv_group_kernel<2>;
-        // Cooperative launch (all CTAs co-resident: phase 2 spins on data of other CTAs) plus programmatic stream
-        // serialization, so that this kernel's prologue overlaps the previous kernel's tail.  If the driver
-        // refuses the combination once, plain cooperative launches are used from then on.
+        // Programmatic stream serialization, so that this kernel's prologue overlaps the previous kernel's tail.  If the
+        // driver refuses the attribute once, plain launches are used from then on.
         static bool pdl_ok = true;
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(grid);
         cfg.blockDim = dim3(kGemvThreads);
-        cfg.dynamicSmemBytes = smem_for(tn);
+        cfg.dynamicSmemBytes = smem_bytes;
         cfg.stream = as_stream(stream);
-        cudaLaunchAttribute attrs[2];
-        attrs[0].id = cudaLaunchAttributeCooperative;
-        attrs[0].val.cooperative = 1;
-        attrs[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attrs[1].val.programmaticStreamSerializationAllowed = 1;
-        cfg.attrs = attrs;
-        cfg.numAttrs = pdl_ok ? 2 : 1;
+        cudaLaunchAttribute attr;
+        attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr.val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = &attr;
+        cfg.numAttrs = pdl_ok ? 1 : 0;
+        const void* fn = gemv_kernel(dtype, tn);
         cudaError_t e = cudaLaunchKernelExC(&cfg, fn, args);
         if (e != cudaSuccess && pdl_ok) {
             (void)cudaGetLastError();
             pdl_ok = false;
-            cfg.numAttrs = 1;
+            cfg.numAttrs = 0;
             e = cudaLaunchKernelExC(&cfg, fn, args);
         }
         NQ_CUDA_TRY(e);
