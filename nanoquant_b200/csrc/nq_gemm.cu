@@ -43,6 +43,7 @@
 #include <cstring>
 
 #include "nq_common.cuh"
+#include "nq_stage.h"
 
 namespace nq {
 
@@ -115,7 +116,6 @@ struct alignas(64) GemmJob {
     int splits, chunks_per;
     int tile0;             // first grid.x index of this job's tiles
 };
-constexpr int kMaxGemmJobs = 4;
 
 struct GemmParams {
     GemmJob job[kMaxGemmJobs];
@@ -793,26 +793,6 @@ static EncodeTiledFn encode_tiled_fn() {
     return fn;
 }
 
-// One linear's stage as the host sees it.
-struct StageJob {
-    const void* a;          // activations [T, K], row stride lda elements
-    long long lda;
-    const void* tiles;
-    const void* pre;
-    const void* post;
-    void* out;
-    long long ld_out;
-    int K, Nout;
-    const void* bias;       // [Nout] or nullptr
-    const void* resid;      // [T, ld_res] or nullptr
-    long long ld_res;
-    const int* row_exp;     // [T] per-token exponents of the intermediate or nullptr
-};
-// Types of a stage: scales / bias / residual, MMA operands, output; sign of the row exponents (0: none).
-struct StageTypes {
-    int io_bf16, a_bf16, out_bf16, exp_sign;
-};
-
 // Tile shape of a launch and the k split of each of its jobs.
 struct GroupPlan {
     int mh, nh;                       // tile: 128*mh tokens x 128*nh weight rows
@@ -995,6 +975,7 @@ static int launch_stage(const StageJob* jobs, int n, int T, StageTypes ty, int s
         if (S.pre && !aligned16(S.pre)) return NQ_ERR_ALIGN;
         Ks[j] = S.K; Ns[j] = S.Nout;
     }
+    if (T <= batch_max_tokens(jobs, n)) return launch_batch_stage(jobs, n, T, ty, saturate, status, stream);
     { const int st_attr = set_kernel_attributes(); if (st_attr != NQ_OK) return st_attr; }
     const GroupPlan pl = plan_group(T, n, Ks, Ns, counters != nullptr && slabs != nullptr, true);
     const int mh = pl.mh, nh = pl.nh;

@@ -1,0 +1,34 @@
+// One stage of a launch group as the host sees it: Out_j[T, Nout_j] = (A_j[T, K_j] . W_j^T) * post_j for up to four
+// linears.  Implemented by the tensor-core GEMM (nq_gemm.cu) and, for few tokens, by the batch kernel (nq_batch.cu).
+#pragma once
+
+#include <cuda_runtime.h>
+
+namespace nq {
+
+constexpr int kMaxGemmJobs = 4;
+
+struct StageJob {
+    const void* a;          // activations [T, K], row stride lda elements; 16-byte aligned rows, K a multiple of 8
+    long long lda;
+    const void* tiles;
+    const void* pre;        // [K] input scales or nullptr (ones)
+    const void* post;       // [Nout] output scales or nullptr
+    void* out;
+    long long ld_out;
+    int K, Nout;
+    const void* bias;       // [Nout] or nullptr
+    const void* resid;      // [T, ld_res] or nullptr
+    long long ld_res;
+    const int* row_exp;     // [T] per-token exponents of the intermediate or nullptr
+};
+// Types of a stage: scales / bias / residual, MMA operands, output; sign of the row exponents (0: none).
+struct StageTypes {
+    int io_bf16, a_bf16, out_bf16, exp_sign;
+};
+
+// Most tokens of the batch kernel; 0 where it cannot take the jobs.
+int batch_max_tokens(const StageJob* jobs, int n);
+int launch_batch_stage(const StageJob* jobs, int n, int T, StageTypes ty, int saturate, unsigned* status, cudaStream_t stream);
+
+}  // namespace nq
