@@ -11,11 +11,17 @@
 //  * mma.sync m16n8k16 (16 rows x 8 tokens).  The bits of columns {4q, 4q+2} and {4q+1, 4q+3} of a 16-column block are
 //    16 apart in the lane's word, so a shift and ONE LOP3 ((word & 0x80008000) ^ {s, s'}) make an A register +-s: the
 //    product x * (+-s_in) is exact.  The columns of a block may be permuted as long as A and B agree, so the B fragment
-//    of a token is its four consecutive columns 4q..4q+3: one 64-bit load from global memory, no staging.
+//    of a token is its four consecutive columns 4q..4q+3.
+//  * B fragments.  The intermediate is stored in fragment order (see fragment_index): a warp's load of one is 256
+//    contiguous bytes.  Activations come in rows: every warp stages its own columns through shared memory with 16-byte
+//    copies, 192 of them in flight.  (Fragments loaded from rows touch eight lines each, 2 us of L1 tag lookups in a stage of 6.)
 //  * Two barriers; no K split over CTAs, no counters, no slabs.
 //
-// Qwen3-8B decode, eight layers in a graph, GEMM against this kernel: 8 tokens 804 -> 433 us, 16 tokens 825 -> 544 us; 32
-// tokens 842 -> 1141 us, where it stops.
+// Splitting K over the CTAs of a cluster (partial sums exchanged through distributed shared memory) and staging the whole
+// input by bulk copies before the loop both measured slower than this at every size.
+// Qwen3-8B decode, eight layers in a graph, GEMM against this kernel: 8 tokens 804 -> 359 us, 16 tokens 825 -> 438 us.  At 16
+// tokens a stage with little work takes 4.4 us; gate/up's second stage 12 (16 clocks per MMA and scheduler), down's
+// first 11.5 (58 MB of activations from L2 to the SMs, 7 TB/s).
 #include <cstddef>
 #include <cstring>
 
@@ -27,13 +33,14 @@ namespace nq {
 
 constexpr int kBatchThreads = 512;
 constexpr int kBatchWarps = kBatchThreads / 32;
-constexpr int rows_per_pass(int nt) { return nt == 4 ? 2 : 4; }     // row groups a warp keeps accumulators for
-constexpr int blocks_in_flight(int nt) { return nt == 1 ? 8 : 4; }  // 16-column blocks whose B fragments are loaded together
+// 16-column blocks of the intermediate whose B fragments a warp loads together
+constexpr int blocks_in_flight(int nt, int rows) { return nt == 1 || rows < 4 ? 8 : 4; }
+constexpr int kPieces = 3;               // pieces of 64 columns a warp has in flight
+constexpr int kPieceStride = 128 + 32;   // bytes of a staged row: 32 mod 128, so the eight tokens of a fragment fall on
+                                         // different banks
 constexpr int kBatchSlots = 8;           // weight blocks in flight
 constexpr int kBatchMaxCtas = 256;
 constexpr size_t kOffParams = 64, kFixedBytes = 1024;
-constexpr size_t kSlotBytes = 64 << 10;  // weights of a row block
-constexpr size_t kPartBytes = 64 << 10;  // partial sums of a row block
 constexpr unsigned kWeightWaitLimit = 1u << 20;   // attempts of up to ~2 us each
 
 struct alignas(16) BatchJob {
@@ -57,7 +64,8 @@ struct alignas(16) BatchParams {
     BatchJob job[kMaxGemmJobs];
     unsigned* status;
     int T, io_bf16, out_bf16, saturate, exp_sign;
-    int slots, slot_bytes, part_off, pad[2];
+    int slots, slot_bytes, part_off;
+    int stage_off, frag_out;      // activation staging buffers; output in fragment order
     uint8_t cta_job[kBatchMaxCtas];
 };
 constexpr int kBatchWords = (int)offsetof(BatchParams, cta_job) / 16;
@@ -79,10 +87,23 @@ __device__ __forceinline__ float float_of(uint16_t h, int bf16) {
 __device__ __forceinline__ uint32_t even_columns(uint2 v) { return __byte_perm(v.x, v.y, 0x5410); }
 __device__ __forceinline__ uint32_t odd_columns(uint2 v) { return __byte_perm(v.x, v.y, 0x7632); }
 
-// NT: column groups of eight tokens.
-template <bool BF16, int NT>
+// Fragment order of an intermediate [T, K]: per chunk, 16-column block (32 j + 16 h) and group of eight tokens, the 8
+// bytes {columns 4q, 4q+2, 4q+1, 4q+3} of lane 4g + q (token g of the group).  Element index; the layout has
+// chunks * 16 * NT * 128 elements, those of columns and tokens that do not exist are never used.
+template <int NT>
+__device__ __forceinline__ long long fragment_index(int tok, int k) {
+    const int b = k & 3;
+    return (((long long)(k >> 4) * NT + (tok >> 3)) * 32 + 4 * (tok & 7) + ((k >> 2) & 3)) * 4 + ((b >> 1) | ((b & 1) << 1));
+}
+__device__ __forceinline__ void copy16_or_zero(uint32_t dst, const void* src, bool there) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(there ? 16 : 0) : "memory");
+}
+
+// NT: column groups of eight tokens.  ROWS: row groups a warp takes in a pass.  FRAG: the input is in fragment order
+// and has no scale (the second stage); otherwise it is [T, lda].
+template <bool BF16, int NT, int ROWS, bool FRAG>
 __global__ void __launch_bounds__(kBatchThreads, 1) batch_stage_kernel(const __grid_constant__ BatchParams Pc) {
-    constexpr int kRows = rows_per_pass(NT), kB = blocks_in_flight(NT);
+    constexpr int kRows = ROWS, kB = blocks_in_flight(NT, ROWS);
     extern __shared__ __align__(128) unsigned char smem[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, q = lane & 3;
     const uint32_t bars = smem_u32(smem);
@@ -136,10 +157,30 @@ __global__ void __launch_bounds__(kBatchThreads, 1) batch_stage_kernel(const __g
     const int c0 = (kw * chunks * jb.wk_magic) >> 16, c1 = ((kw + 1) * chunks * jb.wk_magic) >> 16;
     const int wr_magic = jb.wr_magic, K = jb.K, tok_stride = gb * 16 + 4;   // 4 mod 16: an accumulator's 32 stores fall on 32 banks
     const uint16_t* const pre = static_cast<const uint16_t*>(jb.pre);
-    const uint16_t* a_row[NT];
+    const uint16_t* const a_in = static_cast<const uint16_t*>(jb.a);
+    const long long lda = jb.lda;
+    // staging: buffers of T + 1 rows (the scales last) of 64 columns, one piece each
+    const int piece_bytes = (T + 1) * kPieceStride;
+    unsigned char* const stage = smem + P.stage_off + warp * kPieces * piece_bytes;
+    int a_row[NT];
 #pragma unroll
-    for (int nt = 0; nt < NT; ++nt)
-        a_row[nt] = static_cast<const uint16_t*>(jb.a) + (long long)min(8 * nt + g, T - 1) * jb.lda + 4 * q;   // tokens beyond T: not stored
+    for (int nt = 0; nt < NT; ++nt) a_row[nt] = min(8 * nt + g, T - 1) * kPieceStride + 8 * q;   // tokens beyond T: not stored
+    int s_in = 0, s_out = 0;             // next buffer to fill, to read
+    // piece `pc` (columns 64 pc ..): eight lanes per row
+    auto stage_piece = [&](int pc) {
+        if (pc < 4 * c1) {
+            const int col = pc * 64 + (lane & 7) * 8, t0 = lane >> 3;
+            const bool there = col < K;          // K is a multiple of 8
+            const uint32_t dst = smem_u32(stage + s_in * piece_bytes) + (uint32_t)(t0 * kPieceStride + (lane & 7) * 16);
+            const uint16_t* src = a_in + (there ? col : 0);
+#pragma unroll
+            for (int t = 0; t < 8 * NT; t += 4)
+                if (t + t0 < T) copy16_or_zero(dst + (uint32_t)(t * kPieceStride), src + (t + t0) * lda, there);
+            if (pre && lane < 8) copy16_or_zero(dst + (uint32_t)(T * kPieceStride), pre + (there ? col : 0), there);
+            s_in = s_in + 1 == kPieces ? 0 : s_in + 1;
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
@@ -149,6 +190,13 @@ __global__ void __launch_bounds__(kBatchThreads, 1) batch_stage_kernel(const __g
     for (int blk = 0; blk < groups; blk += gb) {
         const int nb = min(gb, groups - blk);
         const int r0 = (rw * nb * wr_magic) >> 16, r1 = rw < wr ? ((rw + 1) * nb * wr_magic) >> 16 : r0;
+        // output scale and bias of row `tid` of the block (asm: a plain 16-bit load is widened, that is waited for, at once)
+        const int row0 = (first + blk) * 16;
+        uint16_t post_raw = 0, bias_raw = 0;
+        if (tid < nb * 16 && row0 + tid < rows) {
+            if (jb.post) asm volatile("ld.global.nc.u16 %0, [%1];" : "=h"(post_raw) : "l"(static_cast<const uint16_t*>(jb.post) + row0 + tid));
+            if (jb.bias) asm volatile("ld.global.nc.u16 %0, [%1];" : "=h"(bias_raw) : "l"(static_cast<const uint16_t*>(jb.bias) + row0 + tid));
+        }
 #pragma unroll 1
         for (int rb = r0; rb < r1; rb += kRows) {
             const int nr = min(kRows, r1 - rb);
@@ -159,49 +207,83 @@ __global__ void __launch_bounds__(kBatchThreads, 1) batch_stage_kernel(const __g
                 for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
                     for (int i = 0; i < 4; ++i) acc[r][nt][i] = 0.f;
+            if (!FRAG && c0 < c1) {
+#pragma unroll 1
+                for (int i = 0; i < kPieces; ++i) stage_piece(4 * c0 + i);
+            }
+            if (rb == r0) {
+#pragma unroll 1
+                for (unsigned spins = 0; !mbar_try(bars + 8 * slot, parity); ++spins)
+                    if (spins >= kWeightWaitLimit) { atomicExch(P.status, (unsigned)(-NQ_ERR_TIMEOUT)); break; }
+            }
+            const uint32_t one2 = BF16 ? 0x3F803F80u : 0x3C003C00u;
+            // block b of a chunk (columns 32 j + 16 h + ..) against all row groups
+            auto block = [&](const uint4 (&w)[kRows], int b, uint32_t se, uint32_t so, const uint32_t (&be)[NT], const uint32_t (&bo)[NT]) {
+                const int j = b >> 1, h = b & 1;
+#pragma unroll
+                for (int r = 0; r < kRows; ++r)
+                    if (r < nr) {
+                        const uint32_t w0 = h ? w[r].z : w[r].x, w1 = h ? w[r].w : w[r].y;   // rows g, g + 8
+                        const uint32_t a0 = ((w0 << (15 - j)) & 0x80008000u) ^ se, a2 = ((w0 << (7 - j)) & 0x80008000u) ^ so;
+                        const uint32_t a1 = ((w1 << (15 - j)) & 0x80008000u) ^ se, a3 = ((w1 << (7 - j)) & 0x80008000u) ^ so;
+#pragma unroll
+                        for (int nt = 0; nt < NT; ++nt) mma_16816<BF16>(acc[r][nt], a0, a1, a2, a3, be[nt], bo[nt]);
+                    }
+            };
 #pragma unroll 1
             for (int c = c0; c < c1; ++c) {
+                uint4 w[kRows];
 #pragma unroll
-                for (int b0 = 0; b0 < 16; b0 += kB) {
-                    uint2 x[NT][kB], s[kB];
+                for (int r = 0; r < kRows; ++r)
+                    w[r] = *reinterpret_cast<const uint4*>(weights + slot * slot_bytes + ((rb + min(r, nr - 1)) * chunks + c) * 512 + lane * 16);
+                if (FRAG) {
+                    const uint2* src = reinterpret_cast<const uint2*>(a_in) + (size_t)c * (16 * NT * 32) + lane;
 #pragma unroll
-                    for (int b = 0; b < kB; ++b) {
-                        const int k = c * 256 + (b0 + b) * 16;        // + 4q in a_row: K is a multiple of 8
-                        const bool in = k + 4 * q < K;
+                    for (int b0 = 0; b0 < 16; b0 += kB) {
+                        uint2 x[kB][NT];
 #pragma unroll
-                        for (int nt = 0; nt < NT; ++nt)
-                            x[nt][b] = in ? *reinterpret_cast<const uint2*>(a_row[nt] + k) : make_uint2(0u, 0u);
-                        s[b] = pre && in ? __ldg(reinterpret_cast<const uint2*>(pre + k + 4 * q))
-                                         : (BF16 ? make_uint2(0x3F803F80u, 0x3F803F80u) : make_uint2(0x3C003C00u, 0x3C003C00u));
+                        for (int b = 0; b < kB; ++b) {
+                            const bool in = c * 256 + (b0 + b) * 16 + 4 * q < K;
+#pragma unroll
+                            for (int nt = 0; nt < NT; ++nt) x[b][nt] = in ? src[((b0 + b) * NT + nt) * 32] : make_uint2(0u, 0u);
+                        }
+#pragma unroll
+                        for (int b = 0; b < kB; ++b) {
+                            uint32_t be[NT], bo[NT];
+#pragma unroll
+                            for (int nt = 0; nt < NT; ++nt) { be[nt] = x[b][nt].x; bo[nt] = x[b][nt].y; }
+                            block(w, b0 + b, one2, one2, be, bo);
+                        }
                     }
-                    if (b0 == 0 && c == c0 && rb == r0) {
-#pragma unroll 1
-                        for (unsigned spins = 0; !mbar_try(bars + 8 * slot, parity); ++spins)
-                            if (spins >= kWeightWaitLimit) { atomicExch(P.status, (unsigned)(-NQ_ERR_TIMEOUT)); break; }
-                    }
-                    uint4 w[kRows];
+                } else {
 #pragma unroll
-                    for (int r = 0; r < kRows; ++r)
-                        w[r] = *reinterpret_cast<const uint4*>(weights + slot * slot_bytes +
-                                                               ((size_t)(rb + min(r, nr - 1)) * chunks + c) * 512 + lane * 16);
+                    for (int pc = 0; pc < 4; ++pc) {
+                        asm volatile("cp.async.wait_group %0;" ::"n"(kPieces - 1) : "memory");
+                        __syncwarp();
+                        const unsigned char* buf = stage + s_out * piece_bytes;
+                        s_out = s_out + 1 == kPieces ? 0 : s_out + 1;
 #pragma unroll
-                    for (int b = 0; b < kB; ++b) {
-                        const int j = (b0 + b) >> 1, h = b & 1;       // block = columns 32 j + 16 h + ..
-                        const uint32_t se = even_columns(s[b]), so = odd_columns(s[b]);
-                        uint32_t be[NT], bo[NT];
-#pragma unroll
-                        for (int nt = 0; nt < NT; ++nt) { be[nt] = even_columns(x[nt][b]); bo[nt] = odd_columns(x[nt][b]); }
-#pragma unroll
-                        for (int r = 0; r < kRows; ++r)
-                            if (r < nr) {
-                                const uint32_t w0 = h ? w[r].z : w[r].x, w1 = h ? w[r].w : w[r].y;   // rows g, g + 8
-                                const uint32_t a0 = ((w0 << (15 - j)) & 0x80008000u) ^ se, a2 = ((w0 << (7 - j)) & 0x80008000u) ^ so;
-                                const uint32_t a1 = ((w1 << (15 - j)) & 0x80008000u) ^ se, a3 = ((w1 << (7 - j)) & 0x80008000u) ^ so;
-#pragma unroll
-                                for (int nt = 0; nt < NT; ++nt) mma_16816<BF16>(acc[r][nt], a0, a1, a2, a3, be[nt], bo[nt]);
+                        for (int b = 0; b < 4; ++b) {
+                            uint32_t se = one2, so = one2, be[NT], bo[NT];
+                            if (pre) {
+                                const uint2 sv = *reinterpret_cast<const uint2*>(buf + T * kPieceStride + 8 * q + b * 32);
+                                se = even_columns(sv); so = odd_columns(sv);
                             }
+#pragma unroll
+                            for (int nt = 0; nt < NT; ++nt) {
+                                const uint2 xv = *reinterpret_cast<const uint2*>(buf + a_row[nt] + b * 32);
+                                be[nt] = even_columns(xv); bo[nt] = odd_columns(xv);
+                            }
+                            block(w, 4 * pc + b, se, so, be, bo);
+                        }
+                        __syncwarp();            // the buffer has been read
+                        stage_piece(4 * c + pc + kPieces);
                     }
                 }
+            }
+            if (!FRAG) {
+                asm volatile("cp.async.wait_group 0;" ::: "memory");
+                __syncwarp();
             }
             // lane (g, q): rows g, g + 8 of each row group, tokens 8 nt + 2q, + 1
             float* dst = part + (size_t)kw * T * tok_stride + (2 * q) * tok_stride + rb * 16 + g;
@@ -215,32 +297,34 @@ __global__ void __launch_bounds__(kBatchThreads, 1) batch_stage_kernel(const __g
                             if (8 * nt + 2 * q + (i & 1) < T) dst[(8 * nt + (i & 1)) * tok_stride + r * 16 + 8 * (i >> 1)] = acc[r][nt][i];
                 }
         }
+        const int io_bf16 = P.io_bf16, out_bf16 = P.out_bf16;
+        float2* const scale = reinterpret_cast<float2*>(part + (size_t)wk * T * tok_stride);   // {output scale, bias} of a row
+        if (tid < nb * 16) scale[tid] = make_float2(jb.post ? float_of(post_raw, io_bf16) : 1.f, jb.bias ? float_of(bias_raw, io_bf16) : 0.f);
         __syncthreads();   // partial sums complete, this block's weights have been read
         if (++slot == slots) { slot = 0; parity ^= 1u; }
         if (loader) load_block();
         // outputs: lanes take rows, warps take tokens
-        const int io_bf16 = P.io_bf16, out_bf16 = P.out_bf16, kslice = T * tok_stride;
         const float lim = P.saturate ? (out_bf16 ? 3.3895313892515355e+38f : 64504.0f) : 3.4e38f;
         const uint16_t* const resid = static_cast<const uint16_t*>(jb.resid);
-        const int row0 = (first + blk) * 16;
+        const int* const row_exp = jb.row_exp;
+        const int kslice = T * tok_stride, frag_out = P.frag_out;
 #pragma unroll 1
-        for (int idx = lane; idx < nb * 16 && row0 + idx < rows; idx += 32) {
-            const int row = row0 + idx;
-            const float post = jb.post ? float_of(static_cast<const uint16_t*>(jb.post)[row], io_bf16) : 1.f;
-            const float bias = jb.bias ? float_of(static_cast<const uint16_t*>(jb.bias)[row], io_bf16) : 0.f;
+        for (int tok = warp; tok < T; tok += kBatchWarps) {
+            const float rs = row_exp ? exp2f((float)(P.exp_sign * row_exp[tok])) : 1.f;
+            uint16_t* const out = static_cast<uint16_t*>(jb.out) + (frag_out ? 0 : tok * jb.ld_out + row0);
 #pragma unroll 1
-            for (int tok = warp; tok < T; tok += kBatchWarps) {
+            for (int idx = lane; idx < nb * 16; idx += 32) {
                 const float* src = part + tok * tok_stride + idx;
                 float v = 0.f;
 #pragma unroll 4
                 for (int k = 0; k < wk; ++k, src += kslice) v += *src;
-                const float rs = jb.row_exp ? exp2f((float)(P.exp_sign * jb.row_exp[tok])) : 1.f;
-                float extra = bias;
-                if (resid) extra += float_of(resid[tok * jb.ld_res + row], io_bf16);
-                v = fminf(fmaxf(v * (post * rs) + extra, -lim), lim);
-                const long long at = tok * jb.ld_out + row;
-                if (out_bf16) static_cast<__nv_bfloat16*>(jb.out)[at] = __float2bfloat16(v);
-                else static_cast<__half*>(jb.out)[at] = __float2half(v);
+                const float2 sc = scale[idx];
+                if (row0 + idx < rows) {
+                    float extra = sc.y;
+                    if (resid) extra += float_of(resid[tok * jb.ld_res + row0 + idx], io_bf16);
+                    v = fminf(fmaxf(v * (sc.x * rs) + extra, -lim), lim);
+                    out[frag_out ? fragment_index<NT>(tok, row0 + idx) : idx] = out_bf16 ? __bfloat16_as_ushort(__float2bfloat16(v)) : __half_as_ushort(__float2half(v));
+                }
             }
         }
         if (blk + gb < groups) __syncthreads();   // the partial sums have been read
@@ -250,12 +334,19 @@ __global__ void __launch_bounds__(kBatchThreads, 1) batch_stage_kernel(const __g
 // ---------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------
-constexpr int kMostTokens = 16;    // above, every CTA's fetch of the whole input outweighs the GEMM's fixed costs (see the figures above)
 
-static const void* batch_kernel(int bf16, int T) {
-    const int nt = T <= 8 ? 1 : T <= 16 ? 2 : 4;
-    if (bf16) return nt == 1 ? (const void*)batch_stage_kernel<true, 1> : nt == 2 ? (const void*)batch_stage_kernel<true, 2> : (const void*)batch_stage_kernel<true, 4>;
-    return nt == 1 ? (const void*)batch_stage_kernel<false, 1> : nt == 2 ? (const void*)batch_stage_kernel<false, 2> : (const void*)batch_stage_kernel<false, 4>;
+template <bool BF16, int NT, bool FRAG>
+static const void* batch_kernel_of(int rows) {
+    return rows == 1 ? (const void*)batch_stage_kernel<BF16, NT, 1, FRAG> : rows == 2 ? (const void*)batch_stage_kernel<BF16, NT, 2, FRAG>
+                                                                                      : (const void*)batch_stage_kernel<BF16, NT, 4, FRAG>;
+}
+static const void* batch_kernel(int bf16, int T, int rows, bool frag) {
+    if (frag) {
+        if (bf16) return T <= 8 ? batch_kernel_of<true, 1, true>(rows) : batch_kernel_of<true, 2, true>(rows);
+        return T <= 8 ? batch_kernel_of<false, 1, true>(rows) : batch_kernel_of<false, 2, true>(rows);
+    }
+    if (bf16) return T <= 8 ? batch_kernel_of<true, 1, false>(rows) : batch_kernel_of<true, 2, false>(rows);
+    return T <= 8 ? batch_kernel_of<false, 1, false>(rows) : batch_kernel_of<false, 2, false>(rows);
 }
 static int batch_smem_limit(int* out) {
     static int cached[64];
@@ -264,8 +355,8 @@ static int batch_smem_limit(int* out) {
     if (cached[dev & 63] == 0) {
         int optin = 0;
         NQ_CUDA_TRY(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-        for (int i = 0; i < 6; ++i)
-            NQ_CUDA_TRY(cudaFuncSetAttribute(batch_kernel(i & 1, 8 << (i >> 1)), cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
+        for (int i = 0; i < 24; ++i)
+            NQ_CUDA_TRY(cudaFuncSetAttribute(batch_kernel(i & 1, i & 2 ? 16 : 8, 1 << (i / 8), (i & 4) != 0), cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
         cached[dev & 63] = optin;
     }
     *out = cached[dev & 63];
@@ -274,11 +365,18 @@ static int batch_smem_limit(int* out) {
 
 int batch_max_tokens(const StageJob* jobs, int n) {
     for (int i = 0; i < n; ++i)
-        if (jobs[i].K > 65536) return 0;    // one row group's weights have to fit beside its partial sums
-    return kMostTokens;
+        if (jobs[i].K > 32768) return 0;    // one row group's weights have to fit beside staging and partial sums
+    return kBatchMostTokens;
 }
 
-int launch_batch_stage(const StageJob* jobs, int n, int T, StageTypes ty, int saturate, unsigned* status, cudaStream_t stream) {
+size_t batch_fragment_bytes(int T, int K) { return (size_t)((K + 255) / 256) * 16 * (T <= 8 ? 1 : 2) * 256; }
+
+int launch_batch_stage(const StageJob* jobs, int n, int T, StageTypes ty, int saturate, bool frag_in, bool frag_out, unsigned* status,
+                       cudaStream_t stream) {
+    for (int i = 0; i < n; ++i) {      // 16-byte copies of rows and scales
+        if (jobs[i].K % 8 != 0 || (!frag_in && (!aligned16(jobs[i].a) || jobs[i].lda % 8 != 0))) return NQ_ERR_ALIGN;
+        if (jobs[i].pre && !aligned16(jobs[i].pre)) return NQ_ERR_ALIGN;
+    }
     int limit = 0;
     { const int st = batch_smem_limit(&limit); if (st != NQ_OK) return st; }
     BatchParams P;
@@ -286,7 +384,7 @@ int launch_batch_stage(const StageJob* jobs, int n, int T, StageTypes ty, int sa
     P.status = status;
     P.T = T;
     P.io_bf16 = ty.io_bf16; P.out_bf16 = ty.out_bf16; P.saturate = saturate; P.exp_sign = ty.exp_sign;
-    const int nt = T <= 8 ? 1 : T <= 16 ? 2 : 4;
+    const int nt = T <= 8 ? 1 : 2;
     int groups[kMaxGemmJobs], chunks[kMaxGemmJobs], ncta[kMaxGemmJobs], total = 0;
     for (int i = 0; i < n; ++i) {
         groups[i] = (jobs[i].Nout + 15) / 16;
@@ -297,8 +395,10 @@ int launch_batch_stage(const StageJob* jobs, int n, int T, StageTypes ty, int sa
     if (grid > total) grid = total;
     if (grid < n) grid = n;
     deal_ctas(grid, n, groups, chunks, ncta);
+    const size_t stage_bytes = frag_in ? 0 : (size_t)kBatchWarps * kPieces * (T + 1) * kPieceStride;
+    const size_t room = limit - kFixedBytes - stage_bytes;      // weights and partial sums of a block
     size_t slot_used = 0, part_used = 0;
-    int cta = 0, most_blocks = 1;
+    int cta = 0, most_blocks = 1, most_rows = 1;
     for (int i = 0; i < n; ++i) {
         const StageJob& S = jobs[i];
         BatchJob& j = P.job[i];
@@ -312,37 +412,51 @@ int launch_batch_stage(const StageJob* jobs, int n, int T, StageTypes ty, int sa
         j.g_r = groups[i] % ncta[i];
         memset(P.cta_job + cta, i, (size_t)ncta[i]);
         cta += ncta[i];
-        const int most = j.g_q + (j.g_r ? 1 : 0);
-        for (int blocks = 1;; ++blocks) {   // row blocks whose weights and partial sums fit, as equal as possible
-            j.gb = (most + blocks - 1) / blocks;
-            // Chunk slices x row slices: a step (a row group's chunk) against fetching a chunk's B fragments, which a
-            // warp does once per pass over its row groups.
-            int best = 1 << 30;
-            for (int k = 1; k <= kBatchWarps && k <= chunks[i]; ++k) {
-                int r = kBatchWarps / k;
-                if (r > j.gb) r = j.gb;
-                const int per = (j.gb + r - 1) / r;
-                const int cost = ((chunks[i] + k - 1) / k) * (per * (2 + T / 8) + ((per + rows_per_pass(nt) - 1) / rows_per_pass(nt)) * (2 + T / 4));
-                if (cost < best) { best = cost; j.wk = (uint16_t)k; j.wr = (uint16_t)r; }
+    }
+    // Row blocks, as equal as possible: each job's weights and partial sums fit the room together; where the largest of
+    // both over the jobs do not, each of them gets half; and where one row group does not fit half, one row group per
+    // block (64 KB of weights at the largest K, 21 KB of partial sums).
+    for (int attempt = 0; attempt < 3; ++attempt) {
+        slot_used = part_used = 0;
+        most_blocks = most_rows = 1;
+        for (int i = 0; i < n; ++i) {
+            BatchJob& j = P.job[i];
+            const int most = j.g_q + (j.g_r ? 1 : 0);
+            size_t part = 0, slot = 0;
+            for (int blocks = 1;; ++blocks) {
+                j.gb = attempt == 2 ? 1 : (most + blocks - 1) / blocks;
+                // Chunk slices x row slices: a step (a row group's chunk) against a chunk's B fragments, once per pass
+                int best = 1 << 30;
+                for (int k = 1; k <= kBatchWarps && k <= chunks[i]; ++k) {
+                    int r = kBatchWarps / k;
+                    if (r > j.gb) r = j.gb;
+                    const int per = (j.gb + r - 1) / r;
+                    const int cost = ((chunks[i] + k - 1) / k) * (per * (8 + 2 * nt) + ((per + 3) / 4) * (3 + 3 * nt));
+                    if (cost < best) { best = cost; j.wk = (uint16_t)k; j.wr = (uint16_t)r; }
+                }
+                part = (size_t)j.wk * T * (j.gb * 16 + 4) * 4 + (size_t)j.gb * 16 * 8;
+                slot = (size_t)j.gb * chunks[i] * 512;
+                const bool fits = attempt == 0 ? part + slot <= room : part <= room / 2 && slot <= room / 2;
+                if (j.gb == 1 || (fits && j.gb <= kBatchThreads / 16)) break;
             }
-            const size_t part = (size_t)j.wk * T * (j.gb * 16 + 4) * 4, slot = (size_t)j.gb * chunks[i] * 512;
-            if (j.gb == 1 || (part <= kPartBytes && slot <= kSlotBytes && j.gb <= 128)) {
-                part_used = part > part_used ? part : part_used;
-                slot_used = slot > slot_used ? slot : slot_used;
-                break;
-            }
+            part_used = part > part_used ? part : part_used;
+            slot_used = slot > slot_used ? slot : slot_used;
+            j.wk_magic = (65536 + j.wk - 1) / j.wk;
+            j.wr_magic = (65536 + j.wr - 1) / j.wr;
+            const int blocks = (most + j.gb - 1) / j.gb, per_warp = (j.gb + j.wr - 1) / j.wr;
+            most_blocks = blocks > most_blocks ? blocks : most_blocks;
+            most_rows = per_warp > most_rows ? per_warp : most_rows;
         }
-        j.wk_magic = (65536 + j.wk - 1) / j.wk;
-        j.wr_magic = (65536 + j.wr - 1) / j.wr;
-        const int blocks = (most + j.gb - 1) / j.gb;
-        most_blocks = blocks > most_blocks ? blocks : most_blocks;
+        if (part_used + slot_used <= room) break;
     }
     int slots = most_blocks < kBatchSlots ? most_blocks : kBatchSlots;
-    while (slots > 1 && kFixedBytes + part_used + slots * slot_used > (size_t)limit) --slots;
+    while (slots > 1 && part_used + slots * slot_used > room) --slots;
     P.slots = slots;
     P.slot_bytes = (int)slot_used;
+    P.frag_out = frag_out;
     P.part_off = (int)(kFixedBytes + slots * slot_used);
-    const size_t smem = P.part_off + part_used;
+    P.stage_off = (P.part_off + (int)part_used + 15) / 16 * 16;
+    const size_t smem = P.stage_off + stage_bytes;
     if (smem > (size_t)limit) return NQ_ERR_UNSUPPORTED;
     static bool pdl_ok = true;
     cudaLaunchConfig_t cfg = {};
@@ -356,7 +470,7 @@ int launch_batch_stage(const StageJob* jobs, int n, int T, StageTypes ty, int sa
     cfg.attrs = &attr;
     cfg.numAttrs = pdl_ok ? 1 : 0;
     void* args[] = {&P};
-    const void* fn = batch_kernel(ty.a_bf16, T);
+    const void* fn = batch_kernel(ty.a_bf16, T, most_rows == 1 ? 1 : most_rows == 2 ? 2 : 4, frag_in);
     cudaError_t e = cudaLaunchKernelExC(&cfg, fn, args);
     if (e != cudaSuccess && pdl_ok) {
         (void)cudaGetLastError();

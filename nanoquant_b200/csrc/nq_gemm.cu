@@ -975,7 +975,7 @@ static int launch_stage(const StageJob* jobs, int n, int T, StageTypes ty, int s
         if (S.pre && !aligned16(S.pre)) return NQ_ERR_ALIGN;
         Ks[j] = S.K; Ns[j] = S.Nout;
     }
-    if (T <= batch_max_tokens(jobs, n)) return launch_batch_stage(jobs, n, T, ty, saturate, status, stream);
+    if (T <= batch_max_tokens(jobs, n)) return launch_batch_stage(jobs, n, T, ty, saturate, false, false, status, stream);
     { const int st_attr = set_kernel_attributes(); if (st_attr != NQ_OK) return st_attr; }
     const GroupPlan pl = plan_group(T, n, Ks, Ns, counters != nullptr && slabs != nullptr, true);
     const int mh = pl.mh, nh = pl.nh;
@@ -1075,7 +1075,9 @@ static size_t gemm_group_layout(const nq_linear_desc* d, int n, int T, size_t* t
     int K1[kMaxGemmJobs], N1[kMaxGemmJobs], K2[kMaxGemmJobs], N2[kMaxGemmJobs];
     for (int j = 0; j < n; ++j) {
         if (t_off) t_off[j] = off;
-        off += ((size_t)T * (size_t)d[j].R * 2 + 255) / 256 * 256;
+        size_t t_bytes = (size_t)T * (size_t)d[j].R * 2;
+        if (T <= kBatchMostTokens && batch_fragment_bytes(T, d[j].R) > t_bytes) t_bytes = batch_fragment_bytes(T, d[j].R);
+        off += (t_bytes + 255) / 256 * 256;
         K1[j] = d[j].N; N1[j] = d[j].R; K2[j] = d[j].R; N2[j] = d[j].M;
     }
     for (int j = 0; j < n; ++j) {
@@ -1144,12 +1146,20 @@ int nq_gemm_group_fwd(const nq_linear_desc* d, int n_linears, int T, int dtype, 
         s1[j] = {L.x, L.ldx, L.v_tiles, L.s_in, L.s_mid, t, L.R, L.N, L.R, nullptr, nullptr, 0, row_exp};
         s2[j] = {t, L.R, L.u_tiles, nullptr, L.s_out, L.y, L.ldy, L.R, L.M, L.bias, L.residual, L.ldr, row_exp};
     }
+    // few tokens: both stages by the batch kernel, which keeps the intermediate in its own order
+    const bool batch = T <= batch_max_tokens(s1, n_linears) && T <= batch_max_tokens(s2, n_linears);
+    auto stages = [&](StageTypes ty1, StageTypes ty2) -> int {
+        if (batch) {
+            const int st = launch_batch_stage(s1, n_linears, T, ty1, 0, false, true, status, as_stream(stream));
+            return st != NQ_OK ? st : launch_batch_stage(s2, n_linears, T, ty2, 1, true, false, status, as_stream(stream));
+        }
+        const int st = launch_stage(s1, n_linears, T, ty1, 0, status, counters, slabs, as_stream(stream));
+        return st != NQ_OK ? st : launch_stage(s2, n_linears, T, ty2, 1, status, counters, slabs, as_stream(stream));
+    };
     if (dtype == NQ_F16 || !g_precise_intermediate) {   // the intermediate in the I/O type, as it comes
         const int b16 = dtype == NQ_BF16;
         const StageTypes ty = {b16, b16, b16, 0};
-        const int st = launch_stage(s1, n_linears, T, ty, 0, status, counters, slabs, as_stream(stream));
-        if (st != NQ_OK) return st;
-        return launch_stage(s2, n_linears, T, ty, 1, status, counters, slabs, as_stream(stream));
+        return stages(ty, ty);
     }
     // bf16 with the precise intermediate switched on: a bf16 intermediate carries 8 significant bits into stage 2
     // (its rounding alone is up to 1.6e-3 of the output's maximum); here it is kept as fp16 times a per-token
@@ -1184,9 +1194,7 @@ int nq_gemm_group_fwd(const nq_linear_desc* d, int n_linears, int T, int dtype, 
         }
         NQ_CUDA_TRY(e);
     }
-    const int st = launch_stage(s1, n_linears, T, StageTypes{1, 1, 0, +1}, 0, status, counters, slabs, as_stream(stream));
-    if (st != NQ_OK) return st;
-    return launch_stage(s2, n_linears, T, StageTypes{1, 0, 1, -1}, 1, status, counters, slabs, as_stream(stream));
+    return stages(StageTypes{1, 1, 0, +1}, StageTypes{1, 0, 1, -1});
 }
 
 int nq_gemm_fwd(const void* x, const void* s_in, const void* v_tiles, const void* s_mid, const void* u_tiles,

@@ -27,8 +27,13 @@ struct StageTypes {
     int io_bf16, a_bf16, out_bf16, exp_sign;
 };
 
-// Most tokens of the batch kernel; 0 where it cannot take the jobs.
+constexpr int kBatchMostTokens = 16;    // of the batch kernel (see nq_batch.cu)
+// The same, or 0 where it cannot take the jobs.
 int batch_max_tokens(const StageJob* jobs, int n);
-int launch_batch_stage(const StageJob* jobs, int n, int T, StageTypes ty, int saturate, unsigned* status, cudaStream_t stream);
+// `frag_in` / `frag_out`: the activations / the output are an intermediate in the batch kernel's fragment order, of
+// batch_fragment_bytes each, without an input scale.
+size_t batch_fragment_bytes(int T, int K);
+int launch_batch_stage(const StageJob* jobs, int n, int T, StageTypes ty, int saturate, bool frag_in, bool frag_out, unsigned* status,
+                       cudaStream_t stream);
 
 }  // namespace nq
