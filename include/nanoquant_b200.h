@@ -216,10 +216,9 @@ unsigned nq_gemv_set_wait_limit(unsigned polls);
  * ------------------------------------------------------------------------ */
 
 /* Bytes of scratch nq_gemm_fwd needs: a 256-byte header (status word at byte 8,
- * the same place as in the GEMV scratch; tile counters of the split-K path in
- * bytes 32..255) followed by the rank-R intermediate t[T, R] in the I/O dtype
- * and, for up to 24 tokens, the fp32 partial sums of the k splits (above that
- * a k split runs over the CTAs of a thread-block cluster and needs no scratch). */
+ * the same place as in the GEMV scratch) followed by the rank-R intermediate
+ * t[T, R] in the I/O dtype (padded to its fragment order for up to 32 tokens)
+ * and per-token exponents. */
 size_t nq_gemm_scratch_bytes(int T, int N, int R, int M);
 
 /* Precision of the rank-R intermediate of bf16 linears in the GEMM path (process-wide; returns the old setting).
@@ -236,8 +235,7 @@ int nq_gemm_set_precise_intermediate(int on);
  * intermediate is rounded to the I/O dtype between the stages, accumulation is
  * fp32, the products x * (+-s_in) are exact.  Requires N % 8 == 0, R % 8 == 0,
  * 16-byte aligned x, y, scales and scratch.  The scratch header must be zeroed
- * once by the caller (the tile counters return to zero by themselves); a
- * device-side wait that gives up sets its status word (nq_scratch_status).
+ * once by the caller; a device-side wait that gives up sets its status word (nq_scratch_status).
  * Consecutive launches overlap through programmatic dependent launch: a
  * kernel loads activations and stores results only after the previous kernel
  * of the stream has completed.

@@ -19,9 +19,9 @@
 //
 // Splitting K over the CTAs of a cluster (partial sums exchanged through distributed shared memory) and staging the whole
 // input by bulk copies before the loop both measured slower than this at every size.
-// Qwen3-8B decode, eight layers in a graph, GEMM against this kernel: 8 tokens 804 -> 359 us, 16 tokens 825 -> 438 us.  At 16
-// tokens a stage with little work takes 4.4 us; gate/up's second stage 12 (16 clocks per MMA and scheduler), down's
-// first 11.5 (58 MB of activations from L2 to the SMs, 7 TB/s).
+// Qwen3-8B decode, eight layers in a graph, GEMM against this kernel: 8 tokens 804 -> 359 us, 16 tokens 825 -> 438, 20 tokens
+// 865 -> 631, 24 tokens 860 -> 721, 32 tokens 826 -> 801.  At 16 tokens a stage with little work takes 4.4 us; gate/up's
+// second stage 12 (16 clocks per MMA and scheduler), down's first 11.5 (58 MB of activations from L2 to the SMs, 7 TB/s).
 #include <cstddef>
 #include <cstring>
 
@@ -34,8 +34,11 @@ namespace nq {
 constexpr int kBatchThreads = 512;
 constexpr int kBatchWarps = kBatchThreads / 32;
 // 16-column blocks of the intermediate whose B fragments a warp loads together
-constexpr int blocks_in_flight(int nt, int rows) { return nt == 1 || rows < 4 ? 8 : 4; }
-constexpr int kPieces = 3;               // pieces of 64 columns a warp has in flight
+constexpr int blocks_in_flight(int nt, int rows) { return nt == 1 || (nt == 2 && rows < 4) ? 8 : nt == 4 && rows == 2 ? 2 : 4; }
+constexpr int tokens_groups(int T) { return T <= 8 ? 1 : T <= 16 ? 2 : T <= 24 ? 3 : 4; }
+// row groups of a pass: four, two where the accumulators of four do not leave registers for the operands
+constexpr int most_rows_of(int nt) { return nt <= 2 ? 4 : 2; }
+constexpr int pieces(int nt) { return nt <= 2 ? 3 : nt == 3 ? 2 : 1; }   // pieces of 64 columns a warp has in flight
 constexpr int kPieceStride = 128 + 32;   // bytes of a staged row: 32 mod 128, so the eight tokens of a fragment fall on
                                          // different banks
 constexpr int kBatchSlots = 8;           // weight blocks in flight
@@ -103,7 +106,7 @@ __device__ __forceinline__ void copy16_or_zero(uint32_t dst, const void* src, bo
 // and has no scale (the second stage); otherwise it is [T, lda].
 template <bool BF16, int NT, int ROWS, bool FRAG>
 __global__ void __launch_bounds__(kBatchThreads, 1) batch_stage_kernel(const __grid_constant__ BatchParams Pc) {
-    constexpr int kRows = ROWS, kB = blocks_in_flight(NT, ROWS);
+    constexpr int kRows = ROWS, kB = blocks_in_flight(NT, ROWS), kPieces = pieces(NT);
     extern __shared__ __align__(128) unsigned char smem[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, q = lane & 3;
     const uint32_t bars = smem_u32(smem);
@@ -336,17 +339,19 @@ __global__ void __launch_bounds__(kBatchThreads, 1) batch_stage_kernel(const __g
 // ---------------------------------------------------------------------------
 
 template <bool BF16, int NT, bool FRAG>
-static const void* batch_kernel_of(int rows) {
-    return rows == 1 ? (const void*)batch_stage_kernel<BF16, NT, 1, FRAG> : rows == 2 ? (const void*)batch_stage_kernel<BF16, NT, 2, FRAG>
-                                                                                      : (const void*)batch_stage_kernel<BF16, NT, 4, FRAG>;
+static const void* batch_kernel_rows(int rows) {
+    if (rows == 1) return (const void*)batch_stage_kernel<BF16, NT, 1, FRAG>;
+    if (rows == 2 || most_rows_of(NT) == 2) return (const void*)batch_stage_kernel<BF16, NT, 2, FRAG>;
+    return (const void*)batch_stage_kernel<BF16, NT, most_rows_of(NT), FRAG>;
 }
-static const void* batch_kernel(int bf16, int T, int rows, bool frag) {
-    if (frag) {
-        if (bf16) return T <= 8 ? batch_kernel_of<true, 1, true>(rows) : batch_kernel_of<true, 2, true>(rows);
-        return T <= 8 ? batch_kernel_of<false, 1, true>(rows) : batch_kernel_of<false, 2, true>(rows);
-    }
-    if (bf16) return T <= 8 ? batch_kernel_of<true, 1, false>(rows) : batch_kernel_of<true, 2, false>(rows);
-    return T <= 8 ? batch_kernel_of<false, 1, false>(rows) : batch_kernel_of<false, 2, false>(rows);
+template <bool BF16, bool FRAG>
+static const void* batch_kernel_tokens(int nt, int rows) {
+    return nt == 1 ? batch_kernel_rows<BF16, 1, FRAG>(rows) : nt == 2 ? batch_kernel_rows<BF16, 2, FRAG>(rows)
+           : nt == 3 ? batch_kernel_rows<BF16, 3, FRAG>(rows) : batch_kernel_rows<BF16, 4, FRAG>(rows);
+}
+static const void* batch_kernel(int bf16, int nt, int rows, bool frag) {
+    if (frag) return bf16 ? batch_kernel_tokens<true, true>(nt, rows) : batch_kernel_tokens<false, true>(nt, rows);
+    return bf16 ? batch_kernel_tokens<true, false>(nt, rows) : batch_kernel_tokens<false, false>(nt, rows);
 }
 static int batch_smem_limit(int* out) {
     static int cached[64];
@@ -355,8 +360,8 @@ static int batch_smem_limit(int* out) {
     if (cached[dev & 63] == 0) {
         int optin = 0;
         NQ_CUDA_TRY(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-        for (int i = 0; i < 24; ++i)
-            NQ_CUDA_TRY(cudaFuncSetAttribute(batch_kernel(i & 1, i & 2 ? 16 : 8, 1 << (i / 8), (i & 4) != 0), cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
+        for (int i = 0; i < 48; ++i)
+            NQ_CUDA_TRY(cudaFuncSetAttribute(batch_kernel(i & 1, 1 + (i / 4) % 4, 1 << (i / 16), (i & 2) != 0), cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
         cached[dev & 63] = optin;
     }
     *out = cached[dev & 63];
@@ -369,7 +374,7 @@ int batch_max_tokens(const StageJob* jobs, int n) {
     return kBatchMostTokens;
 }
 
-size_t batch_fragment_bytes(int T, int K) { return (size_t)((K + 255) / 256) * 16 * (T <= 8 ? 1 : 2) * 256; }
+size_t batch_fragment_bytes(int T, int K) { return (size_t)((K + 255) / 256) * 16 * tokens_groups(T) * 256; }
 
 int launch_batch_stage(const StageJob* jobs, int n, int T, StageTypes ty, int saturate, bool frag_in, bool frag_out, unsigned* status,
                        cudaStream_t stream) {
@@ -384,7 +389,7 @@ int launch_batch_stage(const StageJob* jobs, int n, int T, StageTypes ty, int sa
     P.status = status;
     P.T = T;
     P.io_bf16 = ty.io_bf16; P.out_bf16 = ty.out_bf16; P.saturate = saturate; P.exp_sign = ty.exp_sign;
-    const int nt = T <= 8 ? 1 : 2;
+    const int nt = tokens_groups(T), rows_most = most_rows_of(nt);
     int groups[kMaxGemmJobs], chunks[kMaxGemmJobs], ncta[kMaxGemmJobs], total = 0;
     for (int i = 0; i < n; ++i) {
         groups[i] = (jobs[i].Nout + 15) / 16;
@@ -395,7 +400,7 @@ int launch_batch_stage(const StageJob* jobs, int n, int T, StageTypes ty, int sa
     if (grid > total) grid = total;
     if (grid < n) grid = n;
     deal_ctas(grid, n, groups, chunks, ncta);
-    const size_t stage_bytes = frag_in ? 0 : (size_t)kBatchWarps * kPieces * (T + 1) * kPieceStride;
+    const size_t stage_bytes = frag_in ? 0 : (size_t)kBatchWarps * pieces(nt) * (T + 1) * kPieceStride;
     const size_t room = limit - kFixedBytes - stage_bytes;      // weights and partial sums of a block
     size_t slot_used = 0, part_used = 0;
     int cta = 0, most_blocks = 1, most_rows = 1;
@@ -431,7 +436,7 @@ int launch_batch_stage(const StageJob* jobs, int n, int T, StageTypes ty, int sa
                     int r = kBatchWarps / k;
                     if (r > j.gb) r = j.gb;
                     const int per = (j.gb + r - 1) / r;
-                    const int cost = ((chunks[i] + k - 1) / k) * (per * (8 + 2 * nt) + ((per + 3) / 4) * (3 + 3 * nt));
+                    const int cost = ((chunks[i] + k - 1) / k) * (per * (8 + 2 * nt) + ((per + rows_most - 1) / rows_most) * (3 + 3 * nt));
                     if (cost < best) { best = cost; j.wk = (uint16_t)k; j.wr = (uint16_t)r; }
                 }
                 part = (size_t)j.wk * T * (j.gb * 16 + 4) * 4 + (size_t)j.gb * 16 * 8;
@@ -470,7 +475,7 @@ int launch_batch_stage(const StageJob* jobs, int n, int T, StageTypes ty, int sa
     cfg.attrs = &attr;
     cfg.numAttrs = pdl_ok ? 1 : 0;
     void* args[] = {&P};
-    const void* fn = batch_kernel(ty.a_bf16, T, most_rows == 1 ? 1 : most_rows == 2 ? 2 : 4, frag_in);
+    const void* fn = batch_kernel(ty.a_bf16, nt, most_rows == 1 ? 1 : most_rows == 2 ? 2 : 4, frag_in);
     cudaError_t e = cudaLaunchKernelExC(&cfg, fn, args);
     if (e != cudaSuccess && pdl_ok) {
         (void)cudaGetLastError();

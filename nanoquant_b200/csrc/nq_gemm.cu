@@ -23,10 +23,9 @@
 //   epilogue    tcgen05.ld of the accumulator(s) (lane = token, column = output row),
 //               * post[n], saturate, convert, 16-byte stores.
 //
-// Launches with fewer output tiles than SMs split K: over independent CTAs with fp32 slabs in global
-// memory and a last-CTA reduction (up to 24 tokens), or over the CTAs of a thread-block cluster that
-// exchange their partial sums through distributed shared memory (more tokens); see GemmParams::csplit
-// and plan_group.  bf16 linears may keep their intermediate as fp16 times a per-token power of two
+// Launches with fewer output tiles than SMs split K over the CTAs of a thread-block cluster that exchange their partial
+// sums through distributed shared memory; see GemmParams::csplit and plan_group.  Few tokens (up to kBatchMostTokens) are
+// nq_batch.cu's.  bf16 linears may keep their intermediate as fp16 times a per-token power of two
 // (row_bound_kernel, nq_gemm_set_precise_intermediate).
 //
 // The packed operand is the same tile layout the decode GEMV streams (nq_rows_to_tiles),
@@ -106,22 +105,19 @@ struct alignas(64) GemmJob {
     const void* bias;      // [Nout] (I/O dtype) or nullptr, added behind the output scale
     const void* resid;     // [T, ld_res] (I/O dtype) or nullptr, added behind the bias
     long long ld_out, ld_res;
-    // split-K (few tokens, few output tiles): `splits` CTAs along grid.z share an output tile, each over
-    // `chunks_per` 256-column chunks; partial sums go to fp32 slabs [split][Nout][t_pad] and the CTA that
-    // arrives last at the tile's counter adds them up in split order and writes the output.
-    float* slabs;
-    unsigned* counters;    // one per output tile of this job, zero between launches
     int K, Nout;
     int chunks, row_groups;
-    int splits, chunks_per;
-    int tile0;             // first grid.x index of this job's tiles
+    int chunks_per;        // 256-column chunks of a CTA (all of them unless the launch is split)
 };
 
 struct GemmParams {
     GemmJob job[kMaxGemmJobs];
+    // The parameter bank is cold at every launch and a first touch of a line costs some 700 cycles: what every CTA needs to
+    // find its job lies together.
     int njobs;
+    int tile0[kMaxGemmJobs];   // first grid.x index of each job's tiles
     unsigned* status;      // device status word (0 = ok)
-    int T, t_pad;          // tokens; slab row length (tokens, multiple of 4)
+    int T;                 // tokens
     int is_bf16;           // type of the scales, bias and residual (the I/O type of the linear)
     int a_bf16;            // type of the MMA operands: activations and expanded weights (bf16, else fp16)
     int out_bf16;          // type of the output (bf16, else fp16)
@@ -130,7 +126,7 @@ struct GemmParams {
     // instead of 8): stage 1 multiplies row t by 2^row_exp[t] (exp_sign = +1), stage 2 by 2^-row_exp[t] (-1).
     // The exponents come from row_bound_kernel; 0: no row scaling.
     int exp_sign;
-    // Cluster split-K (more than 24 tokens, fewer output tiles than SMs): the `csplit` CTAs of a thread-block
+    // Cluster split-K (fewer output tiles than SMs): the `csplit` CTAs of a thread-block
     // cluster along grid.z share an output tile, each over `chunks_per` 256-column chunks of every job.  After the
     // main loops the accumulators are exchanged through distributed shared memory: 32-column blocks of the tile
     // are dealt round-robin to the CTAs of the cluster, every CTA stores the blocks it does not own into the
@@ -234,11 +230,9 @@ __global__ void __launch_bounds__(GemmCfg<MH, NH>::kThreads) gemm_stage_kernel(c
     const uint32_t sbase = smem_u32(smem);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     int ji = 0;
-    while (ji + 1 < P.njobs && (int)blockIdx.x >= P.job[ji + 1].tile0) ++ji;
+    while (ji + 1 < P.njobs && (int)blockIdx.x >= P.tile0[ji + 1]) ++ji;
     const GemmJob& J = P.job[ji];
-    // grid.z is the largest split count of the launch; the CTAs of a cluster all stay (they meet at its barriers)
-    if (P.csplit == 1 && (int)blockIdx.z >= J.splits) return;
-    const int tile = (int)blockIdx.x - J.tile0;
+    const int tile = (int)blockIdx.x - P.tile0[ji];
     const int n0 = tile * kBN;   // first weight row of the tile
     const int m0 = blockIdx.y * (kBM * MH);   // first token of the tile
     // k range of this CTA (all of K unless the launch is split): whole 256-column chunks
@@ -283,14 +277,15 @@ __global__ void __launch_bounds__(GemmCfg<MH, NH>::kThreads) gemm_stage_kernel(c
     // input-scale slots start finite: a partial last k block leaves older (finite) values behind
     for (int i = threadIdx.x; i < kBitsSlots * kPreBytes / 4; i += kGemmThreads)
         reinterpret_cast<uint32_t*>(smem + kOffPre)[i] = 0;
-    // Output scales and bias of this tile: expand thread i loads those of column i now (the values are needed
-    // only in the epilogue, and nothing here waits for them) and puts them into shared memory behind its main loop.
-    uint32_t raw_post = 0, raw_bias = 0;
+    // Output scales and bias of this tile: expand thread i loads those of column i now and puts them into shared memory
+    // behind its main loop.  (asm: a 16-bit load into a wider type is widened, that is waited for, at once, here by the
+    // whole CTA at the barrier below.)
+    uint16_t raw_post = 0, raw_bias = 0;
     {
         const int i = (int)threadIdx.x - 32 * kFirstExpandWarp;
         if (i >= 0 && i < kBN && n0 + i < J.Nout) {
-            if (J.post) raw_post = 0x10000u | static_cast<const uint16_t*>(J.post)[n0 + i];
-            if (J.bias) raw_bias = 0x10000u | static_cast<const uint16_t*>(J.bias)[n0 + i];
+            if (J.post) asm volatile("ld.global.nc.u16 %0, [%1];" : "=h"(raw_post) : "l"(static_cast<const uint16_t*>(J.post) + n0 + i));
+            if (J.bias) asm volatile("ld.global.nc.u16 %0, [%1];" : "=h"(raw_bias) : "l"(static_cast<const uint16_t*>(J.bias) + n0 + i));
         }
     }
     if (warp == 1) {  // tensor-memory allocation: 128 fp32 columns per accumulator, by one whole warp
@@ -428,12 +423,11 @@ __global__ void __launch_bounds__(GemmCfg<MH, NH>::kThreads) gemm_stage_kernel(c
             if (((kb + kGroups) >> 2) != c || kb + kGroups >= nkb) mbar_arrive(bar_bits_empty(b));
         }
         if (tu < kBN) {
-            auto as_float = [&](uint32_t raw, float dflt) {
-                if (!(raw & 0x10000u)) return dflt;
-                return P.is_bf16 ? __uint_as_float(raw << 16) : __half2float(__ushort_as_half((unsigned short)raw));
+            auto as_float = [&](uint16_t raw) {
+                return P.is_bf16 ? __uint_as_float((uint32_t)raw << 16) : __half2float(__ushort_as_half(raw));
             };
-            reinterpret_cast<float*>(smem + kOffPost)[tu] = as_float(raw_post, 1.f);
-            reinterpret_cast<float*>(smem + kOffBias)[tu] = as_float(raw_bias, 0.f);
+            reinterpret_cast<float*>(smem + kOffPost)[tu] = J.post ? as_float(raw_post) : 1.f;
+            reinterpret_cast<float*>(smem + kOffBias)[tu] = J.bias ? as_float(raw_bias) : 0.f;
         }
         asm volatile("bar.sync 2, %0;" ::"n"(kExpandThreads) : "memory");   // scales visible to every expand thread
         if (ok) ok = mbar_wait(bar_accum, 0, abort_flag, P.status);   // this CTA's MMAs are complete
@@ -533,14 +527,7 @@ __global__ void __launch_bounds__(GemmCfg<MH, NH>::kThreads) gemm_stage_kernel(c
                 // lane without a valid output only skips the stores.
                 const bool valid = row < P.T && n0 + c0 < J.Nout;
                 const float rs = MH == 1 ? rs_mh[0] : (mh == 0 ? rs_mh[0] : rs_mh[MH - 1]);
-                if (J.splits > 1) {   // partial sums of this k range: a warp writes 32 consecutive tokens per column
-                    if (valid) {
-                        float* slab = J.slabs + ((size_t)blockIdx.z * J.Nout + n0 + c0) * P.t_pad + row;
-#pragma unroll
-                        for (int e = 0; e < 32; ++e)
-                            if (n0 + c0 + e < J.Nout) slab[(size_t)e * P.t_pad] = __uint_as_float(r[e]);
-                    }
-                } else if (valid) {
+                if (valid) {
                 const float4* bias4 = reinterpret_cast<const float4*>(smem + kOffBias);
                 const uint16_t* res_row = J.resid ? static_cast<const uint16_t*>(J.resid) + (size_t)row * J.ld_res + n0 + c0 : nullptr;
                 uint32_t packed[16];
@@ -588,90 +575,6 @@ __global__ void __launch_bounds__(GemmCfg<MH, NH>::kThreads) gemm_stage_kernel(c
                         if (n0 + c0 + e < J.Nout)
                             reinterpret_cast<uint16_t*>(dst)[e] = (uint16_t)(packed[e >> 1] >> (16 * (e & 1)));
                 }
-                }
-            }
-        }
-    }
-    if (J.splits > 1 && warp >= kFirstExpandWarp) {
-        // Split-K tail.  Every expand thread passes both barriers whatever happened before, so an expired wait
-        // elsewhere cannot leave threads behind.  The CTA that finds the other splits' arrivals at the tile's
-        // counter adds the slabs up in split order (the result does not depend on arrival order).
-        volatile int* last_flag = reinterpret_cast<volatile int*>(smem + kOffMisc + 8);
-        const int tu = threadIdx.x - 32 * kFirstExpandWarp;
-        __threadfence();
-        asm volatile("bar.sync 1, %0;" ::"n"(kExpandThreads) : "memory");
-        if (tu == 0) {
-            int last = 0;
-            if (!*abort_flag) {
-                const unsigned old = atomicAdd(J.counters + tile, 1u);
-                last = old == (unsigned)(J.splits - 1);
-                if (last) J.counters[tile] = 0u;   // ready for the next launch
-            }
-            *last_flag = last;
-        }
-        asm volatile("bar.sync 1, %0;" ::"n"(kExpandThreads) : "memory");
-        if (*last_flag) {
-            __threadfence();
-            const int tp4 = P.t_pad >> 2;
-            const int ncols = min(kBN, J.Nout - n0);
-            const float lim = P.saturate ? (P.out_bf16 ? 3.3895313892515355e+38f : 64504.0f) : 3.4e38f;
-            const float* post_s = reinterpret_cast<const float*>(smem + kOffPost);
-            const float* bias_s = reinterpret_cast<const float*>(smem + kOffBias);
-            // Items: (column, group of four tokens).  Two items and eight splits per round keep 16 independent
-            // 16-byte loads in flight per thread; the sums are formed in split order.
-            constexpr int kZ = 8;
-            const int nitems = ncols * tp4;
-            for (int it0 = tu; it0 < nitems; it0 += 2 * kExpandThreads) {
-                float4 acc[2];
-                const float* src[2];
-#pragma unroll
-                for (int w = 0; w < 2; ++w) {
-                    const int it = min(it0 + w * kExpandThreads, nitems - 1);   // clamped: a duplicate is not stored
-                    const int col = it / tp4, r4 = it - col * tp4;
-                    src[w] = J.slabs + ((size_t)n0 + col) * P.t_pad + 4 * r4;
-                    acc[w] = make_float4(0.f, 0.f, 0.f, 0.f);
-                }
-                const size_t zstride = (size_t)J.Nout * P.t_pad;
-                for (int z0 = 0; z0 < J.splits; z0 += kZ) {
-                    float4 v[2][kZ];
-#pragma unroll
-                    for (int u = 0; u < kZ; ++u)
-#pragma unroll
-                        for (int w = 0; w < 2; ++w)
-                            v[w][u] = z0 + u < J.splits
-                                          ? __ldcg(reinterpret_cast<const float4*>(src[w] + (size_t)(z0 + u) * zstride))
-                                          : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-                    for (int u = 0; u < kZ; ++u)
-#pragma unroll
-                        for (int w = 0; w < 2; ++w) {
-                            acc[w].x += v[w][u].x; acc[w].y += v[w][u].y; acc[w].z += v[w][u].z; acc[w].w += v[w][u].w;
-                        }
-                }
-#pragma unroll
-                for (int w = 0; w < 2; ++w) {
-                    const int it = it0 + w * kExpandThreads;
-                    if (it >= nitems) continue;
-                    const int col = it / tp4, r4 = it - col * tp4;
-                    const float sc = post_s[col], bv = bias_s[col];
-                    const float o[4] = {acc[w].x, acc[w].y, acc[w].z, acc[w].w};
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        const int row = 4 * r4 + j;
-                        if (row < P.T) {
-                            float ex = bv;
-                            if (J.resid) {
-                                const size_t ra = (size_t)row * J.ld_res + n0 + col;
-                                ex += P.is_bf16 ? __bfloat162float(static_cast<const __nv_bfloat16*>(J.resid)[ra])
-                                                : __half2float(static_cast<const __half*>(J.resid)[ra]);
-                            }
-                            const float rs = J.row_exp ? exp2f((float)(P.exp_sign * J.row_exp[row])) : 1.f;
-                            const float v1 = fminf(fmaxf(o[j] * (sc * rs) + ex, -lim), lim);
-                            const size_t at = (size_t)row * J.ld_out + n0 + col;
-                            if (P.out_bf16) static_cast<__nv_bfloat16*>(J.out)[at] = __float2bfloat16(v1);
-                            else static_cast<__half*>(J.out)[at] = __float2half(v1);
-                        }
-                    }
                 }
             }
         }
@@ -796,27 +699,11 @@ static EncodeTiledFn encode_tiled_fn() {
 // Tile shape of a launch and the k split of each of its jobs.
 struct GroupPlan {
     int mh, nh;                       // tile: 128*mh tokens x 128*nh weight rows
-    int t_pad;                        // slab row length (tokens, multiple of 4)
     int tiles_total;                  // grid.x
-    int max_splits;                   // grid.z
     int csplit;                       // CTAs per cluster along grid.z that share an output tile (1: no cluster)
     int tile0[kMaxGemmJobs];          // first grid.x index of each job
-    int splits[kMaxGemmJobs];         // CTAs per output tile along K (1 = no split)
-    int chunks_per[kMaxGemmJobs];     // 256-column chunks per split
-    int counter0[kMaxGemmJobs];       // first tile counter of the job (index into the counter words)
-    size_t slab0[kMaxGemmJobs];       // first slab float of the job
-    size_t slab_floats;               // slab floats of the launch
+    int chunks_per[kMaxGemmJobs];     // 256-column chunks of a CTA
 };
-constexpr size_t kMaxSlabBytes = (size_t)16 << 20;
-// The tile counters live in words 8..63 of the 256-byte scratch header, which no other kernel writes
-// (the decode kernel that may share the scratch uses words 0..2 and the bytes behind the header).
-constexpr int kCounterWord0 = 8, kMaxSplitTiles = 56;
-// Up to 24 tokens the k split goes over independent CTAs with slabs in global memory (any number of splits, as
-// many as there are idle SMs); beyond, the serial slab reduction of the last CTA costs more than the split saves
-// and the split goes over the CTAs of a cluster instead.  Qwen3-8B decode step, slabs against clusters: 16 tokens
-// 3.59 against 3.76 ms, 32 tokens 3.79 against 3.73 ms, 48 tokens 4.38 against 3.83 ms.
-constexpr int kMaxSplitTokens = 24;
-
 // The four tile configurations as the host sees them.
 struct KernelInfo {
     const void* fn;
@@ -884,10 +771,9 @@ static int cluster_capacity(int mh, int nh, int s) {
 // cycles per 64-column step (bounded by the tensor pipe for the 256 x 256 tile, by shared-memory traffic and the
 // per-step waits of the issuing threads for the smaller ones); the grid runs in ceil(CTAs/resident CTAs) waves, each
 // with a fixed prologue/epilogue cost.  Launches that would leave SMs idle split the k dimension of every job
-// (whole 256-column chunks per CTA): above 24 tokens over the CTAs of a cluster, which add their partial sums
-// through distributed shared memory; up to 24 tokens over independent CTAs with fp32 slabs in global memory, as
-// far as counters and slab budget allow.
-static GroupPlan plan_group(int T, int n, const int* K, const int* Nout, bool allow_split, bool allow_cluster) {
+// (whole 256-column chunks per CTA) over the CTAs of a cluster, which add their partial sums through distributed
+// shared memory.
+static GroupPlan plan_group(int T, int n, const int* K, const int* Nout) {
     GroupPlan pl;
     memset(&pl, 0, sizeof(pl));
     pl.mh = 1; pl.nh = 1; pl.csplit = 1;
@@ -899,7 +785,6 @@ static GroupPlan plan_group(int T, int n, const int* K, const int* Nout, bool al
         min_chunks = c < min_chunks ? c : min_chunks;
         max_chunks = c > max_chunks ? c : max_chunks;
     }
-    const bool cluster_ok = allow_cluster && T > kMaxSplitTokens;
     long long best = -1;
     for (const auto& c : cand) {
         if (c[0] == 2 && T <= kBM) continue;
@@ -910,7 +795,7 @@ static GroupPlan plan_group(int T, int n, const int* K, const int* Nout, bool al
         const long long per_step = c[0] * c[1] == 4 ? 990 : (c[0] == 2 ? 580 : (c[1] == 2 ? 830 : 485));
         const long long fixed = 6000 + 2000LL * c[0] * c[1];
         const KernelInfo ki = kernel_info(c[0], c[1]);
-        for (int s = 1; s <= (cluster_ok && c[0] * c[1] < 4 ? 8 : 1); ++s) {
+        for (int s = 1; s <= (c[0] * c[1] < 4 ? 8 : 1); ++s) {
             if (s > 1) {
                 if (s > min_chunks) break;
                 if ((long long)s * ((ki.blocks + s - 1) / s) * (128 * 32 * 4) > ki.pipe_bytes) continue;
@@ -923,48 +808,16 @@ static GroupPlan plan_group(int T, int n, const int* K, const int* Nout, bool al
             if (best < 0 || cost < best) { best = cost; pl.mh = c[0]; pl.nh = c[1]; pl.csplit = s; }
         }
     }
-    pl.t_pad = (T + 3) / 4 * 4;
-    pl.max_splits = 1;
-    int tiles_n[kMaxGemmJobs];
     for (int j = 0; j < n; ++j) {
-        tiles_n[j] = (Nout[j] + 128 * pl.nh - 1) / (128 * pl.nh);
         pl.tile0[j] = pl.tiles_total;
-        pl.tiles_total += tiles_n[j];
-        pl.splits[j] = 1;
-        pl.chunks_per[j] = (K[j] + 255) / 256;
-    }
-    if (pl.csplit > 1) {
-        pl.max_splits = pl.csplit;
-        for (int j = 0; j < n; ++j) pl.chunks_per[j] = ((K[j] + 255) / 256 + pl.csplit - 1) / pl.csplit;
-    }
-    if (allow_split && T <= kMaxSplitTokens) {
-        long long want_all = sms / pl.tiles_total;   // CTAs per tile that the idle SMs allow
-        int counters_used = 0;
-        size_t slab_budget = kMaxSlabBytes / sizeof(float);
-        for (int j = 0; j < n && want_all >= 2; ++j) {
-            const int chunks = (K[j] + 255) / 256;
-            const size_t per_split = (size_t)pl.t_pad * (size_t)Nout[j];
-            long long want = want_all;
-            const long long by_mem = (long long)((slab_budget - pl.slab_floats) / per_split);
-            want = want < by_mem ? want : by_mem;
-            want = want < chunks ? want : chunks;
-            if (want < 2 || counters_used + tiles_n[j] > kMaxSplitTiles) continue;
-            pl.chunks_per[j] = (int)((chunks + want - 1) / want);
-            pl.splits[j] = (chunks + pl.chunks_per[j] - 1) / pl.chunks_per[j];
-            pl.counter0[j] = counters_used;
-            counters_used += tiles_n[j];
-            pl.slab0[j] = pl.slab_floats;
-            pl.slab_floats += (size_t)pl.splits[j] * per_split;
-            pl.max_splits = pl.max_splits > pl.splits[j] ? pl.max_splits : pl.splits[j];
-        }
+        pl.tiles_total += (Nout[j] + 128 * pl.nh - 1) / (128 * pl.nh);
+        pl.chunks_per[j] = ((K[j] + 255) / 256 + pl.csplit - 1) / pl.csplit;
     }
     return pl;
 }
 
-// One stage of up to four linears: out_j[T, Nout_j] = (a_j[T, K_j] . W_j^T) * post_j.  `counters` (zero
-// between launches) and `slabs` may be nullptr: no k split.
-static int launch_stage(const StageJob* jobs, int n, int T, StageTypes ty, int saturate, unsigned* status,
-                        unsigned* counters, float* slabs, cudaStream_t stream) {
+// One stage of up to four linears: out_j[T, Nout_j] = (a_j[T, K_j] . W_j^T) * post_j.
+static int launch_stage(const StageJob* jobs, int n, int T, StageTypes ty, int saturate, unsigned* status, cudaStream_t stream) {
     if (n < 1 || n > kMaxGemmJobs) return NQ_ERR_UNSUPPORTED;
     EncodeTiledFn enc = encode_tiled_fn();
     if (!enc) return NQ_ERR_UNSUPPORTED;
@@ -977,7 +830,7 @@ static int launch_stage(const StageJob* jobs, int n, int T, StageTypes ty, int s
     }
     if (T <= batch_max_tokens(jobs, n)) return launch_batch_stage(jobs, n, T, ty, saturate, false, false, status, stream);
     { const int st_attr = set_kernel_attributes(); if (st_attr != NQ_OK) return st_attr; }
-    const GroupPlan pl = plan_group(T, n, Ks, Ns, counters != nullptr && slabs != nullptr, true);
+    const GroupPlan pl = plan_group(T, n, Ks, Ns);
     const int mh = pl.mh, nh = pl.nh;
     const int m_tiles = (T + kBM * mh - 1) / (kBM * mh);
     GemmParams P;
@@ -985,7 +838,6 @@ static int launch_stage(const StageJob* jobs, int n, int T, StageTypes ty, int s
     P.njobs = n;
     P.status = status;
     P.T = T;
-    P.t_pad = pl.t_pad;
     P.is_bf16 = ty.io_bf16;
     P.a_bf16 = ty.a_bf16;
     P.out_bf16 = ty.out_bf16;
@@ -1016,11 +868,8 @@ static int launch_stage(const StageJob* jobs, int n, int T, StageTypes ty, int s
         J.K = S.K; J.Nout = S.Nout;
         J.chunks = (S.K + 255) / 256;
         J.row_groups = (S.Nout + 15) / 16;
-        J.splits = pl.splits[j];
         J.chunks_per = pl.chunks_per[j];
-        J.tile0 = pl.tile0[j];
-        J.counters = counters ? counters + pl.counter0[j] : nullptr;
-        J.slabs = slabs ? slabs + pl.slab0[j] : nullptr;
+        P.tile0[j] = pl.tile0[j];
     }
     const KernelInfo ki = kernel_info(mh, nh);
     const void* fn = ki.fn;
@@ -1031,7 +880,7 @@ static int launch_stage(const StageJob* jobs, int n, int T, StageTypes ty, int s
     // launches are used from then on.
     static bool pdl_ok = true;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(pl.tiles_total, m_tiles, pl.max_splits);
+    cfg.gridDim = dim3(pl.tiles_total, m_tiles, pl.csplit);
     cfg.blockDim = dim3(threads);
     cfg.dynamicSmemBytes = smem_bytes;
     cfg.stream = stream;
@@ -1066,27 +915,21 @@ using namespace nq;
 
 extern "C" {
 
-// Scratch of a GEMM group: header (status word, tile counters), the intermediates t_j[T, R_j] (16-bit,
-// 256-byte aligned each), the per-token exponents of each intermediate (T words each; used by bf16 linears),
-// split-K slabs (shared by the two stages).
-static size_t gemm_group_layout(const nq_linear_desc* d, int n, int T, size_t* t_off, size_t* slab_off,
-                                size_t* exp_off = nullptr) {
+// Scratch of a GEMM group: header (status word), the intermediates t_j[T, R_j] (16-bit, 256-byte aligned each; in the
+// batch kernel's order for few tokens), the per-token exponents of each intermediate (T words each; used by bf16 linears).
+static size_t gemm_group_layout(const nq_linear_desc* d, int n, int T, size_t* t_off, size_t* exp_off) {
     size_t off = 256;
-    int K1[kMaxGemmJobs], N1[kMaxGemmJobs], K2[kMaxGemmJobs], N2[kMaxGemmJobs];
     for (int j = 0; j < n; ++j) {
         if (t_off) t_off[j] = off;
         size_t t_bytes = (size_t)T * (size_t)d[j].R * 2;
         if (T <= kBatchMostTokens && batch_fragment_bytes(T, d[j].R) > t_bytes) t_bytes = batch_fragment_bytes(T, d[j].R);
         off += (t_bytes + 255) / 256 * 256;
-        K1[j] = d[j].N; N1[j] = d[j].R; K2[j] = d[j].R; N2[j] = d[j].M;
     }
     for (int j = 0; j < n; ++j) {
         if (exp_off) exp_off[j] = off;
         off += ((size_t)T * sizeof(int) + 255) / 256 * 256;
     }
-    if (slab_off) *slab_off = off;
-    const size_t a = plan_group(T, n, K1, N1, true, false).slab_floats, b = plan_group(T, n, K2, N2, true, false).slab_floats;
-    return off + (a > b ? a : b) * sizeof(float);
+    return off;
 }
 
 size_t nq_gemm_group_scratch_bytes(const nq_linear_desc* d, int n_linears, int T) {
@@ -1112,8 +955,7 @@ int nq_onebit_gemm_fwd(const void* x, const void* tiles, const void* s_in, const
     if (!aligned16(tiles)) return NQ_ERR_ALIGN;
     const StageJob job = {x, K, tiles, s_in, s_out, y, Nout, K, Nout, nullptr, nullptr, 0, nullptr};
     const int b16 = dtype == NQ_BF16;
-    return launch_stage(&job, 1, T, StageTypes{b16, b16, b16, 0}, 1, static_cast<unsigned*>(status_word) + 2, nullptr, nullptr,
-                        as_stream(stream));
+    return launch_stage(&job, 1, T, StageTypes{b16, b16, b16, 0}, 1, static_cast<unsigned*>(status_word) + 2, as_stream(stream));
 }
 
 int nq_gemm_group_fwd(const nq_linear_desc* d, int n_linears, int T, int dtype, void* scratch,
@@ -1131,13 +973,9 @@ int nq_gemm_group_fwd(const nq_linear_desc* d, int n_linears, int T, int dtype, 
         if (L.N % 8 || L.R % 8) return NQ_ERR_SHAPE;
         if (!aligned16(L.v_tiles) || !aligned16(L.u_tiles)) return NQ_ERR_ALIGN;
     }
-    size_t t_off[kMaxGemmJobs], exp_off[kMaxGemmJobs], slab_off = 0;
-    if (scratch_bytes < gemm_group_layout(d, n_linears, T, t_off, &slab_off, exp_off)) return NQ_ERR_SCRATCH;
+    size_t t_off[kMaxGemmJobs], exp_off[kMaxGemmJobs];
+    if (scratch_bytes < gemm_group_layout(d, n_linears, T, t_off, exp_off)) return NQ_ERR_SCRATCH;
     unsigned* status = static_cast<unsigned*>(scratch) + 2;   // same word as the GEMV header's status
-    // Both stages use the same counters and slab space: a stage touches them only after the kernel before it
-    // has completed (its stores come behind the dependency wait).
-    unsigned* counters = static_cast<unsigned*>(scratch) + kCounterWord0;
-    float* slabs = reinterpret_cast<float*>(static_cast<char*>(scratch) + slab_off);
     StageJob s1[kMaxGemmJobs], s2[kMaxGemmJobs];
     for (int j = 0; j < n_linears; ++j) {
         const nq_linear_desc& L = d[j];
@@ -1153,8 +991,8 @@ int nq_gemm_group_fwd(const nq_linear_desc* d, int n_linears, int T, int dtype, 
             const int st = launch_batch_stage(s1, n_linears, T, ty1, 0, false, true, status, as_stream(stream));
             return st != NQ_OK ? st : launch_batch_stage(s2, n_linears, T, ty2, 1, true, false, status, as_stream(stream));
         }
-        const int st = launch_stage(s1, n_linears, T, ty1, 0, status, counters, slabs, as_stream(stream));
-        return st != NQ_OK ? st : launch_stage(s2, n_linears, T, ty2, 1, status, counters, slabs, as_stream(stream));
+        const int st = launch_stage(s1, n_linears, T, ty1, 0, status, as_stream(stream));
+        return st != NQ_OK ? st : launch_stage(s2, n_linears, T, ty2, 1, status, as_stream(stream));
     };
     if (dtype == NQ_F16 || !g_precise_intermediate) {   // the intermediate in the I/O type, as it comes
         const int b16 = dtype == NQ_BF16;
@@ -1216,7 +1054,7 @@ int nq_gemm_set_precise_intermediate(int on) {
     return old;
 }
 
-// One decode launch handles four tokens; from five tokens on the split-K GEMM is faster than two launches.
+// One decode launch handles four tokens; from five tokens on the batch kernel's two stages are faster than two launches.
 int nq_gemv_max_tokens(void) { return 4; }
 
 size_t nq_linear_scratch_bytes(int T, int N, int R, int M) {

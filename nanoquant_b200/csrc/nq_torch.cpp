@@ -394,8 +394,31 @@ PyObject* py_dense_gemv_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
     END_HANDLE_TH_ERRORS
 }
 
-// repack(op, src, rows, cols, order) -> out or None: the pack / layout kernels on a contiguous CUDA tensor
-//   0 pack_rows, 1 unpack_rows, 2 rows_to_tiles, 3 tiles_to_rows, 4 pack_marlin (rows = out features)
+// The pack / layout kernels on a contiguous CUDA tensor.
+enum RepackOp : int { kPackRows, kUnpackRows, kRowsToTiles, kTilesToRows, kPackMarlin };
+Tensor repack(RepackOp op, const Tensor& src, int64_t rows, int64_t cols, int order) {
+    const int64_t words = (cols + 31) / 32, row_groups = (rows + 15) / 16, chunks = (cols + 255) / 256;
+    const auto ints = src.options().dtype(at::kInt);
+    Tensor out = op == kUnpackRows    ? at::empty({rows, cols}, src.options().dtype(at::kChar))
+                 : op == kRowsToTiles ? at::empty({row_groups, chunks, 128}, ints)
+                 : op == kPackMarlin  ? at::empty({cols / 16, rows / 2}, ints)
+                                      : at::empty({rows, words}, ints);
+    const int dev = src.get_device();
+    OnDevice on(dev);
+    const nq_stream_t stream = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)dev).stream();
+    const void* in = src.const_data_ptr();
+    void* o = out.mutable_data_ptr();
+    static const char* const kNames[5] = {"nq_pack_rows", "nq_unpack_rows", "nq_rows_to_tiles", "nq_tiles_to_rows", "nq_pack_marlin"};
+    const int st = op == kPackRows      ? nq_pack_rows(static_cast<const int8_t*>(in), static_cast<int32_t*>(o), rows, cols, order, stream)
+                   : op == kUnpackRows  ? nq_unpack_rows(static_cast<const int32_t*>(in), static_cast<int8_t*>(o), rows, cols, order, stream)
+                   : op == kRowsToTiles ? nq_rows_to_tiles(static_cast<const int32_t*>(in), o, rows, cols, order, stream)
+                   : op == kTilesToRows ? nq_tiles_to_rows(in, static_cast<int32_t*>(o), rows, cols, order, stream)
+                                        : nq_pack_marlin(static_cast<const int8_t*>(in), static_cast<int32_t*>(o), rows, cols, stream);
+    if (st < 0) fail(st, kNames[op]);
+    return out;
+}
+
+// repack(op, src, rows, cols, order) -> out or None (rows = out features for the Marlin layout)
 PyObject* py_repack(PyObject*, PyObject* const* a, Py_ssize_t n) {
     HANDLE_TH_ERRORS
     TORCH_CHECK(n == 5, "repack takes 5 arguments");
@@ -403,30 +426,37 @@ PyObject* py_repack(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const long op = PyLong_AsLong(a[0]), order = PyLong_AsLong(a[4]);
     const int64_t rows = PyLong_AsLongLong(a[2]), cols = PyLong_AsLongLong(a[3]);
     if (PyErr_Occurred()) return nullptr;
-    const bool dense = op == 0 || op == 4;
-    if (!src || !src->is_contiguous() || src->scalar_type() != (dense ? at::kChar : at::kInt)) Py_RETURN_NONE;
-    const int64_t words = (cols + 31) / 32, row_groups = (rows + 15) / 16, chunks = (cols + 255) / 256;
-    Tensor out;
-    const auto ints = src->options().dtype(at::kInt);
-    if (op == 0) out = at::empty({rows, words}, ints);
-    else if (op == 1) out = at::empty({rows, cols}, src->options().dtype(at::kChar));
-    else if (op == 2) out = at::empty({row_groups, chunks, 128}, ints);
-    else if (op == 3) out = at::empty({rows, words}, ints);
-    else if (op == 4) out = at::empty({cols / 16, rows / 2}, ints);
-    else Py_RETURN_NONE;
-    const int dev = src->get_device();
-    OnDevice on(dev);
-    const nq_stream_t stream = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)dev).stream();
-    const void* in = src->const_data_ptr();
-    void* o = out.mutable_data_ptr();
-    static const char* const kNames[5] = {"nq_pack_rows", "nq_unpack_rows", "nq_rows_to_tiles", "nq_tiles_to_rows", "nq_pack_marlin"};
-    const int st = op == 0   ? nq_pack_rows(static_cast<const int8_t*>(in), static_cast<int32_t*>(o), rows, cols, (int)order, stream)
-                   : op == 1 ? nq_unpack_rows(static_cast<const int32_t*>(in), static_cast<int8_t*>(o), rows, cols, (int)order, stream)
-                   : op == 2 ? nq_rows_to_tiles(static_cast<const int32_t*>(in), o, rows, cols, (int)order, stream)
-                   : op == 3 ? nq_tiles_to_rows(in, static_cast<int32_t*>(o), rows, cols, (int)order, stream)
-                             : nq_pack_marlin(static_cast<const int8_t*>(in), static_cast<int32_t*>(o), rows, cols, stream);
-    if (st < 0) fail(st, kNames[op]);
-    return THPVariable_Wrap(out);
+    const bool dense = op == kPackRows || op == kPackMarlin;
+    if (!src || op < kPackRows || op > kPackMarlin || !src->is_contiguous() || src->scalar_type() != (dense ? at::kChar : at::kInt))
+        Py_RETURN_NONE;
+    return THPVariable_Wrap(repack((RepackOp)op, *src, rows, cols, (int)order));
+    END_HANDLE_TH_ERRORS
+}
+
+// pack_rows(dense, order) -> words; words_to(op, words, shape, order) -> unpacked or tiles.  None: not a plain CUDA
+// tensor of the right type, or not of the shape it is said to have; the caller sorts that out.
+PyObject* py_pack_rows(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    TORCH_CHECK(n == 2, "pack_rows takes 2 arguments");
+    const Tensor* src = plain(a[0]);
+    const long order = PyLong_AsLong(a[1]);
+    if (PyErr_Occurred()) return nullptr;
+    if (!src || src->dim() != 2 || !src->is_contiguous() || src->scalar_type() != at::kChar) Py_RETURN_NONE;
+    return THPVariable_Wrap(repack(kPackRows, *src, src->size(0), src->size(1), (int)order));
+    END_HANDLE_TH_ERRORS
+}
+PyObject* py_words_to(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    TORCH_CHECK(n == 4, "words_to takes 4 arguments");
+    const Tensor* src = plain(a[1]);
+    if (!src || src->dim() != 2 || !src->is_contiguous() || src->scalar_type() != at::kInt || !PyTuple_Check(a[2]) ||
+        PyTuple_GET_SIZE(a[2]) != 2 || !PyLong_Check(PyTuple_GET_ITEM(a[2], 0)) || !PyLong_Check(PyTuple_GET_ITEM(a[2], 1)))
+        Py_RETURN_NONE;
+    const long op = PyLong_AsLong(a[0]), order = PyLong_AsLong(a[3]);
+    const int64_t rows = PyLong_AsLongLong(PyTuple_GET_ITEM(a[2], 0)), cols = PyLong_AsLongLong(PyTuple_GET_ITEM(a[2], 1));
+    if (PyErr_Occurred()) return nullptr;
+    if ((op != kUnpackRows && op != kRowsToTiles) || src->size(0) != rows || src->size(1) != (cols + 31) / 32) Py_RETURN_NONE;
+    return THPVariable_Wrap(repack((RepackOp)op, *src, rows, cols, (int)order));
     END_HANDLE_TH_ERRORS
 }
 
@@ -485,6 +515,8 @@ PyMethodDef kMethods[] = {
     {"group_forward", (PyCFunction)(void*)py_group_forward, METH_FASTCALL, nullptr},
     {"dense_gemv_forward", (PyCFunction)(void*)py_dense_gemv_forward, METH_FASTCALL, nullptr},
     {"repack", (PyCFunction)(void*)py_repack, METH_FASTCALL, nullptr},
+    {"pack_rows", (PyCFunction)(void*)py_pack_rows, METH_FASTCALL, nullptr},
+    {"words_to", (PyCFunction)(void*)py_words_to, METH_FASTCALL, nullptr},
     {"permute_scale", (PyCFunction)(void*)py_permute_scale, METH_FASTCALL, nullptr},
     {"set_scratch", py_set_scratch, METH_VARARGS, nullptr},
     {"set_thread_scratch", py_set_thread_scratch, METH_VARARGS, nullptr},

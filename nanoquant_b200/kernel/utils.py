@@ -76,6 +76,11 @@ def get_kernel_function(namespace: str, dtype: torch.dtype, kernel_type: str):
 def pack_binary_gemv(tensor: torch.Tensor, method: str = "lsb_first") -> torch.Tensor:
     """±1 int8 ``(rows, cols)`` -> int32 ``(rows, ceil(cols/32))``; reference
     ``pack_binary_gemv`` (``kernel/utils.py:51-113``)."""
+    order = _lib.ORDER_ID.get(method)
+    if order is not None:      # the plain case in one native call
+        out = _lib.ext().pack_rows(tensor, order)
+        if out is not None:
+            return out
     if tensor.dtype != torch.int8:
         raise TypeError("Input tensor must be int8.")
     order = _check_method(method)
@@ -87,6 +92,11 @@ def unpack_binary_gemv(packed_tensor: torch.Tensor, original_shape: Tuple[int, i
                        method: str = "lsb_first") -> torch.Tensor:
     """Inverse of :func:`pack_binary_gemv`; reference ``unpack_binary_gemv``
     (``kernel/utils.py:116-183``)."""
+    order = _lib.ORDER_ID.get(method)
+    if order is not None:
+        out = _lib.ext().words_to(_UNPACK_ROWS, packed_tensor, original_shape, order)
+        if out is not None:
+            return out
     if packed_tensor.dim() != 2:
         raise ValueError(
             f"Unsupported packed tensor format. Expected 2D tensor, got {packed_tensor.dim()} dimensions.")
@@ -170,6 +180,11 @@ def pack_tiles(packed: torch.Tensor, shape: Tuple[int, int], method: str = "lsb_
     """rows layout ``(rows, ceil(cols/32))`` -> int32 ``(ceil(rows/16), ceil(cols/256), 128)``
     tile layout consumed by the GEMV kernel (``nq_rows_to_tiles``)."""
     rows, cols = int(shape[0]), int(shape[1])
+    order = _lib.ORDER_ID.get(method)
+    out = None if order is None else _lib.ext().words_to(_ROWS_TO_TILES, packed, (rows, cols), order)
+    if out is not None:
+        out._nq_rows, out._nq_cols = rows, cols   # exact shape: the tiles pad rows to 16 and columns to 256
+        return out
     if tuple(packed.shape) != (rows, (cols + 31) // 32):
         raise ValueError(f"packed tensor of shape {tuple(packed.shape)} does not hold a {rows}x{cols} matrix")
     packed = _int32(packed if packed.is_cuda else _to_cuda(packed))
