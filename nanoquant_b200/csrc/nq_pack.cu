@@ -19,6 +19,26 @@ static inline unsigned grid_for(int64_t n, int threads) {
     return static_cast<unsigned>(g < 1 ? 1 : (g > cap ? cap : g));
 }
 
+// Launches with programmatic stream serialization and no early trigger: packing is a run of such calls, and the blocks of the
+// next one are set up while this one's last blocks finish (pack, tiles and unpack of 12288 x 2432 in a stream: 33.7 -> 28.4
+// us).  The kernels touch memory only behind enter().  They do NOT let a successor in early: the linears load their weight
+// tiles ahead of their own dependency wait, so the tiles have to be complete by then.
+template <typename... P, typename... A>
+static int launch(void (*kernel)(P...), unsigned grid, unsigned threads, nq_stream_t stream, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(threads);
+    cfg.stream = as_stream(stream);
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    NQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...));
+    return NQ_OK;
+}
+__device__ __forceinline__ void enter() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // sign bits of four int8 values held in one register -> 4-bit field (byte b -> bit b)
 __device__ __forceinline__ uint32_t sign_nibble(uint32_t v) {
     uint32_t x = (v >> 7) & 0x01010101u;
@@ -33,51 +53,151 @@ __device__ __forceinline__ uint32_t spread_nibble(uint32_t n) {
 // ---------------------------------------------------------------------------
 // rows layout
 // ---------------------------------------------------------------------------
-__global__ void pack_rows_kernel(const int8_t* __restrict__ w, uint32_t* __restrict__ out,
-                                 int64_t rows, int64_t cols, int64_t words, int order, bool vec) {
-    const int64_t total = rows * words;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t r = i / words, wi = i - r * words;
-        const int64_t c0 = wi * 32;
-        const int8_t* src = w + r * cols + c0;
-        uint32_t bits = 0;
-        if (vec && c0 + 32 <= cols) {
-            const uint4 a = __ldg(reinterpret_cast<const uint4*>(src));
-            const uint4 b = __ldg(reinterpret_cast<const uint4*>(src) + 1);
-            bits = sign_nibble(a.x) | (sign_nibble(a.y) << 4) | (sign_nibble(a.z) << 8) |
-                   (sign_nibble(a.w) << 12) | (sign_nibble(b.x) << 16) | (sign_nibble(b.y) << 20) |
-                   (sign_nibble(b.z) << 24) | (sign_nibble(b.w) << 28);
-        } else {
-            const int n = (int)((cols - c0) < 32 ? (cols - c0) : 32);
-            for (int k = 0; k < n; ++k) bits |= (uint32_t)(src[k] < 0) << k;  // padding stays +1 (bit 0)
+// Matrices of any width at any address.  The rows are one run of bytes, in which a word starts at any byte, so a thread
+// that fetches its own 32 bytes can only do so byte by byte.  Here a warp takes 64 consecutive words: the up to 129 aligned
+// 16-byte pieces that cover them come in with contiguous loads, each piece leaves its 16 sign bits in shared memory, and a
+// word is 32 bits of that string.  The instructions bound it, hence one division per 2 KB and offsets inside a step in 32
+// bits (they are small: sums modulo 2^32 will do).  12291 x 2435: 8.7 us (29.7 with byte loads).
+constexpr int kAnyThreads = 128;      // small blocks: a matrix of a few hundred KB is a few hundred warps
+
+// a / b for a >= 0, b > 0, in 32 bits where that will do (the same branch in the whole warp)
+__device__ __forceinline__ int64_t quotient(int64_t a, int64_t b) {
+    return ((a | b) >> 32) == 0 ? (int64_t)((uint32_t)a / (uint32_t)b) : a / b;
+}
+// Element `d` behind element `col` of a row of `n` elements: rows crossed, and the column in its row; 0 <= d <= 2048
+__device__ __forceinline__ uint32_t advance(int64_t& col, int d, int64_t n) {
+    col += d;
+    if (n >= 2048) {                            // col < n before: one row at most
+        if (col < n) return 0;
+        col -= n;
+        return 1;
+    }
+    const uint32_t q = (uint32_t)col / (uint32_t)n;
+    col -= (int64_t)(q * (uint32_t)n);
+    return q;
+}
+// signs of 16 int8 values -> 16 bits.  The products put bits 7, 15, 23, 31 of a word at 28..31.
+__device__ __forceinline__ uint32_t sign_bits16(const uint4& v) {
+    auto top4 = [](uint32_t x) { return (x & 0x80808080u) * 0x00204081u; };
+    uint32_t h = top4(v.w) >> 28;
+    h = __funnelshift_l(top4(v.z), h, 4);
+    h = __funnelshift_l(top4(v.y), h, 4);
+    return __funnelshift_l(top4(v.x), h, 4);
+}
+// 16 bits -> int8 +1 (0) / -1 (1): bit b of a nibble goes to bit 8b + 7, whose byte is filled with it, lowest bit set
+__device__ __forceinline__ uint4 signs_of16(uint32_t h) {
+    auto four = [](uint32_t product) {
+        uint32_t fill;     // selector values 8..11: the sign of byte 0..3, repeated (__byte_perm drops that bit)
+        asm("prmt.b32 %0, %1, 0, 0xBA98;" : "=r"(fill) : "r"(product));
+        return fill | 0x01010101u;
+    };
+    const uint32_t g = h >> 8;
+    return make_uint4(four((h & 0x0Fu) * 0x10204080u), four((h & 0xF0u) * 0x01020408u), four((g & 0x0Fu) * 0x10204080u),
+                      four((g & 0xF0u) * 0x01020408u));
+}
+
+__global__ void __launch_bounds__(kAnyThreads) pack_rows_kernel(const int8_t* __restrict__ w, uint32_t* __restrict__ out,
+                                                                int64_t rows, int64_t cols, int64_t words, int order) {
+    enter();
+    __shared__ uint32_t signs[kAnyThreads / 32][66];     // 16 bits per piece, piece 2i in the low half of word i
+    const int lane = threadIdx.x & 31;
+    uint32_t* const mine = signs[threadIdx.x >> 5];
+    const int64_t total = rows * words, bytes = rows * cols, step = (int64_t)gridDim.x * (kAnyThreads / 32) * 64;
+    const uint32_t tail = (uint32_t)(cols - 32 * (words - 1));                   // columns in a row's last word
+    for (int64_t base = ((int64_t)blockIdx.x * (kAnyThreads / 32) + (threadIdx.x >> 5)) * 64; base < total; base += step) {
+        const int64_t r0 = quotient(base, words), wi0 = base - r0 * words, b0 = r0 * cols + 32 * wi0;
+        const int mis = (int)((reinterpret_cast<uintptr_t>(w) + (uintptr_t)b0) & 15);
+        // pieces [lo, hi) lie inside the matrix; the one before and the one after may do so in part
+        const int lo = b0 < mis ? 1 : 0, hi = bytes - b0 + mis < 129 * 16 ? (int)(bytes - b0 + mis) >> 4 : 129;
+        const int8_t* const from = w + (b0 - mis);
+        uint4 v[5];
+#pragma unroll
+        for (int k = 0; k < 5; ++k) {
+            const int p = 32 * k + lane;
+            v[k] = p >= lo && p < hi ? __ldcs(reinterpret_cast<const uint4*>(from) + p) : make_uint4(0u, 0u, 0u, 0u);
         }
-        out[i] = convert_order(bits, NQ_LSB_FIRST, order);
+        uint16_t* const piece = reinterpret_cast<uint16_t*>(mine);
+        __syncwarp();                                                            // the previous step's string has been read
+#pragma unroll
+        for (int k = 0; k < 5; ++k)
+            if (k < 4 || lane < 4) piece[32 * k + lane] = (uint16_t)sign_bits16(v[k]);
+        if (lo > 0 || hi < 129) {                                                // (the whole warp) an end of the matrix
+            __syncwarp();
+            const int p = lane == 0 ? 0 : hi;
+            if ((lane == 0 && lo > 0) || (lane == 1 && hi < 129)) {
+                uint32_t h = 0;
+                const int64_t f = b0 - mis + 16 * p;
+#pragma unroll
+                for (int e = 0; e < 16; ++e)
+                    if (f + e >= 0 && f + e < bytes) h |= (uint32_t)(w[f + e] < 0) << e;
+                piece[p] = (uint16_t)h;
+            }
+        }
+        __syncwarp();
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            int64_t wi = wi0;
+            const uint32_t dr = advance(wi, 32 * k + lane, words);
+            if (base + 32 * k + lane < total) {
+                const uint32_t at = (uint32_t)mis + dr * (uint32_t)cols + 32u * (uint32_t)(wi - wi0);   // below 16 + 2048
+                uint32_t v32 = __funnelshift_r(mine[at >> 5], mine[(at >> 5) + 1], at & 31);
+                if (wi == words - 1) v32 &= 0xFFFFFFFFu >> (32 - tail);          // padding stays +1 (bit 0)
+                out[base + 32 * k + lane] = convert_order(v32, NQ_LSB_FIRST, order);
+            }
+        }
     }
 }
 
-__global__ void unpack_rows_kernel(const uint32_t* __restrict__ packed, int8_t* __restrict__ w,
-                                   int64_t rows, int64_t cols, int64_t words, int order, bool vec) {
-    const int64_t total = rows * words;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t r = i / words, wi = i - r * words;
-        const int64_t c0 = wi * 32;
-        const uint32_t bits = convert_order(packed[i], order, NQ_LSB_FIRST);
-        int8_t* dst = w + r * cols + c0;
-        if (vec && c0 + 32 <= cols) {
-            uint32_t v[8];
+// The way back: a warp writes 32 * P of the aligned 16-byte pieces of the run of bytes.  A lane gathers the 16 bits of a
+// piece from the one or two words that hold them, the words of all its pieces in flight together; pieces that span rows, or
+// an end of the matrix, go bit run by bit run.  12291 x 2435: 12.5 us (172 with byte stores).
+template <int P>
+__global__ void __launch_bounds__(kAnyThreads) unpack_rows_kernel(const uint32_t* __restrict__ packed, int8_t* __restrict__ w,
+                                                                  int64_t rows, int64_t cols, int64_t words, int order) {
+    enter();
+    const int lane = threadIdx.x & 31, mis = (int)(reinterpret_cast<uintptr_t>(w) & 15);
+    const int64_t bytes = rows * cols, pieces = (bytes + mis + 15) / 16, step = (int64_t)gridDim.x * (kAnyThreads * P);
+    for (int64_t base = ((int64_t)blockIdx.x * (kAnyThreads / 32) + (threadIdx.x >> 5)) * (32 * P); base < pieces; base += step) {
+        const int64_t fb = 16 * base - mis > 0 ? 16 * base - mis : 0;            // the step's first byte of the matrix
+        const int64_t r0 = quotient(fb, cols), c0 = fb - r0 * cols;
+        const uint32_t* const row = packed + r0 * words;
+        uint32_t lo[P], hi[P];
+        bool whole[P];                                                           // in one row
 #pragma unroll
-            for (int k = 0; k < 8; ++k) {
-                // bit b of the nibble -> byte b; +1 = 0x01, -1 = 0xFF  (1 - 2*bit)
-                const uint32_t s = spread_nibble(bits >> (4 * k));
-                v[k] = 0x01010101u + s * 0xFEu;
+        for (int k = 0; k < P; ++k) {
+            const int64_t f = 16 * (base + 32 * k + lane) - mis;                 // the piece's first byte, below 0 in the first
+            int64_t c = c0;
+            const uint32_t dr = advance(c, f < fb ? 0 : (int)(f - fb), cols);
+            whole[k] = f >= 0 && f + 16 <= bytes && c + 16 <= cols;
+            const uint32_t* const src = row + dr * words + (c >> 5);
+            lo[k] = whole[k] ? __ldg(src) : 0u;
+            hi[k] = whole[k] && (c & 31) > 16 ? __ldg(src + 1) : 0u;
+        }
+#pragma unroll
+        for (int k = 0; k < P; ++k) {
+            const int64_t f = 16 * (base + 32 * k + lane) - mis;
+            int64_t c = c0;
+            uint32_t dr = advance(c, f < fb ? 0 : (int)(f - fb), cols);
+            uint4* const dst = reinterpret_cast<uint4*>(w + f);
+            if (whole[k]) {
+                const uint32_t a = convert_order(lo[k], order, NQ_LSB_FIRST), b = convert_order(hi[k], order, NQ_LSB_FIRST);
+                __stcs(dst, signs_of16(__funnelshift_r(a, b, (uint32_t)c & 31u)));
+            } else if (f < bytes) {
+                const int first = f < 0 ? (int)-f : 0, end = bytes - f < 16 ? (int)(bytes - f) : 16;
+                uint32_t h = 0;
+                for (int e = first; e < end;) {
+                    int n = 32 - (int)(c & 31);
+                    n = n < end - e ? n : end - e;
+                    n = cols - c < n ? (int)(cols - c) : n;
+                    const uint32_t word = convert_order(__ldg(row + dr * words + (c >> 5)), order, NQ_LSB_FIRST);
+                    h |= ((word >> (c & 31)) & ((1u << n) - 1u)) << e;           // n <= 16
+                    e += n; c += n;
+                    if (c == cols) { c = 0; ++dr; }
+                }
+                if (end - first == 16) __stcs(dst, signs_of16(h));
+                else
+                    for (int e = first; e < end; ++e) w[f + e] = ((h >> e) & 1u) ? (int8_t)-1 : (int8_t)1;
             }
-            reinterpret_cast<uint4*>(dst)[0] = make_uint4(v[0], v[1], v[2], v[3]);
-            reinterpret_cast<uint4*>(dst)[1] = make_uint4(v[4], v[5], v[6], v[7]);
-        } else {
-            const int n = (int)((cols - c0) < 32 ? (cols - c0) : 32);
-            for (int k = 0; k < n; ++k) dst[k] = ((bits >> k) & 1u) ? (int8_t)-1 : (int8_t)1;
         }
     }
 }
@@ -86,9 +206,10 @@ __global__ void unpack_rows_kernel(const uint32_t* __restrict__ packed, int8_t* 
 // access of a warp contiguous: the dense side moves in 512-byte pieces (one 16-byte piece per lane), the packed
 // side in 128-byte pieces (one word per lane), and the lanes trade their halves with shuffles.  A warp handles
 // 32 consecutive words (1 KB of weights) per step; `n_words` is a multiple of 32 here, the tail goes to the
-// word-per-thread kernels above.
+// kernels above.
 __global__ void __launch_bounds__(256) pack_rows_warp_kernel(const uint4* __restrict__ w, uint32_t* __restrict__ out,
                                                              int64_t n_words, int order) {
+    enter();
     const int lane = threadIdx.x & 31;
     const int64_t warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
     for (int64_t base = ((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5) * 32; base < n_words; base += warps * 32) {
@@ -107,6 +228,7 @@ __global__ void __launch_bounds__(256) pack_rows_warp_kernel(const uint4* __rest
 
 __global__ void __launch_bounds__(256) unpack_rows_warp_kernel(const uint32_t* __restrict__ packed, uint4* __restrict__ w,
                                                                int64_t n_words, int order) {
+    enter();
     const int lane = threadIdx.x & 31;
     const int64_t warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
     for (int64_t base = ((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5) * 32; base < n_words; base += warps * 32) {
@@ -268,49 +390,37 @@ __global__ void permute_scale16_kernel(const uint16_t* __restrict__ s, uint16_t*
 // A-fragment register of an m16n8k32 MMA over columns [32j, 32j+32) with values
 // {0, 2^j} (j = 7: {0, -128}).  Rows and columns beyond the matrix are +1 (bit 0).
 // ---------------------------------------------------------------------------
-// Through shared memory: a work item is one row group (16 rows) by eight chunks (64 words per row); a block
-// reads the 16 row pieces of 256 bytes with contiguous loads and writes eight whole tiles (one uint4 per thread).
-// (One thread per output lane reading its 16 words straight from global memory touches a 32-byte sector per word.)
-// Blocks stride over the items and load the next item's words into registers before they convert the current one.
-__global__ void __launch_bounds__(256) rows_to_tiles_staged_kernel(const uint32_t* __restrict__ packed, uint4* __restrict__ tiles,
-                                                                   int64_t rows, int64_t words, int64_t chunks, int64_t cblocks,
-                                                                   int64_t items, int order) {
-    __shared__ uint32_t s[16][65];
-    const int cl = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
-    uint32_t nxt[4];
-    auto fetch = [&](int64_t item) {
-        const int64_t rg = item / cblocks, c0 = (item - rg * cblocks) * 8;
+// A warp per tile: its 16 pieces of 32 bytes come in with four loads of four pieces each (the neighbouring warp's tile has the
+// rest of a line), are turned around in shared memory and leave as one contiguous store.  Tiles are dealt one by one, so
+// that a matrix of any number of chunks keeps every warp busy: blocks of eight chunks of a row group, which had idle warps
+// at ragged ends and a block barrier, took 6.1 us for 12288 x 2432, this takes 4.7.
+__global__ void __launch_bounds__(256) rows_to_tiles_kernel(const uint32_t* __restrict__ packed, uint4* __restrict__ tiles,
+                                                            int64_t rows, int64_t words, int64_t chunks, int64_t n_tiles, int order) {
+    enter();
+    __shared__ uint32_t s[8][16 * 9];
+    const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
+    uint32_t* const mine = s[threadIdx.x >> 5];
+    const int64_t step = (int64_t)gridDim.x * 8;
+    for (int64_t tile = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5); tile < n_tiles; tile += step) {
+        const int64_t rg = quotient(tile, chunks), wi = (tile - rg * chunks) * 8 + (lane & 7), r0 = rg * 16 + (lane >> 3);
+        uint32_t v[4];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const int i = threadIdx.x + 256 * k, r = i >> 6, wl = i & 63;
-            const int64_t gr = rg * 16 + r, gw = c0 * 8 + wl;
-            nxt[k] = (gr < rows && gw < words) ? __ldcs(packed + gr * words + gw) : 0u;
-        }
-    };
-    int64_t item = blockIdx.x;
-    if (item < items) fetch(item);
-    for (; item < items; item += gridDim.x) {
+        for (int k = 0; k < 4; ++k) v[k] = r0 + 4 * k < rows && wi < words ? __ldg(packed + (r0 + 4 * k) * words + wi) : 0u;
+        __syncwarp();       // the previous tile has been read
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const int i = threadIdx.x + 256 * k;
-            s[i >> 6][i & 63] = convert_order(nxt[k], order, NQ_LSB_FIRST);   // padding words are 0 in either order
-        }
-        __syncthreads();
-        if (item + gridDim.x < items) fetch(item + gridDim.x);
-        const int64_t rg = item / cblocks, c0 = (item - rg * cblocks) * 8;
-        if (c0 + cl < chunks) {
-            uint32_t o[4] = {0, 0, 0, 0};
+        for (int k = 0; k < 4; ++k)   // padding words are 0 in either order
+            mine[(4 * k + (lane >> 3)) * 9 + (lane & 7)] = convert_order(v[k], order, NQ_LSB_FIRST);
+        __syncwarp();
+        uint32_t o[4] = {0, 0, 0, 0};
 #pragma unroll
-            for (int half_row = 0; half_row < 2; ++half_row)
+        for (int half_row = 0; half_row < 2; ++half_row)
 #pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    const uint32_t src = s[g + 8 * half_row][cl * 8 + j];
-                    o[half_row] |= spread_nibble(src >> (4 * q)) << j;           // h = 0
-                    o[2 + half_row] |= spread_nibble(src >> (16 + 4 * q)) << j;  // h = 1
-                }
-            __stcs(tiles + ((rg * chunks + c0 + cl) << 5) + lane, make_uint4(o[0], o[1], o[2], o[3]));
-        }
-        __syncthreads();
+            for (int j = 0; j < 8; ++j) {
+                const uint32_t src = mine[(g + 8 * half_row) * 9 + j];
+                o[half_row] |= spread_nibble(src >> (4 * q)) << j;           // h = 0
+                o[2 + half_row] |= spread_nibble(src >> (16 + 4 * q)) << j;  // h = 1
+            }
+        __stcs(tiles + tile * 32 + lane, make_uint4(o[0], o[1], o[2], o[3]));
     }
 }
 
@@ -358,26 +468,22 @@ int nq_pack_rows(const int8_t* w, int32_t* packed, int64_t rows, int64_t cols, i
     if (rows == 0 || cols == 0) return NQ_OK;
     if (!w || !packed) return NQ_ERR_NULL;
     const int64_t words = (cols + 31) / 32;
-    const bool vec = (cols % 16 == 0) && aligned16(w);
+    uint32_t* const out = reinterpret_cast<uint32_t*>(packed);
     // whole words at an aligned address: the rows form one run of words; the leading rows whose words are a multiple
-    // of 32 go to the warp-contiguous kernel, the remaining rows to the word-per-thread kernel
-    int64_t done_rows = 0;
+    // of 32 go to the kernel without index arithmetic, the remaining rows to the general one
+    int64_t done = 0;
     if (cols % 32 == 0 && aligned16(w)) {
         const int64_t step = 32 / gcd32(words), head_rows = rows / step * step, head = head_rows * words;
         if (head > 0) {
-            pack_rows_warp_kernel<<<grid_for(head, kPackThreads), kPackThreads, 0, as_stream(stream)>>>(
-                reinterpret_cast<const uint4*>(w), reinterpret_cast<uint32_t*>(packed), head, bit_order);
-            NQ_LAUNCH_CHECK();
-            done_rows = head_rows;
+            const int st = launch(pack_rows_warp_kernel, grid_for(head, kPackThreads), kPackThreads, stream,
+                                  reinterpret_cast<const uint4*>(w), out, head, bit_order);
+            if (st != NQ_OK) return st;
+            done = head_rows;
         }
     }
-    if (done_rows < rows) {
-        pack_rows_kernel<<<grid_for((rows - done_rows) * words, kPackThreads), kPackThreads, 0, as_stream(stream)>>>(
-            w + done_rows * cols, reinterpret_cast<uint32_t*>(packed) + done_rows * words, rows - done_rows, cols, words,
-            bit_order, vec);
-        NQ_LAUNCH_CHECK();
-    }
-    return NQ_OK;
+    if (done == rows) return NQ_OK;
+    return launch(pack_rows_kernel, grid_for(((rows - done) * words + 1) / 2, kAnyThreads), kAnyThreads, stream, w + done * cols,
+                  out + done * words, rows - done, cols, words, bit_order);
 }
 
 int nq_unpack_rows(const int32_t* packed, int8_t* w, int64_t rows, int64_t cols, int bit_order,
@@ -387,24 +493,24 @@ int nq_unpack_rows(const int32_t* packed, int8_t* w, int64_t rows, int64_t cols,
     if (rows == 0 || cols == 0) return NQ_OK;
     if (!w || !packed) return NQ_ERR_NULL;
     const int64_t words = (cols + 31) / 32;
-    const bool vec = (cols % 16 == 0) && aligned16(w);
-    int64_t done_rows = 0;
+    const uint32_t* const in = reinterpret_cast<const uint32_t*>(packed);
+    int64_t done = 0;
     if (cols % 32 == 0 && aligned16(w)) {   // see nq_pack_rows
         const int64_t step = 32 / gcd32(words), head_rows = rows / step * step, head = head_rows * words;
         if (head > 0) {
-            unpack_rows_warp_kernel<<<grid_for(head, kPackThreads), kPackThreads, 0, as_stream(stream)>>>(
-                reinterpret_cast<const uint32_t*>(packed), reinterpret_cast<uint4*>(w), head, bit_order);
-            NQ_LAUNCH_CHECK();
-            done_rows = head_rows;
+            const int st = launch(unpack_rows_warp_kernel, grid_for(head, kPackThreads), kPackThreads, stream, in,
+                                  reinterpret_cast<uint4*>(w), head, bit_order);
+            if (st != NQ_OK) return st;
+            done = head_rows;
         }
     }
-    if (done_rows < rows) {
-        unpack_rows_kernel<<<grid_for((rows - done_rows) * words, kPackThreads), kPackThreads, 0, as_stream(stream)>>>(
-            reinterpret_cast<const uint32_t*>(packed) + done_rows * words, w + done_rows * cols, rows - done_rows, cols, words,
-            bit_order, vec);
-        NQ_LAUNCH_CHECK();
-    }
-    return NQ_OK;
+    if (done == rows) return NQ_OK;
+    // Four pieces per lane share the row arithmetic and are in flight together (12291 x 2435: 13.8 us with two, 12.5 with
+    // four), where that leaves every SM a few blocks; else one (1000 x 777: 3.3 us with four).
+    const int64_t pieces = ((rows - done) * cols + 15) / 16 + 1;
+    const bool many = pieces >= (int64_t)sm_count() * 8 * kAnyThreads * 4;
+    return launch(many ? unpack_rows_kernel<4> : unpack_rows_kernel<1>, grid_for(many ? (pieces + 3) / 4 : pieces, kAnyThreads),
+                  kAnyThreads, stream, in + done * words, w + done * cols, rows - done, cols, words, bit_order);
 }
 
 int nq_reorder_words(const int32_t* in, int32_t* out, int64_t n_words, int order_in, int order_out,
@@ -473,13 +579,9 @@ int nq_rows_to_tiles(const int32_t* packed, void* tiles, int64_t rows, int64_t c
     if (check_order(bit_order) != NQ_OK) return NQ_ERR_DTYPE;
     if (!packed || !tiles) return NQ_ERR_NULL;
     if (!aligned16(tiles)) return NQ_ERR_ALIGN;
-    const int64_t words = (cols + 31) / 32, rgs = (rows + 15) / 16, chunks = (cols + 255) / 256;
-    const int64_t cblocks = (chunks + 7) / 8, items = rgs * cblocks;
-    const int64_t resident = (int64_t)sm_count() * 8;   // 256-thread blocks that are resident at once
-    rows_to_tiles_staged_kernel<<<(unsigned)(items < resident ? items : resident), 256, 0, as_stream(stream)>>>(
-        reinterpret_cast<const uint32_t*>(packed), static_cast<uint4*>(tiles), rows, words, chunks, cblocks, items, bit_order);
-    NQ_LAUNCH_CHECK();
-    return NQ_OK;
+    const int64_t words = (cols + 31) / 32, chunks = (cols + 255) / 256, n_tiles = (rows + 15) / 16 * chunks;
+    return launch(rows_to_tiles_kernel, grid_for(n_tiles * 32, 256), 256, stream, reinterpret_cast<const uint32_t*>(packed),
+                  static_cast<uint4*>(tiles), rows, words, chunks, n_tiles, bit_order);
 }
 
 int nq_tiles_to_rows(const void* tiles, int32_t* packed, int64_t rows, int64_t cols, int bit_order,
