@@ -274,7 +274,7 @@ class Step:
                   "i": torch.randn(T, INTER, generator=g, device=device).to(dtype)}
         self.keep, self.launches, self.bytes = [], [], 0
         scratch_bytes = 0
-        # more tokens than one decode launch takes: the groups go through nq_gemm_group_fwd (split-K GEMM)
+        # more tokens than one decode launch takes: the groups go through nq_gemm_group_fwd (batch kernel or GEMM)
         self.per_linear = T >= (GEMM_MIN_TOKENS or self.L.nq_gemv_max_tokens() + 1)
         self.n_linears = 0
         for _ in range(layers):
@@ -297,7 +297,8 @@ class Step:
         self.last_y = self.keep[-1]["y"]
         self.scratch = torch.zeros(scratch_bytes, dtype=torch.uint8, device=device)
         self.kernels_per_step = (2 if self.per_linear else 1) * len(self.launches)
-        self.kernel_name = "gemm_stage_kernel (split-K)" if self.per_linear else "gemv_group_kernel"
+        self.kernel_name = ("gemv_group_kernel" if not self.per_linear else
+                            "batch_stage_kernel" if T <= 32 else "gemm_stage_kernel")
         self.graph = None
 
     def run(self):
@@ -751,9 +752,8 @@ def measure_tp(T, layers, steps, warmup, collective, device, world, rank, shard=
 
     # One GPU, or the peer-memory collective: the step is replayed as a CUDA graph.  With NCCL the launches
     # and the collectives are issued eagerly in stream order: a captured NCCL collective runs on a stream of
-    # its own beside the next cooperative launch, which cannot become resident while the collective's CTAs hold
-    # SMs and wait for a peer that is itself waiting for its cooperative launch: that combination can deadlock
-    # and is not used.
+    # its own beside the next launch of this rank while its CTAs hold SMs and wait for a peer: a combination in
+    # which the ranks can end up waiting for one another, and it is not used.
     graph = None
     for _ in range(2):
         run()
