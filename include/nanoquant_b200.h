@@ -176,6 +176,13 @@ int nq_gemv_fwd(const void* x, const void* s_in, const void* v_tiles, const void
 int nq_gemv_group_fwd(const nq_linear_desc* linears_host, int n_linears, int T, int dtype,
                       void* scratch, size_t scratch_bytes, nq_stream_t stream);
 
+/* nq_gemv_group_fwd as the dispatchers call it: large groups of four tokens run as two launches with a matrix
+ * instruction over 16-bit floats, the intermediate kept as two bf16 words per element (16 significant bits, like the
+ * fixed point of the GEMV).  Same arguments, scratch and accuracy; the results differ from nq_gemv_fwd's in the
+ * last bits. */
+int nq_decode_group_fwd(const nq_linear_desc* linears_host, int n_linears, int T, int dtype,
+                        void* scratch, size_t scratch_bytes, nq_stream_t stream);
+
 /* nq_gemv_fwd for callers that cannot hand the library any device memory of their own
  * beyond inputs and outputs: code running where allocation is forbidden or already frozen
  * (inside a serving loop whose memory plan is fixed, a plugin host that owns the allocator,

@@ -51,6 +51,7 @@ SIGNATURES = {
     "nq_gemv_group_fwd": (c_int, [ctypes.POINTER(LinearDesc), c_int, c_int, c_int, c_void_p, c_size_t, c_void_p]),
     "nq_scratch_status": (c_int, [c_void_p, c_void_p]),
     "nq_gemv_set_wait_limit": (ctypes.c_uint, [ctypes.c_uint]),
+    "nq_decode_group_fwd": (c_int, [ctypes.POINTER(LinearDesc), c_int, c_int, c_int, c_void_p, c_size_t, c_void_p]),
     "nq_gemv_fwd_static": (c_int, [c_void_p] * 7 + [c_int, c_int, c_int, c_int, c_int, c_void_p]),
     "nq_gemv_static_max_rank": (c_size_t, []),
     "nq_gemm_scratch_bytes": (c_size_t, [c_int, c_int, c_int, c_int]),

@@ -66,7 +66,7 @@ static_assert(sizeof(BatchJob) == 128, "128 bytes");
 struct alignas(16) BatchParams {
     BatchJob job[kMaxGemmJobs];
     unsigned* status;
-    int T, io_bf16, out_bf16, saturate, exp_sign;
+    int T, io_bf16, out_bf16, saturate, exp_sign;   // T: columns of partial sums (tokens, or 8 for a split input)
     int slots, slot_bytes, part_off;
     int stage_off, frag_out;      // activation staging buffers; output in fragment order
     uint8_t cta_job[kBatchMaxCtas];
@@ -103,8 +103,9 @@ __device__ __forceinline__ void copy16_or_zero(uint32_t dst, const void* src, bo
 }
 
 // NT: column groups of eight tokens.  ROWS: row groups a warp takes in a pass.  FRAG: the input is in fragment order
-// and has no scale (the second stage); otherwise it is [T, lda].
-template <bool BF16, int NT, int ROWS, bool FRAG>
+// and has no scale (the second stage); otherwise it is [T, lda].  SPLIT: the intermediate is value and remainder (see
+// kSplitTokens).
+template <bool BF16, int NT, int ROWS, bool FRAG, bool SPLIT>
 __global__ void __launch_bounds__(kBatchThreads, 1) batch_stage_kernel(const __grid_constant__ BatchParams Pc) {
     constexpr int kRows = ROWS, kB = blocks_in_flight(NT, ROWS), kPieces = pieces(NT);
     extern __shared__ __align__(128) unsigned char smem[];
@@ -307,12 +308,13 @@ __global__ void __launch_bounds__(kBatchThreads, 1) batch_stage_kernel(const __g
         if (++slot == slots) { slot = 0; parity ^= 1u; }
         if (loader) load_block();
         // outputs: lanes take rows, warps take tokens
-        const float lim = P.saturate ? (out_bf16 ? 3.3895313892515355e+38f : 64504.0f) : 3.4e38f;
+        const float lim = P.saturate || (SPLIT && !FRAG) ? (out_bf16 ? 3.3895313892515355e+38f : 64504.0f) : 3.4e38f;
         const uint16_t* const resid = static_cast<const uint16_t*>(jb.resid);
         const int* const row_exp = jb.row_exp;
         const int kslice = T * tok_stride, frag_out = P.frag_out;
+        const int tokens = SPLIT ? kSplitTokens : T;
 #pragma unroll 1
-        for (int tok = warp; tok < T; tok += kBatchWarps) {
+        for (int tok = warp; tok < tokens; tok += kBatchWarps) {
             const float rs = row_exp ? exp2f((float)(P.exp_sign * row_exp[tok])) : 1.f;
             uint16_t* const out = static_cast<uint16_t*>(jb.out) + (frag_out ? 0 : tok * jb.ld_out + row0);
 #pragma unroll 1
@@ -321,11 +323,24 @@ __global__ void __launch_bounds__(kBatchThreads, 1) batch_stage_kernel(const __g
                 float v = 0.f;
 #pragma unroll 4
                 for (int k = 0; k < wk; ++k, src += kslice) v += *src;
+                if (SPLIT && FRAG) {
+                    const float* rest = part + (kSplitTokens + tok) * tok_stride + idx;
+                    float v2 = 0.f;
+#pragma unroll 4
+                    for (int k = 0; k < wk; ++k, rest += kslice) v2 += *rest;
+                    v += v2;
+                }
                 const float2 sc = scale[idx];
                 if (row0 + idx < rows) {
                     float extra = sc.y;
                     if (resid) extra += float_of(resid[tok * jb.ld_res + row0 + idx], io_bf16);
                     v = fminf(fmaxf(v * (sc.x * rs) + extra, -lim), lim);
+                    if (SPLIT && !FRAG) {
+                        const __nv_bfloat16 value = __float2bfloat16(v);
+                        out[fragment_index<1>(tok, row0 + idx)] = __bfloat16_as_ushort(value);
+                        out[fragment_index<1>(kSplitTokens + tok, row0 + idx)] = __bfloat16_as_ushort(__float2bfloat16(v - __bfloat162float(value)));
+                        continue;
+                    }
                     out[frag_out ? fragment_index<NT>(tok, row0 + idx) : idx] = out_bf16 ? __bfloat16_as_ushort(__float2bfloat16(v)) : __half_as_ushort(__float2half(v));
                 }
             }
@@ -340,14 +355,22 @@ __global__ void __launch_bounds__(kBatchThreads, 1) batch_stage_kernel(const __g
 
 template <bool BF16, int NT, bool FRAG>
 static const void* batch_kernel_rows(int rows) {
-    if (rows == 1) return (const void*)batch_stage_kernel<BF16, NT, 1, FRAG>;
-    if (rows == 2 || most_rows_of(NT) == 2) return (const void*)batch_stage_kernel<BF16, NT, 2, FRAG>;
-    return (const void*)batch_stage_kernel<BF16, NT, most_rows_of(NT), FRAG>;
+    if (rows == 1) return (const void*)batch_stage_kernel<BF16, NT, 1, FRAG, false>;
+    if (rows == 2 || most_rows_of(NT) == 2) return (const void*)batch_stage_kernel<BF16, NT, 2, FRAG, false>;
+    return (const void*)batch_stage_kernel<BF16, NT, most_rows_of(NT), FRAG, false>;
 }
 template <bool BF16, bool FRAG>
 static const void* batch_kernel_tokens(int nt, int rows) {
     return nt == 1 ? batch_kernel_rows<BF16, 1, FRAG>(rows) : nt == 2 ? batch_kernel_rows<BF16, 2, FRAG>(rows)
            : nt == 3 ? batch_kernel_rows<BF16, 3, FRAG>(rows) : batch_kernel_rows<BF16, 4, FRAG>(rows);
+}
+template <bool BF16, bool FRAG>
+static const void* split_kernel_rows(int rows) {
+    return rows == 1 ? (const void*)batch_stage_kernel<BF16, 1, 1, FRAG, true>
+           : rows == 2 ? (const void*)batch_stage_kernel<BF16, 1, 2, FRAG, true> : (const void*)batch_stage_kernel<BF16, 1, 4, FRAG, true>;
+}
+static const void* split_kernel(int bf16, int rows, bool frag) {     // (a split intermediate is bf16)
+    return frag ? split_kernel_rows<true, true>(rows) : bf16 ? split_kernel_rows<true, false>(rows) : split_kernel_rows<false, false>(rows);
 }
 static const void* batch_kernel(int bf16, int nt, int rows, bool frag) {
     if (frag) return bf16 ? batch_kernel_tokens<true, true>(nt, rows) : batch_kernel_tokens<false, true>(nt, rows);
@@ -362,6 +385,8 @@ static int batch_smem_limit(int* out) {
         NQ_CUDA_TRY(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
         for (int i = 0; i < 48; ++i)
             NQ_CUDA_TRY(cudaFuncSetAttribute(batch_kernel(i & 1, 1 + (i / 4) % 4, 1 << (i / 16), (i & 2) != 0), cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
+        for (int i = 0; i < 12; ++i)
+            NQ_CUDA_TRY(cudaFuncSetAttribute(split_kernel(i & 1, 1 << (i / 4), (i & 2) != 0), cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
         cached[dev & 63] = optin;
     }
     *out = cached[dev & 63];
@@ -376,8 +401,23 @@ int batch_max_tokens(const StageJob* jobs, int n) {
 
 size_t batch_fragment_bytes(int T, int K) { return (size_t)((K + 255) / 256) * 16 * tokens_groups(T) * 256; }
 
-int launch_batch_stage(const StageJob* jobs, int n, int T, StageTypes ty, int saturate, bool frag_in, bool frag_out, unsigned* status,
-                       cudaStream_t stream) {
+// Chunk slices x row slices of the warps for a block of `gb` row groups: a step (a row group's chunk) against a chunk's B
+// fragments, once per pass.
+static void split_warps(int gb, int chunks, int nt, int& wk, int& wr) {
+    const int rows_most = most_rows_of(nt);
+    int best = 1 << 30;
+    for (int k = 1; k <= kBatchWarps && k <= chunks; ++k) {
+        int r = kBatchWarps / k;
+        if (r > gb) r = gb;
+        const int per = (gb + r - 1) / r;
+        const int cost = ((chunks + k - 1) / k) * (per * (8 + 2 * nt) + ((per + rows_most - 1) / rows_most) * (3 + 3 * nt));
+        if (cost < best) { best = cost; wk = k; wr = r; }
+    }
+}
+
+int launch_batch_stage(const StageJob* jobs, int n, int tokens, StageTypes ty, int saturate, bool frag_in, bool frag_out, bool split,
+                       unsigned* status, cudaStream_t stream) {
+    const int T = split && frag_in ? 2 * kSplitTokens : tokens;
     for (int i = 0; i < n; ++i) {      // 16-byte copies of rows and scales
         if (jobs[i].K % 8 != 0 || (!frag_in && (!aligned16(jobs[i].a) || jobs[i].lda % 8 != 0))) return NQ_ERR_ALIGN;
         if (jobs[i].pre && !aligned16(jobs[i].pre)) return NQ_ERR_ALIGN;
@@ -389,7 +429,7 @@ int launch_batch_stage(const StageJob* jobs, int n, int T, StageTypes ty, int sa
     P.status = status;
     P.T = T;
     P.io_bf16 = ty.io_bf16; P.out_bf16 = ty.out_bf16; P.saturate = saturate; P.exp_sign = ty.exp_sign;
-    const int nt = tokens_groups(T), rows_most = most_rows_of(nt);
+    const int nt = tokens_groups(T);
     int groups[kMaxGemmJobs], chunks[kMaxGemmJobs], ncta[kMaxGemmJobs], total = 0;
     for (int i = 0; i < n; ++i) {
         groups[i] = (jobs[i].Nout + 15) / 16;
@@ -430,15 +470,11 @@ int launch_batch_stage(const StageJob* jobs, int n, int T, StageTypes ty, int sa
             size_t part = 0, slot = 0;
             for (int blocks = 1;; ++blocks) {
                 j.gb = attempt == 2 ? 1 : (most + blocks - 1) / blocks;
-                // Chunk slices x row slices: a step (a row group's chunk) against a chunk's B fragments, once per pass
-                int best = 1 << 30;
-                for (int k = 1; k <= kBatchWarps && k <= chunks[i]; ++k) {
-                    int r = kBatchWarps / k;
-                    if (r > j.gb) r = j.gb;
-                    const int per = (j.gb + r - 1) / r;
-                    const int cost = ((chunks[i] + k - 1) / k) * (per * (8 + 2 * nt) + ((per + rows_most - 1) / rows_most) * (3 + 3 * nt));
-                    if (cost < best) { best = cost; j.wk = (uint16_t)k; j.wr = (uint16_t)r; }
-                }
+                int wk = 1, wr = 1;
+                // the sums of a split linear have to be the same alone and in a group: slices as for the linear alone
+                split_warps(split ? (groups[i] + sm_count() - 1) / sm_count() : j.gb, chunks[i], nt, wk, wr);
+                if (split) wr = kBatchWarps / wk < j.gb ? kBatchWarps / wk : j.gb;
+                j.wk = (uint16_t)wk; j.wr = (uint16_t)wr;
                 part = (size_t)j.wk * T * (j.gb * 16 + 4) * 4 + (size_t)j.gb * 16 * 8;
                 slot = (size_t)j.gb * chunks[i] * 512;
                 const bool fits = attempt == 0 ? part + slot <= room : part <= room / 2 && slot <= room / 2;
@@ -475,7 +511,8 @@ int launch_batch_stage(const StageJob* jobs, int n, int T, StageTypes ty, int sa
     cfg.attrs = &attr;
     cfg.numAttrs = pdl_ok ? 1 : 0;
     void* args[] = {&P};
-    const void* fn = batch_kernel(ty.a_bf16, nt, most_rows == 1 ? 1 : most_rows == 2 ? 2 : 4, frag_in);
+    const int rows = most_rows == 1 ? 1 : most_rows == 2 ? 2 : 4;
+    const void* fn = split ? split_kernel(ty.a_bf16, rows, frag_in) : batch_kernel(ty.a_bf16, nt, rows, frag_in);
     cudaError_t e = cudaLaunchKernelExC(&cfg, fn, args);
     if (e != cudaSuccess && pdl_ok) {
         (void)cudaGetLastError();

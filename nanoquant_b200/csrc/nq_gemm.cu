@@ -831,7 +831,7 @@ static int launch_stage(const StageJob* jobs, int n, int T, StageTypes ty, int s
         if (S.pre && !aligned16(S.pre)) return NQ_ERR_ALIGN;
         Ks[j] = S.K; Ns[j] = S.Nout;
     }
-    if (T <= batch_max_tokens(jobs, n)) return launch_batch_stage(jobs, n, T, ty, saturate, false, false, status, stream);
+    if (T <= batch_max_tokens(jobs, n)) return launch_batch_stage(jobs, n, T, ty, saturate, false, false, false, status, stream);
     { const int st_attr = set_kernel_attributes(); if (st_attr != NQ_OK) return st_attr; }
     const GroupPlan pl = plan_group(T, n, Ks, Ns);
     const int mh = pl.mh, nh = pl.nh;
@@ -991,8 +991,8 @@ int nq_gemm_group_fwd(const nq_linear_desc* d, int n_linears, int T, int dtype, 
     const bool batch = T <= batch_max_tokens(s1, n_linears) && T <= batch_max_tokens(s2, n_linears);
     auto stages = [&](StageTypes ty1, StageTypes ty2) -> int {
         if (batch) {
-            const int st = launch_batch_stage(s1, n_linears, T, ty1, 0, false, true, status, as_stream(stream));
-            return st != NQ_OK ? st : launch_batch_stage(s2, n_linears, T, ty2, 1, true, false, status, as_stream(stream));
+            const int st = launch_batch_stage(s1, n_linears, T, ty1, 0, false, true, false, status, as_stream(stream));
+            return st != NQ_OK ? st : launch_batch_stage(s2, n_linears, T, ty2, 1, true, false, false, status, as_stream(stream));
         }
         const int st = launch_stage(s1, n_linears, T, ty1, 0, status, as_stream(stream));
         return st != NQ_OK ? st : launch_stage(s2, n_linears, T, ty2, 1, status, as_stream(stream));
@@ -1057,7 +1057,8 @@ int nq_gemm_set_precise_intermediate(int on) {
     return old;
 }
 
-// One decode launch handles four tokens; from five tokens on the batch kernel's two stages are faster than two launches.
+// The decode path takes up to four tokens (the largest groups of four by the batch kernel, see nq_decode_group_fwd); from five
+// on the batch kernel's two stages are faster than two decode launches, and keep the intermediate in the I/O type.
 int nq_gemv_max_tokens(void) { return 4; }
 
 size_t nq_linear_scratch_bytes(int T, int N, int R, int M) {
@@ -1068,9 +1069,13 @@ size_t nq_linear_scratch_bytes(int T, int N, int R, int M) {
 int nq_linear_fwd(const void* x, const void* s_in, const void* v_tiles, const void* s_mid, const void* u_tiles,
                   const void* s_out, void* y, void* scratch, size_t scratch_bytes, int T, int N, int R, int M,
                   int dtype, nq_stream_t stream) {
-    if (T <= nq_gemv_max_tokens() || (N % 8) || (R % 8))
-        return nq_gemv_fwd(x, s_in, v_tiles, s_mid, u_tiles, s_out, y, scratch, scratch_bytes, T, N, R, M, dtype,
-                           stream);
+    if (T <= nq_gemv_max_tokens() || (N % 8) || (R % 8)) {
+        nq_linear_desc d;
+        memset(&d, 0, sizeof(d));
+        d.x = x; d.s_in = s_in; d.v_tiles = v_tiles; d.s_mid = s_mid; d.u_tiles = u_tiles; d.s_out = s_out; d.y = y;
+        d.N = N; d.R = R; d.M = M; d.ldx = N; d.ldy = M;
+        return nq_decode_group_fwd(&d, 1, T, dtype, scratch, scratch_bytes, stream);
+    }
     return nq_gemm_fwd(x, s_in, v_tiles, s_mid, u_tiles, s_out, y, scratch, scratch_bytes, T, N, R, M, dtype, stream);
 }
 

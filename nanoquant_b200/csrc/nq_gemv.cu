@@ -49,6 +49,7 @@
 
 #include "nq_common.cuh"
 #include "nq_plan.h"
+#include "nq_stage.h"
 
 namespace nq {
 
@@ -752,6 +753,36 @@ static int static_scratch_ptr(void** out) {
 // {fp32, tag} words of a linear's intermediate, rows padded to eight elements
 static size_t intermediate_bytes(int R) { return round_up((size_t)kMaxTok * (size_t)((R + 7) / 8 * 8) * sizeof(uint2), 256); }
 
+// Tokens [t0, t0 + T) of a group by the batch kernel's two launches, or NQ_ERR_UNSUPPORTED.  Every CTA of the decode kernel
+// converts the whole input and the whole intermediate of its linear to fixed point, and at four tokens that is the largest
+// part of a launch; the batch kernel takes 16-bit floats as they come, with the intermediate as value and remainder, at eight
+// columns of which it computes all anyway.  Eight layers of an 8B-class model in a graph: 421 -> 359 us; three tokens take
+// 363 in one launch each and 361 in two, and stay.  The line: from 20 chunks of input and intermediate on (N + R about 5000)
+// the conversion is worth the second launch.  Below, and below 1 MB of factors, a call in a stream is bound by the host, which
+// pays some 5 us for it (a 1B-class layer of 2048 columns: 143 us per four layers, 163 with two launches throughout, 137
+// by this rule).
+constexpr int kTwoStageChunks = 20;
+constexpr size_t kTwoStageBytes = (size_t)1 << 20;
+static int launch_two_stages(const nq_linear_desc* d, int n, int t0, int T, int dtype, void* scratch, cudaStream_t stream) {
+    StageJob s1[kMaxJobs], s2[kMaxJobs];
+    size_t off = kHeaderBytes;
+    for (int i = 0; i < n; ++i) {
+        const nq_linear_desc& L = d[i];
+        if (L.N % 8 || L.R % 8 || L.ldx % 8 || !aligned16(L.x) || !aligned16(L.s_in)) return NQ_ERR_UNSUPPORTED;
+        if (batch_fragment_bytes(2 * kSplitTokens, L.R) > intermediate_bytes(L.R)) return NQ_ERR_UNSUPPORTED;   // ranks below 128
+        void* t = static_cast<char*>(scratch) + off;
+        off += intermediate_bytes(L.R);
+        s1[i] = {static_cast<const uint16_t*>(L.x) + (size_t)t0 * L.ldx, L.ldx, L.v_tiles, L.s_in, L.s_mid, t, L.R, L.N, L.R, nullptr, nullptr, 0, nullptr};
+        s2[i] = {t, L.R, L.u_tiles, nullptr, L.s_out, static_cast<uint16_t*>(L.y) + (size_t)t0 * L.ldy, L.ldy, L.R, L.M, L.bias,
+                 L.residual ? static_cast<const uint16_t*>(L.residual) + (size_t)t0 * L.ldr : nullptr, L.ldr, nullptr};
+    }
+    if (T > batch_max_tokens(s1, n) || T > batch_max_tokens(s2, n)) return NQ_ERR_UNSUPPORTED;
+    const int b16 = dtype == NQ_BF16;
+    unsigned* status = static_cast<unsigned*>(scratch) + 2;
+    const int st = launch_batch_stage(s1, n, T, StageTypes{b16, b16, 1, 0}, 0, false, true, true, status, stream);
+    return st != NQ_OK ? st : launch_batch_stage(s2, n, T, StageTypes{b16, 1, b16, 0}, 1, true, false, true, status, stream);
+}
+
 static unsigned g_spin_limit = kSpinLimit;   // polls before a wait for the tagged intermediate gives up
 
 }  // namespace nq
@@ -775,8 +806,8 @@ size_t nq_gemv_group_scratch_bytes(const nq_linear_desc* d, int n_linears, int T
     return b;
 }
 
-int nq_gemv_group_fwd(const nq_linear_desc* d, int n_linears, int T, int dtype, void* scratch,
-                      size_t scratch_bytes, nq_stream_t stream) {
+static int gemv_group(const nq_linear_desc* d, int n_linears, int T, int dtype, void* scratch, size_t scratch_bytes,
+                      bool two_stages, nq_stream_t stream) {
     if (!d || !scratch) return NQ_ERR_NULL;
     if (n_linears <= 0 || n_linears > kMaxJobs) return NQ_ERR_UNSUPPORTED;
     if (T <= 0) return NQ_ERR_SHAPE;
@@ -784,7 +815,7 @@ int nq_gemv_group_fwd(const nq_linear_desc* d, int n_linears, int T, int dtype, 
     if (!aligned16(scratch)) return NQ_ERR_ALIGN;
     if (scratch_bytes < nq_gemv_group_scratch_bytes(d, n_linears, T)) return NQ_ERR_SCRATCH;
 
-    int max_chunks = 0;
+    int max_chunks = 0, most_conversion = 0;   // chunks of a phase, of both phases of a linear
     int rg[2][kMaxJobs], ck[2][kMaxJobs];      // row groups and chunks of the two phases
     size_t packed = 0;
     for (int i = 0; i < n_linears; ++i) {
@@ -799,6 +830,7 @@ int nq_gemv_group_fwd(const nq_linear_desc* d, int n_linears, int T, int dtype, 
         rg[1][i] = (L.M + 15) / 16; ck[1][i] = (L.R + 255) / 256;
         for (int ph = 0; ph < 2; ++ph) max_chunks = ck[ph][i] > max_chunks ? ck[ph][i] : max_chunks;
         packed += (size_t)L.R * ((size_t)L.N + L.M) / 8;
+        most_conversion = ck[0][i] + ck[1][i] > most_conversion ? ck[0][i] + ck[1][i] : most_conversion;
     }
     int dev = 0, smem_limit = 0;
     NQ_CUDA_TRY(cudaGetDevice(&dev));
@@ -839,6 +871,11 @@ int nq_gemv_group_fwd(const nq_linear_desc* d, int n_linears, int T, int dtype, 
     const size_t esz = 2;
     for (int t0 = 0; t0 < T; t0 += tg) {
         const int tn = (T - t0) < tg ? (T - t0) : tg;
+        if (two_stages && tn == kSplitTokens && most_conversion >= kTwoStageChunks && packed >= kTwoStageBytes) {
+            const int st = launch_two_stages(d, n_linears, t0, tn, dtype, scratch, as_stream(stream));
+            if (st == NQ_OK) continue;
+            if (st != NQ_ERR_UNSUPPORTED) return st;
+        }
         P.T = tn;
         memset(P.cta_job, kMaxJobs * 17, sizeof(P.cta_job));
         // room for a block's partial sums and weights; a single row group is always allowed (see above)
@@ -939,6 +976,16 @@ int nq_gemv_group_fwd(const nq_linear_desc* d, int n_linears, int T, int dtype, 
         NQ_CUDA_TRY(e);
     }
     return NQ_OK;
+}
+
+int nq_gemv_group_fwd(const nq_linear_desc* d, int n_linears, int T, int dtype, void* scratch, size_t scratch_bytes,
+                      nq_stream_t stream) {
+    return gemv_group(d, n_linears, T, dtype, scratch, scratch_bytes, false, stream);
+}
+
+int nq_decode_group_fwd(const nq_linear_desc* d, int n_linears, int T, int dtype, void* scratch, size_t scratch_bytes,
+                        nq_stream_t stream) {
+    return gemv_group(d, n_linears, T, dtype, scratch, scratch_bytes, true, stream);
 }
 
 int nq_gemv_fwd(const void* x, const void* s_in, const void* v_tiles, const void* s_mid,

@@ -33,7 +33,10 @@ int batch_max_tokens(const StageJob* jobs, int n);
 // `frag_in` / `frag_out`: the activations / the output are an intermediate in the batch kernel's fragment order, of
 // batch_fragment_bytes each, without an input scale.
 size_t batch_fragment_bytes(int T, int K);
-int launch_batch_stage(const StageJob* jobs, int n, int T, StageTypes ty, int saturate, bool frag_in, bool frag_out, unsigned* status,
-                       cudaStream_t stream);
+// `split` (with a fragment-order side, kSplitTokens tokens): the intermediate is bf16 twice, value and remainder, as the
+// columns t and 4 + t of eight; 16 significant bits at fp32's range.  A linear's results are then the same bits in any group.
+constexpr int kSplitTokens = 4;
+int launch_batch_stage(const StageJob* jobs, int n, int T, StageTypes ty, int saturate, bool frag_in, bool frag_out, bool split,
+                       unsigned* status, cudaStream_t stream);
 
 }  // namespace nq

@@ -109,7 +109,7 @@ void launch(nq_linear_desc* d, int n, int64_t T, int dtype, int dev) {
     if (!gemv && n == 1 && (d->N % 8 != 0 || d->R % 8 != 0)) gemv = true;
     OnDevice on(dev);
     const nq_stream_t stream = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)dev).stream();
-    const auto fwd = gemv ? nq_gemv_group_fwd : nq_gemm_group_fwd;
+    const auto fwd = gemv ? nq_decode_group_fwd : nq_gemm_group_fwd;
     Scratch s = scratch_of(dev);
     int st = s.ptr ? fwd(d, n, (int)T, dtype, s.ptr, s.bytes, stream) : (int)NQ_ERR_SCRATCH;
     if (st == NQ_ERR_SCRATCH) {   // nothing has been launched: the scratch is checked first
@@ -117,7 +117,7 @@ void launch(nq_linear_desc* d, int n, int64_t T, int dtype, int dev) {
         s = scratch_of(dev);
         st = fwd(d, n, (int)T, dtype, s.ptr, s.bytes, stream);
     }
-    if (st < 0) fail(st, gemv ? "nq_gemv_group_fwd" : "nq_gemm_group_fwd");
+    if (st < 0) fail(st, gemv ? "nq_decode_group_fwd" : "nq_gemm_group_fwd");
 }
 
 // A linear's operands.  `rank` comes from the caller: the tile layout pads it.

@@ -2,7 +2,7 @@
 
 The reference runs one operator call per projection (``modules/linear.py:121-132``, two kernel launches each);
 at decode batch sizes a launch is a chain of latencies, so the step time is set by the number of launches.
-``LinearGroup`` issues ``nq_gemv_group_fwd`` (up to four tokens) or ``nq_gemm_group_fwd`` for up to four
+``LinearGroup`` issues ``nq_decode_group_fwd`` (up to four tokens) or ``nq_gemm_group_fwd`` for up to four
 prepared :class:`~nanoquant_b200.modules.linear.NanoQuantLinear` modules, with their biases and optional
 residuals in the kernel's epilogue.
 """

@@ -169,7 +169,7 @@ def as_tiles(bits: torch.Tensor, cols: int) -> torch.Tensor:
 
 def gemv_forward(x: torch.Tensor, s_in: torch.Tensor, v_tiles: torch.Tensor, s_mid: Optional[torch.Tensor],
                  u_tiles: torch.Tensor, s_out: torch.Tensor, R: int) -> torch.Tensor:
-    """Launch ``nq_gemv_fwd`` on the current stream; ``x`` is ``[T, N]``."""
+    """The decode path on the current stream at any token count; ``x`` is ``[T, N]``."""
     T, N = x.shape
     M = s_out.size(0)
     y = torch.empty((T, M), dtype=x.dtype, device=x.device)
@@ -178,12 +178,13 @@ def gemv_forward(x: torch.Tensor, s_in: torch.Tensor, v_tiles: torch.Tensor, s_m
     L = _lib.lib()
     nbytes = L.nq_gemv_scratch_bytes(T, N, R, M)
     scratch = scratch_for(x.device, nbytes)
+    fwd = L.nq_linear_fwd if T <= L.nq_gemv_max_tokens() else L.nq_gemv_fwd
     with torch.cuda.device(x.device):
-        st = L.nq_gemv_fwd(x.data_ptr(), s_in.data_ptr(), v_tiles.data_ptr(),
-                           s_mid.data_ptr() if s_mid is not None else None,
-                           u_tiles.data_ptr(), s_out.data_ptr(), y.data_ptr(),
-                           scratch.data_ptr(), scratch.numel(), T, N, R, M, _dtype_id(x),
-                           torch.cuda.current_stream(x.device).cuda_stream)
+        st = fwd(x.data_ptr(), s_in.data_ptr(), v_tiles.data_ptr(),
+                 s_mid.data_ptr() if s_mid is not None else None,
+                 u_tiles.data_ptr(), s_out.data_ptr(), y.data_ptr(),
+                 scratch.data_ptr(), scratch.numel(), T, N, R, M, _dtype_id(x),
+                 torch.cuda.current_stream(x.device).cuda_stream)
     _lib.check(st, "nq_gemv_fwd")
     return y
 
@@ -274,7 +275,7 @@ def _nanoquant_dyn_forward_fake(x, scale_g, Ubits, scale_l, Vbits, scale_h, *arg
 
 def group_forward(xs, layers, T: int, dtype: torch.dtype, device: torch.device, biases=None, residuals=None,
                   out: Optional[torch.Tensor] = None):
-    """One launch group: up to four linears in one ``nq_gemv_group_fwd`` (T <= 4) or ``nq_gemm_group_fwd`` call.
+    """One launch group: up to four linears in one ``nq_decode_group_fwd`` (T <= 4) or ``nq_gemm_group_fwd`` call.
 
     ``xs[i]`` ``[T, N_i]`` (row stride free, unit inner stride), ``layers[i] = (s_in, v_tiles, s_mid, u_tiles, s_out, R)``,
     optional ``biases[i]`` ``[M_i]`` and ``residuals[i]`` ``[T, M_i]`` (added in fp32 behind the output scale).  The
@@ -310,13 +311,13 @@ def group_forward(xs, layers, T: int, dtype: torch.dtype, device: torch.device, 
         col += Ms[i]
     arr = (_lib.LinearDesc * n)(*descs)
     gemv = T <= L.nq_gemv_max_tokens()
-    size_fn, fwd = ((L.nq_gemv_group_scratch_bytes, L.nq_gemv_group_fwd) if gemv
+    size_fn, fwd = ((L.nq_gemv_group_scratch_bytes, L.nq_decode_group_fwd) if gemv
                     else (L.nq_gemm_group_scratch_bytes, L.nq_gemm_group_fwd))
     scratch = scratch_for(device, size_fn(arr, n, T))
     with torch.cuda.device(device):
         st = fwd(arr, n, T, _dtype_id(out), scratch.data_ptr(), scratch.numel(),
                  torch.cuda.current_stream(device).cuda_stream)
-    _lib.check(st, "nq_gemv_group_fwd" if gemv else "nq_gemm_group_fwd")
+    _lib.check(st, "nq_decode_group_fwd" if gemv else "nq_gemm_group_fwd")
     return views
 
 
