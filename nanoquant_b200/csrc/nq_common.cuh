@@ -51,12 +51,14 @@ int sm_count();
 // adds 1, with a reduction nobody waits for), so the bits above the span are the same for every CTA of a
 // launch whenever it reads them (fewer than a span's worth of arrivals can precede the read) and differ from
 // those of every recent launch.  Reads and arrivals of a launch must come after the previous launch on the
-// scratch has completed (behind griddepcontrol.wait).  The tag is 0x7FF in its upper 12 bits (a NaN pattern
-// as fp32 and in both halves as fp16 / bf16 pairs, which no kernel that shares the scratch ever stores, and
-// never the 0 of a zeroed scratch) and the launch count modulo 2^20 below; an element is rewritten by every
-// launch that uses its address, so a stale tag can only match after 2^20 launches in a row that leave it
-// alone.  Waits are bounded: on expiry a status word is set and the thread goes on with what it has (the
-// host reports the status).
+// scratch has completed (behind griddepcontrol.wait).
+//
+// The tag (launch_tag) is the launch count modulo 2^20 spread over a NaN pattern that no kernel sharing the scratch stores:
+// its upper half is 0x7FF0..0x7FF7 or 0xFFF0..0xFFF7, in fp32 as in both 16-bit formats a NaN, but not the 0x7FFF that
+// arithmetic and conversions make of one and that a GEMM stage stores for a token with a NaN (nor the 0xFFFF of a negative
+// exponent word, nor the 0 of a zeroed scratch).  An element is rewritten by every launch that uses its address, so a
+// stale tag can only match after 2^20 launches in a row that leave it alone.  Waits are bounded: on expiry a status word is
+// set and the thread goes on with what it has (the host reports the status).
 constexpr unsigned kTagSpan = 1024u;        // > CTAs per tagged launch
 constexpr unsigned kSpinLimit = 4000000u;   // default number of polls before a wait gives up
 struct TagCtx {
@@ -76,8 +78,13 @@ __device__ __forceinline__ void tag_read(TagRaw& r, const unsigned* header) {
     asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(r.counter) : "l"(header) : "memory");
     asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(r.status) : "l"(header + 2) : "memory");
 }
+// Bits 0..18 of the launch count below 0x7FF0'0000, bit 19 as the sign.
+__device__ __forceinline__ unsigned launch_tag(unsigned long long counter) {
+    const unsigned n = (unsigned)(counter / kTagSpan);
+    return 0x7FF00000u | (n & 0x7FFFFu) | ((n << 12) & 0x80000000u);
+}
 __device__ __forceinline__ void tag_finish(TagCtx& tc, const TagRaw& r, unsigned* header, unsigned limit) {
-    tc.tag = 0x7FF00000u | ((unsigned)(r.counter / kTagSpan) & 0xFFFFFu);
+    tc.tag = launch_tag(r.counter);
     tc.limit = r.status ? 0u : limit;
     tc.status = header + 2;
 }

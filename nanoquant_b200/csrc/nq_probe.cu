@@ -33,7 +33,7 @@ __global__ void __launch_bounds__(512, 1) probe_chain_kernel(const __grid_consta
     if (tid < p.n_x16) v = p.x[tid];                       // every CTA reads all of the input
     unsigned long long c;
     asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(c) : "l"(p.counter) : "memory");
-    const unsigned tag = 0x7FF00000u | ((unsigned)(c / kTagSpan) & 0xFFFFFu);
+    const unsigned tag = launch_tag(c);
     float m = __uint_as_float(v.x) + __uint_as_float(v.y) + __uint_as_float(v.z) + __uint_as_float(v.w);
     for (int o = 16; o; o >>= 1) m += __shfl_xor_sync(0xffffffffu, m, o);
     if ((tid & 31) == 0) red[tid >> 5] = m;
