@@ -107,6 +107,22 @@ __device__ __forceinline__ void store_tagged(void* base, long long i, float val,
 }
 
 // ---------------------------------------------------------------------------
+// values that are not finite
+// ---------------------------------------------------------------------------
+// A NaN operand gives NaN (fmaxf and fminf return the other operand and so hide it).
+__device__ __forceinline__ float max_or_nan(float a, float b) {
+    float r;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float min_or_nan(float a, float b) {
+    float r;
+    asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float clamp_or_nan(float v, float lim) { return min_or_nan(max_or_nan(v, -lim), lim); }
+
+// ---------------------------------------------------------------------------
 // mbarriers and bulk copies
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }

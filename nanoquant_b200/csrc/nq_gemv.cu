@@ -136,12 +136,18 @@ __device__ __forceinline__ void quantise_unit(float (&p)[8], unsigned char* xq_c
     const int lane = threadIdx.x & 31, j = lane >> 2;
     float m = 0.f;
 #pragma unroll
-    for (int e = 0; e < 8; ++e) m = fmaxf(m, fabsf(p[e]));
-    m = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(m)));
-    if (!(m > 1e-31f && m < 3.0e38f)) {   // zero (below 1e-31 the reciprocal would overflow) or not finite: zeros
-        m = 1.f;
+    for (int e = 0; e < 8; ++e) m = max_or_nan(m, fabsf(p[e]));
+    m = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(m)));   // as bits: a NaN is above infinity
+    float unit = m * (1.0f / (128.f * kQMax));
+    if (!(m > 1e-31f && m <= 3.4028235e38f)) {
+        const bool tiny = m > 0.f && m <= 1e-31f;       // the reciprocal would overflow: the same integers from p * 2^64
+        // All zero, or not finite.  A value that is not finite makes the unit a NaN, and with it every sum over this
+        // chunk and every output of this token, as the same sums in floating point would be (an infinity meets another of
+        // the opposite sign); left in, its bits would spill into the bytes of neighbouring columns.
+        if (!tiny && m != 0.f) unit = __uint_as_float(0x7FFFFFFFu);
+        m = tiny ? m * 1.8446744e19f : 1.f;
 #pragma unroll
-        for (int e = 0; e < 8; ++e) p[e] = 0.f;
+        for (int e = 0; e < 8; ++e) p[e] = tiny ? p[e] * 1.8446744e19f : 0.f;
     }
     // times 2^(7-j), negative for j = 7 (the A operand of class 7 is -128)
     const float inv_j = kQMax * __frcp_rn(m) * __uint_as_float(j == 7 ? 0xBF800000u : (uint32_t)(127 + 7 - j) << 23);
@@ -169,7 +175,7 @@ __device__ __forceinline__ void quantise_unit(float (&p)[8], unsigned char* xq_c
     }
     int sum = (int)(zsum - 8u * (0x4B400000u + 0x8080u));    // |sum| * 2^j <= 2^25
     sum = __reduce_add_sync(0xffffffffu, j == 7 ? sum * -128 : sum * (1 << j));
-    if (lane == 0) *meta = make_int2(__float_as_int(m * (1.0f / (128.f * kQMax))), sum);
+    if (lane == 0) *meta = make_int2(__float_as_int(unit), sum);
 }
 
 template <int KIND>
@@ -494,7 +500,7 @@ __device__ __forceinline__ void emit_block(const Job& jb, int row0, int nb, int 
                 if (jb.bias) v += to_float<KIND>((uint16_t)raw.bias);
                 if (jb.resid) v += to_float<KIND>((uint16_t)raw.resid);
                 constexpr float lim = KIND == KIND_F16 ? 64504.0f : 3.3895313892515355e+38f;
-                v = fminf(fmaxf(v, -lim), lim);
+                v = clamp_or_nan(v, lim);
                 if (KIND == KIND_F16) static_cast<__half*>(jb.out)[tok * jb.ld_out + row] = __float2half(v);
                 else static_cast<__nv_bfloat16*>(jb.out)[tok * jb.ld_out + row] = __float2bfloat16(v);
             }

@@ -1,0 +1,60 @@
+"""Activations that are not finite, and activations far below one: a token with a NaN or an infinity has NaN in every
+output and leaves the other tokens' bits alone; a token scaled by a power of two gives the scaled result."""
+import pytest
+import torch
+
+from tests.util import assert_parity, exact_np, make_layer, tiles_on_gpu
+
+pytestmark = pytest.mark.gpu
+
+SHAPES = [(520, 136, 96), (4104, 264, 1000), (1003, 333, 77)]
+
+
+def gemv(L, x):
+    """The decode kernel through the C ABI."""
+    from nanoquant_b200 import _lib
+    Lb = _lib.lib()
+    (T, N), R, M = x.shape, L["R"], L["M"]
+    st = torch.cuda.current_stream().cuda_stream
+    nb = Lb.nq_gemv_scratch_bytes(T, N, R, M)
+    scratch = torch.zeros(nb, dtype=torch.uint8, device="cuda")
+    y = torch.empty((T, M), dtype=x.dtype, device="cuda")
+    vt, ut = tiles_on_gpu(L["V"]), tiles_on_gpu(L["U"])
+    _lib.check(Lb.nq_gemv_fwd(x.data_ptr(), L["s_pre"].data_ptr(), vt.data_ptr(), L["s_mid"].data_ptr(), ut.data_ptr(),
+                              L["s_post"].data_ptr(), y.data_ptr(), scratch.data_ptr(), nb, T, N, R, M,
+                              _lib.NQ_BF16 if x.dtype == torch.bfloat16 else _lib.NQ_F16, st), "nq_gemv_fwd")
+    assert Lb.nq_scratch_status(scratch.data_ptr(), st) == 0
+    return y
+
+
+def spoil(x, tok, value):
+    """`value` in two columns of token `tok`, in different chunks of 256 columns."""
+    x = x.clone()
+    x[tok, 7] = value
+    x[tok, x.size(1) - 2] = value
+    return x
+
+
+@pytest.mark.parametrize("value", [float("nan"), float("inf"), float("-inf")])
+@pytest.mark.parametrize("T,dtype", [(1, torch.bfloat16), (2, torch.float16), (3, torch.bfloat16), (4, torch.float16)])
+@pytest.mark.parametrize("N,R,M", SHAPES)
+def test_decode_kernel_not_finite(N, R, M, T, dtype, value):
+    L = make_layer(N, R, M, T, dtype, seed=N + T)
+    clean = gemv(L, L["x"])
+    y = gemv(L, spoil(L["x"], T - 1, value))
+    assert torch.isnan(y[T - 1]).all()
+    assert torch.equal(y[:T - 1], clean[:T - 1])
+
+
+@pytest.mark.parametrize("exponent", [-40, -96, -100, -104])
+@pytest.mark.parametrize("T", [1, 4])
+def test_decode_kernel_small_activations(T, exponent):
+    # products s_in * x from 1e-14 down to 1e-33, whose fixed-point scale has no fp32 reciprocal; the unit of a chunk is
+    # then a subnormal of 18 bits or more, and outputs (1e-34 and above) are normal in bf16
+    N, R, M = 1032, 136, 520
+    L = make_layer(N, R, M, T, torch.bfloat16, seed=5)
+    L["s_mid"] = torch.ones_like(L["s_mid"])
+    from oracle import nanoquant_oracle as oc
+    want = oc.forward_fp64(exact_np(L["x"]), L["V"], L["U"], exact_np(L["s_pre"]), None, exact_np(L["s_post"]))
+    y = gemv(L, L["x"] * 2.0 ** exponent)
+    assert_parity(exact_np(y) * 2.0 ** -exponent, want, torch.bfloat16, rel=1e-4, what=f"2^{exponent}")
