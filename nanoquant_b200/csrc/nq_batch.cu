@@ -308,6 +308,8 @@ __global__ void __launch_bounds__(kBatchThreads, 1) batch_stage_kernel(const __g
         if (++slot == slots) { slot = 0; parity ^= 1u; }
         if (loader) load_block();
         // outputs: lanes take rows, warps take tokens
+        // An intermediate that is not a pair becomes infinite beyond its type's range, as in the GEMM; the value of a pair
+        // stays finite, and it is the remainder that an infinity goes to.  NaN passes every clamp.
         const float lim = P.saturate || (SPLIT && !FRAG) ? (out_bf16 ? 3.3895313892515355e+38f : 64504.0f) : 3.4e38f;
         const uint16_t* const resid = static_cast<const uint16_t*>(jb.resid);
         const int* const row_exp = jb.row_exp;
@@ -334,11 +336,12 @@ __global__ void __launch_bounds__(kBatchThreads, 1) batch_stage_kernel(const __g
                 if (row0 + idx < rows) {
                     float extra = sc.y;
                     if (resid) extra += float_of(resid[tok * jb.ld_res + row0 + idx], io_bf16);
-                    v = fminf(fmaxf(v * (sc.x * rs) + extra, -lim), lim);
+                    const float exact = v * (sc.x * rs) + extra;
+                    v = clamp_or_nan(exact, lim);
                     if (SPLIT && !FRAG) {
                         const __nv_bfloat16 value = __float2bfloat16(v);
                         out[fragment_index<1>(tok, row0 + idx)] = __bfloat16_as_ushort(value);
-                        out[fragment_index<1>(kSplitTokens + tok, row0 + idx)] = __bfloat16_as_ushort(__float2bfloat16(v - __bfloat162float(value)));
+                        out[fragment_index<1>(kSplitTokens + tok, row0 + idx)] = __bfloat16_as_ushort(__float2bfloat16(exact - __bfloat162float(value)));
                         continue;
                     }
                     out[frag_out ? fragment_index<NT>(tok, row0 + idx) : idx] = out_bf16 ? __bfloat16_as_ushort(__float2bfloat16(v)) : __half_as_ushort(__float2half(v));

@@ -120,7 +120,6 @@ struct GemmParams {
     int T;                 // tokens
     int is_bf16;           // type of the scales, bias and residual (the I/O type of the linear)
     int a_bf16;            // type of the MMA operands: activations and expanded weights (bf16, else fp16)
-    int out_bf16;          // type of the output (bf16, else fp16)
     int saturate;          // apply the reference's output saturation bounds
     // bf16 linears keep their rank-R intermediate as fp16 times a per-token power of two (11 significant bits
     // instead of 8): stage 1 multiplies row t by 2^row_exp[t] (exp_sign = +1), stage 2 by 2^-row_exp[t] (-1).
@@ -212,13 +211,16 @@ __device__ __forceinline__ void cluster_store4(uint32_t addr, uint32_t a, uint32
     asm volatile("st.shared::cluster.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
 }
 
+// OUT: conversion of the outputs.  Chosen at run time in the epilogue's loop, the third kind cost 0.7 % of a 517-token layer.
+enum : int { kOutFp16, kOutBf16, kOutBf16Saturated };
+
 // ---------------------------------------------------------------------------
 // the kernel: one 128 x 128 output tile per CTA
 // ---------------------------------------------------------------------------
 // The ", 1" matters: its shared memory allows one CTA per SM anyway, but without the word the compiler saves registers (64
 // instead of 89 for the largest tile) and puts the loads of the expansion and of the epilogue one behind the other.  Layer of
 // 517 tokens 249 -> 244 us, 2048 tokens 720 -> 702, 128 tokens 188 -> 180, eight layers of 64 tokens 876 -> 844.
-template <int MH, int NH>
+template <int MH, int NH, int OUT>
 __global__ void __launch_bounds__(GemmCfg<MH, NH>::kThreads, 1) gemm_stage_kernel(const __grid_constant__ GemmParams P) {
     using C = GemmCfg<MH, NH>;
     constexpr int kGemmStages = C::kStages, kBN = C::kBN, kBitsSlotBytes = C::kBitsSlotBytes;
@@ -494,7 +496,7 @@ __global__ void __launch_bounds__(GemmCfg<MH, NH>::kThreads, 1) gemm_stage_kerne
         // 32-column blocks of the MH accumulators, dealt round-robin to the warps that share a lane quarter
         if (ok) {
             tc_fence_after();
-            const float lim = P.saturate ? (P.out_bf16 ? 3.3895313892515355e+38f : 64504.0f) : 3.4e38f;
+            constexpr float lim = 64504.0f;      // of fp16 outputs
             const float4* post4 = reinterpret_cast<const float4*>(smem + kOffPost);
             // per-token power of two of the intermediate (exact: the exponent is an integer), one load per
             // token and thread ahead of the blocks (inside the loop its latency would repeat for every block)
@@ -551,15 +553,18 @@ __global__ void __launch_bounds__(GemmCfg<MH, NH>::kThreads, 1) gemm_stage_kerne
                     }
                     float v0 = __uint_as_float(r[4 * e4 + 0]) * sc.x + ad.x, v1 = __uint_as_float(r[4 * e4 + 1]) * sc.y + ad.y;
                     float v2 = __uint_as_float(r[4 * e4 + 2]) * sc.z + ad.z, v3 = __uint_as_float(r[4 * e4 + 3]) * sc.w + ad.w;
-                    if (P.out_bf16) {
+                    if (OUT == kOutBf16Saturated) {
                         // the reference's bound for bf16 is the largest finite bf16: the saturating conversion applies it
                         // (this arithmetic, two clamps per output at half rate, was half of a large tile's epilogue)
                         asm("cvt.rn.satfinite.bf16x2.f32 %0, %1, %2;" : "=r"(packed[2 * e4]) : "f"(v1), "f"(v0));
                         asm("cvt.rn.satfinite.bf16x2.f32 %0, %1, %2;" : "=r"(packed[2 * e4 + 1]) : "f"(v3), "f"(v2));
+                    } else if (OUT == kOutBf16) {     // an intermediate keeps its infinities: cut off, they could cancel
+                        asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(packed[2 * e4]) : "f"(v1), "f"(v0));
+                        asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(packed[2 * e4 + 1]) : "f"(v3), "f"(v2));
                     } else {
                         if (P.saturate) {
-                            v0 = fminf(fmaxf(v0, -lim), lim); v1 = fminf(fmaxf(v1, -lim), lim);
-                            v2 = fminf(fmaxf(v2, -lim), lim); v3 = fminf(fmaxf(v3, -lim), lim);
+                            v0 = clamp_or_nan(v0, lim); v1 = clamp_or_nan(v1, lim);
+                            v2 = clamp_or_nan(v2, lim); v3 = clamp_or_nan(v3, lim);
                         }
                         const __half2 a2 = __floats2half2_rn(v0, v1), b2 = __floats2half2_rn(v2, v3);
                         packed[2 * e4] = *reinterpret_cast<const uint32_t*>(&a2);
@@ -709,7 +714,7 @@ struct GroupPlan {
 };
 // The four tile configurations as the host sees them.
 struct KernelInfo {
-    const void* fn;
+    const void* fn[3];   // by kind of output
     size_t smem;
     int threads;
     int pipe_bytes;   // pipeline buffers (activation + weight stages): receive space of a cluster split
@@ -718,7 +723,8 @@ struct KernelInfo {
 template <int MH, int NH>
 static KernelInfo kernel_info_of() {
     using C = GemmCfg<MH, NH>;
-    return {(const void*)gemm_stage_kernel<MH, NH>, (size_t)C::kSmemBytes, C::kThreads, C::kStages * (C::kABytes + C::kWBytes),
+    return {{(const void*)gemm_stage_kernel<MH, NH, kOutFp16>, (const void*)gemm_stage_kernel<MH, NH, kOutBf16>,
+             (const void*)gemm_stage_kernel<MH, NH, kOutBf16Saturated>}, (size_t)C::kSmemBytes, C::kThreads, C::kStages * (C::kABytes + C::kWBytes),
             MH * (C::kBN / 32)};
 }
 static KernelInfo kernel_info(int mh, int nh) {
@@ -736,7 +742,7 @@ static int set_kernel_attributes() {
         for (int mh = 1; mh <= 2; ++mh)
             for (int nh = 1; nh <= 2; ++nh) {
                 const KernelInfo ki = kernel_info(mh, nh);
-                NQ_CUDA_TRY(cudaFuncSetAttribute(ki.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ki.smem));
+                for (const void* fn : ki.fn) NQ_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ki.smem));
             }
         attr_set[dev & 63] = true;
     }
@@ -760,7 +766,7 @@ static int cluster_capacity(int mh, int nh, int s) {
         cfg.attrs = &attr;
         cfg.numAttrs = 1;
         int clusters = 0;
-        if (set_kernel_attributes() != NQ_OK || cudaOccupancyMaxActiveClusters(&clusters, ki.fn, &cfg) != cudaSuccess ||
+        if (set_kernel_attributes() != NQ_OK || cudaOccupancyMaxActiveClusters(&clusters, ki.fn[kOutFp16], &cfg) != cudaSuccess ||
             clusters <= 0) {
             (void)cudaGetLastError();
             clusters = 0;   // this cluster size cannot be launched here: the planner leaves it out
@@ -843,7 +849,6 @@ static int launch_stage(const StageJob* jobs, int n, int T, StageTypes ty, int s
     P.T = T;
     P.is_bf16 = ty.io_bf16;
     P.a_bf16 = ty.a_bf16;
-    P.out_bf16 = ty.out_bf16;
     P.exp_sign = ty.exp_sign;
     P.saturate = saturate;
     P.csplit = pl.csplit;
@@ -875,7 +880,7 @@ static int launch_stage(const StageJob* jobs, int n, int T, StageTypes ty, int s
         P.tile0[j] = pl.tile0[j];
     }
     const KernelInfo ki = kernel_info(mh, nh);
-    const void* fn = ki.fn;
+    const void* fn = ki.fn[!ty.out_bf16 ? kOutFp16 : saturate ? kOutBf16Saturated : kOutBf16];
     const size_t smem_bytes = ki.smem;
     const int threads = ki.threads;
     // Programmatic stream serialization lets this grid start while the previous kernel of the stream drains

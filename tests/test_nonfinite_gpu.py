@@ -58,3 +58,40 @@ def test_decode_kernel_small_activations(T, exponent):
     want = oc.forward_fp64(exact_np(L["x"]), L["V"], L["U"], exact_np(L["s_pre"]), None, exact_np(L["s_post"]))
     y = gemv(L, L["x"] * 2.0 ** exponent)
     assert_parity(exact_np(y) * 2.0 ** -exponent, want, torch.bfloat16, rel=1e-4, what=f"2^{exponent}")
+
+
+def dispatched(L, x, resid=None, precise=False):
+    """A launch group of one, as the module calls it."""
+    from nanoquant_b200 import ops
+    tens = [(L["s_pre"], tiles_on_gpu(L["V"]), L["s_mid"], tiles_on_gpu(L["U"]), L["s_post"], L["R"])]
+    old = ops.set_precise_intermediate(precise)
+    try:
+        return ops.group_forward([x], tens, x.size(0), x.dtype, x.device, [None], None if resid is None else [resid])[0]
+    finally:
+        ops.set_precise_intermediate(old)
+
+
+# four tokens of a linear large enough for the pair of bf16 words; batch kernel at one and three column groups; GEMM with
+# the K split over a cluster and without
+@pytest.mark.parametrize("value", [float("nan"), float("inf")])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("T,N,R,M", [(1, 520, 136, 96), (4, 4104, 1032, 8000), (8, 520, 136, 96), (20, 1032, 264, 1000),
+                                     (40, 520, 136, 96), (300, 1032, 264, 8200)])
+def test_dispatch_not_finite(T, N, R, M, dtype, value):
+    L = make_layer(N, R, M, T, dtype, seed=N + T)
+    bad = spoil(L["x"], T - 1, value)
+    for precise in ((False, True) if T > 4 and dtype == torch.bfloat16 else (False,)):
+        clean = dispatched(L, L["x"], precise=precise)
+        y = dispatched(L, bad, precise=precise)
+        assert torch.isnan(y[T - 1]).all()
+        assert torch.equal(y[:T - 1], clean[:T - 1]) and torch.isfinite(clean).all()
+    # a residual that is not finite belongs to its element
+    resid = torch.zeros(T, M, dtype=dtype, device="cuda")
+    resid[0, 1] = value
+    y = dispatched(L, L["x"], resid)
+    bound = 64512.0 if dtype == torch.float16 else torch.finfo(dtype).max      # 64504 as fp16
+    assert torch.isnan(y[0, 1]) if value != value else y[0, 1].item() == bound
+    y[0, 1] = 0
+    clean = dispatched(L, L["x"], torch.zeros_like(resid))
+    clean[0, 1] = 0
+    assert torch.equal(y, clean)
