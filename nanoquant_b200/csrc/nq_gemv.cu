@@ -29,9 +29,9 @@
 // linears that share the two phases (q/k/v, gate/up) are processed in one launch.
 // There is no device-wide barrier between the phases: every element of t is stored
 // together with a tag of the launch and phase 2 polls the elements it needs until
-// they carry this launch's tag (nq_common.cuh).  A CTA that polls in vain computes the missing rows itself, so no wait
-// depends on CTAs that are not running (help_phase1); beyond that the poll is bounded: on expiry a status word is set and
-// the thread goes on.  The launch has programmatic stream serialization: the weight loads of both phases are started
+// they carry this launch's tag (nq_common.cuh).  A CTA that polls in vain computes the missing rows itself, once, so no wait
+// depends on CTAs that are not running (help_phase1); what a thread polls in vain in a launch is bounded all the same (two
+// launches that share a scratch by mistake overwrite each other's tags): then a status word is set and the thread goes on.  The launch has programmatic stream serialization: the weight loads of both phases are started
 // before griddepcontrol.wait.
 //
 // Measured against the first versions of this kernel (cooperative launch, one scale per token, partial sums added with
@@ -71,7 +71,8 @@ constexpr size_t kPartBytes = 32 << 10;    // partial sums of a row block
 constexpr size_t kSlotBytes = 64 << 10;    // weights of a row block
 constexpr unsigned kWeightWaitLimit = 1u << 20;   // attempts of up to ~2 us each
 constexpr unsigned kPollBackoffNs = 100;   // pause between two polls of the tagged intermediate (20: equal, 300: slower)
-constexpr unsigned kHelpAfter = 256;       // polls (about 0.1 ms) before a CTA helps
+constexpr unsigned kHelpAfter = 256;       // polls (about 0.1 ms) before a CTA helps; 1/16 of the limit where that is less,
+                                           // never with a limit below 16
 
 enum : int { KIND_F16 = 0, KIND_BF16 = 1 };
 
@@ -98,8 +99,8 @@ static_assert(sizeof(Job) == 128 && offsetof(Job, cta0) == 88, "cta0..g_r are re
 
 struct alignas(16) GemvParams {
     Job job[2 * kMaxJobs];  // phase 1, phase 2
-    unsigned* header;       // [0..1] 64-bit arrival counter (launch tags), [2] status
-    unsigned spin_limit;    // polls before a wait for the tagged intermediate gives up
+    unsigned* header;       // [0..1] 64-bit arrival counter (launch tags), [2] status, [3] CTAs that have helped
+    unsigned spin_limit;    // polls in vain before a thread gives the tagged intermediate up
     unsigned help_after;    // polls before a CTA computes missing rows of the intermediate itself
     int T;
     int slots, slot_bytes;  // weight blocks in shared memory
@@ -273,7 +274,8 @@ __device__ __noinline__ void quantise_x_any(const Job& jb, int T, unsigned char*
 }
 // Phase 2: the tagged intermediate, polled until every element of a share's chunk (MT tokens at most) carries this
 // launch's tag.  Every element is one 64-bit word {value, tag}: a 64-bit access is single-copy atomic, so a matching
-// tag implies its value.  Returns false (for the whole warp) after `help_after` polls in vain.
+// tag implies its value.  Returns false (for the whole warp) after `help_after` polls in vain for one element, and goes
+// on without the data when the launch's limit is spent.
 template <int MT>
 __device__ __forceinline__ bool quantise_t(const Job& jb, int T, unsigned char* xq, int2* meta, TagCtx& tc, unsigned help_after) {
     constexpr int B = MT > 2 ? 2 : MT;       // tokens whose loads are in flight together
@@ -321,7 +323,8 @@ __device__ __forceinline__ bool quantise_t(const Job& jb, int T, unsigned char* 
                         }
                 }
                 if (__all_sync(0xffffffffu, wrong == 0u)) break;
-                if (spins >= tc.limit) { tag_wait_expired(tc); break; }   // the same in every lane
+                if (tc.limit == 0u) { tag_wait_expired(tc); break; }      // the same in every lane
+                --tc.limit;
                 if (spins >= help_after) return false;
                 __nanosleep(kPollBackoffNs);   // failed polls of 148 CTAs load the L2 lines the producers are storing to
             }
@@ -511,10 +514,12 @@ __device__ __forceinline__ void emit_block(const Job& jb, int row0, int nb, int 
 // Phase 1 of a job for every CTA whose rows are not there yet: called by a CTA that has polled in vain for a while.  The
 // missing CTAs may not be running (other work holds their SMs), so a wait must not depend on them: this makes the
 // launch finish however few of its CTAs run at a time, without the cooperative attribute (which cost 0.5 us per launch in
-// a graph and 3 us in a stream).  A row computed twice is written with the same bits.
+// a graph and 3 us in a stream).  A row computed twice is written with the same bits.  The header counts the helpers.
 template <int KIND, int CG>
-__device__ __noinline__ void help_phase1(const Job& jb, int T, unsigned char* xq, int2* meta, float* part, unsigned tag) {
+__device__ __noinline__ void help_phase1(const Job& jb, int T, unsigned char* xq, int2* meta, float* part, unsigned tag,
+                                         unsigned* helpers) {
     const int tid = threadIdx.x;
+    if (tid == 0) atomicAdd(helpers, 1u);
     const Slice sl = slice_of(jb);
     bool have_input = false;
     for (int k = 0; k < jb.ncta; ++k) {
@@ -593,7 +598,7 @@ __global__ void __launch_bounds__(kGemvThreads, 1) gemv_group_kernel(const __gri
     unsigned char* xq = smem + P.xq_off;
     float* part = reinterpret_cast<float*>(smem + P.part_off);
     unsigned* const header = P.header;
-    const unsigned help_after = P.help_after;
+    unsigned help_after = P.help_after;
     // This CTA's job in each phase and its row groups of it: every job has a contiguous range of CTAs of its own, so a
     // CTA prepares the input of one job per phase.
     int first[2], groups[2], ji[2];
@@ -659,8 +664,10 @@ __global__ void __launch_bounds__(kGemvThreads, 1) gemv_group_kernel(const __gri
             tag_finish(tc, tag_raw, header, P.spin_limit);
         } else if (my_groups > 0) {
             load_raw_out(raw0, jb, row0, min(jb.gb, my_groups) * 16, T, tid >> 2);
-            while (!__syncthreads_and(quantise_t<2 * CG>(jb, T, xq, meta, tc, help_after)))
-                help_phase1<KIND, CG>(jobs[ji[1] - kMaxJobs], T, xq, meta, part, tc.tag);
+            while (!__syncthreads_and(quantise_t<2 * CG>(jb, T, xq, meta, tc, help_after))) {
+                help_phase1<KIND, CG>(jobs[ji[1] - kMaxJobs], T, xq, meta, part, tc.tag, header + 3);
+                help_after = ~0u;     // every row has carried the tag now: what is missing again, another launch overwrites
+            }
         }
 #pragma unroll 1
         for (int blk = 0; blk < my_groups; blk += jb.gb) {
@@ -789,7 +796,7 @@ static int launch_two_stages(const nq_linear_desc* d, int n, int t0, int T, int 
     return st != NQ_OK ? st : launch_batch_stage(s2, n, T, StageTypes{b16, 1, b16, 0}, 1, true, false, true, status, stream);
 }
 
-static unsigned g_spin_limit = kSpinLimit;   // polls before a wait for the tagged intermediate gives up
+static unsigned g_spin_limit = kSpinLimit;   // polls in vain before a thread gives the tagged intermediate up
 
 }  // namespace nq
 
@@ -848,7 +855,7 @@ static int gemv_group(const nq_linear_desc* d, int n_linears, int T, int dtype, 
     memset(&P, 0, sizeof(P));
     P.header = static_cast<unsigned*>(scratch);
     P.spin_limit = g_spin_limit;
-    P.help_after = g_spin_limit / 16 < kHelpAfter ? g_spin_limit / 16 : kHelpAfter;
+    P.help_after = g_spin_limit < 16 ? ~0u : g_spin_limit / 16 < kHelpAfter ? g_spin_limit / 16 : kHelpAfter;
 
     // One CTA per SM, fewer for launches with less than 3 MB of packed factors (the o projection of an 8B-class layer and
     // everything smaller): their row groups do not divide any finer by 148, and every CTA fetches the whole input and polls

@@ -39,6 +39,35 @@ def test_gemv_wait_for_a_stale_intermediate_expires():
         assert Lb.nq_gemv_set_wait_limit(old) == 64
 
 
+def test_gemv_wait_that_runs_out():
+    # Four row groups of 128 chunks each: four CTAs produce the intermediate while the others poll for it from the start.
+    # With a limit of one poll in vain, too small for a CTA to help, their wait runs out long before the rows are there.
+    from nanoquant_b200 import _lib
+    Lb = _lib.lib()
+    T, N, R, M = 1, 32768, 64, 4096
+    L = make_layer(N, R, M, T, torch.float16, seed=3)
+    vt, ut = tiles_on_gpu(L["V"]), tiles_on_gpu(L["U"])
+    st = torch.cuda.current_stream().cuda_stream
+    nb = Lb.nq_gemv_scratch_bytes(T, N, R, M)
+    scratch = torch.zeros(nb, dtype=torch.uint8, device="cuda")
+    y = torch.empty(T, M, dtype=torch.float16, device="cuda")
+    args = (L["x"].data_ptr(), L["s_pre"].data_ptr(), vt.data_ptr(), L["s_mid"].data_ptr(), ut.data_ptr(),
+            L["s_post"].data_ptr(), y.data_ptr(), scratch.data_ptr(), nb, T, N, R, M, _lib.NQ_F16, st)
+    old = Lb.nq_gemv_set_wait_limit(1)
+    try:
+        _lib.check(Lb.nq_gemv_fwd(*args), "nq_gemv_fwd")
+        assert Lb.nq_scratch_status(scratch.data_ptr(), st) == _lib.NQ_ERR_TIMEOUT
+        assert scratch.view(torch.int32)[3].item() == 0                 # nobody helped
+    finally:
+        Lb.nq_gemv_set_wait_limit(old)
+    _lib.check(Lb.nq_gemv_fwd(*args), "nq_gemv_fwd")
+    assert Lb.nq_scratch_status(scratch.data_ptr(), st) == _lib.NQ_ERR_TIMEOUT     # stays until the scratch is zeroed
+    scratch.zero_()
+    _lib.check(Lb.nq_gemv_fwd(*args), "nq_gemv_fwd")
+    assert Lb.nq_scratch_status(scratch.data_ptr(), st) == 0
+    assert_parity(exact_np(y), L["y64"], torch.float16, what="after re-zeroing")
+
+
 def test_allgather_wait_for_an_absent_peer_expires():
     # world = 2 on one GPU, both "ranks" pointing at this process's buffer; slot 1's flag is never written, so the
     # wait for rank 1 runs out: the kernel returns, the status says so, and after re-zeroing a world of 1 works.

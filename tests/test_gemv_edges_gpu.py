@@ -26,7 +26,7 @@ def _run(L, T, N, R, M, dtype):
     torch.cuda.synchronize()
     assert Lb.nq_scratch_status(scratch.data_ptr(), st) == 0
     assert torch.equal(first, y)
-    return y
+    return y, scratch.view(torch.int32)[3].item()       # result, number of CTAs that computed others' rows
 
 
 @pytest.mark.parametrize("T", [1, 2, 3, 4])
@@ -39,22 +39,27 @@ def _run(L, T, N, R, M, dtype):
 def test_tile_edges(N, R, M, T):
     dtype = torch.bfloat16 if T % 2 or N < 200 else torch.float16     # (eight columns: outputs below fp16's normal range)
     L = make_layer(N, R, M, T, dtype, seed=N + R + M)
-    y = _run(L, T, N, R, M, dtype)
+    y, _ = _run(L, T, N, R, M, dtype)
     assert_parity(exact_np(y), L["y64"], dtype, what=f"N={N} R={R} M={M} T={T}")
 
 
 @pytest.mark.parametrize("T", [1, 4])
-@pytest.mark.parametrize("N,R,M", [(1003, 333, 777), (4096, 608, 1024)])
+@pytest.mark.parametrize("N,R,M", [(1003, 333, 777), (4096, 608, 1024), (32768, 64, 4096)])
 def test_rows_polled_for_in_vain_are_computed(N, R, M, T):
     # a short wait limit makes a CTA compute the other CTAs' rows soon after its first failed poll: same bits
     from nanoquant_b200 import _lib
     Lb = _lib.lib()
     L = make_layer(N, R, M, T, torch.float16, seed=7)
-    want = _run(L, T, N, R, M, torch.float16)
-    # help comes after 1/16 of the limit: after the first poll, with time enough for the helper's own check of every row
+    want, _ = _run(L, T, N, R, M, torch.float16)
+    # help comes after 1/16 of the limit: after the second poll in vain
     old = Lb.nq_gemv_set_wait_limit(31)
     try:
+        helpers = 0
         for _ in range(4):
-            assert torch.equal(_run(L, T, N, R, M, torch.float16), want)
+            y, h = _run(L, T, N, R, M, torch.float16)
+            assert torch.equal(y, want)
+            helpers += h
+        # four row groups of 128 chunks: most CTAs have no row of the intermediate and poll while four compute it
+        assert helpers > 0 or N != 32768
     finally:
         Lb.nq_gemv_set_wait_limit(old)
