@@ -211,9 +211,9 @@ size_t nq_gemv_static_max_rank(void);
  * nq_gemv_fwd_static on the current device. */
 int nq_scratch_status(const void* scratch, nq_stream_t stream);
 
-/* Number of polls in vain a thread may spend on the tagged intermediate in one launch, over all its waits,
- * before it gives up and sets the status word (after an expiry it does not spin again).  Well before that, after
- * 256 polls or a sixteenth of the limit if that is less, a block computes the missing rows itself, once per launch,
+/* Number of polls a wait for the tagged intermediate may spend before it gives up and sets the status word
+ * (per thread and launch: after its first expiry a thread does not spin again).  Well before that, after 256 polls
+ * or a sixteenth of the limit if that is less, a block computes the missing rows itself, once per launch,
  * and adds one to the 32-bit word at byte 12 of the scratch header; with a limit below 16 it never does.
  * 0 restores the default (4e6, seconds).  Host-side setting read at launch time;
  * returns the previous value.  For failure-path tests and for callers that want a

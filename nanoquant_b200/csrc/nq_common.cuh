@@ -63,8 +63,8 @@ constexpr unsigned kTagSpan = 1024u;        // > CTAs per tagged launch
 constexpr unsigned kSpinLimit = 4000000u;   // default number of polls before a wait gives up
 struct TagCtx {
     unsigned tag;        // tag of this launch
-    unsigned limit;      // polls in vain that this thread may still spend in this launch, over all its waits; 0 after an
-                         // expiry (sticky: one missing producer costs every thread one limit, not one per element)
+    unsigned limit;      // polls a wait of this thread may spend; 0 after an expiry (sticky: one missing
+                         // producer costs every thread one limit, not one limit per element it waits for)
     unsigned* status;    // device status word (header word 2)
 };
 // The launch counter and the status word of the scratch header as they are read: issue the read with the first data

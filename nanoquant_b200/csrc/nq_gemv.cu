@@ -30,9 +30,9 @@
 // There is no device-wide barrier between the phases: every element of t is stored
 // together with a tag of the launch and phase 2 polls the elements it needs until
 // they carry this launch's tag (nq_common.cuh).  A CTA that polls in vain computes the missing rows itself, once, so no wait
-// depends on CTAs that are not running (help_phase1); what a thread polls in vain in a launch is bounded all the same (two
-// launches that share a scratch by mistake overwrite each other's tags): then a status word is set and the thread goes on.  The launch has programmatic stream serialization: the weight loads of both phases are started
-// before griddepcontrol.wait.
+// depends on CTAs that are not running (help_phase1).  From then on only the poll limit ends a wait (two launches that share
+// a scratch by mistake overwrite each other's tags): a status word is set and the thread goes on.  The launch has
+// programmatic stream serialization: the weight loads of both phases are started before griddepcontrol.wait.
 //
 // Measured against the first versions of this kernel (cooperative launch, one scale per token, partial sums added with
 // shared-memory atomics, weights by cp.async per warp): Qwen3-8B decode, eight layers in a graph, one token 291 -> 250 us,
@@ -100,7 +100,7 @@ static_assert(sizeof(Job) == 128 && offsetof(Job, cta0) == 88, "cta0..g_r are re
 struct alignas(16) GemvParams {
     Job job[2 * kMaxJobs];  // phase 1, phase 2
     unsigned* header;       // [0..1] 64-bit arrival counter (launch tags), [2] status, [3] CTAs that have helped
-    unsigned spin_limit;    // polls in vain before a thread gives the tagged intermediate up
+    unsigned spin_limit;    // polls before a wait for the tagged intermediate gives up
     unsigned help_after;    // polls before a CTA computes missing rows of the intermediate itself
     int T;
     int slots, slot_bytes;  // weight blocks in shared memory
@@ -275,7 +275,7 @@ __device__ __noinline__ void quantise_x_any(const Job& jb, int T, unsigned char*
 // Phase 2: the tagged intermediate, polled until every element of a share's chunk (MT tokens at most) carries this
 // launch's tag.  Every element is one 64-bit word {value, tag}: a 64-bit access is single-copy atomic, so a matching
 // tag implies its value.  Returns false (for the whole warp) after `help_after` polls in vain for one element, and goes
-// on without the data when the launch's limit is spent.
+// on without the data when the limit is spent.
 template <int MT>
 __device__ __forceinline__ bool quantise_t(const Job& jb, int T, unsigned char* xq, int2* meta, TagCtx& tc, unsigned help_after) {
     constexpr int B = MT > 2 ? 2 : MT;       // tokens whose loads are in flight together
@@ -323,8 +323,7 @@ __device__ __forceinline__ bool quantise_t(const Job& jb, int T, unsigned char* 
                         }
                 }
                 if (__all_sync(0xffffffffu, wrong == 0u)) break;
-                if (tc.limit == 0u) { tag_wait_expired(tc); break; }      // the same in every lane
-                --tc.limit;
+                if (spins >= tc.limit) { tag_wait_expired(tc); break; }   // the same in every lane
                 if (spins >= help_after) return false;
                 __nanosleep(kPollBackoffNs);   // failed polls of 148 CTAs load the L2 lines the producers are storing to
             }
@@ -796,7 +795,7 @@ static int launch_two_stages(const nq_linear_desc* d, int n, int t0, int T, int 
     return st != NQ_OK ? st : launch_batch_stage(s2, n, T, StageTypes{b16, 1, b16, 0}, 1, true, false, true, status, stream);
 }
 
-static unsigned g_spin_limit = kSpinLimit;   // polls in vain before a thread gives the tagged intermediate up
+static unsigned g_spin_limit = kSpinLimit;   // polls before a wait for the tagged intermediate gives up
 
 }  // namespace nq
 
