@@ -176,10 +176,12 @@ int nq_gemv_fwd(const void* x, const void* s_in, const void* v_tiles, const void
 int nq_gemv_group_fwd(const nq_linear_desc* linears_host, int n_linears, int T, int dtype,
                       void* scratch, size_t scratch_bytes, nq_stream_t stream);
 
-/* nq_gemv_group_fwd as the dispatchers call it: large groups of four tokens run as two launches with a matrix
- * instruction over 16-bit floats, the intermediate kept as two bf16 words per element (16 significant bits, like the
- * fixed point of the GEMV).  Same arguments, scratch and accuracy; the results differ from nq_gemv_fwd's in the
- * last bits. */
+/* nq_gemv_group_fwd as the dispatchers call it: four tokens of a linear with N > 3328 (N, R and ldx multiples of 8, x and
+ * s_in 16-byte aligned, R >= 128) run as two launches with a matrix instruction over 16-bit floats, the intermediate kept
+ * as two bf16 words per element (16 significant bits, like the fixed point of the GEMV).  Same arguments, scratch and
+ * accuracy.  The route is a property of the linear: alone or in a group, whose other linears may take the other route, it
+ * has the same bits.  At four tokens these differ from nq_gemv_fwd's, and from those of the same token in a call of one
+ * to three, in the last bits.  T > 4: four at a time, the rest as nq_gemv_group_fwd. */
 int nq_decode_group_fwd(const nq_linear_desc* linears_host, int n_linears, int T, int dtype,
                         void* scratch, size_t scratch_bytes, nq_stream_t stream);
 

@@ -765,34 +765,44 @@ static int static_scratch_ptr(void** out) {
 // {fp32, tag} words of a linear's intermediate, rows padded to eight elements
 static size_t intermediate_bytes(int R) { return round_up((size_t)kMaxTok * (size_t)((R + 7) / 8 * 8) * sizeof(uint2), 256); }
 
-// Tokens [t0, t0 + T) of a group by the batch kernel's two launches, or NQ_ERR_UNSUPPORTED.  Every CTA of the decode kernel
-// converts the whole input and the whole intermediate of its linear to fixed point, and at four tokens that is the largest
-// part of a launch; the batch kernel takes 16-bit floats as they come, with the intermediate as value and remainder, at eight
-// columns of which it computes all anyway.  Eight layers of an 8B-class model in a graph: 421 -> 359 us; three tokens take
-// 363 in one launch each and 361 in two, and stay.  The line: from 20 chunks of input and intermediate on (N + R about 5000)
-// the conversion is worth the second launch.  Below, and below 1 MB of factors, a call in a stream is bound by the host, which
-// pays some 5 us for it (a 1B-class layer of 2048 columns: 143 us per four layers, 163 with two launches throughout, 137
-// by this rule).
-constexpr int kTwoStageChunks = 20;
-constexpr size_t kTwoStageBytes = (size_t)1 << 20;
-static int launch_two_stages(const nq_linear_desc* d, int n, int t0, int T, int dtype, void* scratch, cudaStream_t stream) {
+// Four tokens of a linear by the batch kernel's two launches instead of one of the decode kernel.  Every CTA of the
+// decode kernel converts the whole input and the whole intermediate of its linear to fixed point, and at four tokens that
+// is the largest part of a launch; the batch kernel takes 16-bit floats as they come, with the intermediate as value and
+// remainder, at eight columns of which it computes all anyway.  (Three tokens measured level and stay.)
+//
+// The rule looks at the linear alone, so that a module and a launch group give it the same bits, and at the size that the
+// linears of a group share, so that a group is not torn apart.  The line: input of 14 chunks and more (above 3328
+// columns).  us at four tokens, 0.8 bits per weight, one launch -> two:
+//                                    2048 columns       3072              3584              4096              8192
+//   q/k/v, in a graph                6.6 -> 5.9        8.5 -> 6.5        9.2 -> 7.2       10.1 -> 7.9       17.4 -> 17.3
+//   gate/up, in a graph              9.3 -> 7.6       11.5 -> 11.2      13.9 -> 13.8      15.4 -> 16.4      39.5 -> 48.3
+//   square linear alone, in a graph  6.7 -> 6.1        8.4 -> 6.2        9.0 -> 6.5        9.5 -> 6.6       15.7 -> 13.2
+//   square linear called eagerly     6.8 -> 8.5        8.5 -> 8.6        9.4 -> 9.1        9.8 -> 8.9       15.9 -> 13.5
+//   its quarter (k) called eagerly   6.3 -> 8.4        6.6 -> 8.5        7.1 -> 8.4        7.2 -> 8.6       11.0 -> 8.7
+// A graph gains from 2048 columns on, but a call in a stream is bound by the host there, which pays 2.3 us for the second
+// launch; from 3584 on the seven linears of a layer gain called one by one as well, though not the smallest of them.  Groups
+// of more than some 9 MB of factors lose (gate/up at 8192 columns), because the batch kernel computes all eight columns:
+// that is the price of a rule that does not see the group.
+constexpr int kTwoStageChunks = 14;
+static bool takes_two_stages(const nq_linear_desc& L) {
+    return (L.N + 255) / 256 >= kTwoStageChunks && L.N % 8 == 0 && L.R % 8 == 0 && L.ldx % 8 == 0 && aligned16(L.x) &&
+           aligned16(L.s_in) && batch_fragment_bytes(2 * kSplitTokens, L.R) <= intermediate_bytes(L.R);   // (ranks from 128)
+}
+static int launch_two_stages(const nq_linear_desc* d, int n, int t0, int dtype, void* scratch, cudaStream_t stream) {
     StageJob s1[kMaxJobs], s2[kMaxJobs];
     size_t off = kHeaderBytes;
     for (int i = 0; i < n; ++i) {
         const nq_linear_desc& L = d[i];
-        if (L.N % 8 || L.R % 8 || L.ldx % 8 || !aligned16(L.x) || !aligned16(L.s_in)) return NQ_ERR_UNSUPPORTED;
-        if (batch_fragment_bytes(2 * kSplitTokens, L.R) > intermediate_bytes(L.R)) return NQ_ERR_UNSUPPORTED;   // ranks below 128
         void* t = static_cast<char*>(scratch) + off;
         off += intermediate_bytes(L.R);
         s1[i] = {static_cast<const uint16_t*>(L.x) + (size_t)t0 * L.ldx, L.ldx, L.v_tiles, L.s_in, L.s_mid, t, L.R, L.N, L.R, nullptr, nullptr, 0, nullptr};
         s2[i] = {t, L.R, L.u_tiles, nullptr, L.s_out, static_cast<uint16_t*>(L.y) + (size_t)t0 * L.ldy, L.ldy, L.R, L.M, L.bias,
                  L.residual ? static_cast<const uint16_t*>(L.residual) + (size_t)t0 * L.ldr : nullptr, L.ldr, nullptr};
     }
-    if (T > batch_max_tokens(s1, n) || T > batch_max_tokens(s2, n)) return NQ_ERR_UNSUPPORTED;
     const int b16 = dtype == NQ_BF16;
     unsigned* status = static_cast<unsigned*>(scratch) + 2;
-    const int st = launch_batch_stage(s1, n, T, StageTypes{b16, b16, 1, 0}, 0, false, true, true, status, stream);
-    return st != NQ_OK ? st : launch_batch_stage(s2, n, T, StageTypes{b16, 1, b16, 0}, 1, true, false, true, status, stream);
+    const int st = launch_batch_stage(s1, n, kSplitTokens, StageTypes{b16, b16, 1, 0}, 0, false, true, true, status, stream);
+    return st != NQ_OK ? st : launch_batch_stage(s2, n, kSplitTokens, StageTypes{b16, 1, b16, 0}, 1, true, false, true, status, stream);
 }
 
 static unsigned g_spin_limit = kSpinLimit;   // polls before a wait for the tagged intermediate gives up
@@ -818,18 +828,13 @@ size_t nq_gemv_group_scratch_bytes(const nq_linear_desc* d, int n_linears, int T
     return b;
 }
 
-static int gemv_group(const nq_linear_desc* d, int n_linears, int T, int dtype, void* scratch, size_t scratch_bytes,
-                      bool two_stages, nq_stream_t stream) {
+static int check_group(const nq_linear_desc* d, int n_linears, int T, int dtype, const void* scratch, size_t scratch_bytes) {
     if (!d || !scratch) return NQ_ERR_NULL;
     if (n_linears <= 0 || n_linears > kMaxJobs) return NQ_ERR_UNSUPPORTED;
     if (T <= 0) return NQ_ERR_SHAPE;
     if (dtype != NQ_F16 && dtype != NQ_BF16) return NQ_ERR_DTYPE;
     if (!aligned16(scratch)) return NQ_ERR_ALIGN;
     if (scratch_bytes < nq_gemv_group_scratch_bytes(d, n_linears, T)) return NQ_ERR_SCRATCH;
-
-    int max_chunks = 0, most_conversion = 0;   // chunks of a phase, of both phases of a linear
-    int rg[2][kMaxJobs], ck[2][kMaxJobs];      // row groups and chunks of the two phases
-    size_t packed = 0;
     for (int i = 0; i < n_linears; ++i) {
         const nq_linear_desc& L = d[i];
         if (!L.x || !L.s_in || !L.v_tiles || !L.u_tiles || !L.s_out || !L.y) return NQ_ERR_NULL;
@@ -838,11 +843,21 @@ static int gemv_group(const nq_linear_desc* d, int n_linears, int T, int dtype, 
         if (L.residual && L.ldr < L.M) return NQ_ERR_SHAPE;
         if (L.N > kMaxK || L.R > kMaxK) return NQ_ERR_UNSUPPORTED;
         if (!aligned16(L.v_tiles) || !aligned16(L.u_tiles)) return NQ_ERR_ALIGN;
+    }
+    return NQ_OK;
+}
+
+// Tokens [t_first, T) of a group that check_group has passed, by the decode kernel.
+static int launch_decode(const nq_linear_desc* d, int n_linears, int t_first, int T, int dtype, void* scratch, nq_stream_t stream) {
+    int max_chunks = 0;
+    int rg[2][kMaxJobs], ck[2][kMaxJobs];      // row groups and chunks of the two phases
+    size_t packed = 0;
+    for (int i = 0; i < n_linears; ++i) {
+        const nq_linear_desc& L = d[i];
         rg[0][i] = (L.R + 15) / 16; ck[0][i] = (L.N + 255) / 256;
         rg[1][i] = (L.M + 15) / 16; ck[1][i] = (L.R + 255) / 256;
         for (int ph = 0; ph < 2; ++ph) max_chunks = ck[ph][i] > max_chunks ? ck[ph][i] : max_chunks;
         packed += (size_t)L.R * ((size_t)L.N + L.M) / 8;
-        most_conversion = ck[0][i] + ck[1][i] > most_conversion ? ck[0][i] + ck[1][i] : most_conversion;
     }
     int dev = 0, smem_limit = 0;
     NQ_CUDA_TRY(cudaGetDevice(&dev));
@@ -856,10 +871,14 @@ static int gemv_group(const nq_linear_desc* d, int n_linears, int T, int dtype, 
     P.spin_limit = g_spin_limit;
     P.help_after = g_spin_limit < 16 ? ~0u : g_spin_limit / 16 < kHelpAfter ? g_spin_limit / 16 : kHelpAfter;
 
-    // One CTA per SM, fewer for launches with less than 3 MB of packed factors (the o projection of an 8B-class layer and
-    // everything smaller): their row groups do not divide any finer by 148, and every CTA fetches the whole input and polls
-    // the whole intermediate.  Measured on Qwen3-8B at one token: all SMs 255, 7/10 of them 250, half of them 267 us per
-    // eight layers; with 7/8 for up to 20 MB 254.
+    // One CTA per SM, fewer for launches with less than 3 MB of packed factors: their row groups do not divide any finer by
+    // 148, and every CTA fetches the whole input and polls the whole intermediate.  One token, us per launch in a graph by
+    // CTAs (52 / 74 / 103 / 148):
+    //   0.4 MB (4096 -> 1024)  5.0 / 5.1 / 5.1 / 5.1      2.3 MB (q/k/v of 4096)          6.8 / 6.5 / 6.3 / 6.6
+    //   1.6 MB (4096 -> 4096)  5.9 / 6.0 / 6.0 / 6.2      3.9 MB (gate/up of 2048)        9.7 / 7.7 / 7.3 / 7.1
+    //   1.7 MB (3072 -> 3072)  6.2 / 6.0 / 6.7 / 7.0      4.8 MB (12288 -> 4096)         10.7 / 10.3 / 9.4 / 8.7
+    // Below 3 MB 7/10 of the SMs are within 5 % of the best of these but for a few sizes (a square linear of 3072 columns;
+    // of 2048 at two tokens, 5.3 at 74 CTAs and 6.1 here).
     int grid = sm_count() < kMaxCtas ? sm_count() : kMaxCtas;
     if (packed < ((size_t)3 << 20)) grid = grid * 7 / 10;
     {   // no more CTAs than the larger phase has row groups
@@ -871,7 +890,7 @@ static int gemv_group(const nq_linear_desc* d, int n_linears, int T, int dtype, 
     }
     // tokens are processed in groups that fit the MMA columns (3 per token) and shared memory: the quantised input,
     // one row group's weights and its partial sums at least
-    int tg = T < kMaxTok ? T : kMaxTok;
+    int tg = T - t_first < kMaxTok ? T - t_first : kMaxTok;
     auto fixed_bytes = [&](int t) { return kFixedBytes + (size_t)3 * t * max_chunks * 256; };
     const size_t least = (size_t)max_chunks * 512, least_part = (size_t)max_chunks * (16 + 8) * 4;   // part: per token
     while (tg > 1 && fixed_bytes(tg) + least + tg * least_part > (size_t)smem_limit) --tg;
@@ -881,13 +900,8 @@ static int gemv_group(const nq_linear_desc* d, int n_linears, int T, int dtype, 
     for (int ph = 0; ph < 2; ++ph) deal_ctas(grid, n_linears, rg[ph], ck[ph], cta_n[ph]);
 
     const size_t esz = 2;
-    for (int t0 = 0; t0 < T; t0 += tg) {
+    for (int t0 = t_first; t0 < T; t0 += tg) {
         const int tn = (T - t0) < tg ? (T - t0) : tg;
-        if (two_stages && tn == kSplitTokens && most_conversion >= kTwoStageChunks && packed >= kTwoStageBytes) {
-            const int st = launch_two_stages(d, n_linears, t0, tn, dtype, scratch, as_stream(stream));
-            if (st == NQ_OK) continue;
-            if (st != NQ_ERR_UNSUPPORTED) return st;
-        }
         P.T = tn;
         memset(P.cta_job, kMaxJobs * 17, sizeof(P.cta_job));
         // room for a block's partial sums and weights; a single row group is always allowed (see above)
@@ -992,12 +1006,28 @@ static int gemv_group(const nq_linear_desc* d, int n_linears, int T, int dtype, 
 
 int nq_gemv_group_fwd(const nq_linear_desc* d, int n_linears, int T, int dtype, void* scratch, size_t scratch_bytes,
                       nq_stream_t stream) {
-    return gemv_group(d, n_linears, T, dtype, scratch, scratch_bytes, false, stream);
+    const int st = check_group(d, n_linears, T, dtype, scratch, scratch_bytes);
+    return st != NQ_OK ? st : launch_decode(d, n_linears, 0, T, dtype, scratch, stream);
 }
 
 int nq_decode_group_fwd(const nq_linear_desc* d, int n_linears, int T, int dtype, void* scratch, size_t scratch_bytes,
                         nq_stream_t stream) {
-    return gemv_group(d, n_linears, T, dtype, scratch, scratch_bytes, true, stream);
+    int st = check_group(d, n_linears, T, dtype, scratch, scratch_bytes);
+    const int whole = T - T % kSplitTokens;
+    if (st != NQ_OK || whole == 0) return st != NQ_OK ? st : launch_decode(d, n_linears, 0, T, dtype, scratch, stream);
+    // Each linear by its own rule (the linears of a layer that share their input share it, too), one set of launches for
+    // those of a kind; the launches follow one another, so they use the same scratch.
+    nq_linear_desc two[kMaxJobs], one[kMaxJobs];
+    int n_two = 0, n_one = 0;
+    for (int i = 0; i < n_linears; ++i) {
+        if (takes_two_stages(d[i])) two[n_two++] = d[i];
+        else one[n_one++] = d[i];
+    }
+    for (int t0 = 0; n_two > 0 && st == NQ_OK && t0 < whole; t0 += kSplitTokens)
+        st = launch_two_stages(two, n_two, t0, dtype, scratch, as_stream(stream));
+    if (n_two > 0 && st == NQ_OK && whole < T) st = launch_decode(two, n_two, whole, T, dtype, scratch, stream);
+    if (n_one > 0 && st == NQ_OK) st = launch_decode(one, n_one, 0, T, dtype, scratch, stream);
+    return st;
 }
 
 int nq_gemv_fwd(const void* x, const void* s_in, const void* v_tiles, const void* s_mid,

@@ -4,7 +4,8 @@ The reference runs one operator call per projection (``modules/linear.py:121-132
 at decode batch sizes a launch is a chain of latencies, so the step time is set by the number of launches.
 ``LinearGroup`` issues ``nq_decode_group_fwd`` (up to four tokens) or ``nq_gemm_group_fwd`` for up to four
 prepared :class:`~nanoquant_b200.modules.linear.NanoQuantLinear` modules, with their biases and optional
-residuals in the kernel's epilogue.
+residuals in the kernel's epilogue.  Up to four tokens the results are the modules' own, bit for bit; above, the
+order of the fp32 sums depends on the whole launch and the last bits may differ.
 """
 from __future__ import annotations
 

@@ -1,5 +1,7 @@
-"""Four tokens through the decode dispatch: groups large enough for the two launches with a split intermediate, at ragged
+"""Four tokens through the decode dispatch: linears wide enough for the two launches with a split intermediate, at ragged
 rows, ranks and chunks, against the oracle within what the decode GEMV reaches, and beside the same linears alone."""
+import ctypes
+
 import pytest
 import torch
 
@@ -10,8 +12,8 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 @pytest.mark.parametrize("shapes", [
-    [(4104, 1032, 20001)], [(12296, 2440, 4100)], [(1024, 2056, 9000), (1024, 136, 64), (1024, 1000, 5000)],
-    [(1032, 6000, 4096), (1032, 8, 16)],       # a rank whose fragments do not fit: stays with the GEMV
+    [(4104, 1032, 20001)], [(12296, 2440, 4100)], [(3592, 2056, 9000), (3592, 136, 64), (3592, 1000, 5000)],
+    [(4104, 6000, 4096), (4104, 8, 16)],       # a rank whose fragments do not fit: that linear stays with the GEMV
 ])
 def test_four_tokens_large_groups(shapes, dtype):
     from nanoquant_b200 import ops
@@ -32,3 +34,40 @@ def test_four_tokens_large_groups(shapes, dtype):
             want += exact_np(resid[i])
         assert_parity(exact_np(ys[i]), want, dtype, rel=1e-4, what=f"linear {i} of {shapes}")
         assert torch.equal(ys[i], again[i])
+
+
+def call(layers, tiles, T, dtype):
+    """One nq_decode_group_fwd of the first T tokens."""
+    from nanoquant_b200 import _lib
+    Lb = _lib.lib()
+    st = torch.cuda.current_stream().cuda_stream
+    ys = [torch.empty(T, L["M"], dtype=dtype, device="cuda") for L in layers]
+    d = (_lib.LinearDesc * len(layers))(*[
+        _lib.LinearDesc(L["x"].data_ptr(), L["s_pre"].data_ptr(), v.data_ptr(), L["s_mid"].data_ptr(), u.data_ptr(),
+                        L["s_post"].data_ptr(), y.data_ptr(), L["N"], L["R"], L["M"], L["N"], L["M"])
+        for L, (v, u), y in zip(layers, tiles, ys)])
+    nb = Lb.nq_gemv_group_scratch_bytes(d, len(layers), T)
+    scratch = torch.zeros(nb, dtype=torch.uint8, device="cuda")
+    _lib.check(Lb.nq_decode_group_fwd(d, len(layers), T, _lib.NQ_BF16 if dtype == torch.bfloat16 else _lib.NQ_F16,
+                                      scratch.data_ptr(), ctypes.c_size_t(nb), st), "nq_decode_group_fwd")
+    assert Lb.nq_scratch_status(scratch.data_ptr(), st) == 0
+    return ys
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("shapes", [
+    [(4096, 1600, 4096), (4096, 608, 1024), (4096, 608, 1024)],          # q/k/v: k alone is a quarter of a megabyte
+    [(3328, 264, 512), (3329 + 7, 264, 512)],                            # on both sides of the line
+    [(4096, 1600, 1000), (4096, 64, 500), (4096, 1001, 40), (1003, 333, 77)],   # a rank below 128, ragged ranks and widths
+    [(12288, 2432, 4096), (2048, 384, 512)],
+])
+def test_group_equals_linears_alone(shapes, dtype):
+    T = 7
+    layers = make_group(shapes, T, dtype, seed=11)
+    tiles = [(tiles_on_gpu(L["V"]), tiles_on_gpu(L["U"])) for L in layers]
+    group = {n: call(layers, tiles, n, dtype) for n in (3, 4, 7)}
+    for i, L in enumerate(layers):
+        for n in (3, 4, 7):
+            assert torch.equal(group[n][i], call([L], tiles[i:i + 1], n, dtype)[0]), f"linear {i} of {shapes}, {n} tokens"
+        assert_parity(exact_np(group[7][i]), L["y64"], dtype, what=f"linear {i} of {shapes}")
+        assert torch.equal(group[7][i][:4], group[4][i])         # four tokens at a time, the rest by the decode kernel

@@ -129,6 +129,25 @@ def test_launch_group_equals_separate_modules():
     assert g.shape == (2, 3, m.I) and torch.equal(g, m.gate(x3))
 
 
+@pytest.mark.parametrize("T", [1, 2, 3, 4])
+def test_launch_group_equals_separate_modules_at_model_width(T):
+    # q/k/v of a 4096-column model at 0.8 bits per weight: at four tokens k alone must take the route that it takes in the
+    # group, whose factors are six times as large
+    from nanoquant_b200.modules.group import LinearGroup
+    from nanoquant_b200.modules.linear import NanoQuantLinear
+    g = torch.Generator(device="cuda").manual_seed(T)
+    words = lambda r, c: torch.randint(-2 ** 31, 2 ** 31 - 1, (r, c // 32), generator=g, device="cuda", dtype=torch.int32)
+    scale = lambda n: ((torch.rand(n, generator=g, device="cuda") + 0.5) * 0.01).to(DT)
+    mods = []
+    for M, R in ((4096, 1600), (1024, 608), (1024, 608)):
+        m = NanoQuantLinear(4096, M, R)
+        m.load_packed(words(R, 4096), (R, 4096), words(M, R), (M, R), scale(4096), scale(M), scale(R), dtype=DT, kernel_type="gemv")
+        mods.append(m)
+    x = torch.randn(T, 1, 4096, generator=g, device="cuda").to(DT)
+    for y, m in zip(LinearGroup(mods)(x), mods):
+        assert torch.equal(y, m(x))
+
+
 def grouped_step(m, groups, x):
     """The toy layer with folded norm weights, launch groups and residuals in the epilogues: 4 launches."""
     xf = x.float()
