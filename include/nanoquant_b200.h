@@ -150,8 +150,10 @@ size_t nq_gemv_scratch_bytes(int T, int N, int R, int M);
 size_t nq_gemv_group_scratch_bytes(const nq_linear_desc* linears_host, int n_linears, int T);
 
 /* The decode GEMV.  Accumulation is exact integer arithmetic on a 16-bit
- * fixed-point image of (s_in * x) and of the rank-R intermediate (per-token
- * scale), results are converted once per output in fp32.  `scratch` holds a
+ * fixed-point image of (s_in * x) and of the rank-R intermediate (one scale per
+ * token and 256 columns); the sums of the 256-column chunks are added in fp32 in
+ * an order that only their number decides.  A NaN or an infinity in a token makes
+ * every output of that token NaN.  `scratch` holds a
  * 256-byte header (a free-running launch counter + status word) followed by
  * the fp32 intermediate, each element stored with the tag of the launch that
  * wrote it (8 bytes per element); it must be 16-byte aligned, at least

@@ -1,12 +1,30 @@
 """Batch kernel (5 tokens up to its limit) at the edges of its tiles: column groups of 8 tokens, row groups of 16,
 chunks of 256 columns, more row groups per CTA than a pass takes, with bias and residual, in a launch group."""
+import numpy as np
 import pytest
 import torch
 
-from oracle import nanoquant_oracle as oc
-from tests.util import assert_parity, exact_np, make_group, tiles_on_gpu
+from tests.util import exact_np, make_group, tiles_on_gpu
 
 pytestmark = pytest.mark.gpu
+
+
+def bound(L, y, want, dtype):
+    """What rounding the intermediate t and the output to `dtype` and summing in fp32 may cost, element by element.
+
+    Every t_r is rounded once, by at most half a unit in its last place d_r, uniform and independent, so the sum over r stays
+    within six standard deviations of d_r / sqrt(3) each, and never exceeds the sum of the d_r.  fp32 sums: 2^-24 a step in a random walk over up to 4104 steps, 2^-18 of the norm of the terms.  The output
+    is rounded once: half a unit in its last place.  (2e-3 of the largest output, the bar of the other tests, is not a bound
+    for a handful of outputs: the largest of five may be small beside the norm of its terms.)"""
+    half = dtype == torch.float16
+    xs = exact_np(L["x"]) * exact_np(L["s_pre"])
+    mid = exact_np(L["s_mid"]) if L["s_mid"] is not None else np.ones(L["R"])
+    t = (xs @ L["V"].T.astype(np.float64)) * mid
+    half_ulp = lambda v: 2.0 ** (np.floor(np.log2(np.maximum(np.abs(v), 2.0 ** (-14 if half else -126)))) - (11 if half else 8))
+    d = half_ulp(t)
+    rounding_t = np.minimum(d.sum(axis=1), 6 / np.sqrt(3) * np.sqrt((d * d).sum(axis=1)))
+    fp32 = 2.0 ** -18 * np.sqrt(L["R"]) * np.abs(mid).max() * np.sqrt((xs * xs).sum(axis=1))
+    return np.outer(rounding_t + fp32, np.abs(exact_np(L["s_post"]))) + half_ulp(np.maximum(np.abs(y), np.abs(want)))
 
 
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
@@ -32,7 +50,6 @@ def test_batch_tile_edges(shapes, T, dtype):
             want += exact_np(biases[i])
         if resid[i] is not None:
             want += exact_np(resid[i])
-        if dtype == torch.float16 and scale[i] < 1e-3:      # outputs near fp16's subnormals: only the magnitude is checked
-            assert oc.rel_err(exact_np(ys[i]), want) < 0.05
-        else:
-            assert_parity(exact_np(ys[i]), want, dtype, rel=2.5e-3, what=f"linear {i} of {shapes}, {T} tokens")
+        y = exact_np(ys[i])
+        worst = float((np.abs(y - want) - bound(layers[i], y, want, dtype)).max())
+        assert worst <= 0, f"linear {i} of {shapes}, {T} tokens: {worst:.3e} beyond the bound"

@@ -1,65 +1,104 @@
-"""The integer identities the decode GEMV kernel relies on, checked in numpy (no GPU).
+"""The integer arithmetic of the decode kernel, restated in numpy (no GPU).
 
-The kernel feeds `word & (0x01010101 << j)` (an int8x4 with values {0, 2^j}, {0, -128} for j = 7) to an s8 MMA as
-the A operand and the activations, quantised to a fixed-point X with |X| <= 64000, as B operands X * 2^(7-j)
-(-X for j = 7) split into three signed bytes.  Every product is then 128 * X on the columns whose bit is set, the
-three byte terms recombine exactly, and sum(+-X) = sum(X) - 2 * sum_{bit=1}(X) = sum(X) - terms / 64.
+A unit is one token's 256 products p = s_in * x of a chunk.  With m = max |p| and the class j = (column % 256) / 32, a
+column becomes Z = round(p * 32500 / m * 2^(7-j)), negated for j = 7, by adding 1.5 * 2^23 in fp32; the low mantissa bits
+of that sum, 0x8080 added, are the three signed bytes of Z.  The kernel feeds `word & (0x01010101 << j)` (an int8x4 with
+values {0, 2^j}, {0, -128} for j = 7) to an s8 MMA against the bytes, so every class has the weight 128 * p * 32500 / m,
+and sum(+-p) = unit * (sum - 2 * S) with unit = m / (128 * 32500), S the sum over the set bits, both modulo 2^32.
 """
 import numpy as np
 
-Q_MAX = 64000
+Q_MAX = 32500
+MAGIC = np.float32(12582912.0 + 32896.0)      # 1.5 * 2^23 + 0x8080
+J = np.arange(256) // 32
+A = np.where(J == 7, -128, 1 << J)            # what a set bit of class j is worth to the MMA
 
 
-def byte_terms(y):
-    """Split Y (int64 array, |Y| < 2^23) into signed bytes b0, b1, b2 with Y = 65536*b2 + 256*b1 + b0, the way
-    the kernel does it on 32-bit registers: b0 = byte 0 of Y, b1 = byte 1 of Y + 0x80, b2 = byte 2 of Y + 0x8080."""
-    u = y.astype(np.int64) & 0xFFFFFFFF
-    as_s8 = lambda v: ((v & 0xFF) ^ 0x80) - 0x80
-    b0 = as_s8(u)
-    b1 = as_s8((u + 0x80) >> 8)
-    b2 = as_s8((u + 0x8080) >> 16)
-    return b0, b1, b2
+def words_of(p):
+    """fp32 words of the conversion, and m, for the 256 products of a unit (finite, m above 1e-31)."""
+    m = np.float32(np.abs(p).max())
+    inv = np.float32(Q_MAX) * (np.float32(1) / m)
+    inv_j = inv * np.where(J == 7, np.float32(-1), np.float32(2.0) ** (7 - J)).astype(np.float32)
+    # the product of two fp32 numbers is exact in fp64; the sum is rounded to an integer by the size of MAGIC
+    y = (p.astype(np.float64) * inv_j.astype(np.float64) + np.float64(MAGIC)).astype(np.float32)
+    return y.view(np.uint32), m
 
 
-def test_three_signed_bytes_recombine_exactly():
-    g = np.random.default_rng(0)
-    x = np.concatenate([g.integers(-Q_MAX, Q_MAX + 1, size=200000), [Q_MAX, -Q_MAX, 0, 1, -1, 127, 128, -128, -129, 32767, -32768]])
-    for j in range(8):
-        y = -x if j == 7 else x << (7 - j)           # class-shifted operand, |Y| <= 64000 * 128 < 2^23
-        b0, b1, b2 = byte_terms(y)
-        assert np.all(np.abs(b0) <= 128) and np.all(np.abs(b1) <= 128) and np.all(np.abs(b2) <= 128)
-        assert np.array_equal(65536 * b2 + 256 * b1 + b0, y)
+def bytes_of(w):
+    """The kernel's three bytes of a word, as signed values: packed adds and exclusive ors, without carries between bytes."""
+    s8 = lambda b: ((b & 0xFF).astype(np.int64) ^ 0x80) - 0x80
+    b2 = (w >> 16) & 0xFF
+    assert np.all(b2 + 0x40 <= 0xFF)           # the packed addition of 0x40404040 carries nothing into a neighbour
+    return s8((w & 0xFF) ^ 0x80), s8(((w >> 8) & 0xFF) ^ 0x80), s8((b2 + 0x40) ^ 0x80)
 
 
-def test_masked_bits_times_shifted_operand_is_128_x():
-    # A value of class j: 2^j as a signed byte (-128 for j = 7); operand: X * 2^(7-j) (-X for j = 7)
-    x = np.arange(-Q_MAX, Q_MAX + 1, 997, dtype=np.int64)
-    for j in range(8):
-        a = -128 if j == 7 else 1 << j
-        y = -x if j == 7 else x << (7 - j)
-        assert np.array_equal(a * y, 128 * x)
+def test_three_signed_bytes_recombine_for_every_integer():
+    most = int(Q_MAX * 128 * (1 + 2.0 ** -20)) + 1       # the reciprocal and its products are rounded
+    assert most < 2 ** 22
+    z = np.arange(-most, most + 1, dtype=np.int64)
+    w = (np.float32(12582912.0) + (z + 0x8080).astype(np.float32)).view(np.uint32)
+    assert np.array_equal(w, (0x4B400000 + 0x8080 + z).astype(np.uint32))
+    b0, b1, b2 = bytes_of(w)
+    assert np.array_equal(65536 * b2 + 256 * b1 + b0, z)
 
 
-def test_sign_sum_from_the_three_accumulators():
-    g = np.random.default_rng(1)
-    K = 4096
-    x = g.integers(-Q_MAX, Q_MAX + 1, size=K).astype(np.int64)
-    bits = g.integers(0, 2, size=(32, K)).astype(np.int64)          # 1 = weight -1
-    j = (np.arange(K) % 256) // 32                                   # class of a column inside its 256-column chunk
-    a = np.where(j == 7, -128, 1 << j) * bits                        # what the masked registers hold
-    y = np.where(j == 7, -x, x << (7 - j))
-    b0, b1, b2 = byte_terms(y)
-    c0, c1, c2 = a @ b0, a @ b1, a @ b2                              # the three int32 accumulators per row
-    assert np.all(np.abs(c0) < 2**31) and np.all(np.abs(c1) < 2**31) and np.all(np.abs(c2) < 2**31)
-    terms = 65536 * c2 + 256 * c1 + c0
-    assert np.all(terms % 128 == 0)
-    got = x.sum() - (terms >> 6)
-    want = ((1 - 2 * bits) * x).sum(axis=1)
-    assert np.array_equal(got, want)
+def unit_of(p):
+    """{unit value, sum} and the three byte rows, as quantise_unit leaves them in shared memory."""
+    w, m = words_of(p)
+    lanes = w.reshape(32, 8).astype(np.uint64).sum(axis=1)
+    part = (lanes - 8 * (0x4B400000 + 0x8080)).astype(np.uint32).view(np.int32).astype(np.int64)      # modulo 2^32, per lane
+    part = part * A[::8]
+    assert np.abs(part).max() <= 2 ** 25
+    total = int(part.sum())
+    assert abs(total) < 2 ** 30
+    return np.float32(m) * np.float32(1.0 / (128 * Q_MAX)), total, bytes_of(w)
 
 
-def test_accumulators_stay_inside_int32_at_the_largest_k():
-    # worst case per accumulator: every bit set, every byte term at its extreme, K = 32768 columns
-    K = 32768
-    assert K * 128 * 128 < 2**31
-    assert K * Q_MAX < 2**31       # sum(X)
+def products(seed, n=256):
+    g = np.random.default_rng(seed)
+    p = (g.standard_normal(n) * 10.0 ** g.uniform(-8, 8)).astype(np.float32)
+    p[g.integers(n, size=seed % 64)] = 0
+    return p
+
+
+def test_sums_over_signs_are_exact_and_in_range():
+    for seed in range(40):
+        p = products(seed) if seed else np.full(256, 3.0, np.float32)      # seed 0: every column at the bound
+        unit, total, (b0, b1, b2) = unit_of(p)
+        z = 65536 * b2 + 256 * b1 + b0
+        assert np.abs(A * z).sum() < 2 ** 30
+        bits = np.random.default_rng(seed).integers(0, 2, size=(64, 256)).astype(np.int64)
+        bits[0], bits[1] = 0, 1
+        c0, c1, c2 = (bits * A) @ b0, (bits * A) @ b1, (bits * A) @ b2
+        assert max(np.abs(c).max() for c in (c0, c1, c2)) < 2 ** 31         # int32 accumulators
+        S = (c0 + (c1 << 8) + (c2 << 16)) & 0xFFFFFFFF
+        got = ((total - 2 * S) & 0xFFFFFFFF).astype(np.uint32).view(np.int32).astype(np.int64)
+        assert np.array_equal(got, ((1 - 2 * bits) * (A * z)).sum(axis=1))
+
+
+def test_quantisation_error():
+    for seed in range(1, 40):
+        p = products(seed)
+        unit, _, (b0, b1, b2) = unit_of(p)
+        q = (A * (65536 * b2 + 256 * b1 + b0)) * np.float64(unit)
+        # half an integer of class j is 2^j / 2 <= 64 of 128 * 32500 units; the rest is the rounding of reciprocal and unit
+        assert np.abs(q - p).max() <= np.abs(p).max() * (64 / (128 * Q_MAX) + 2.0 ** -21)
+
+
+def test_small_products_scaled_by_a_power_of_two_give_the_same_integers():
+    # below 1e-31 the reciprocal of the maximum times 32500 * 128 would overflow fp32
+    assert np.float32(Q_MAX) * (np.float32(1) / np.float32(1e-31)) * np.float32(128) < np.finfo(np.float32).max
+    p = (products(3) / np.abs(products(3)).max()).astype(np.float32)
+    tiny = p * np.float32(2.0 ** -110)
+    assert np.abs(tiny).max() <= 1e-31
+    want, _ = words_of(p)
+    got, m = words_of(tiny * np.float32(2.0 ** 64))
+    assert np.array_equal(got, want) and m == np.float32(2.0 ** -46)
+
+
+def test_the_largest_finite_maximum_stays_in_range():
+    p = np.zeros(256, np.float32)
+    p[::32] = np.finfo(np.float32).max
+    _, _, (b0, b1, b2) = unit_of(p)
+    z = 65536 * b2 + 256 * b1 + b0
+    assert np.abs(z).max() < 2 ** 22 and np.abs(A * z).max() <= 128 * Q_MAX * (1 + 2.0 ** -20)

@@ -1,7 +1,7 @@
 """``nq_gemv_group_fwd`` with several linears per launch (the launches a decode step is made of) through the
 C ABI: every output against the fp64 oracle on the same seeded inputs, and bit-equal to the same linear run
-alone through ``nq_gemv_fwd`` (all accumulation is exact integer arithmetic on a per-token fixed-point image,
-so the way rows are dealt to CTAs and launches cannot change a result)."""
+alone through ``nq_gemv_fwd`` (a chunk's sums are exact integers of a fixed-point image, and the chunks are added in
+fp32 in an order of their own, so the way rows are dealt to CTAs and launches cannot change a result)."""
 import ctypes
 
 import pytest

@@ -7,7 +7,7 @@ from oracle import nanoquant_oracle as oc
 # Parity bar against the fp64 oracle, element by element:
 #     |y - y64| <= 2e-3 * max|y64| + half a unit in the last place of the output type at that element
 # (`parity_excess` / `assert_parity` below).  The representation error of a rounded output belongs to the
-# element (2^-9 of it for bf16, 2^-12 for fp16), not to the largest one, so a 2e-3 error before the final rounding
+# element (up to 2^-8 of it for bf16, 2^-11 for fp16), not to the largest one, so a 2e-3 error before the final rounding
 # cannot hide behind it.  TOL is the older max-normalised bar, kept for comparisons between two rounded results.
 TOL = {torch.float16: 2e-3, torch.bfloat16: 2e-3 + 2.0 ** -8}
 
