@@ -8,8 +8,8 @@ Workload (``config.workload``): the quantised linears of a Qwen3-8B-shaped decod
 factors and scales ``(U[0,1)+0.5)*0.01``, synthetic N(0,1) activations — executed for one decode
 step of ``--batch`` tokens (default 1).  A *step* is one pass over all 252 linears, i.e. the
 hot-path work of one generated token per sequence.  Per layer the launches are q/k/v (one group),
-o, gate/up (one group), down: 4 launches of the group GEMV kernel, 144 per step, captured in a
-CUDA graph.  The packed factors (690 MB) exceed L2, so every step streams them from HBM.
+o, gate/up (one group), down: 4 launches of the group GEMV kernel, 144 per step (288 of the batch
+kernel or the GEMM from 4 tokens on), captured in a CUDA graph.  The packed factors (690 MB) exceed L2, so every step streams them from HBM.
 
 * ``value``      tokens/s of the device-resident step (CUDA events around K graph replays).
 * ``e2e``        the same through host buffers: per step the activations are copied from pinned
@@ -256,6 +256,31 @@ def dram_traffic_ratio():
     return None
 
 
+def group_call(L, T, gemm_from=0):
+    """The C entry point that a launch group of modules takes at T tokens, and its scratch size."""
+    if T >= (gemm_from or L.nq_gemv_max_tokens() + 1):
+        return L.nq_gemm_group_fwd, L.nq_gemm_group_scratch_bytes
+    return L.nq_decode_group_fwd, L.nq_gemv_group_scratch_bytes
+
+
+def group_kernels(L, shapes, T, gemm_from=0):
+    """Kernels that one call of `group_call` launches for linears of `shapes` [(N, R, M)], in order: above the decode limit
+    one per stage (up to 32 tokens the batch kernel); below it one launch of the decode kernel per four tokens, except that
+    linears with more than 3328 columns and a rank from 128 run four tokens as the two stages of the batch kernel."""
+    if T >= (gemm_from or L.nq_gemv_max_tokens() + 1):
+        return ["batch_stage_kernel" if T <= 32 else "gemm_stage_kernel"] * 2
+    two = [N > 3328 and R >= 128 and N % 8 == 0 and R % 8 == 0 for (N, R, _) in shapes]
+    if T < 4 or not any(two):
+        return ["gemv_group_kernel"] * -(-T // 4)
+    return (["batch_stage_kernel"] * (2 * (T // 4)) + ["gemv_group_kernel"] * (T % 4 > 0) +
+            ["gemv_group_kernel"] * (0 if all(two) else -(-T // 4)))
+
+
+ARITHMETIC = {"gemv_group_kernel": "s8 mma / s32 accumulate on 16-bit fixed point; bf16 in/out",
+              "batch_stage_kernel": "bf16 mma / f32 accumulate; bf16 in/out",
+              "gemm_stage_kernel": "bf16 tcgen05 mma / f32 accumulate; bf16 in/out"}
+
+
 class Step:
     """Device-resident weights of the decoder layers and the launch list of one decode step."""
 
@@ -274,9 +299,8 @@ class Step:
                   "i": torch.randn(T, INTER, generator=g, device=device).to(dtype)}
         self.keep, self.launches, self.bytes = [], [], 0
         scratch_bytes = 0
-        # more tokens than one decode launch takes: the groups go through nq_gemm_group_fwd (batch kernel or GEMM)
-        self.per_linear = T >= (GEMM_MIN_TOKENS or self.L.nq_gemv_max_tokens() + 1)
-        self.n_linears = 0
+        self.fwd, size_fn = group_call(self.L, T, GEMM_MIN_TOKENS)
+        self.n_linears, kernels = 0, []
         for _ in range(layers):
             groups = {}
             for (name, N, R, M, src, grp) in layer_linears():
@@ -291,28 +315,20 @@ class Step:
                 self.n_linears += 1
             for grp in sorted(groups):
                 arr = (_lib.LinearDesc * len(groups[grp]))(*groups[grp])
-                size_fn = self.L.nq_gemm_group_scratch_bytes if self.per_linear else self.L.nq_gemv_group_scratch_bytes
                 scratch_bytes = max(scratch_bytes, size_fn(arr, len(arr), T))
                 self.launches.append(arr)
+                kernels += group_kernels(self.L, [(d.N, d.R, d.M) for d in arr], T, GEMM_MIN_TOKENS)
         self.last_y = self.keep[-1]["y"]
         self.scratch = torch.zeros(scratch_bytes, dtype=torch.uint8, device=device)
-        self.kernels_per_step = (2 if self.per_linear else 1) * len(self.launches)
-        self.kernel_name = ("gemv_group_kernel" if not self.per_linear else
-                            "batch_stage_kernel" if T <= 32 else "gemm_stage_kernel")
+        self.kernels_per_step = len(kernels)
+        self.kernel_name = max(set(kernels), key=kernels.count)      # (the one with most launches)
         self.graph = None
 
     def run(self):
         st = self.torch.cuda.current_stream(self.device).cuda_stream
-        if self.per_linear:
-            for arr in self.launches:
-                rc = self.L.nq_gemm_group_fwd(arr, len(arr), self.T, self.dt_id, self.scratch.data_ptr(),
-                                              self.scratch.numel(), st)
-                self.lib.check(rc, "nq_gemm_group_fwd")
-            return
         for arr in self.launches:
-            rc = self.L.nq_gemv_group_fwd(arr, len(arr), self.T, self.dt_id, self.scratch.data_ptr(),
-                                          self.scratch.numel(), st)
-            self.lib.check(rc, "nq_gemv_group_fwd")
+            rc = self.fwd(arr, len(arr), self.T, self.dt_id, self.scratch.data_ptr(), self.scratch.numel(), st)
+            self.lib.check(rc, "group launch")
 
     def capture(self):
         torch = self.torch
@@ -356,7 +372,7 @@ class StepCycle:
         self.i = 0
         s0 = self.steps[0]
         self.bytes, self.kernels_per_step = s0.bytes, s0.kernels_per_step
-        self.per_linear, self.kernel_name = s0.per_linear, s0.kernel_name
+        self.kernel_name = s0.kernel_name
 
     def capture(self):
         for st in self.steps:
@@ -400,9 +416,7 @@ def check_step(T, dtype, device):
         groups.setdefault(grp, []).append(
             _lib.LinearDesc(x[src].data_ptr(), t["s_in"].data_ptr(), t["v"].data_ptr(), t["s_mid"].data_ptr(),
                             t["u"].data_ptr(), t["s_out"].data_ptr(), t["y"].data_ptr(), N, R, M, N, M))
-    use_gemm = T >= (GEMM_MIN_TOKENS or L.nq_gemv_max_tokens() + 1)
-    fwd = L.nq_gemm_group_fwd if use_gemm else L.nq_gemv_group_fwd
-    size_fn = L.nq_gemm_group_scratch_bytes if use_gemm else L.nq_gemv_group_scratch_bytes
+    fwd, size_fn = group_call(L, T, GEMM_MIN_TOKENS)
     st = torch.cuda.current_stream(device).cuda_stream
     for grp in sorted(groups):
         arr = (_lib.LinearDesc * len(groups[grp]))(*groups[grp])
@@ -609,7 +623,7 @@ def gpu_arm(args):
         return
 
     peak, peak_src = hbm_peak()
-    ratio = dram_traffic_ratio()
+    ratio = dram_traffic_ratio() if step.kernel_name == "gemv_group_kernel" else None
     step_s = ms * 1e-3 / args.steps
     achieved = step.bytes / step_s / 1e9
     if args.layers != LAYERS:   # profiling aid: fewer layers resident; report per-step numbers of what ran
@@ -621,15 +635,14 @@ def gpu_arm(args):
         "metric": "decode tok/s (quantised linears of one decode step)", "value": world * T / step_s,
         "unit": "tokens/s", "n_gpus": world, "steps": args.steps, "warmup": max(args.warmup, 3),
         "ms_per_step": step_s * 1e3, "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
-        "dtype": ("bf16 tcgen05 mma / f32 accumulate; bf16 in/out" if step.per_linear
-                  else "s8 mma / s32 accumulate on 16-bit fixed point; bf16 in/out"), "data": "synthetic",
+        "dtype": ARITHMETIC[step.kernel_name], "data": "synthetic",
         "config": workload_config(T),
         "parallelism": "single gpu" if world == 1 else f"{world} independent replicas",
         "layers_timed": args.layers,
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                     "traffic": (step.bytes / step.kernels_per_step * ratio if (ratio and not step.per_linear) else None),
+                     "traffic": (step.bytes / step.kernels_per_step * ratio if ratio else None),
                      "traffic_source": ("dram__bytes_read+write over algorithmic bytes of three launches captured with ncu, "
-                                        "scaled to the average launch" if (ratio and not step.per_linear) else None),
+                                        "scaled to the average launch" if ratio else None),
                      "kernel": step.kernel_name,
                      "bytes_per_launch": step.bytes / step.kernels_per_step, "us_per_launch": launch_us,
                      "peak_source": peak_src},
@@ -709,9 +722,8 @@ def measure_tp(T, layers, steps, warmup, collective, device, world, rank, shard=
         dist.all_reduce(ok, op=dist.ReduceOp.MIN)
         if ok.item() == 0:
             peer = None
-    use_gemm = T > L.nq_gemv_max_tokens()   # more tokens than a decode launch takes: the group GEMM (two launches)
-    group_fwd = L.nq_gemm_group_fwd if use_gemm else L.nq_gemv_group_fwd
-    group_bytes = L.nq_gemm_group_scratch_bytes if use_gemm else L.nq_gemv_group_scratch_bytes
+    group_fwd, group_bytes = group_call(L, T)
+    kernels = []
     for _ in range(layers):
         groups = {}
         for spec in tp_layer_linears():
@@ -737,9 +749,10 @@ def measure_tp(T, layers, steps, warmup, collective, device, world, rank, shard=
                 nbytes += R * N // 8 + R * m // 8 + 2 * (N + R + m) + 2 * T * (N + m)
             arr = (_lib.LinearDesc * len(descs))(*descs)
             scratch_bytes = max(scratch_bytes, group_bytes(arr, len(arr), T))
+            kernels += group_kernels(L, [(d.N, d.R, d.M) for d in arr], T)
             steps_.append((arr, ybuf, full))
     scratch = torch.zeros(scratch_bytes, dtype=torch.uint8, device=device)
-    launches_per_step = (2 if use_gemm else 1) * len(steps_)
+    launches_per_step = len(kernels)
 
     def run():
         st = torch.cuda.current_stream(device).cuda_stream
@@ -797,7 +810,7 @@ def measure_tp(T, layers, steps, warmup, collective, device, world, rank, shard=
     res = {"tokens_per_s": T / step_s, "ms_per_step": step_s * 1e3, "per_gpu_gbs": per_gpu,
            "hbm_frac_per_gpu": per_gpu / hbm_peak()[0], "gpus": G, "batch": T, "layers_timed": layers,
            "collective": ("none" if G == 1 else "peer-memory kernel, CUDA graph" if peer is not None else "NCCL, eager"),
-           "kernel": "gemm_stage_kernel" if use_gemm else "gemv_group_kernel", "launches_per_step": launches_per_step}
+           "kernel": max(set(kernels), key=kernels.count), "launches_per_step": launches_per_step}
     del keep, steps_, scratch, graph, peer
     torch.cuda.empty_cache()
     return res
@@ -1010,9 +1023,7 @@ def measure_group(shapes, T, dtype, device, steps, resident, profile=False, max_
     copies = 1 if resident else max(2, int(2 * L2_BYTES // packed) + 1)
     if max_copies:
         copies = min(copies, max_copies)
-    use_gemm = T > L.nq_gemv_max_tokens()
-    fwd = L.nq_gemm_group_fwd if use_gemm else L.nq_gemv_group_fwd
-    size_fn = L.nq_gemm_group_scratch_bytes if use_gemm else L.nq_gemv_group_scratch_bytes
+    fwd, size_fn = group_call(L, T)
     xs = {N: torch.randn(T, N, generator=g, device=device).to(dtype) for N in {n for (n, _, _) in shapes}}
     keep, arrs = [], []
     for _ in range(copies):
@@ -1058,7 +1069,7 @@ def measure_group(shapes, T, dtype, device, steps, resident, profile=False, max_
     if L.nq_scratch_status(scratch.data_ptr(), torch.cuda.current_stream(device).cuda_stream) != 0:
         raise SystemExit("bench.py: a device-side wait timed out")
     us = e0.elapsed_time(e1) * 1e3 / (steps * copies * reps)
-    return us, copies, (2 if use_gemm else (T + 3) // 4)
+    return us, copies, len(group_kernels(L, shapes, T))
 
 
 def linear_arm(args):
