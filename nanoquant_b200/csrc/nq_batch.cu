@@ -14,14 +14,20 @@
 //    of a token is its four consecutive columns 4q..4q+3.
 //  * B fragments.  The intermediate is stored in fragment order (see fragment_index): a warp's load of one is 256
 //    contiguous bytes.  Activations come in rows: every warp stages its own columns through shared memory with 16-byte
-//    copies, 192 of them in flight.  (Fragments loaded from rows touch eight lines each, 2 us of L1 tag lookups in a stage of 6.)
+//    copies, 192 of them in flight.  (Fragments loaded from rows touch eight lines each.)
 //  * Two barriers; no K split over CTAs, no counters, no slabs.
 //
 // Splitting K over the CTAs of a cluster (partial sums exchanged through distributed shared memory) and staging the whole
 // input by bulk copies before the loop both measured slower than this at every size.
-// Qwen3-8B decode, eight layers in a graph, GEMM against this kernel: 8 tokens 804 -> 359 us, 16 tokens 825 -> 438, 20 tokens
-// 865 -> 631, 24 tokens 860 -> 721, 32 tokens 826 -> 801.  At 16 tokens a stage with little work takes 4.4 us; gate/up's
-// second stage 12 (16 clocks per MMA and scheduler), down's first 11.5 (58 MB of activations from L2 to the SMs, 7 TB/s).
+// Qwen3-8B decode, eight layers in a graph, all through the GEMM against this kernel: 8 tokens 813 and 353 us, 16 tokens 822
+// and 435, 20 tokens 821 and 626, 24 tokens 818 and 702, 28 tokens 816 and 736, 32 tokens 816 and 752.
+//
+// What bounds it (counters of single launches at 16 tokens, cold): no throughput limit is near.  DRAM 3 to 6 % of its peak,
+// L2 4 to 16, tensor pipe 12 to 19.  The two stages of a group with little work take 8.8 us together, two launches of a fixed
+// chain (dependency, weights' arrival, a loop of a few steps, two barriers, output).  In first stages the 16 warps issue in
+// 56 to 60 % of the active cycles: copies, shifts and LOP3 around the MMAs; down's reads 56 MB through L2, since every CTA
+// stages the whole input.  Gate/up's second stage waits for the fragments of t (long scoreboard, 3.1 warps per issue, is its
+// largest stall) with four warps per scheduler to hide that.
 #include <cstddef>
 #include <cstring>
 

@@ -217,9 +217,10 @@ enum : int { kOutFp16, kOutBf16, kOutBf16Saturated };
 // ---------------------------------------------------------------------------
 // the kernel: one 128 x 128 output tile per CTA
 // ---------------------------------------------------------------------------
-// The ", 1" matters: its shared memory allows one CTA per SM anyway, but without the word the compiler saves registers (64
-// instead of 89 for the largest tile) and puts the loads of the expansion and of the epilogue one behind the other.  Layer of
-// 517 tokens 249 -> 244 us, 2048 tokens 720 -> 702, 128 tokens 188 -> 180, eight layers of 64 tokens 876 -> 844.
+// The ", 1" matters: its shared memory allows one CTA per SM anyway, but without the word the compiler saves registers (70
+// instead of 88 for the largest tile) and puts the loads of the expansion and of the epilogue one behind the other.  Without
+// and with it, the same source: layer of 128 tokens 184.6 and 176.1 us, 517 tokens 246.2 and 243.6, 2048 tokens 741.6 and
+// 731.1, eight layers of 64 tokens 871 and 843.
 template <int MH, int NH, int OUT>
 __global__ void __launch_bounds__(GemmCfg<MH, NH>::kThreads, 1) gemm_stage_kernel(const __grid_constant__ GemmParams P) {
     using C = GemmCfg<MH, NH>;

@@ -27,7 +27,8 @@ struct StageTypes {
     int io_bf16, a_bf16, out_bf16, exp_sign;
 };
 
-constexpr int kBatchMostTokens = 32;    // of the batch kernel (see nq_batch.cu)
+constexpr int kBatchMostTokens = 32;    // of the batch kernel: all that its four column groups hold, and there it is
+                                        // still ahead of the GEMM (see the figures in nq_batch.cu)
 // The same, or 0 where it cannot take the jobs.
 int batch_max_tokens(const StageJob* jobs, int n);
 // `frag_in` / `frag_out`: the activations / the output are an intermediate in the batch kernel's fragment order, of
