@@ -65,9 +65,11 @@ def test_group_equals_linears_alone(shapes, dtype):
     T = 7
     layers = make_group(shapes, T, dtype, seed=11)
     tiles = [(tiles_on_gpu(L["V"]), tiles_on_gpu(L["U"])) for L in layers]
-    group = {n: call(layers, tiles, n, dtype) for n in (3, 4, 7)}
+    group = {n: call(layers, tiles, n, dtype) for n in (1, 2, 3, 4, 7)}
     for i, L in enumerate(layers):
         for n in (3, 4, 7):
             assert torch.equal(group[n][i], call([L], tiles[i:i + 1], n, dtype)[0]), f"linear {i} of {shapes}, {n} tokens"
         assert_parity(exact_np(group[7][i]), L["y64"], dtype, what=f"linear {i} of {shapes}")
         assert torch.equal(group[7][i][:4], group[4][i])         # four tokens at a time, the rest by the decode kernel
+        # up to three tokens: the same bits however many ride along
+        assert torch.equal(group[1][i], group[3][i][:1]) and torch.equal(group[2][i], group[3][i][:2])
