@@ -230,7 +230,7 @@ unsigned nq_gemv_set_wait_limit(unsigned polls);
 
 /* Bytes of scratch nq_gemm_fwd needs: a 256-byte header (status word at byte 8,
  * the same place as in the GEMV scratch) followed by the rank-R intermediate
- * t[T, R] in the I/O dtype (padded to its fragment order for up to 32 tokens)
+ * t[T, R] in the I/O dtype (padded to its fragment order for up to 16 tokens)
  * and per-token exponents. */
 size_t nq_gemm_scratch_bytes(int T, int N, int R, int M);
 

@@ -1,4 +1,4 @@
-// One stage of a decode batch (a handful to a few dozen tokens): Out[T, rows] = (A[T, K] . W[rows, K]^T) * post.
+// One stage of a decode batch (5 to 16 tokens, and split four): Out[T, rows] = (A[T, K] . W[rows, K]^T) * post.
 //
 // At these sizes a stage is a few microseconds of fixed chain around very little arithmetic.  The tcgen05 GEMM spends 12 to
 // 13 us on it: 128-row tiles leave most SMs idle unless K is split, and the split costs slabs or a cluster exchange.
@@ -19,8 +19,8 @@
 //
 // Splitting K over the CTAs of a cluster (partial sums exchanged through distributed shared memory) and staging the whole
 // input by bulk copies before the loop both measured slower than this at every size.
-// Qwen3-8B decode, eight layers in a graph, all through the GEMM against this kernel: 8 tokens 813 and 353 us, 16 tokens 822
-// and 435, 20 tokens 821 and 626, 24 tokens 818 and 702, 28 tokens 816 and 736, 32 tokens 816 and 752.
+// It ends at 16 tokens: eight layers in a graph with this kernel, and through nq_wgemm.cu, us: Qwen3-8B 8 tokens 359 and 453,
+// 16 tokens 436 and 455, 17 tokens (three column groups, a variant that is gone) 625 and 473; Llama-3.2-1B 16 tokens 313 and 302.
 //
 // What bounds it (counters of single launches at 16 tokens, cold): no throughput limit is near.  DRAM 3 to 6 % of its peak,
 // L2 4 to 16, tensor pipe 12 to 19.  The two stages of a group with little work take 8.8 us together, two launches of a fixed
@@ -40,11 +40,10 @@ namespace nq {
 constexpr int kBatchThreads = 512;
 constexpr int kBatchWarps = kBatchThreads / 32;
 // 16-column blocks of the intermediate whose B fragments a warp loads together
-constexpr int blocks_in_flight(int nt, int rows) { return nt == 1 || (nt == 2 && rows < 4) ? 8 : nt == 4 && rows == 2 ? 2 : 4; }
-constexpr int tokens_groups(int T) { return T <= 8 ? 1 : T <= 16 ? 2 : T <= 24 ? 3 : 4; }
-// row groups of a pass: four, two where the accumulators of four do not leave registers for the operands
-constexpr int most_rows_of(int nt) { return nt <= 2 ? 4 : 2; }
-constexpr int pieces(int nt) { return nt <= 2 ? 3 : nt == 3 ? 2 : 1; }   // pieces of 64 columns a warp has in flight
+constexpr int blocks_in_flight(int nt, int rows) { return nt == 1 || rows < 4 ? 8 : 4; }
+constexpr int tokens_groups(int T) { return T <= 8 ? 1 : 2; }
+constexpr int kMostRows = 4;             // row groups of a pass
+constexpr int kPieces = 3;               // pieces of 64 columns a warp has in flight
 constexpr int kPieceStride = 128 + 32;   // bytes of a staged row: 32 mod 128, so the eight tokens of a fragment fall on
                                          // different banks
 constexpr int kBatchSlots = 8;           // weight blocks in flight
@@ -113,7 +112,7 @@ __device__ __forceinline__ void copy16_or_zero(uint32_t dst, const void* src, bo
 // kSplitTokens).
 template <bool BF16, int NT, int ROWS, bool FRAG, bool SPLIT>
 __global__ void __launch_bounds__(kBatchThreads, 1) batch_stage_kernel(const __grid_constant__ BatchParams Pc) {
-    constexpr int kRows = ROWS, kB = blocks_in_flight(NT, ROWS), kPieces = pieces(NT);
+    constexpr int kRows = ROWS, kB = blocks_in_flight(NT, ROWS);
     extern __shared__ __align__(128) unsigned char smem[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, q = lane & 3;
     const uint32_t bars = smem_u32(smem);
@@ -365,13 +364,12 @@ __global__ void __launch_bounds__(kBatchThreads, 1) batch_stage_kernel(const __g
 template <bool BF16, int NT, bool FRAG>
 static const void* batch_kernel_rows(int rows) {
     if (rows == 1) return (const void*)batch_stage_kernel<BF16, NT, 1, FRAG, false>;
-    if (rows == 2 || most_rows_of(NT) == 2) return (const void*)batch_stage_kernel<BF16, NT, 2, FRAG, false>;
-    return (const void*)batch_stage_kernel<BF16, NT, most_rows_of(NT), FRAG, false>;
+    if (rows == 2) return (const void*)batch_stage_kernel<BF16, NT, 2, FRAG, false>;
+    return (const void*)batch_stage_kernel<BF16, NT, kMostRows, FRAG, false>;
 }
 template <bool BF16, bool FRAG>
 static const void* batch_kernel_tokens(int nt, int rows) {
-    return nt == 1 ? batch_kernel_rows<BF16, 1, FRAG>(rows) : nt == 2 ? batch_kernel_rows<BF16, 2, FRAG>(rows)
-           : nt == 3 ? batch_kernel_rows<BF16, 3, FRAG>(rows) : batch_kernel_rows<BF16, 4, FRAG>(rows);
+    return nt == 1 ? batch_kernel_rows<BF16, 1, FRAG>(rows) : batch_kernel_rows<BF16, 2, FRAG>(rows);
 }
 template <bool BF16, bool FRAG>
 static const void* split_kernel_rows(int rows) {
@@ -392,8 +390,8 @@ static int batch_smem_limit(int* out) {
     if (cached[dev & 63] == 0) {
         int optin = 0;
         NQ_CUDA_TRY(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-        for (int i = 0; i < 48; ++i)
-            NQ_CUDA_TRY(cudaFuncSetAttribute(batch_kernel(i & 1, 1 + (i / 4) % 4, 1 << (i / 16), (i & 2) != 0), cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
+        for (int i = 0; i < 24; ++i)
+            NQ_CUDA_TRY(cudaFuncSetAttribute(batch_kernel(i & 1, 1 + (i / 4) % 2, 1 << (i / 8), (i & 2) != 0), cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
         for (int i = 0; i < 12; ++i)
             NQ_CUDA_TRY(cudaFuncSetAttribute(split_kernel(i & 1, 1 << (i / 4), (i & 2) != 0), cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
         cached[dev & 63] = optin;
@@ -413,13 +411,12 @@ size_t batch_fragment_bytes(int T, int K) { return (size_t)((K + 255) / 256) * 1
 // Chunk slices x row slices of the warps for a block of `gb` row groups: a step (a row group's chunk) against a chunk's B
 // fragments, once per pass.
 static void split_warps(int gb, int chunks, int nt, int& wk, int& wr) {
-    const int rows_most = most_rows_of(nt);
     int best = 1 << 30;
     for (int k = 1; k <= kBatchWarps && k <= chunks; ++k) {
         int r = kBatchWarps / k;
         if (r > gb) r = gb;
         const int per = (gb + r - 1) / r;
-        const int cost = ((chunks + k - 1) / k) * (per * (8 + 2 * nt) + ((per + rows_most - 1) / rows_most) * (3 + 3 * nt));
+        const int cost = ((chunks + k - 1) / k) * (per * (8 + 2 * nt) + ((per + kMostRows - 1) / kMostRows) * (3 + 3 * nt));
         if (cost < best) { best = cost; wk = k; wr = r; }
     }
 }
@@ -449,7 +446,7 @@ int launch_batch_stage(const StageJob* jobs, int n, int tokens, StageTypes ty, i
     if (grid > total) grid = total;
     if (grid < n) grid = n;
     deal_ctas(grid, n, groups, chunks, ncta);
-    const size_t stage_bytes = frag_in ? 0 : (size_t)kBatchWarps * pieces(nt) * (T + 1) * kPieceStride;
+    const size_t stage_bytes = frag_in ? 0 : (size_t)kBatchWarps * kPieces * (T + 1) * kPieceStride;
     const size_t room = limit - kFixedBytes - stage_bytes;      // weights and partial sums of a block
     size_t slot_used = 0, part_used = 0;
     int cta = 0, most_blocks = 1, most_rows = 1;

@@ -43,6 +43,7 @@
 
 #include "nq_common.cuh"
 #include "nq_stage.h"
+#include "nq_tcgen05.cuh"
 
 namespace nq {
 
@@ -51,7 +52,6 @@ constexpr int kBK = 64;             // k per pipeline stage: 128 bytes of bf16 =
 constexpr int kGroupThreads = 256;                          // expand threads that share one k block
 constexpr int kTileBytes = kBM * kBK * 2;          // 16 KB: one 128-row operand tile
 constexpr int kPreBytes = 256 * 2;                 // input scales of one 256-column chunk
-constexpr unsigned kWaitLimit = 1u << 21;   // attempts of up to ~2 us each
 
 // Tile configuration: MH x 128 tokens by NH x 128 weight rows per CTA.  One expanded weight
 // tile feeds MH MMAs and one activation tile meets 128 * NH weight rows, which sets the
@@ -137,36 +137,6 @@ struct GemmParams {
 // ---------------------------------------------------------------------------
 // PTX wrappers
 // ---------------------------------------------------------------------------
-// Bounded wait on an mbarrier phase.  Returns false when the limit expired or another
-// thread of the CTA already gave up; the caller then leaves its loop.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag,
-                                          unsigned* status) {
-    if (mbar_try(bar, parity)) return true;   // the common case: already complete
-    for (unsigned i = 0; i < kWaitLimit; ++i) {
-        if (mbar_try(bar, parity)) return true;
-        if (*abort_flag) return false;
-    }
-    *abort_flag = 1;
-    atomicExch(status, (unsigned)(-NQ_ERR_TIMEOUT));
-    return false;
-}
-
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int c0, int c1, uint32_t bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-        ::"r"(dst), "l"(map), "r"(c0), "r"(c1), "r"(bar)
-        : "memory");
-}
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-
-// K-major, 128-byte swizzle: rows of 128 bytes, 8-row groups 1024 bytes apart.
-__device__ __forceinline__ uint64_t umma_desc(uint32_t smem_addr) {
-    const uint32_t lo = ((smem_addr >> 4) & 0x3FFFu) | (1u << 16);          // start address, LBO = 1 (unused)
-    const uint32_t hi = (1024u >> 4) | (1u << 14) | (2u << 29);             // SBO, version 1, SWIZZLE_128B
-    return ((uint64_t)hi << 32) | lo;
-}
-
 __device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
                                          uint32_t accumulate) {
     asm volatile(
@@ -201,16 +171,6 @@ __device__ __forceinline__ void cluster_sync_all() {
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-// address of this CTA's shared-memory location `local` in the CTA of rank `rank` of the cluster
-__device__ __forceinline__ uint32_t cluster_map(uint32_t local, uint32_t rank) {
-    uint32_t r;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local), "r"(rank));
-    return r;
-}
-__device__ __forceinline__ void cluster_store4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
-    asm volatile("st.shared::cluster.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
-}
-
 // OUT: conversion of the outputs.  Chosen at run time in the epilogue's loop, the third kind cost 0.7 % of a 517-token layer.
 enum : int { kOutFp16, kOutBf16, kOutBf16Saturated };
 
@@ -826,6 +786,20 @@ static GroupPlan plan_group(int T, int n, const int* K, const int* Nout) {
     return pl;
 }
 
+int encode_activations(CUtensorMap* map, const StageJob& S, int bf16, int T, int box_rows) {
+    EncodeTiledFn enc = encode_tiled_fn();
+    if (!enc) return NQ_ERR_UNSUPPORTED;
+    const cuuint64_t dims[2] = {(cuuint64_t)S.K, (cuuint64_t)T};
+    const cuuint64_t strides[1] = {(cuuint64_t)S.lda * 2};
+    const cuuint32_t box[2] = {(cuuint32_t)kBK, (cuuint32_t)box_rows};
+    const cuuint32_t estr[2] = {1, 1};
+    const CUresult r = enc(map, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16,
+                           2, const_cast<void*>(S.a), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                           CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? NQ_OK : NQ_ERR_UNSUPPORTED;
+}
+
 // One stage of up to four linears: out_j[T, Nout_j] = (a_j[T, K_j] . W_j^T) * post_j.
 static int launch_stage(const StageJob* jobs, int n, int T, StageTypes ty, int saturate, unsigned* status, cudaStream_t stream) {
     if (n < 1 || n > kMaxGemmJobs) return NQ_ERR_UNSUPPORTED;
@@ -839,6 +813,10 @@ static int launch_stage(const StageJob* jobs, int n, int T, StageTypes ty, int s
         Ks[j] = S.K; Ns[j] = S.Nout;
     }
     if (T <= batch_max_tokens(jobs, n)) return launch_batch_stage(jobs, n, T, ty, saturate, false, false, false, status, stream);
+    if (T <= kWgemmMostTokens) {
+        const int st = launch_wgemm_stage(jobs, n, T, ty, saturate, status, stream);
+        if (st != NQ_ERR_UNSUPPORTED) return st;     // (input scales of more columns than shared memory holds: below)
+    }
     { const int st_attr = set_kernel_attributes(); if (st_attr != NQ_OK) return st_attr; }
     const GroupPlan pl = plan_group(T, n, Ks, Ns);
     const int mh = pl.mh, nh = pl.nh;

@@ -2,6 +2,7 @@
 // linears.  Implemented by the tensor-core GEMM (nq_gemm.cu) and, for few tokens, by the batch kernel (nq_batch.cu).
 #pragma once
 
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 namespace nq {
@@ -27,8 +28,7 @@ struct StageTypes {
     int io_bf16, a_bf16, out_bf16, exp_sign;
 };
 
-constexpr int kBatchMostTokens = 32;    // of the batch kernel: all that its four column groups hold, and there it is
-                                        // still ahead of the GEMM (see the figures in nq_batch.cu)
+constexpr int kBatchMostTokens = 16;    // of the batch kernel: its two column groups (beyond, nq_wgemm.cu is faster; figures in nq_batch.cu)
 // The same, or 0 where it cannot take the jobs.
 int batch_max_tokens(const StageJob* jobs, int n);
 // `frag_in` / `frag_out`: the activations / the output are an intermediate in the batch kernel's fragment order, of
@@ -39,5 +39,13 @@ size_t batch_fragment_bytes(int T, int K);
 constexpr int kSplitTokens = 4;
 int launch_batch_stage(const StageJob* jobs, int n, int T, StageTypes ty, int saturate, bool frag_in, bool frag_out, bool split,
                        unsigned* status, cudaStream_t stream);
+
+// Tensor map of a stage's activations: boxes of 64 columns x `box_rows` tokens, 128-byte swizzle.
+int encode_activations(CUtensorMap* map, const StageJob& S, int bf16, int T, int box_rows);
+
+// GEMM with the weights on the row side (nq_wgemm.cu).  Up to this many tokens it was faster on each of 14 shapes (at 384 tokens by
+// 4 to 60 %); at 517 a layer takes 257 us with it and 241 with the 256-token tiles.
+constexpr int kWgemmMostTokens = 384;
+int launch_wgemm_stage(const StageJob* jobs, int n, int T, StageTypes ty, int saturate, unsigned* status, cudaStream_t stream);
 
 }  // namespace nq
