@@ -20,7 +20,7 @@ EXT_PATH = os.path.join(PKG_DIR, "_nq_torch.so")
 EXT_SOURCE = "nq_torch.cpp"
 INCLUDE = os.path.join(os.path.dirname(PKG_DIR), "include")
 
-SOURCES = ["nq_core.cu", "nq_pack.cu", "nq_gemv.cu", "nq_gemm.cu", "nq_wgemm.cu", "nq_batch.cu", "nq_comm.cu", "nq_dense.cu", "nq_probe.cu"]
+SOURCES = ["nq_core.cu", "nq_pack.cu", "nq_gemv.cu", "nq_gemm.cu", "nq_wgemm.cu", "nq_pgemm.cu", "nq_batch.cu", "nq_comm.cu", "nq_dense.cu", "nq_probe.cu"]
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",

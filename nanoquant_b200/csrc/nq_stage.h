@@ -1,5 +1,5 @@
 // One stage of a launch group as the host sees it: Out_j[T, Nout_j] = (A_j[T, K_j] . W_j^T) * post_j for up to four
-// linears.  Implemented by the tensor-core GEMM (nq_gemm.cu) and, for few tokens, by the batch kernel (nq_batch.cu).
+// linears.  Implemented by the tensor-core GEMMs (nq_wgemm.cu, nq_pgemm.cu) and, for few tokens, by the batch kernel (nq_batch.cu).
 #pragma once
 
 #include <cuda.h>
@@ -26,7 +26,11 @@ struct StageJob {
 // Types of a stage: scales / bias / residual, MMA operands, output; sign of the row exponents (0: none).
 struct StageTypes {
     int io_bf16, a_bf16, out_bf16, exp_sign;
+    int order = 0;          // kOrderOut, kOrderIn
 };
+// The intermediate between two stages of nq_wgemm.cu or nq_pgemm.cu has the middle two of every four columns swapped, which costs the
+// first stage nothing (its MMA rows may have any order) and halves the expansion of the second.
+enum : int { kOrderOut = 1, kOrderIn = 2 };
 
 constexpr int kBatchMostTokens = 16;    // of the batch kernel: its two column groups (beyond, nq_wgemm.cu is faster; figures in nq_batch.cu)
 // The same, or 0 where it cannot take the jobs.
@@ -43,9 +47,22 @@ int launch_batch_stage(const StageJob* jobs, int n, int T, StageTypes ty, int sa
 // Tensor map of a stage's activations: boxes of 64 columns x `box_rows` tokens, 128-byte swizzle.
 int encode_activations(CUtensorMap* map, const StageJob& S, int bf16, int T, int box_rows);
 
-// GEMM with the weights on the row side (nq_wgemm.cu).  Up to this many tokens it was faster on each of 14 shapes (at 384 tokens by
-// 4 to 60 %); at 517 a layer takes 257 us with it and 241 with the 256-token tiles.
-constexpr int kWgemmMostTokens = 384;
-int launch_wgemm_stage(const StageJob* jobs, int n, int T, StageTypes ty, int saturate, unsigned* status, cudaStream_t stream);
+// GEMMs with the weights on the row side of the MMA; `us` is the predicted time of the launch.
+// nq_wgemm.cu: tiles of 128 rows, K split over a cluster, two CTAs per SM.  False: no plan (input scales of too many columns).
+struct WgemmPlan {
+    float us;
+    int ntok, stages, csplit, owned, off_recv, off_pre, smem;
+};
+bool plan_wgemm(const StageJob* jobs, int n, int T, int order, WgemmPlan& plan);
+int launch_wgemm_stage(const StageJob* jobs, int n, int T, StageTypes ty, int saturate, const WgemmPlan& plan, unsigned* status,
+                       cudaStream_t stream);
+// nq_pgemm.cu: tiles of 256 rows by pairs of CTAs, several tiles each.  Takes everything.
+struct PgemmPlan {
+    float us;
+    int ntok, accs;
+};
+PgemmPlan plan_pgemm(const StageJob* jobs, int n, int T, int order);
+int launch_pgemm_stage(const StageJob* jobs, int n, int T, StageTypes ty, int saturate, const PgemmPlan& plan, unsigned* status,
+                       cudaStream_t stream);
 
 }  // namespace nq

@@ -84,4 +84,50 @@ __device__ __forceinline__ bool mbar_try_cluster(uint32_t bar, uint32_t parity) 
     return ok != 0;
 }
 
+// ---------------------------------------------------------------------------
+// sign bits -> the A operand in tensor memory
+// ---------------------------------------------------------------------------
+// tcgen05.st 16x256b: of a 16-column block of 16 rows, lane 4g + q has the columns 4q..4q+3 (two words) of the rows g and g + 8: what the
+// same lane holds in the tile layout.
+__device__ __forceinline__ void tmem_st_frag4(uint32_t taddr, const uint32_t (&v)[16]) {
+    asm volatile("tcgen05.st.sync.aligned.16x256b.x4.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
+                 ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]),
+                 "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
+                 : "memory");
+}
+// Selector nibble 8 + b: the sign of byte b in every bit.
+__device__ __forceinline__ uint32_t spread_signs(uint32_t u, uint32_t sel) {
+    uint32_t r;
+    asm("prmt.b32 %0, %1, 0, %2;" : "=r"(r) : "r"(u), "r"(sel));
+    return r;
+}
+// 64 columns of 16 rows: `w` with the bits of column class j at 8 b + j + 4 - (j & 4), half `hf` of the 128 columns -> the words of
+// tcgen05.st 16x256b.x4, +-pn.  Two ALU operations per two weights.
+__device__ __forceinline__ void expand_columns(const uint4& w, int hf, const uint2 (&pn)[4], uint32_t (&v)[16]) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int sh = 3 - (2 * hf + (i >> 1));
+        const uint32_t u0 = ((i & 1) ? w.z : w.x) << sh, u1 = ((i & 1) ? w.w : w.y) << sh;
+        v[4 * i + 0] = (spread_signs(u0, 0x9988u) & 0x80008000u) ^ pn[i].x;
+        v[4 * i + 1] = (spread_signs(u0, 0xBBAAu) & 0x80008000u) ^ pn[i].y;
+        v[4 * i + 2] = (spread_signs(u1, 0x9988u) & 0x80008000u) ^ pn[i].x;
+        v[4 * i + 3] = (spread_signs(u1, 0xBBAAu) & 0x80008000u) ^ pn[i].y;
+    }
+}
+// The same for +-1 and columns whose middle two of every four are swapped (kOrderIn): the bits of a pair are 16 apart, one ALU
+// operation per two weights.
+__device__ __forceinline__ void expand_swapped(const uint4& w, int hf, uint32_t one2, uint32_t (&v)[16]) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int sh = 3 - (2 * hf + (i >> 1));
+        const uint32_t w0 = (i & 1) ? w.z : w.x, w1 = (i & 1) ? w.w : w.y;
+        v[4 * i + 0] = ((w0 << (sh + 8)) & 0x80008000u) ^ one2;
+        v[4 * i + 1] = ((w0 << sh) & 0x80008000u) ^ one2;
+        v[4 * i + 2] = ((w1 << (sh + 8)) & 0x80008000u) ^ one2;
+        v[4 * i + 3] = ((w1 << sh) & 0x80008000u) ^ one2;
+    }
+}
+// 0 2 1 3 4 6 5 7
+__device__ __forceinline__ int swap_middle(int g) { return (g & 4) | ((g & 1) << 1) | ((g >> 1) & 1); }
+
 }  // namespace nq

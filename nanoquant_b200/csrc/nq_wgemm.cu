@@ -26,7 +26,8 @@
 // of it the expansion (64 half-rate ALU operations of every warp per step, plus wait, store and signal), and 64 tokens of MMA are half
 // of that.  k blocks of 64 cost 0.24 each: the signalling.  An issuing branch by lane number instead of elect.sync costs 0.05 more.
 //
-// Stages through the 128-row-token GEMM and through this kernel (one launch after another in a graph, us):
+// Stages through tiles of 128 tokens whose weights were expanded into shared memory, and through this kernel, one launch after another in a
+// graph, us, before the second stage's swapped column order (kOrderIn), which takes 5 to 10 % off it:
 //   K -> rows            33 tokens       64              128             256             384
 //   4096 -> 2016         9.8 -> 5.8      9.8 -> 7.0      10.9 -> 7.7     12.3 -> 9.7     15.1 -> 13
 //   2944 -> 11008        15.9 -> 8.6     16.1 -> 9.3     18.2 -> 13.6    23.5 -> 19.6    31.4 -> 21.1
@@ -68,6 +69,7 @@ struct alignas(16) WHead {
     int T;
     int ntok, stages;      // tokens of a tile (a multiple of 16), pipeline stages of 128 columns
     int is_bf16, a_bf16, saturate, exp_sign;
+    int order;             // kOrderOut, kOrderIn
     int csplit, owned;
     int off_recv, off_pre;
 };
@@ -94,12 +96,6 @@ __device__ __forceinline__ void umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64
 __device__ __forceinline__ void umma_commit_w(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
-__device__ __forceinline__ void tmem_st_frag4(uint32_t taddr, const uint32_t (&v)[16]) {
-    asm volatile("tcgen05.st.sync.aligned.16x256b.x4.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
-                 ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]),
-                 "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
-                 : "memory");
-}
 __device__ __forceinline__ void tmem_ld_frag2(uint32_t taddr, float (&r)[8]) {
     asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
                  : "=f"(r[0]), "=f"(r[1]), "=f"(r[2]), "=f"(r[3]), "=f"(r[4]), "=f"(r[5]), "=f"(r[6]), "=f"(r[7])
@@ -116,13 +112,6 @@ __device__ __forceinline__ void tmem_ld_frag8(uint32_t taddr, float (&r)[4][8]) 
                  : "r"(taddr) : "memory");
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
-// selector nibble 8 + b: the sign of byte b in every bit
-__device__ __forceinline__ uint32_t spread_signs(uint32_t u, uint32_t sel) {
-    uint32_t r;
-    asm("prmt.b32 %0, %1, 0, %2;" : "=r"(r) : "r"(u), "r"(sel));
-    return r;
-}
-
 template <int OUT>
 __global__ void __launch_bounds__(kWThreads, 2) wgemm_kernel(const __grid_constant__ WParams Pc) {
     extern __shared__ unsigned char smem_raw[];
@@ -246,8 +235,9 @@ __global__ void __launch_bounds__(kWThreads, 2) wgemm_kernel(const __grid_consta
         const int grp = ew >> 2, rg0 = (n0 >> 4) + 2 * (warp & 3);
         const bool there0 = rg0 < J.row_groups, there1 = rg0 + 1 < J.row_groups;
         const int chunks = J.chunks;
-        const uint4* wt0 = J.tiles + ((size_t)(there0 ? rg0 : 0) * chunks + c_begin) * 32 + lane;
-        const uint4* wt1 = J.tiles + ((size_t)(there1 ? rg0 + 1 : 0) * chunks + c_begin) * 32 + lane;
+        const int src_lane = P.order == kOrderOut ? 4 * swap_middle(lane >> 2) + q : lane;
+        const uint4* wt0 = J.tiles + ((size_t)(there0 ? rg0 : 0) * chunks + c_begin) * 32 + src_lane;
+        const uint4* wt1 = J.tiles + ((size_t)(there1 ? rg0 + 1 : 0) * chunks + c_begin) * 32 + src_lane;
         uint4 w0n = make_uint4(0u, 0u, 0u, 0u), w1n = w0n, w0nn = w0n, w1nn = w0n;
         if (c_begin < c_end) {
             if (there0) w0n = __ldg(wt0);
@@ -258,7 +248,7 @@ __global__ void __launch_bounds__(kWThreads, 2) wgemm_kernel(const __grid_consta
             if (there1) w1nn = __ldg(wt1 + 32);
         }
         if (lane == 0 && c_begin + 2 < c_end && (grp ? there1 : there0))
-            asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"((grp ? wt1 : wt0) + 64), "r"((uint32_t)(c_end - c_begin - 2) * 512u) : "memory");
+            asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"((grp ? wt1 : wt0) - src_lane + 64), "r"((uint32_t)(c_end - c_begin - 2) * 512u) : "memory");
         const int tu = (int)threadIdx.x - 128;
         uint16_t raw_post = 0, raw_bias = 0;
         if (tu < kWRows && n0 + tu < J.Nout) {
@@ -266,7 +256,7 @@ __global__ void __launch_bounds__(kWThreads, 2) wgemm_kernel(const __grid_consta
             if (J.bias) asm volatile("ld.global.nc.u16 %0, [%1];" : "=h"(raw_bias) : "l"(static_cast<const uint16_t*>(J.bias) + n0 + tu));
         }
         const uint32_t one2 = P.a_bf16 ? 0x3F803F80u : 0x3C003C00u;
-        const bool pre = J.pre != nullptr;
+        const bool pre = J.pre != nullptr, in_order = P.order != kOrderIn;
         const uint2* s_pre = reinterpret_cast<const uint2*>(smem + P.off_pre) + q;
         const int K_left = J.K - 256 * c_begin;
         const uint32_t a_lane = tmem_a + ((uint32_t)(32 * (warp & 3)) << 16);
@@ -287,30 +277,21 @@ __global__ void __launch_bounds__(kWThreads, 2) wgemm_kernel(const __grid_consta
 #pragma unroll
             for (int hf = 0; hf < 2; ++hf) {       // 64 columns
                 uint2 pn[4];
-                if (pre) {
+                if (in_order) {
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        const int k = 128 * ks + 64 * hf + 16 * i;
-                        pn[i] = s_pre[k >> 2];
-                        if (k + 4 * q >= K_left) pn[i] = make_uint2(0u, 0u);     // columns beyond K
+                    for (int i = 0; i < 4; ++i) pn[i] = pre ? s_pre[(128 * ks + 64 * hf + 16 * i) >> 2] : make_uint2(one2, one2);
+                    if (pre && 128 * ks + 64 * hf + 64 > K_left) {       // columns beyond K
+#pragma unroll
+                        for (int i = 0; i < 4; ++i)
+                            if (128 * ks + 64 * hf + 16 * i + 4 * q >= K_left) pn[i] = make_uint2(0u, 0u);
                     }
-                } else {
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) pn[i] = make_uint2(one2, one2);
                 }
 #pragma unroll
                 for (int rr = 0; rr < 2; ++rr) {
                     const uint4& w = rr ? w1 : w0;
                     uint32_t v[16];
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        const int sh = 3 - (2 * hf + (i >> 1));
-                        const uint32_t u0 = ((i & 1) ? w.z : w.x) << sh, u1 = ((i & 1) ? w.w : w.y) << sh;
-                        v[4 * i + 0] = (spread_signs(u0, 0x9988u) & 0x80008000u) ^ pn[i].x;
-                        v[4 * i + 1] = (spread_signs(u0, 0xBBAAu) & 0x80008000u) ^ pn[i].y;
-                        v[4 * i + 2] = (spread_signs(u1, 0x9988u) & 0x80008000u) ^ pn[i].x;
-                        v[4 * i + 3] = (spread_signs(u1, 0xBBAAu) & 0x80008000u) ^ pn[i].y;
-                    }
+                    if (in_order) expand_columns(w, hf, pn, v);
+                    else expand_swapped(w, hf, one2, v);
                     if (hf == 0 && rr == 0) {
                         ok = mbar_wait_warp(bar_free(s), ph ^ 1, abort_flag, P.status);
                         tc_fence_after();
@@ -321,7 +302,7 @@ __global__ void __launch_bounds__(kWThreads, 2) wgemm_kernel(const __grid_consta
             asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(bar_ready(s));
+            if (lane == 0 && ok) mbar_arrive(bar_ready(s));
             s += 2;
             if (s >= stages) { s -= stages; ph ^= 1; }
         }
@@ -373,8 +354,8 @@ __global__ void __launch_bounds__(kWThreads, 2) wgemm_kernel(const __grid_consta
         asm volatile("bar.sync 2, 256;" ::: "memory");        // scales visible
         const int g = lane >> 2, q = lane & 3;
         if (ok) {
-            const int r0 = 16 * rgl + g;
-            const float sc0 = s_post[r0], sc1 = s_post[r0 + 8], bi0 = s_bias[r0], bi1 = s_bias[r0 + 8];
+            const int r0 = 16 * rgl + g, rs = 16 * rgl + (P.order == kOrderOut ? swap_middle(g) : g);
+            const float sc0 = s_post[rs], sc1 = s_post[rs + 8], bi0 = s_bias[rs], bi1 = s_bias[rs + 8];
             const uint16_t* resid = static_cast<const uint16_t*>(J.resid);
             int idx = 0;
             for (int b = crank; b < live; b += csplit, ++idx) {
@@ -476,10 +457,7 @@ static const void* w_kernel(int out) {
 constexpr int kWSmemMost = 112 * 1024;   // two CTAs per SM
 
 // Shared memory of a plan; false if it does not fit half an SM.
-struct WPlan {
-    int ntok, stages, csplit, owned, off_recv, off_pre, smem;
-};
-static bool w_layout(int ntok, int csplit, int pre_bytes, WPlan& p) {
+static bool w_layout(int ntok, int csplit, int pre_bytes, WgemmPlan& p) {
     const int owned = (ntok / 16 + csplit - 1) / csplit;
     const int recv = (csplit - 1) * owned * 8192;
     p.ntok = ntok; p.csplit = csplit; p.owned = owned;
@@ -539,7 +517,7 @@ static int w_capacity(int s) {
 // 608..11008 columns, 33 to 384 tokens, 1 to 8 CTAs per cluster, all tile widths): the plan it picks is 1.3 % above the best on
 // average.  A CTA's steps cost less while it has its SM for itself (`one`) than when two share it (`two`); up to 56 tokens the
 // expansion hides the MMA; every CTA more is contention; clusters above four exchange more and fit less well.
-static bool w_plan(const StageJob* jobs, int n, int T, WPlan& best) {
+bool plan_wgemm(const StageJob* jobs, int n, int T, int order, WgemmPlan& best) {
     int most_chunks = 0, most_pre = 0;
     for (int j = 0; j < n; ++j) {
         const int c = (jobs[j].K + 255) / 256;
@@ -550,14 +528,13 @@ static bool w_plan(const StageJob* jobs, int n, int T, WPlan& best) {
     for (int j = 0; j < n; ++j) rows += (jobs[j].Nout + kWRows - 1) / kWRows;
     const int all = (T + 15) / 16 * 16;
     static const int sizes[] = {16, 32, 48, 64, 80, 96, 112, 128};
-    float least = 0.f;
     bool found = false;
     const int sms = sm_count();
     for (int ntok : sizes) {
         if (ntok > all || (ntok < 32 && ntok < all)) continue;
         const int tiles = rows * ((T + ntok - 1) / ntok);
         for (int s = 1; s <= kWMaxSplit && s <= most_chunks; ++s) {
-            WPlan p;
+            WgemmPlan p;
             if (!w_layout(ntok, s, (most_pre + s - 1) / s * 512, p)) continue;
             const int resident = w_capacity(s);
             if (resident <= 0) continue;
@@ -566,23 +543,22 @@ static bool w_plan(const StageJob* jobs, int n, int T, WPlan& best) {
             const float one = 0.38f + 0.002f * over, two = 0.46f + 0.0024f * over;
             const int full = ctas / resident, rest = ctas % resident;
             float t = 0.5f + 0.03f * ntok + 2.2f * ctas / sms + (ctas > sms ? -0.7f : 0.f) + (s > 1 ? -0.18f + 0.01f * s + (s > 4 ? 0.22f * (s - 4) : 0.f) : 0.f);
-            t += (most_pre ? 1.14f : 1.f) * steps * (full * (resident > sms ? two : one) + (rest == 0 ? 0.f : rest > sms ? two : one));
-            if (!found || t < least) { least = t; best = p; found = true; }
+            t += (order == kOrderIn ? 0.82f : most_pre ? 1.14f : 1.f) * steps * (full * (resident > sms ? two : one) + (rest == 0 ? 0.f : rest > sms ? two : one));
+            if (!found || t < best.us) { best = p; best.us = t; found = true; }
         }
     }
     return found;
 }
 
-int launch_wgemm_stage(const StageJob* jobs, int n, int T, StageTypes ty, int saturate, unsigned* status, cudaStream_t stream) {
+int launch_wgemm_stage(const StageJob* jobs, int n, int T, StageTypes ty, int saturate, const WgemmPlan& pl, unsigned* status,
+                       cudaStream_t stream) {
     { const int st = w_attributes(); if (st != NQ_OK) return st; }
-    WPlan pl;
-    if (!w_plan(jobs, n, T, pl)) return NQ_ERR_UNSUPPORTED;
     WParams P;
     memset(&P, 0, sizeof(P));
     WHead& H = P.head;
     H.njobs = n; H.status = status; H.T = T; H.ntok = pl.ntok; H.stages = pl.stages; H.csplit = pl.csplit;
     H.owned = pl.owned; H.off_recv = pl.off_recv; H.off_pre = pl.off_pre;
-    H.is_bf16 = ty.io_bf16; H.a_bf16 = ty.a_bf16; H.saturate = saturate; H.exp_sign = ty.exp_sign;
+    H.is_bf16 = ty.io_bf16; H.a_bf16 = ty.a_bf16; H.saturate = saturate; H.exp_sign = ty.exp_sign; H.order = ty.order;
     int tiles = 0;
     for (int j = 0; j < n; ++j) {
         const StageJob& S = jobs[j];

@@ -1,6 +1,7 @@
-"""GEMM with the weights on the row side (17 tokens up to its limit) at the edges of its tiles: widths of 16 to 128 tokens and
-their remainders, 128-row tiles, steps of 128 columns and scales beyond the last column, clusters whose last CTAs have no columns of a
-job, with bias and residual, in a launch group; results that do not change from run to run."""
+"""The two GEMMs with the weights on the row side (17 tokens and more) at the edges of their tiles: widths of 16 to 256 tokens and
+their remainders, tiles of 128 and 256 rows, steps of 128 columns and scales beyond the last column, clusters whose last CTAs have no
+columns of a job, pairs with several tiles and an odd number of steps in each (their stages then start anywhere), with bias and residual,
+in a launch group; results that do not change from run to run."""
 import pytest
 import torch
 
@@ -11,7 +12,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
-@pytest.mark.parametrize("T", [17, 48, 65, 129, 200, 384, 385])
+@pytest.mark.parametrize("T", [17, 48, 65, 129, 200, 385])
 @pytest.mark.parametrize("shapes", [
     [(8, 8, 1)], [(264, 136, 17), (264, 256, 400)], [(4104, 264, 1001)], [(192, 1032, 4000)], [(11016, 72, 130)],
     [(1024, 96, 500), (1024, 1288, 64), (1024, 40, 64), (1024, 8, 8)],
@@ -20,7 +21,15 @@ def test_tile_edges(shapes, T, dtype):
     edges.test_batch_tile_edges(shapes, T, dtype)
 
 
-@pytest.mark.parametrize("T", [24, 100])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("T,shapes", [
+    (130, [(328, 200, 30001)]), (513, [(392, 4104, 6001)]), (1030, [(904, 648, 9000), (904, 136, 1001), (904, 264, 2056)]), (2047, [(264, 1160, 3000)]),
+])
+def test_pairs_with_several_tiles(shapes, T, dtype):
+    edges.test_batch_tile_edges(shapes, T, dtype)
+
+
+@pytest.mark.parametrize("T", [24, 100, 600])
 def test_runs_give_the_same_bits(T):
     from nanoquant_b200 import ops
     L = make_group([(4096, 600, 1000)], T, torch.bfloat16, seed=T)[0]
