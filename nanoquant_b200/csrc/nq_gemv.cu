@@ -35,8 +35,8 @@
 // programmatic stream serialization: the weight loads of both phases are started before griddepcontrol.wait.
 //
 // Measured against the first versions of this kernel (cooperative launch, one scale per token, partial sums added with
-// shared-memory atomics, weights by cp.async per warp): Qwen3-8B decode, eight layers in a graph, one token 291 -> 250 us,
-// four tokens 534 -> 430 us; launched eagerly a call took 10.6 us, of which the cooperative attribute 3.
+// shared-memory atomics, weights by cp.async per warp): Qwen3-8B decode, eight layers in a graph, one token 291 -> 250 us, and 217
+// with the token count a constant, whole sectors polled, the tag read once per CTA and the scales prefetched.
 //
 // A SIMT sign-flip-add inner loop issues ~1.5 instructions per weight and tops out
 // near one third of the HBM rate on this part, which is why the integer MMA is
@@ -64,7 +64,7 @@ constexpr int kMaxChunks = kMaxK / 256;
 constexpr size_t kHeaderBytes = 256;
 constexpr int kMaxSlots = 8;        // weight blocks in flight
 // shared memory: mbarriers; the launch's descriptors; {unit value, sum} per chunk and token; weight slots
-constexpr size_t kOffParams = 128, kOffMeta = 1280;
+constexpr size_t kOffTag = 8 * kMaxSlots, kOffParams = 128, kOffMeta = 1280;
 constexpr size_t kFixedBytes = kOffMeta + (size_t)kMaxTok * kMaxChunks * 8;
 static_assert(8 * kMaxSlots <= kOffParams && kFixedBytes % 128 == 0, "shared memory map");
 constexpr size_t kPartBytes = 32 << 10;    // partial sums of a row block
@@ -297,10 +297,10 @@ __device__ __forceinline__ bool quantise_t(const Job& jb, int T, unsigned char* 
                 for (int i = 0; i < B; ++i)
                     if (left > 0 && t0 + i < sh.t1) {
 #pragma unroll
-                        for (int u = 0; u < 4; ++u)
-                            asm volatile("ld.relaxed.gpu.global.v2.b64 {%0,%1}, [%2];"
-                                         : "=l"(e[i][2 * u]), "=l"(e[i][2 * u + 1])
-                                         : "l"(in + (t0 + i) * ld + c * 256 + 2 * u) : "memory");
+                        for (int u = 0; u < 2; ++u)      // whole sectors: in 16-byte loads every sector was asked for twice (231 -> 217 us)
+                            asm volatile("ld.relaxed.gpu.global.v4.b64 {%0,%1,%2,%3}, [%4];"
+                                         : "=l"(e[i][4 * u]), "=l"(e[i][4 * u + 1]), "=l"(e[i][4 * u + 2]), "=l"(e[i][4 * u + 3])
+                                         : "l"(in + (t0 + i) * ld + c * 256 + 4 * u) : "memory");
                     } else {
 #pragma unroll
                         for (int u = 0; u < 8; ++u) e[i][u] = (unsigned long long)tc.tag << 32;
@@ -555,7 +555,9 @@ __device__ __noinline__ void help_phase1(const Job& jb, int T, unsigned char* xq
 // ---------------------------------------------------------------------------
 // the kernel
 // ---------------------------------------------------------------------------
-// CG: column groups of 8 MMA columns (1: up to two tokens, 2: up to four).
+// TOK: tokens of the launch, 1 or 2 (one column group of 8 MMA columns); or 4, three or four of them (two groups).  The count as a
+// constant takes loops and divisions out of a chain of dependent instructions: eight layers in a graph, one token, Qwen3-8B 248 -> 238 us,
+// Llama-3.2-1B 195 -> 188; with a copy of the code per phase 237 and 183.
 //
 // The launch takes about 7 us; its 16 warps need 4 issue cycles of every scheduler, 2 ns, for each instruction of the
 // common path, and most of them wait for something short.  So the descriptors come into shared memory in one round trip,
@@ -563,8 +565,9 @@ __device__ __noinline__ void help_phase1(const Job& jb, int T, unsigned char* xq
 // register is a cold line: 40 bytes of stack made the launch 10 % slower), and ONE thread moves the weights: a CTA's row
 // groups are contiguous in the tile layout, so a block of them is one bulk copy, and the blocks of both phases that fit
 // in shared memory (all of them, for 8B-class layers) are on their way before the dependency wait.
-template <int KIND, int CG>
+template <int KIND, int TOK>
 __global__ void __launch_bounds__(kGemvThreads, 1) gemv_group_kernel(const __grid_constant__ GemvParams Pc) {
+    constexpr int CG = TOK <= 2 ? 1 : 2;
     extern __shared__ __align__(128) unsigned char smem[];
     const int tid = threadIdx.x, lane = tid & 31;
     const uint32_t bars = smem_u32(smem);                                  // weight slot s is full: bars + 8 s
@@ -593,7 +596,7 @@ __global__ void __launch_bounds__(kGemvThreads, 1) gemv_group_kernel(const __gri
     const Job* jobs = P.job;
     int2* meta = reinterpret_cast<int2*>(smem + kOffMeta);                 // [chunk][token] {unit value, sum}
     unsigned char* weights = smem + kFixedBytes;
-    const int T = P.T, slots = P.slots, slot_bytes = P.slot_bytes;
+    const int T = TOK <= 2 ? TOK : P.T, slots = P.slots, slot_bytes = P.slot_bytes;
     unsigned char* xq = smem + P.xq_off;
     float* part = reinterpret_cast<float*>(smem + P.part_off);
     unsigned* const header = P.header;
@@ -630,6 +633,19 @@ __global__ void __launch_bounds__(kGemvThreads, 1) gemv_group_kernel(const __gri
 #pragma unroll 1
         for (int s = 0; s < slots; ++s) load_block();
     }
+    // Scales on their way to L2: a model's are in memory when its turn comes, and the input's would be waited for beside the input
+    // (eight Qwen3-8B layers at one token 223.5 -> 217.0 us; one bulk prefetch of the input's alone 221.9).
+    if (tid < 64) {
+#pragma unroll
+        for (int ph = 0; ph < 2; ++ph) {
+            if (groups[ph] == 0) continue;
+            const Job& jb = jobs[ji[ph]];
+            if (ph == 0)
+                for (int k = 64 * tid; k < jb.K; k += 64 * 64) asm volatile("prefetch.global.L2 [%0];" ::"l"(static_cast<const uint16_t*>(jb.pre) + k));
+            if (jb.post && 64 * tid < 16 * groups[ph])
+                asm volatile("prefetch.global.L2 [%0];" ::"l"(static_cast<const uint16_t*>(jb.post) + min(16 * first[ph] + 64 * tid, jb.rows - 1)));
+        }
+    }
     // Programmatic dependent launch: everything above may overlap with the tail of the previous kernel in the stream;
     // activations and scratch (shared with that kernel) are only touched after it has completed.
     asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -639,10 +655,9 @@ __global__ void __launch_bounds__(kGemvThreads, 1) gemv_group_kernel(const __gri
 
     int slot = 0;                            // of the next weight block, and its barrier's phase
     uint32_t parity = 0;
-    // One copy of the code for both phases up to two tokens, whose launches are short enough to feel the cold instruction
-    // lines of a second one (8B-class layers, 32 launches: 250 -> 254 us at one token); a copy each for more tokens, where
-    // the compiler then keeps the phase's descriptor in fewer registers (four tokens: 432 -> 421 us).
-#pragma unroll CG
+    // A copy of the code for each phase: the compiler then keeps the phase's descriptor in fewer registers.  (One copy for both, while the
+    // token count was not a constant either: 250 us and 254; now 234 and 231.)
+#pragma unroll 2
     for (int ph = 0; ph < 2; ++ph) {
         const int my_groups = ph ? groups[1] : groups[0], row0 = 16 * (ph ? first[1] : first[0]);
         const Job& jb = jobs[ph ? ji[1] : ji[0]];
@@ -651,19 +666,21 @@ __global__ void __launch_bounds__(kGemvThreads, 1) gemv_group_kernel(const __gri
         // not carried around a loop: that would copy the registers, and the copy would wait for the loads.)
         RawOut raw0 = {};
         if (ph == 0) {
-            // tag of this launch: read by every thread, used behind the barrier (the round trip overlaps the input loads)
-            TagRaw tag_raw;
-            tag_read(tag_raw, header);
+            // Tag of this launch: one thread's read, used behind the barrier; the round trip overlaps the input loads.  (Read by every
+            // warp it was 16 requests of each CTA for one line of L2, and the launch 1 to 5 % slower.)
+            TagRaw tag_raw = {};
+            if (tid == kGemvThreads - 1) tag_read(tag_raw, header);
             if (my_groups > 0) {
-                if (jb.vec) quantise_x<KIND, 2 * CG>(jb, T, xq, meta);
+                if (jb.vec) quantise_x<KIND, TOK>(jb, T, xq, meta);
                 else quantise_x_any<KIND>(jb, T, xq, meta);
                 load_raw_out(raw0, jb, row0, min(jb.gb, my_groups) * 16, T, tid >> 2);
             }
+            if (tid == kGemvThreads - 1) *reinterpret_cast<TagRaw*>(smem + kOffTag) = tag_raw;
             __syncthreads();   // quantised input complete
-            tag_finish(tc, tag_raw, header, P.spin_limit);
+            tag_finish(tc, *reinterpret_cast<const TagRaw*>(smem + kOffTag), header, P.spin_limit);
         } else if (my_groups > 0) {
             load_raw_out(raw0, jb, row0, min(jb.gb, my_groups) * 16, T, tid >> 2);
-            while (!__syncthreads_and(quantise_t<2 * CG>(jb, T, xq, meta, tc, help_after))) {
+            while (!__syncthreads_and(quantise_t<TOK>(jb, T, xq, meta, tc, help_after))) {
                 help_phase1<KIND, CG>(jobs[ji[1] - kMaxJobs], T, xq, meta, part, tc.tag, header + 3);
                 help_after = ~0u;     // every row has carried the tag now: what is missing again, another launch overwrites
             }
@@ -696,8 +713,9 @@ __global__ void __launch_bounds__(kGemvThreads, 1) gemv_group_kernel(const __gri
 static size_t round_up(size_t v, size_t m) { return (v + m - 1) / m * m; }
 
 static const void* gemv_kernel(int kind, int tokens) {
-    if (kind == KIND_F16) return tokens <= 2 ? (const void*)gemv_group_kernel<KIND_F16, 1> : (const void*)gemv_group_kernel<KIND_F16, 2>;
-    return tokens <= 2 ? (const void*)gemv_group_kernel<KIND_BF16, 1> : (const void*)gemv_group_kernel<KIND_BF16, 2>;
+    if (kind == KIND_F16)
+        return tokens == 1 ? (const void*)gemv_group_kernel<KIND_F16, 1> : tokens == 2 ? (const void*)gemv_group_kernel<KIND_F16, 2> : (const void*)gemv_group_kernel<KIND_F16, kMaxTok>;
+    return tokens == 1 ? (const void*)gemv_group_kernel<KIND_BF16, 1> : tokens == 2 ? (const void*)gemv_group_kernel<KIND_BF16, 2> : (const void*)gemv_group_kernel<KIND_BF16, kMaxTok>;
 }
 
 // Opt-in shared memory limit of every instantiation, set once per device.
@@ -706,8 +724,8 @@ static int dynamic_smem_limit(int dev, int* out) {
     if (cached[dev & 63] == 0) {
         int optin = 0, lim = 1 << 30;
         NQ_CUDA_TRY(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-        for (int i = 0; i < 4; ++i) {
-            const void* fn = gemv_kernel(i & 1 ? KIND_BF16 : KIND_F16, i & 2 ? kMaxTok : 1);
+        for (int i = 0; i < 6; ++i) {
+            const void* fn = gemv_kernel(i & 1 ? KIND_BF16 : KIND_F16, i / 2 == 0 ? 1 : i / 2 == 1 ? 2 : kMaxTok);
             cudaFuncAttributes fa;
             NQ_CUDA_TRY(cudaFuncGetAttributes(&fa, fn));
             const int v = optin - (int)fa.sharedSizeBytes;  // the opt-in limit covers static + dynamic
@@ -911,7 +929,8 @@ static int launch_decode(const nq_linear_desc* d, int n_linears, int t_first, in
         const size_t part_room = room - slot_most < kPartBytes ? room - slot_most : kPartBytes;
         size_t part_used = 0, slot_used = 0;
         int most_blocks = 0;
-        size_t off = kHeaderBytes;
+        // the intermediate is loaded in 32 bytes: 16 back into the unused end of the header for a scratch between two multiples of 32
+        size_t off = kHeaderBytes - (reinterpret_cast<uintptr_t>(scratch) & 16);
         int cta[2] = {0, 0};            // first CTA of the next job's range in the two phases
         for (int i = 0; i < n_linears; ++i) {
             const nq_linear_desc& L = d[i];

@@ -8,12 +8,13 @@ from tests.util import assert_parity, exact_np, make_layer, tiles_on_gpu
 pytestmark = pytest.mark.gpu
 
 
-def _run(L, T, N, R, M, dtype):
+def _run(L, T, N, R, M, dtype, offset=0):
     from nanoquant_b200 import _lib
     Lb = _lib.lib()
     st = torch.cuda.current_stream().cuda_stream
     nb = Lb.nq_gemv_scratch_bytes(T, N, R, M)
-    scratch = torch.zeros(nb, dtype=torch.uint8, device="cuda")
+    room = torch.zeros(nb + offset + 64, dtype=torch.uint8, device="cuda")
+    scratch = room[offset:offset + nb]
     y = torch.full((T, M), float("nan"), dtype=dtype, device="cuda")
     vt, ut = tiles_on_gpu(L["V"]), tiles_on_gpu(L["U"])
     args = (L["x"].data_ptr(), L["s_pre"].data_ptr(), vt.data_ptr(), L["s_mid"].data_ptr(), ut.data_ptr(),
@@ -26,6 +27,7 @@ def _run(L, T, N, R, M, dtype):
     torch.cuda.synchronize()
     assert Lb.nq_scratch_status(scratch.data_ptr(), st) == 0
     assert torch.equal(first, y)
+    assert not room[:offset].any() and not room[offset + nb:].any()
     return y, scratch.view(torch.int32)[3].item()       # result, number of CTAs that computed others' rows
 
 
@@ -41,6 +43,16 @@ def test_tile_edges(N, R, M, T):
     L = make_layer(N, R, M, T, dtype, seed=N + R + M)
     y, _ = _run(L, T, N, R, M, dtype)
     assert_parity(exact_np(y), L["y64"], dtype, what=f"N={N} R={R} M={M} T={T}")
+
+
+@pytest.mark.parametrize("T", [1, 2, 3, 4])
+@pytest.mark.parametrize("N,R,M", [(256, 16, 16), (1003, 333, 777)])
+def test_scratch_between_two_multiples_of_32(N, R, M, T):
+    # 16 bytes are what the scratch has to be aligned to; the intermediate is loaded in 32
+    L = make_layer(N, R, M, T, torch.bfloat16, seed=3)
+    want, _ = _run(L, T, N, R, M, torch.bfloat16)
+    y, _ = _run(L, T, N, R, M, torch.bfloat16, offset=16)
+    assert torch.equal(y, want)
 
 
 @pytest.mark.parametrize("T", [1, 4])
