@@ -19,8 +19,7 @@
 //
 // Splitting K over the CTAs of a cluster (partial sums exchanged through distributed shared memory) and staging the whole
 // input by bulk copies before the loop both measured slower than this at every size.
-// It ends at 16 tokens: eight layers in a graph with this kernel, and through nq_wgemm.cu, us: Qwen3-8B 8 tokens 359 and 453,
-// 16 tokens 436 and 455, 17 tokens (three column groups, a variant that is gone) 625 and 473; Llama-3.2-1B 16 tokens 313 and 302.
+// It ends at 16 tokens (8 for large launches, see batch_max_tokens): 17 tokens took three column groups, eight Qwen3-8B layers 625 us, 473 through nq_wgemm.cu.
 //
 // What bounds it (counters of single launches at 16 tokens, cold): no throughput limit is near.  DRAM 3 to 6 % of its peak,
 // L2 4 to 16, tensor pipe 12 to 19.  The two stages of a group with little work take 8.8 us together, two launches of a fixed
@@ -30,6 +29,7 @@
 // largest stall) with four warps per scheduler to hide that.
 #include <cstddef>
 #include <cstring>
+#include <type_traits>
 
 #include "nq_common.cuh"
 #include "nq_plan.h"
@@ -199,6 +199,8 @@ __global__ void __launch_bounds__(kBatchThreads, 1) batch_stage_kernel(const __g
     for (int blk = 0; blk < groups; blk += gb) {
         const int nb = min(gb, groups - blk);
         const int r0 = (rw * nb * wr_magic) >> 16, r1 = rw < wr ? ((rw + 1) * nb * wr_magic) >> 16 : r0;
+        // quotient by the rows of a block: exact below 2^22 / rows, and there are at most 16 times as many outputs as rows, 512 of them
+        const unsigned nb16_magic = ((1u << 22) + nb * 16 - 1) / (nb * 16);
         // output scale and bias of row `tid` of the block (asm: a plain 16-bit load is widened, that is waited for, at once)
         const int row0 = (first + blk) * 16;
         uint16_t post_raw = 0, bias_raw = 0;
@@ -226,6 +228,12 @@ __global__ void __launch_bounds__(kBatchThreads, 1) batch_stage_kernel(const __g
                     if (spins >= kWeightWaitLimit) { atomicExch(P.status, (unsigned)(-NQ_ERR_TIMEOUT)); break; }
             }
             const uint32_t one2 = BF16 ? 0x3F803F80u : 0x3C003C00u;
+            // Shifts as products with powers of two the compiler cannot see: multiplications do not wait for the half-rate pipe of the LOP3s
+            // (16 tokens, eight layers: Llama-3.2-1B 315 -> 293 us, Qwen3-8B 438 -> 432, two of 8192 columns 393 -> 399; four and eight: level).
+            uint32_t pw[8], p256;
+            asm volatile("mov.u32 %0, %1;" : "=r"(p256) : "r"(256u));
+#pragma unroll
+            for (int i = 0; i < 8; ++i) asm volatile("mov.u32 %0, %1;" : "=r"(pw[i]) : "r"(1u << i));
             // block b of a chunk (columns 32 j + 16 h + ..) against all row groups
             auto block = [&](const uint4 (&w)[kRows], int b, uint32_t se, uint32_t so, const uint32_t (&be)[NT], const uint32_t (&bo)[NT]) {
                 const int j = b >> 1, h = b & 1;
@@ -233,8 +241,9 @@ __global__ void __launch_bounds__(kBatchThreads, 1) batch_stage_kernel(const __g
                 for (int r = 0; r < kRows; ++r)
                     if (r < nr) {
                         const uint32_t w0 = h ? w[r].z : w[r].x, w1 = h ? w[r].w : w[r].y;   // rows g, g + 8
-                        const uint32_t a0 = ((w0 << (15 - j)) & 0x80008000u) ^ se, a2 = ((w0 << (7 - j)) & 0x80008000u) ^ so;
-                        const uint32_t a1 = ((w1 << (15 - j)) & 0x80008000u) ^ se, a3 = ((w1 << (7 - j)) & 0x80008000u) ^ so;
+                        const uint32_t u0 = w0 * pw[7 - j], u1 = w1 * pw[7 - j];
+                        const uint32_t a0 = ((u0 * p256) & 0x80008000u) ^ se, a2 = (u0 & 0x80008000u) ^ so;
+                        const uint32_t a1 = ((u1 * p256) & 0x80008000u) ^ se, a3 = (u1 & 0x80008000u) ^ so;
 #pragma unroll
                         for (int nt = 0; nt < NT; ++nt) mma_16816<BF16>(acc[r][nt], a0, a1, a2, a3, be[nt], bo[nt]);
                     }
@@ -312,46 +321,59 @@ __global__ void __launch_bounds__(kBatchThreads, 1) batch_stage_kernel(const __g
         __syncthreads();   // partial sums complete, this block's weights have been read
         if (++slot == slots) { slot = 0; parity ^= 1u; }
         if (loader) load_block();
-        // outputs: lanes take rows, warps take tokens
+        // Outputs, [token][row of the block] dealt to all threads, three at a time where there are more: the sums over the chunk slices are
+        // chains of shared-memory loads.  Of a split intermediate two neighbouring lanes sum value and remainder.  (A warp per token left
+        // 12 of 16 warps idle at four tokens: eight Qwen3-8B layers 356 -> 346 us, Llama-3.2-1B 264 -> 244, two of 8192 columns 289 -> 269.)
         // An intermediate that is not a pair becomes infinite beyond its type's range, as in the GEMM; the value of a pair
         // stays finite, and it is the remainder that an infinity goes to.  NaN passes every clamp.
+        constexpr bool kPair = SPLIT && FRAG;
         const float lim = P.saturate || (SPLIT && !FRAG) ? (out_bf16 ? 3.3895313892515355e+38f : 64504.0f) : 3.4e38f;
         const uint16_t* const resid = static_cast<const uint16_t*>(jb.resid);
         const int* const row_exp = jb.row_exp;
-        const int kslice = T * tok_stride, frag_out = P.frag_out;
-        const int tokens = SPLIT ? kSplitTokens : T;
-#pragma unroll 1
-        for (int tok = warp; tok < tokens; tok += kBatchWarps) {
-            const float rs = row_exp ? exp2f((float)(P.exp_sign * row_exp[tok])) : 1.f;
-            uint16_t* const out = static_cast<uint16_t*>(jb.out) + (frag_out ? 0 : tok * jb.ld_out + row0);
-#pragma unroll 1
-            for (int idx = lane; idx < nb * 16; idx += 32) {
-                const float* src = part + tok * tok_stride + idx;
-                float v = 0.f;
+        const int kslice = T * tok_stride, frag_out = P.frag_out, nb16 = nb * 16;
+        const int sums = (SPLIT ? kSplitTokens : T) * nb16 * (kPair ? 2 : 1);
+        auto emit = [&](auto many, int e0) {
+            constexpr int U = decltype(many)::value;
+            float v[U];
+            const float* src[U];
+            int tok[U], idx[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int e = min(e0 + u * kBatchThreads, sums - 1), o = kPair ? e >> 1 : e;
+                tok[u] = (int)((unsigned)o * nb16_magic >> 22);
+                idx[u] = o - tok[u] * nb16;
+                src[u] = part + (tok[u] + (kPair && (e & 1) ? kSplitTokens : 0)) * tok_stride + idx[u];
+                v[u] = 0.f;
+            }
 #pragma unroll 4
-                for (int k = 0; k < wk; ++k, src += kslice) v += *src;
-                if (SPLIT && FRAG) {
-                    const float* rest = part + (kSplitTokens + tok) * tok_stride + idx;
-                    float v2 = 0.f;
-#pragma unroll 4
-                    for (int k = 0; k < wk; ++k, rest += kslice) v2 += *rest;
-                    v += v2;
-                }
-                const float2 sc = scale[idx];
-                if (row0 + idx < rows) {
-                    float extra = sc.y;
-                    if (resid) extra += float_of(resid[tok * jb.ld_res + row0 + idx], io_bf16);
-                    const float exact = v * (sc.x * rs) + extra;
-                    v = clamp_or_nan(exact, lim);
-                    if (SPLIT && !FRAG) {
-                        const __nv_bfloat16 value = __float2bfloat16(v);
-                        out[fragment_index<1>(tok, row0 + idx)] = __bfloat16_as_ushort(value);
-                        out[fragment_index<1>(kSplitTokens + tok, row0 + idx)] = __bfloat16_as_ushort(__float2bfloat16(exact - __bfloat162float(value)));
-                        continue;
-                    }
-                    out[frag_out ? fragment_index<NT>(tok, row0 + idx) : idx] = out_bf16 ? __bfloat16_as_ushort(__float2bfloat16(v)) : __half_as_ushort(__float2half(v));
+            for (int k = 0; k < wk; ++k)
+#pragma unroll
+                for (int u = 0; u < U; ++u) { v[u] += *src[u]; src[u] += kslice; }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                if (kPair) v[u] += __shfl_xor_sync(0xffffffffu, v[u], 1);
+                const float2 sc = scale[idx[u]];
+                const int row = row0 + idx[u];
+                if (e0 + u * kBatchThreads >= sums || row >= rows || (kPair && (lane & 1))) continue;
+                const float rs = row_exp ? exp2f((float)(P.exp_sign * row_exp[tok[u]])) : 1.f;
+                float extra = sc.y;
+                if (resid) extra += float_of(resid[tok[u] * jb.ld_res + row], io_bf16);
+                const float exact = v[u] * (sc.x * rs) + extra, w = clamp_or_nan(exact, lim);
+                uint16_t* const out = static_cast<uint16_t*>(jb.out);
+                if (SPLIT && !FRAG) {
+                    const __nv_bfloat16 value = __float2bfloat16(w);
+                    out[fragment_index<1>(tok[u], row)] = __bfloat16_as_ushort(value);
+                    out[fragment_index<1>(kSplitTokens + tok[u], row)] = __bfloat16_as_ushort(__float2bfloat16(exact - __bfloat162float(value)));
+                } else {
+                    out[frag_out ? fragment_index<NT>(tok[u], row) : tok[u] * jb.ld_out + row] = out_bf16 ? __bfloat16_as_ushort(__float2bfloat16(w)) : __half_as_ushort(__float2half(w));
                 }
             }
+        };
+        if (sums <= kBatchThreads) {
+            if ((tid & ~31) < sums) emit(std::integral_constant<int, 1>{}, tid);
+        } else {
+#pragma unroll 1
+            for (int e0 = tid; (e0 & ~31) < sums; e0 += 3 * kBatchThreads) emit(std::integral_constant<int, 3>{}, e0);
         }
         if (blk + gb < groups) __syncthreads();   // the partial sums have been read
     }
@@ -400,9 +422,21 @@ static int batch_smem_limit(int* out) {
     return NQ_OK;
 }
 
+// From nine tokens on the second column group doubles the matrix instructions, and every CTA stages the whole input of a first stage:
+// launches with much of both are faster through nq_wgemm.cu.  Both stages of a group, 16 tokens, here and there, us:
+//   1.6 MB of packed factors (4096 -> 4096)  8.3 / 9.9      8.3 MB (8192 -> 8192)        16.8 / 20.5     29 MB (28672 -> 8192)      68.6 / 46.0
+//   5.0 MB (12288 -> 4096)                  16.2 / 16.1     10.0 MB (gate/up of 4096)    19.4 / 18.8     58 MB (gate/up of 8192)    88.5 / 73.7
+//   5.8 MB (q/k/v of 5120)                  16.6 / 15.1     10.3 MB (q/k/v of 8192)      24.9 / 21.3
+// Where the two are close (gate/up of 4096) a layer is faster through one kernel: eight layers 432 us, with gate/up there 448.
 int batch_max_tokens(const StageJob* jobs, int n) {
-    for (int i = 0; i < n; ++i)
+    double bytes = 0;                       // of this stage
+    int most_k = 0;
+    for (int i = 0; i < n; ++i) {
         if (jobs[i].K > 32768) return 0;    // one row group's weights have to fit beside staging and partial sums
+        bytes += (double)jobs[i].K * jobs[i].Nout / 8;
+        most_k = jobs[i].K > most_k ? jobs[i].K : most_k;
+    }
+    if (bytes >= 8e6 || (bytes >= 4.5e6 && most_k >= 8192)) return 8;
     return kBatchMostTokens;
 }
 
