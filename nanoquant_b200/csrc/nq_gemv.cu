@@ -696,7 +696,7 @@ __global__ void __launch_bounds__(kGemvThreads, 1) gemv_group_kernel(const __gri
             if (++slot == slots) { slot = 0; parity ^= 1u; }
             if (loader) load_block();
             // every thread has compared or stored the tag, or never will
-            if (ph == 1 && blk == 0 && tid == 0) launch_arrive(reinterpret_cast<unsigned long long*>(header), blockIdx.x == 0, gridDim.x);
+            if (ph == 1 && blk == 0 && tid == kGemvThreads - 1) launch_arrive(reinterpret_cast<unsigned long long*>(header), blockIdx.x == 0, gridDim.x);
             RawOut raw = raw0;
             if (blk > 0) load_raw_out(raw, jb, row0 + blk * 16, nb * 16, T, tid >> 2);
             if (ph == 0) emit_block<KIND, true>(jb, row0 + blk * 16, nb, T, part, tc.tag, raw);
