@@ -61,7 +61,7 @@ def _ext_link(obj: str) -> list:
     import torch
     lib = os.path.join(os.path.dirname(torch.__file__), "lib")
     return ["g++", "-shared", "-o", EXT_PATH, obj, "-L", PKG_DIR, "-l:libnanoquant_b200.so", "-L", lib, "-ltorch_python",
-            "-ltorch", "-ltorch_cpu", "-lc10_cuda", "-lc10", "-Wl,-rpath,$ORIGIN"]
+            "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10_cuda", "-lc10", "-Wl,-rpath,$ORIGIN"]
 
 
 def build(force: bool = False, verbose: bool = False) -> str:

@@ -12,21 +12,24 @@
 //     plain case (other types, tensor subclasses, dispatch modes, odd dimensions); the caller then takes the general route.
 #include <Python.h>
 
+#include <ATen/core/LegacyTypeDispatch.h>
 #include <ATen/core/Tensor.h>
+#include <ATen/cuda/EmptyTensor.h>
 #include <ATen/ops/as_strided.h>
-#include <ATen/ops/empty.h>
 #include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
+#include <torch/csrc/jit/frontend/tracer.h>
 #include <torch/csrc/utils/object_ptr.h>
 #include <torch/csrc/utils/pybind.h>
 #include <torch/library.h>
 
 #include <mutex>
 #include <optional>
+#include <vector>
 
 #include "nanoquant_b200.h"
 
@@ -42,6 +45,7 @@ constexpr int kMaxDevices = 64;
 // Python callbacks, set once by nanoquant_b200.ops
 // ---------------------------------------------------------------------------------------------------------------
 PyObject* g_raise_status = nullptr;    // (status, what): raises
+std::vector<PyObject*> g_global_hooks;
 PyObject* g_grow_scratch = nullptr;    // (device index, bytes): makes the scratch hold that many bytes, or raises
 PyObject* g_dyn_general = nullptr;     // Python implementations of the operators (reference operand layouts)
 PyObject* g_marlin_general = nullptr;
@@ -143,9 +147,12 @@ void describe(nq_linear_desc& d, const Linear& l, const void* x, int64_t N, int6
     d.bias = l.bias ? l.bias->const_data_ptr() : nullptr;
 }
 
-Tensor new_output(at::IntArrayRef shape, const Tensor& like) {
-    return at::empty(shape, like.options().requires_grad(false));
+// Without the dispatcher (1.2 us of a call): nothing that could intercept it is active where a plain call is taken, and the kernel
+// writes every element.
+Tensor new_output(at::IntArrayRef shape, const Tensor& like, at::ScalarType type) {
+    return at::detail::empty_cuda(shape, type, like.device(), std::nullopt);
 }
+Tensor new_output(at::IntArrayRef shape, const Tensor& like) { return new_output(shape, like, like.scalar_type()); }
 
 // y[..., M] for a contiguous x[..., N]
 Tensor linear(const Tensor& x, const Linear& l) {
@@ -293,6 +300,72 @@ PyObject* py_linear_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
     END_HANDLE_TH_ERRORS
 }
 
+// module_call(module.__dict__, x) -> y or None: the call of a prepared NanoQuantLinear that nn.Module.__call__ would pass to its forward and
+// forward to linear_forward, as one function.  None: hooks (the module's or global ones), a replaced forward, tracing, or not a plain call.
+PyObject* py_module_call(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    TORCH_CHECK(n == 2 && PyDict_Check(a[0]), "module_call takes a module's dictionary and its argument");
+    static PyObject* const key[] = {PyUnicode_InternFromString("_forward_hooks"), PyUnicode_InternFromString("_forward_pre_hooks"),
+                                    PyUnicode_InternFromString("_backward_hooks"), PyUnicode_InternFromString("_backward_pre_hooks"),
+                                    PyUnicode_InternFromString("_parameters"), PyUnicode_InternFromString("forward"),
+                                    PyUnicode_InternFromString("_compiled_call_impl"), PyUnicode_InternFromString("do_kernel_inference"),
+                                    PyUnicode_InternFromString("kernel_type"), PyUnicode_InternFromString("V_int8"),
+                                    PyUnicode_InternFromString("U_int8"), PyUnicode_InternFromString("rank")};
+    static PyObject* const scale[2][3] = {{PyUnicode_InternFromString("scale_pre"), PyUnicode_InternFromString("scale_mid"), PyUnicode_InternFromString("scale_post")},
+                                          {PyUnicode_InternFromString("s1"), PyUnicode_InternFromString("s2"), PyUnicode_InternFromString("s3")}};
+    static PyObject* const bias_key = PyUnicode_InternFromString("bias");
+    auto get = [](PyObject* dict, PyObject* k) { return PyDict_GetItemWithError(dict, k); };    // borrowed
+    if (!exact_plain(a[1]) || torch::jit::tracer::isTracing()) Py_RETURN_NONE;
+    for (PyObject* hooks : g_global_hooks)
+        if (PyDict_Size(hooks) != 0) Py_RETURN_NONE;
+    for (int i = 0; i < 4; ++i) {
+        PyObject* hooks = get(a[0], key[i]);
+        if (hooks && PyDict_Size(hooks) != 0) Py_RETURN_NONE;
+    }
+    PyObject* params = get(a[0], key[4]);
+    PyObject* compiled = get(a[0], key[6]);
+    if (!params || !PyDict_Check(params) || get(a[0], key[5]) || (compiled && compiled != Py_None) || get(a[0], key[7]) != Py_True) {
+        PyErr_Clear();
+        Py_RETURN_NONE;
+    }
+    PyObject* type = get(a[0], key[8]);
+    if (!type || !PyUnicode_Check(type)) Py_RETURN_NONE;
+    PyObject* const* s = scale[PyUnicode_CompareWithASCIIString(type, "gemv") == 0 ? 0 : 1];
+    auto or_none = [](PyObject* o) { return o ? o : Py_None; };
+    PyObject* const operands[7] = {get(params, s[0]), get(a[0], key[9]), or_none(get(params, s[1])), get(a[0], key[10]), get(params, s[2]),
+                                   get(a[0], key[11]), or_none(get(params, bias_key))};
+    if (PyErr_Occurred()) return nullptr;
+    for (PyObject* o : operands)
+        if (!o) Py_RETURN_NONE;
+    const Tensor* x = plain(a[1]);
+    Linear l;
+    if (!x || !is_16bit(x->scalar_type()) || (x->dim() != 2 && x->dim() != 3) || !x->is_contiguous() ||
+        !parse_linear(operands, x->scalar_type(), x->size(-1), l))
+        Py_RETURN_NONE;
+    Tensor y;
+    {
+        pybind11::gil_scoped_release no_gil;
+        y = linear(*x, l);
+    }
+    return THPVariable_Wrap(y);
+    END_HANDLE_TH_ERRORS
+}
+
+// set_global_hooks([dict, ...]): nn.Module's dictionaries of hooks on every module
+PyObject* py_set_global_hooks(PyObject*, PyObject* list) {
+    HANDLE_TH_ERRORS
+    TORCH_CHECK(PyList_Check(list), "a list of dictionaries");
+    std::vector<PyObject*> hooks;
+    for (Py_ssize_t i = 0; i < PyList_GET_SIZE(list); ++i) {
+        TORCH_CHECK(PyDict_Check(PyList_GET_ITEM(list, i)), "a list of dictionaries");
+        hooks.push_back(Py_NewRef(PyList_GET_ITEM(list, i)));
+    }
+    g_global_hooks.swap(hooks);
+    for (PyObject* h : hooks) Py_DECREF(h);
+    Py_RETURN_NONE;
+    END_HANDLE_TH_ERRORS
+}
+
 // group_forward(x | [x...], [(s_in, v_tiles, s_mid, u_tiles, s_out, rank, bias)...], residuals | None) -> [y...] or None.
 // The outputs lie side by side in one [T, sum(M)] buffer.
 PyObject* py_group_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
@@ -349,6 +422,8 @@ PyObject* py_group_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
     }
     THPObjectPtr list(PyList_New(count));
     if (!list) return nullptr;
+    // The outputs do not overlap and their buffer is nobody else's, so they need none of a view's bookkeeping.
+    at::AutoDispatchBelowADInplaceOrView below;
     col = 0;
     for (Py_ssize_t i = 0; i < count; ++i) {
         // [..., M] column view with the leading dimensions of x: tokens are `width` elements apart
@@ -398,11 +473,10 @@ PyObject* py_dense_gemv_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
 enum RepackOp : int { kPackRows, kUnpackRows, kRowsToTiles, kTilesToRows, kPackMarlin };
 Tensor repack(RepackOp op, const Tensor& src, int64_t rows, int64_t cols, int order) {
     const int64_t words = (cols + 31) / 32, row_groups = (rows + 15) / 16, chunks = (cols + 255) / 256;
-    const auto ints = src.options().dtype(at::kInt);
-    Tensor out = op == kUnpackRows    ? at::empty({rows, cols}, src.options().dtype(at::kChar))
-                 : op == kRowsToTiles ? at::empty({row_groups, chunks, 128}, ints)
-                 : op == kPackMarlin  ? at::empty({cols / 16, rows / 2}, ints)
-                                      : at::empty({rows, words}, ints);
+    Tensor out = op == kUnpackRows    ? new_output({rows, cols}, src, at::kChar)
+                 : op == kRowsToTiles ? new_output({row_groups, chunks, 128}, src, at::kInt)
+                 : op == kPackMarlin  ? new_output({cols / 16, rows / 2}, src, at::kInt)
+                                      : new_output({rows, words}, src, at::kInt);
     const int dev = src.get_device();
     OnDevice on(dev);
     const nq_stream_t stream = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)dev).stream();
@@ -518,6 +592,8 @@ PyMethodDef kMethods[] = {
     {"pack_rows", (PyCFunction)(void*)py_pack_rows, METH_FASTCALL, nullptr},
     {"words_to", (PyCFunction)(void*)py_words_to, METH_FASTCALL, nullptr},
     {"permute_scale", (PyCFunction)(void*)py_permute_scale, METH_FASTCALL, nullptr},
+    {"module_call", (PyCFunction)(void (*)(void))py_module_call, METH_FASTCALL, nullptr},
+    {"set_global_hooks", py_set_global_hooks, METH_O, nullptr},
     {"set_scratch", py_set_scratch, METH_VARARGS, nullptr},
     {"set_thread_scratch", py_set_thread_scratch, METH_VARARGS, nullptr},
     {"set_callbacks", py_set_callbacks, METH_VARARGS, nullptr},

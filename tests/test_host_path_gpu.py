@@ -56,3 +56,32 @@ def test_group_call_equals_the_general_route(T):
         got = LinearGroup(mods)(x.view(T, 1, 256), residuals=r)
         assert [tuple(y.shape) for y in got] == [(T, 1, 200), (T, 1, 64)]
         assert all(torch.equal(a.reshape(T, -1), b) for a, b in zip(got, want))
+
+
+def test_call_keeps_hooks_and_overrides():
+    # the module's own __call__ passes a call on unless nothing could notice: hooks of every kind, a replaced forward, a subclass's forward
+    from torch.nn.modules.module import register_module_forward_hook
+    from nanoquant_b200.modules.linear import NanoQuantLinear
+    m, _ = _module(256, 96, 200, torch.bfloat16, "gemv", False, seed=5)
+    x = torch.randn(3, 256, device="cuda").to(torch.bfloat16)
+    with torch.no_grad():
+        want = m.forward(x)
+        assert torch.equal(m(x), want) and torch.equal(m(x=x), want)
+        seen = []
+        for register in (m.register_forward_hook, m.register_forward_pre_hook, register_module_forward_hook):
+            handle = register(lambda *a: seen.append(register.__name__))
+            m(x)
+            handle.remove()
+        assert len(seen) == 3
+        handle = m.register_forward_hook(lambda mod, args, y: y + 1)
+        assert torch.equal(m(x), want + 1)
+        handle.remove()
+        m.forward = lambda x: "replaced"
+        assert m(x) == "replaced"
+        del m.forward
+        with pytest.MonkeyPatch.context() as patch:
+            patch.setattr(NanoQuantLinear, "forward", lambda self, x: "patched")
+            assert m(x) == "patched"
+        assert torch.equal(m(x), want)
+        m.__class__ = type("Sub", (NanoQuantLinear,), {"forward": lambda self, x: "subclass"})
+        assert m(x) == "subclass"
