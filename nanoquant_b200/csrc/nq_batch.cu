@@ -138,7 +138,8 @@ __global__ void __launch_bounds__(kBatchThreads, 1) batch_stage_kernel(const __g
     const BatchJob& jb = P.job[my_job];
     unsigned char* weights = smem + kFixedBytes;
     float* part = reinterpret_cast<float*>(smem + P.part_off);        // [chunk slice][token][row of the block]
-    const int T = P.T, slots = P.slots, slot_bytes = P.slot_bytes, chunks = jb.chunks, gb = jb.gb, rows = jb.rows;
+    // (a constant where it is one: eight Qwen3-8B layers of four tokens 347.4 -> 338.9 us, two of 8192 columns 273 -> 267.5)
+    const int T = SPLIT ? (FRAG ? 2 * kSplitTokens : kSplitTokens) : P.T, slots = P.slots, slot_bytes = P.slot_bytes, chunks = jb.chunks, gb = jb.gb, rows = jb.rows;
     int first, groups;
     {
         const int c = (int)blockIdx.x - jb.cta0;
