@@ -102,7 +102,6 @@ struct alignas(16) GemvParams {
     unsigned* header;       // [0..1] 64-bit arrival counter (launch tags), [2] status, [3] CTAs that have helped
     unsigned spin_limit;    // polls before a wait for the tagged intermediate gives up
     unsigned help_after;    // polls before a CTA computes missing rows of the intermediate itself
-    int T;
     int slots, slot_bytes;  // weight blocks in shared memory
     int xq_off, part_off;   // shared-memory offsets behind the weight slots
     uint8_t cta_job[kMaxCtas];   // per CTA: job of phase 1 + 16 * job of phase 2 (kMaxJobs: none)
@@ -555,9 +554,9 @@ __device__ __noinline__ void help_phase1(const Job& jb, int T, unsigned char* xq
 // ---------------------------------------------------------------------------
 // the kernel
 // ---------------------------------------------------------------------------
-// TOK: tokens of the launch, 1 or 2 (one column group of 8 MMA columns); or 4, three or four of them (two groups).  The count as a
-// constant takes loops and divisions out of a chain of dependent instructions: eight layers in a graph, one token, Qwen3-8B 248 -> 238 us,
-// Llama-3.2-1B 195 -> 188; with a copy of the code per phase 237 and 183.
+// TOK: tokens of the launch; one column group of 8 MMA columns up to two of them, two from three on.  The count as a constant takes
+// loops and divisions out of a chain of dependent instructions: eight layers in a graph, one token, Qwen3-8B 248 -> 238 us, Llama-3.2-1B
+// 195 -> 188; with a copy of the code per phase 237 and 183; three tokens 340 -> 332 and 238 -> 234.
 //
 // The launch takes about 7 us; its 16 warps need 4 issue cycles of every scheduler, 2 ns, for each instruction of the
 // common path, and most of them wait for something short.  So the descriptors come into shared memory in one round trip,
@@ -596,7 +595,8 @@ __global__ void __launch_bounds__(kGemvThreads, 1) gemv_group_kernel(const __gri
     const Job* jobs = P.job;
     int2* meta = reinterpret_cast<int2*>(smem + kOffMeta);                 // [chunk][token] {unit value, sum}
     unsigned char* weights = smem + kFixedBytes;
-    const int T = TOK <= 2 ? TOK : P.T, slots = P.slots, slot_bytes = P.slot_bytes;
+    constexpr int T = TOK;
+    const int slots = P.slots, slot_bytes = P.slot_bytes;
     unsigned char* xq = smem + P.xq_off;
     float* part = reinterpret_cast<float*>(smem + P.part_off);
     unsigned* const header = P.header;
@@ -712,11 +712,12 @@ __global__ void __launch_bounds__(kGemvThreads, 1) gemv_group_kernel(const __gri
 
 static size_t round_up(size_t v, size_t m) { return (v + m - 1) / m * m; }
 
-static const void* gemv_kernel(int kind, int tokens) {
-    if (kind == KIND_F16)
-        return tokens == 1 ? (const void*)gemv_group_kernel<KIND_F16, 1> : tokens == 2 ? (const void*)gemv_group_kernel<KIND_F16, 2> : (const void*)gemv_group_kernel<KIND_F16, kMaxTok>;
-    return tokens == 1 ? (const void*)gemv_group_kernel<KIND_BF16, 1> : tokens == 2 ? (const void*)gemv_group_kernel<KIND_BF16, 2> : (const void*)gemv_group_kernel<KIND_BF16, kMaxTok>;
+template <int KIND>
+static const void* gemv_kernel_of(int tokens) {
+    return tokens == 1 ? (const void*)gemv_group_kernel<KIND, 1> : tokens == 2 ? (const void*)gemv_group_kernel<KIND, 2>
+           : tokens == 3 ? (const void*)gemv_group_kernel<KIND, 3> : (const void*)gemv_group_kernel<KIND, kMaxTok>;
 }
+static const void* gemv_kernel(int kind, int tokens) { return kind == KIND_F16 ? gemv_kernel_of<KIND_F16>(tokens) : gemv_kernel_of<KIND_BF16>(tokens); }
 
 // Opt-in shared memory limit of every instantiation, set once per device.
 static int dynamic_smem_limit(int dev, int* out) {
@@ -724,8 +725,8 @@ static int dynamic_smem_limit(int dev, int* out) {
     if (cached[dev & 63] == 0) {
         int optin = 0, lim = 1 << 30;
         NQ_CUDA_TRY(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-        for (int i = 0; i < 6; ++i) {
-            const void* fn = gemv_kernel(i & 1 ? KIND_BF16 : KIND_F16, i / 2 == 0 ? 1 : i / 2 == 1 ? 2 : kMaxTok);
+        for (int i = 0; i < 2 * kMaxTok; ++i) {
+            const void* fn = gemv_kernel(i & 1 ? KIND_BF16 : KIND_F16, 1 + i / 2);
             cudaFuncAttributes fa;
             NQ_CUDA_TRY(cudaFuncGetAttributes(&fa, fn));
             const int v = optin - (int)fa.sharedSizeBytes;  // the opt-in limit covers static + dynamic
@@ -920,7 +921,6 @@ static int launch_decode(const nq_linear_desc* d, int n_linears, int t_first, in
     const size_t esz = 2;
     for (int t0 = t_first; t0 < T; t0 += tg) {
         const int tn = (T - t0) < tg ? (T - t0) : tg;
-        P.T = tn;
         memset(P.cta_job, kMaxJobs * 17, sizeof(P.cta_job));
         // room for a block's partial sums and weights; a single row group is always allowed (see above)
         const size_t room = smem_limit - fixed_bytes(tn);
