@@ -890,16 +890,17 @@ static int launch_decode(const nq_linear_desc* d, int n_linears, int t_first, in
     P.spin_limit = g_spin_limit;
     P.help_after = g_spin_limit < 16 ? ~0u : g_spin_limit / 16 < kHelpAfter ? g_spin_limit / 16 : kHelpAfter;
 
-    // One CTA per SM, fewer for launches with less than 3 MB of packed factors: their row groups do not divide any finer by
-    // 148, and every CTA fetches the whole input and polls the whole intermediate.  One token, us per launch in a graph by
-    // CTAs (52 / 74 / 103 / 148):
-    //   0.4 MB (4096 -> 1024)  5.0 / 5.1 / 5.1 / 5.1      2.3 MB (q/k/v of 4096)          6.8 / 6.5 / 6.3 / 6.6
-    //   1.6 MB (4096 -> 4096)  5.9 / 6.0 / 6.0 / 6.2      3.9 MB (gate/up of 2048)        9.7 / 7.7 / 7.3 / 7.1
-    //   1.7 MB (3072 -> 3072)  6.2 / 6.0 / 6.7 / 7.0      4.8 MB (12288 -> 4096)         10.7 / 10.3 / 9.4 / 8.7
-    // Below 3 MB 7/10 of the SMs are within 5 % of the best of these but for a few sizes (a square linear of 3072 columns;
-    // of 2048 at two tokens, 5.3 at 74 CTAs and 6.1 here).
+    // One CTA per SM, fewer for launches with less than 2.25 MB of packed factors: their row groups do not divide any finer by
+    // 148, every CTA fetches the whole input and polls the whole intermediate, and the SMs left free let CTAs of the next launch in.  One
+    // token, us per launch in a graph by CTAs (52 / 74 / 103 / 148):
+    //   0.4 MB (4096 -> 1024)  4.7 / 4.6 / 4.7 / 4.6      2.1 MB (8192 -> 2048)           6.3 / 6.1 / 5.9 / 5.9
+    //   0.7 MB (q/k/v of 2048) 4.7 / 4.6 / 4.7 / 4.8      2.4 MB (q/k/v of 4096)          6.3 / 5.8 / 5.5 / 5.4
+    //   1.7 MB (4096 -> 4096)  5.7 / 5.4 / 5.3 / 5.3      4.1 MB (gate/up of 2048)        8.8 / 6.8 / 6.5 / 5.9
+    //   1.8 MB (3072 -> 3072)  5.7 / 5.4 / 5.3 / 5.5      5.0 MB (12288 -> 4096)          9.6 / 9.3 / 7.5 / 7.3
+    // (While the intermediate was polled in 16-byte loads the line was at 3 MB.  Eight layers, 3 MB and now, one / two / three tokens: 4096
+    // columns 216.0 / 253.8 / 331.4 -> 215.3 / 252.2 / 328.9, 3072 columns 188.8 / 217.5 / 276.9 -> 187.4 / 215.2 / 273.0.)
     int grid = sm_count() < kMaxCtas ? sm_count() : kMaxCtas;
-    if (packed < ((size_t)3 << 20)) grid = grid * 7 / 10;
+    if (packed < ((size_t)9 << 18)) grid = grid * 7 / 10;
     {   // no more CTAs than the larger phase has row groups
         int g[2] = {0, 0};
         for (int i = 0; i < n_linears; ++i) { g[0] += rg[0][i]; g[1] += rg[1][i]; }
