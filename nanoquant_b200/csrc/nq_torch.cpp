@@ -335,8 +335,13 @@ PyObject* py_module_call(PyObject*, PyObject* const* a, Py_ssize_t n) {
     PyObject* const operands[7] = {get(params, s[0]), get(a[0], key[9]), or_none(get(params, s[1])), get(a[0], key[10]), get(params, s[2]),
                                    get(a[0], key[11]), or_none(get(params, bias_key))};
     if (PyErr_Occurred()) return nullptr;
-    for (PyObject* o : operands)
-        if (!o) Py_RETURN_NONE;
+    // The call's own references, kept until the launch is enqueued: the GIL is released below, and another thread (or Python code that
+    // growing the scratch runs) may replace an operand of the module meanwhile.
+    THPObjectPtr held[7];
+    for (int i = 0; i < 7; ++i) {
+        if (!operands[i]) Py_RETURN_NONE;
+        held[i] = Py_NewRef(operands[i]);
+    }
     const Tensor* x = plain(a[1]);
     Linear l;
     if (!x || !is_16bit(x->scalar_type()) || (x->dim() != 2 && x->dim() != 3) || !x->is_contiguous() ||

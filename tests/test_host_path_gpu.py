@@ -1,4 +1,6 @@
 """The native host path of the modules against the general route, which serves every call it does not take."""
+import sys
+
 import pytest
 import torch
 
@@ -85,3 +87,37 @@ def test_call_keeps_hooks_and_overrides():
         assert torch.equal(m(x), want)
         m.__class__ = type("Sub", (NanoQuantLinear,), {"forward": lambda self, x: "subclass"})
         assert m(x) == "subclass"
+
+
+@pytest.mark.parametrize("kernel,bias", [("gemv", True), ("gemm", False)])
+def test_call_holds_its_operands(kernel, bias):
+    # A module's operands may be replaced by another thread while a call is under way without the GIL.  Python code that the call itself
+    # runs (growing the scratch) stands in for the thread here: it counts the references, and replaces the operands where they are held.
+    from nanoquant_b200 import _lib, ops
+    m, _ = _module(256, 96, 200, torch.bfloat16, kernel, bias, seed=5)
+    x = torch.randn(3, 256, device="cuda").to(torch.bfloat16)
+    ext, buf = _lib.ext(), ops.reserve_scratch(x.device, 256)
+    places = [(m._parameters, n) for n in ("scale_pre", "scale_mid", "scale_post", "s1", "s2", "s3", "bias")] + [(m.__dict__, "V_int8"), (m.__dict__, "U_int8")]
+    places = [(d, n) for d, n in places if d.get(n) is not None]
+    count = lambda: [sys.getrefcount(d[n]) for d, n in places]
+    before, during = count(), []
+    want = m(x)
+    assert count() == before                                         # and gives them back
+
+    def grow(idx, nbytes):
+        during.extend(count())
+        if all(b > a for a, b in zip(before, during)):
+            for d, n in places:
+                d[n] = torch.zeros_like(d[n])
+        ext.set_scratch(idx, buf.data_ptr(), buf.numel())
+
+    ext.set_callbacks(_lib.check, grow, ops._nanoquant_dyn_forward_cuda, ops._marlin_nanoquant_forward_cuda)
+    try:
+        ext.set_scratch(x.device.index or 0, buf.data_ptr(), 0)      # too small: the call asks for more
+        y = m(x)
+    finally:
+        ops.connect_host_path(ext)
+    assert len(places) == 5 + bias and len(during) == len(places)
+    assert all(b > a for a, b in zip(before, during)), (before, during)
+    assert torch.equal(y, want)
+    assert not torch.equal(m(x), want)                               # the operands are the replaced ones from the next call on
