@@ -9,10 +9,12 @@
 //     kernels' tile layout; operands in the reference's layouts go to the Python implementation, which converts them
 //     once and keeps the result on the tensor;
 //   * plain functions for this package's own modules (no dispatcher).  They return None whenever a call is not the
-//     plain case (other types, tensor subclasses, dispatch modes, odd dimensions); the caller then takes the general route.
+//     plain case (other types, tensor subclasses, wrappers of transforms, dispatch modes, odd dimensions, a linear that
+//     autograd would record); the caller then takes the general route.
 #include <Python.h>
 
 #include <ATen/core/LegacyTypeDispatch.h>
+#include <ATen/core/grad_mode.h>
 #include <ATen/core/Tensor.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <ATen/ops/as_strided.h>
@@ -247,11 +249,15 @@ TORCH_LIBRARY_IMPL(binary_kernels, CUDA, m) {
 // ---------------------------------------------------------------------------------------------------------------
 // plain functions
 // ---------------------------------------------------------------------------------------------------------------
-// A tensor argument without anything that would have to go through the dispatcher.
+// A tensor argument without anything that would have to go through the dispatcher: its keys are those of a strided CUDA tensor and of autograd
+// alone.  Not so for the wrappers of transforms (vmap, grad, functionalize), subclasses that dispatch in Python and lazily negated or
+// zero tensors, whose memory (if they have any) does not hold their values.
 const Tensor* plain(PyObject* o) {
+    static const uint64_t keys = c10::DispatchKeySet({c10::DispatchKey::CUDA, c10::DispatchKey::AutogradCUDA, c10::DispatchKey::ADInplaceOrView,
+                                                      c10::DispatchKey::AutocastCUDA}).raw_repr();
     if (!THPVariable_Check(o)) return nullptr;
     const Tensor& t = THPVariable_Unpack(o);
-    return t.is_cuda() && t.layout() == at::kStrided ? &t : nullptr;
+    return t.is_cuda() && (t.key_set().raw_repr() & ~keys) == 0 ? &t : nullptr;
 }
 bool exact_plain(PyObject* o) { return THPVariable_CheckExact(o) && !c10::impl::dispatch_mode_enabled(); }
 
@@ -281,6 +287,15 @@ bool parse_linear(PyObject* const* a, at::ScalarType dt, int64_t N, Linear& l) {
            l.u->size(1) == (l.rank + 255) / 256;
 }
 
+// Autograd would record the operator behind this call (as one without a derivative, which backward then says).  A linear with a bias has
+// no operator.
+bool recorded(const Tensor& x, const Linear& l) {
+    if (l.bias || !at::GradMode::is_enabled()) return false;
+    for (const Tensor* t : {&x, l.s_in, l.s_mid, l.s_out})
+        if (t && t->requires_grad()) return true;
+    return false;
+}
+
 // linear_forward(x, s_in, v_tiles, s_mid, u_tiles, s_out, rank, bias) -> y or None
 PyObject* py_linear_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
     HANDLE_TH_ERRORS
@@ -289,7 +304,7 @@ PyObject* py_linear_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const Tensor* x = plain(a[0]);
     Linear l;
     if (!x || !is_16bit(x->scalar_type()) || (x->dim() != 2 && x->dim() != 3) || !x->is_contiguous() ||
-        !parse_linear(a + 1, x->scalar_type(), x->size(-1), l))
+        !parse_linear(a + 1, x->scalar_type(), x->size(-1), l) || recorded(*x, l))
         Py_RETURN_NONE;
     Tensor y;
     {
@@ -345,7 +360,7 @@ PyObject* py_module_call(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const Tensor* x = plain(a[1]);
     Linear l;
     if (!x || !is_16bit(x->scalar_type()) || (x->dim() != 2 && x->dim() != 3) || !x->is_contiguous() ||
-        !parse_linear(operands, x->scalar_type(), x->size(-1), l))
+        !parse_linear(operands, x->scalar_type(), x->size(-1), l) || recorded(*x, l))
         Py_RETURN_NONE;
     Tensor y;
     {

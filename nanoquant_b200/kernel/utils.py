@@ -27,10 +27,10 @@ def _stream(device: torch.device) -> int:
 
 def _to_cuda(t: torch.Tensor) -> torch.Tensor:
     if t.is_cuda:
-        return t.contiguous()
+        return t.contiguous().resolve_neg()     # (the memory of a lazily negated tensor holds the other sign)
     if not torch.cuda.is_available():
         raise RuntimeError("nanoquant_b200 packers need a CUDA device: there is no CPU implementation")
-    return t.contiguous().cuda()
+    return t.contiguous().resolve_neg().cuda()
 
 
 def _int32(t: torch.Tensor) -> torch.Tensor:
@@ -45,7 +45,10 @@ def _repack(op: int, src: torch.Tensor, rows: int, cols: int, order: int = 0) ->
     ext = _lib.ext()
     out = ext.repack(op, src, rows, cols, order)
     if out is None:   # not a plain contiguous CUDA tensor
-        out = ext.repack(op, _to_cuda(src.detach()), rows, cols, order).to(src.device)
+        out = ext.repack(op, _to_cuda(src.detach()), rows, cols, order)
+        if out is None:
+            raise RuntimeError(f"nanoquant_b200 packers take plain int8 or int32 tensors, got {type(src).__name__} of {src.dtype}")
+        out = out.to(src.device)
     return out
 
 
@@ -129,7 +132,10 @@ def _permute_scale(s: torch.Tensor, kind: int, inverse: bool = False) -> torch.T
         raise TypeError("scale vectors must be fp16 or bf16 (the dtypes the kernels compute in)")
     out = _lib.ext().permute_scale(s, kind, int(inverse))
     if out is None:   # not a plain contiguous CUDA tensor
-        out = _lib.ext().permute_scale(_to_cuda(s.detach().reshape(-1)), kind, int(inverse)).to(s.device)
+        out = _lib.ext().permute_scale(_to_cuda(s.detach().reshape(-1)), kind, int(inverse))
+        if out is None:
+            raise RuntimeError(f"nanoquant_b200 packers take plain fp16 or bf16 scales, got {type(s).__name__} of {s.dtype}")
+        out = out.to(s.device)
     return out
 
 

@@ -156,6 +156,11 @@ def _check_cuda_cont(t: torch.Tensor, name: str, dtype: torch.dtype, dtype_name:
         raise RuntimeError(f"{name} must be {dtype_name} tensor")
 
 
+def _stored(t: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
+    """`t` with its values in memory (those of a lazily negated tensor are there with the other sign)."""
+    return t if t is None else t.resolve_neg()
+
+
 def as_tiles(bits: torch.Tensor, cols: int) -> torch.Tensor:
     """Tile-layout view of a factor given in either accepted layout."""
     if bits.dim() == 3:
@@ -174,6 +179,7 @@ def as_tiles(bits: torch.Tensor, cols: int) -> torch.Tensor:
 def gemv_forward(x: torch.Tensor, s_in: torch.Tensor, v_tiles: torch.Tensor, s_mid: Optional[torch.Tensor],
                  u_tiles: torch.Tensor, s_out: torch.Tensor, R: int) -> torch.Tensor:
     """The decode path on the current stream at any token count; ``x`` is ``[T, N]``."""
+    x, s_in, s_mid, s_out = (_stored(t) for t in (x, s_in, s_mid, s_out))
     T, N = x.shape
     M = s_out.size(0)
     y = torch.empty((T, M), dtype=x.dtype, device=x.device)
@@ -209,6 +215,7 @@ def dense_gemv_forward(x: torch.Tensor, weight: torch.Tensor, bias: Optional[tor
         raise RuntimeError(f"x has {x.size(-1)} columns, weight expects {weight.size(1)}")
     if bias is not None:
         _check_cuda_cont(bias, "bias", weight.dtype, str(weight.dtype))
+    x, weight, bias = _stored(x), _stored(weight), _stored(bias)
     V, N = weight.shape
     x2 = x.reshape(-1, N)
     T = x2.size(0)
@@ -286,6 +293,9 @@ def group_forward(xs, layers, T: int, dtype: torch.dtype, device: torch.device, 
     outputs are written side by side into one ``[T, sum(M_i)]`` buffer (``out`` or a fresh one); returns its
     per-linear column views."""
     n = len(layers)
+    xs = [_stored(x) for x in xs]
+    layers = [tuple(_stored(t) for t in lay[:5]) + (lay[5],) for lay in layers]
+    biases, residuals = ([_stored(t) for t in ts] if ts is not None else None for ts in (biases, residuals))
     Ms = [lay[4].size(0) for lay in layers]
     width = sum(Ms)
     if out is None:
@@ -335,6 +345,7 @@ def linear_forward(x: torch.Tensor, s_in: torch.Tensor, v_tiles: torch.Tensor, s
     if bias is not None or residual is not None:
         return group_forward([x], [(s_in, v_tiles, s_mid, u_tiles, s_out, R)], T, x.dtype, x.device,
                              [bias], [residual])[0]
+    x, s_in, s_mid, s_out = (_stored(t) for t in (x, s_in, s_mid, s_out))
     y = torch.empty((T, M), dtype=x.dtype, device=x.device)
     if T == 0:
         return y

@@ -121,3 +121,40 @@ def test_call_holds_its_operands(kernel, bias):
     assert all(b > a for a, b in zip(before, during)), (before, during)
     assert torch.equal(y, want)
     assert not torch.equal(m(x), want)                               # the operands are the replaced ones from the next call on
+
+
+@pytest.mark.parametrize("kernel,bias", [("gemv", False), ("gemm", False), ("gemv", True)])
+def test_tensors_with_more_than_a_memory(kernel, bias):
+    # wrappers of transforms, lazily negated tensors and calls that autograd records go to the operator (or are resolved first)
+    from nanoquant_b200.modules.group import LinearGroup
+    m, _ = _module(256, 96, 200, torch.bfloat16, kernel, bias, seed=5)
+    x = torch.randn(3, 2, 256, device="cuda").to(torch.bfloat16)
+    want = torch.stack([m(a) for a in x])
+    neg = torch.stack([m(-a) for a in x])
+    for a, y in zip(x, neg):
+        assert torch.equal(m(torch._neg_view(a)), y)
+        assert torch.equal(m.forward(torch._neg_view(a)), y)
+        assert torch.equal(LinearGroup([m])(torch._neg_view(a))[0], y)
+    if bias:
+        return                                     # (behind a bias there is no operator)
+    if kernel == "gemv":                           # (the other operator may write its workspace, which transforms refuse)
+        assert torch.equal(torch.vmap(m)(x), want)
+        assert torch.equal(torch.func.functionalize(m)(x[0]), want[0])
+        assert not torch.func.grad(lambda a: m(a).float().sum())(x[0]).any()      # (no derivative; the value is computed)
+    xg = x[0].clone().requires_grad_()
+    assert m(xg).requires_grad and torch.equal(m(xg), want[0])
+    with torch.no_grad():
+        assert not m(xg).requires_grad
+
+
+def test_lazily_negated_operands_elsewhere():
+    from nanoquant_b200 import ops
+    from nanoquant_b200.kernel import utils as ku
+    x, w = torch.randn(3, 256, device="cuda").half(), torch.randn(40, 256, device="cuda").half()
+    for a, b in ((torch._neg_view(x), w), (x, torch._neg_view(w))):
+        assert torch.equal(ops.dense_gemv_forward(a, b), ops.dense_gemv_forward(-x, w))
+    s = (torch.randint(0, 2, (64, 96), device="cuda") * 2 - 1).to(torch.int8)
+    assert torch.equal(ku.pack_binary_gemv(torch._neg_view(s)), ku.pack_binary_gemv(-s))
+    for got, want in zip(ku.pack_binary_marlin(torch._neg_view(s), torch._neg_view(x[0, :96]), x[0, :64]),
+                         ku.pack_binary_marlin(-s, -x[0, :96], x[0, :64])):
+        assert torch.equal(got, want) if torch.is_tensor(want) else got == want
