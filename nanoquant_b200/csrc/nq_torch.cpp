@@ -316,7 +316,8 @@ PyObject* py_linear_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
 }
 
 // module_call(module.__dict__, x) -> y or None: the call of a prepared NanoQuantLinear that nn.Module.__call__ would pass to its forward and
-// forward to linear_forward, as one function.  None: hooks (the module's or global ones), a replaced forward, tracing, or not a plain call.
+// forward to linear_forward, as one function.  None: hooks (the module's or global ones), a replaced forward or _call_impl of its own,
+// tracing, a Python profiler or debugger, or not a plain call.
 PyObject* py_module_call(PyObject*, PyObject* const* a, Py_ssize_t n) {
     HANDLE_TH_ERRORS
     TORCH_CHECK(n == 2 && PyDict_Check(a[0]), "module_call takes a module's dictionary and its argument");
@@ -325,12 +326,16 @@ PyObject* py_module_call(PyObject*, PyObject* const* a, Py_ssize_t n) {
                                     PyUnicode_InternFromString("_parameters"), PyUnicode_InternFromString("forward"),
                                     PyUnicode_InternFromString("_compiled_call_impl"), PyUnicode_InternFromString("do_kernel_inference"),
                                     PyUnicode_InternFromString("kernel_type"), PyUnicode_InternFromString("V_int8"),
-                                    PyUnicode_InternFromString("U_int8"), PyUnicode_InternFromString("rank")};
+                                    PyUnicode_InternFromString("U_int8"), PyUnicode_InternFromString("rank"),
+                                    PyUnicode_InternFromString("_call_impl")};
     static PyObject* const scale[2][3] = {{PyUnicode_InternFromString("scale_pre"), PyUnicode_InternFromString("scale_mid"), PyUnicode_InternFromString("scale_post")},
                                           {PyUnicode_InternFromString("s1"), PyUnicode_InternFromString("s2"), PyUnicode_InternFromString("s3")}};
     static PyObject* const bias_key = PyUnicode_InternFromString("bias");
     auto get = [](PyObject* dict, PyObject* k) { return PyDict_GetItemWithError(dict, k); };    // borrowed
     if (!exact_plain(a[1]) || torch::jit::tracer::isTracing()) Py_RETURN_NONE;
+    // A profiler that records modules knows them by the frame of nn.Module.__call__; a debugger steps into forward.
+    const PyThreadState* const thread = PyThreadState_Get();
+    if (thread->c_profilefunc || thread->c_tracefunc) Py_RETURN_NONE;
     for (PyObject* hooks : g_global_hooks)
         if (PyDict_Size(hooks) != 0) Py_RETURN_NONE;
     for (int i = 0; i < 4; ++i) {
@@ -339,7 +344,7 @@ PyObject* py_module_call(PyObject*, PyObject* const* a, Py_ssize_t n) {
     }
     PyObject* params = get(a[0], key[4]);
     PyObject* compiled = get(a[0], key[6]);
-    if (!params || !PyDict_Check(params) || get(a[0], key[5]) || (compiled && compiled != Py_None) || get(a[0], key[7]) != Py_True) {
+    if (!params || !PyDict_Check(params) || get(a[0], key[5]) || get(a[0], key[12]) || (compiled && compiled != Py_None) || get(a[0], key[7]) != Py_True) {
         PyErr_Clear();
         Py_RETURN_NONE;
     }

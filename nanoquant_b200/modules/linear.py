@@ -60,8 +60,10 @@ class NanoQuantLinear(nn.Module):
     # ------------------------------------------------------------------ forward
     def __call__(self, *args, **kwargs):
         # nn.Module's way from a call to `forward`, and from there to the launch, costs a third of a decode call's time on the host.
-        # It is taken for everything but a call that it would pass on unchanged: no hooks, no tracing, no compiler, the forward below.
+        # It is taken for everything but a call that it would pass on unchanged and unseen: no hooks, no tracing, no compiler, no Python
+        # profiler or debugger, the forward below, and nn.Module's own way of calling (which tools replace to see every module's calls).
         if (len(args) == 1 and not kwargs and self.__class__ is NanoQuantLinear and NanoQuantLinear.forward is _FORWARD
+                and nn.Module.__call__ is _CALL and NanoQuantLinear._call_impl is _CALL_IMPL
                 and not torch.compiler.is_compiling()):
             y = _lib.ext().module_call(self.__dict__, args[0])
             if y is not None:
@@ -238,4 +240,11 @@ class NanoQuantLinear(nn.Module):
         return state
 
 
-_FORWARD = NanoQuantLinear.forward      # (a call goes the long way when somebody has replaced it)
+def _stock(name):
+    """nn.Module's function `name`; something that nothing is when it has been replaced already."""
+    f = getattr(nn.Module, name, None)
+    return f if getattr(f, "__module__", "") == nn.Module.__module__ and not hasattr(f, "__wrapped__") else object()
+
+
+# a call goes the long way when somebody has replaced one of these
+_FORWARD, _CALL, _CALL_IMPL = NanoQuantLinear.forward, _stock("__call__"), _stock("_call_impl")

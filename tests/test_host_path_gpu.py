@@ -158,3 +158,33 @@ def test_lazily_negated_operands_elsewhere():
     for got, want in zip(ku.pack_binary_marlin(torch._neg_view(s), torch._neg_view(x[0, :96]), x[0, :64]),
                          ku.pack_binary_marlin(-s, -x[0, :96], x[0, :64])):
         assert torch.equal(got, want) if torch.is_tensor(want) else got == want
+
+
+def test_call_is_seen_by_whoever_watches_module_calls(tmp_path):
+    from nanoquant_b200.modules import linear
+    from nanoquant_b200.modules.linear import NanoQuantLinear
+    m, _ = _module(256, 96, 200, torch.bfloat16, "gemv", False, seed=5)
+    x = torch.randn(3, 256, device="cuda").to(torch.bfloat16)
+    want, seen = m(x), []
+    assert linear._CALL is torch.nn.Module.__call__ and linear._CALL_IMPL is torch.nn.Module._call_impl   # (unwatched: the short way)
+
+    def watched(f):
+        def call(self, *args, **kwargs):
+            seen.append(type(self))
+            return f(self, *args, **kwargs)
+        return call
+
+    for cls, name in ((torch.nn.Module, "__call__"), (torch.nn.Module, "_call_impl"), (NanoQuantLinear, "_call_impl")):
+        with pytest.MonkeyPatch.context() as patch:
+            patch.setattr(cls, name, watched(getattr(cls, name)))
+            assert torch.equal(m(x), want)
+    m._call_impl = lambda *args: (seen.append(NanoQuantLinear), NanoQuantLinear._call_impl(m, *args))[1]
+    assert torch.equal(m(x), want)
+    del m._call_impl
+    assert seen == 4 * [NanoQuantLinear] and torch.equal(m(x), want) and len(seen) == 4
+    # torch.profiler's module tree
+    from torch.profiler import ProfilerActivity, profile
+    with profile(activities=[ProfilerActivity.CPU], with_stack=True) as prof:
+        assert torch.equal(m(x), want)
+    prof.export_chrome_trace(str(tmp_path / "trace.json"))
+    assert "nn.Module: NanoQuantLinear" in (tmp_path / "trace.json").read_text()
