@@ -47,10 +47,17 @@ constexpr int kMaxDevices = 64;
 // Python callbacks, set once by nanoquant_b200.ops
 // ---------------------------------------------------------------------------------------------------------------
 PyObject* g_raise_status = nullptr;    // (status, what): raises
-std::vector<PyObject*> g_global_hooks;
 PyObject* g_grow_scratch = nullptr;    // (device index, bytes): makes the scratch hold that many bytes, or raises
 PyObject* g_dyn_general = nullptr;     // Python implementations of the operators (reference operand layouts)
 PyObject* g_marlin_general = nullptr;
+
+// What module_call compares with: NanoQuantLinear and its forward, nn.Module and its way from a call to forward, the hooks on every module.
+struct ModuleClass {
+    PyTypeObject *type = nullptr, *base = nullptr;
+    PyObject *forward = nullptr, *call = nullptr, *call_impl = nullptr;
+    std::vector<PyObject*> global_hooks;
+};
+ModuleClass g_module_class;
 
 // Calls a Python function with the GIL held and throws its exception.
 PyObject* call_python(PyObject* fn, PyObject* args) {
@@ -252,12 +259,12 @@ TORCH_LIBRARY_IMPL(binary_kernels, CUDA, m) {
 // A tensor argument without anything that would have to go through the dispatcher: its keys are those of a strided CUDA tensor and of autograd
 // alone.  Not so for the wrappers of transforms (vmap, grad, functionalize), subclasses that dispatch in Python and lazily negated or
 // zero tensors, whose memory (if they have any) does not hold their values.
+const uint64_t kPlainKeys = c10::DispatchKeySet({c10::DispatchKey::CUDA, c10::DispatchKey::AutogradCUDA, c10::DispatchKey::ADInplaceOrView,
+                                                 c10::DispatchKey::AutocastCUDA}).raw_repr();
 const Tensor* plain(PyObject* o) {
-    static const uint64_t keys = c10::DispatchKeySet({c10::DispatchKey::CUDA, c10::DispatchKey::AutogradCUDA, c10::DispatchKey::ADInplaceOrView,
-                                                      c10::DispatchKey::AutocastCUDA}).raw_repr();
     if (!THPVariable_Check(o)) return nullptr;
     const Tensor& t = THPVariable_Unpack(o);
-    return t.is_cuda() && (t.key_set().raw_repr() & ~keys) == 0 ? &t : nullptr;
+    return t.is_cuda() && (t.key_set().raw_repr() & ~kPlainKeys) == 0 ? &t : nullptr;
 }
 bool exact_plain(PyObject* o) { return THPVariable_CheckExact(o) && !c10::impl::dispatch_mode_enabled(); }
 
@@ -315,45 +322,53 @@ PyObject* py_linear_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
     END_HANDLE_TH_ERRORS
 }
 
-// module_call(module.__dict__, x) -> y or None: the call of a prepared NanoQuantLinear that nn.Module.__call__ would pass to its forward and
-// forward to linear_forward, as one function.  None: hooks (the module's or global ones), a replaced forward or _call_impl of its own,
-// tracing, a Python profiler or debugger, or not a plain call.
+// module_call(module, x) -> y or None: the call of a prepared NanoQuantLinear that nn.Module.__call__ would pass to its forward and forward
+// to linear_forward, as one function.  None for everything that nn.Module would not have passed on unchanged and unseen: hooks (the
+// module's or global ones), a replaced forward, nn.Module's way of calling replaced (tools do that to see every module's calls), tracing, a
+// Python profiler or debugger, a subclass, or not a plain call.
 PyObject* py_module_call(PyObject*, PyObject* const* a, Py_ssize_t n) {
     HANDLE_TH_ERRORS
-    TORCH_CHECK(n == 2 && PyDict_Check(a[0]), "module_call takes a module's dictionary and its argument");
+    TORCH_CHECK(n == 2, "module_call takes a module and its argument");
     static PyObject* const key[] = {PyUnicode_InternFromString("_forward_hooks"), PyUnicode_InternFromString("_forward_pre_hooks"),
                                     PyUnicode_InternFromString("_backward_hooks"), PyUnicode_InternFromString("_backward_pre_hooks"),
                                     PyUnicode_InternFromString("_parameters"), PyUnicode_InternFromString("forward"),
                                     PyUnicode_InternFromString("_compiled_call_impl"), PyUnicode_InternFromString("do_kernel_inference"),
                                     PyUnicode_InternFromString("kernel_type"), PyUnicode_InternFromString("V_int8"),
                                     PyUnicode_InternFromString("U_int8"), PyUnicode_InternFromString("rank"),
-                                    PyUnicode_InternFromString("_call_impl")};
+                                    PyUnicode_InternFromString("_call_impl"), PyUnicode_InternFromString("__call__")};
     static PyObject* const scale[2][3] = {{PyUnicode_InternFromString("scale_pre"), PyUnicode_InternFromString("scale_mid"), PyUnicode_InternFromString("scale_post")},
                                           {PyUnicode_InternFromString("s1"), PyUnicode_InternFromString("s2"), PyUnicode_InternFromString("s3")}};
     static PyObject* const bias_key = PyUnicode_InternFromString("bias");
     auto get = [](PyObject* dict, PyObject* k) { return PyDict_GetItemWithError(dict, k); };    // borrowed
+    const ModuleClass& cls = g_module_class;
+    if (!cls.type || Py_TYPE(a[0]) != cls.type || _PyType_Lookup(cls.type, key[5]) != cls.forward ||
+        _PyType_Lookup(cls.type, key[12]) != cls.call_impl || _PyType_Lookup(cls.base, key[13]) != cls.call)
+        Py_RETURN_NONE;
     if (!exact_plain(a[1]) || torch::jit::tracer::isTracing()) Py_RETURN_NONE;
     // A profiler that records modules knows them by the frame of nn.Module.__call__; a debugger steps into forward.
     const PyThreadState* const thread = PyThreadState_Get();
     if (thread->c_profilefunc || thread->c_tracefunc) Py_RETURN_NONE;
-    for (PyObject* hooks : g_global_hooks)
+    THPObjectPtr module_dict(PyObject_GenericGetDict(a[0], nullptr));
+    if (!module_dict) return nullptr;
+    PyObject* const dict = module_dict.get();
+    for (PyObject* hooks : cls.global_hooks)
         if (PyDict_Size(hooks) != 0) Py_RETURN_NONE;
     for (int i = 0; i < 4; ++i) {
-        PyObject* hooks = get(a[0], key[i]);
+        PyObject* hooks = get(dict, key[i]);
         if (hooks && PyDict_Size(hooks) != 0) Py_RETURN_NONE;
     }
-    PyObject* params = get(a[0], key[4]);
-    PyObject* compiled = get(a[0], key[6]);
-    if (!params || !PyDict_Check(params) || get(a[0], key[5]) || get(a[0], key[12]) || (compiled && compiled != Py_None) || get(a[0], key[7]) != Py_True) {
+    PyObject* params = get(dict, key[4]);
+    PyObject* compiled = get(dict, key[6]);
+    if (!params || !PyDict_Check(params) || get(dict, key[5]) || get(dict, key[12]) || (compiled && compiled != Py_None) || get(dict, key[7]) != Py_True) {
         PyErr_Clear();
         Py_RETURN_NONE;
     }
-    PyObject* type = get(a[0], key[8]);
+    PyObject* type = get(dict, key[8]);
     if (!type || !PyUnicode_Check(type)) Py_RETURN_NONE;
     PyObject* const* s = scale[PyUnicode_CompareWithASCIIString(type, "gemv") == 0 ? 0 : 1];
     auto or_none = [](PyObject* o) { return o ? o : Py_None; };
-    PyObject* const operands[7] = {get(params, s[0]), get(a[0], key[9]), or_none(get(params, s[1])), get(a[0], key[10]), get(params, s[2]),
-                                   get(a[0], key[11]), or_none(get(params, bias_key))};
+    PyObject* const operands[7] = {get(params, s[0]), get(dict, key[9]), or_none(get(params, s[1])), get(dict, key[10]), get(params, s[2]),
+                                   get(dict, key[11]), or_none(get(params, bias_key))};
     if (PyErr_Occurred()) return nullptr;
     // The call's own references, kept until the launch is enqueued: the GIL is released below, and another thread (or Python code that
     // growing the scratch runs) may replace an operand of the module meanwhile.
@@ -376,17 +391,24 @@ PyObject* py_module_call(PyObject*, PyObject* const* a, Py_ssize_t n) {
     END_HANDLE_TH_ERRORS
 }
 
-// set_global_hooks([dict, ...]): nn.Module's dictionaries of hooks on every module
-PyObject* py_set_global_hooks(PyObject*, PyObject* list) {
+// set_module_class(class, its forward, nn.Module, nn.Module.__call__, nn.Module._call_impl, [dictionaries of hooks on every module])
+PyObject* py_set_module_class(PyObject*, PyObject* args) {
     HANDLE_TH_ERRORS
-    TORCH_CHECK(PyList_Check(list), "a list of dictionaries");
-    std::vector<PyObject*> hooks;
-    for (Py_ssize_t i = 0; i < PyList_GET_SIZE(list); ++i) {
-        TORCH_CHECK(PyDict_Check(PyList_GET_ITEM(list, i)), "a list of dictionaries");
-        hooks.push_back(Py_NewRef(PyList_GET_ITEM(list, i)));
+    PyObject *type, *forward, *base, *call, *call_impl, *hooks;
+    if (!PyArg_ParseTuple(args, "O!OO!OOO!", &PyType_Type, &type, &forward, &PyType_Type, &base, &call, &call_impl, &PyList_Type, &hooks)) return nullptr;
+    ModuleClass c;
+    for (Py_ssize_t i = 0; i < PyList_GET_SIZE(hooks); ++i) {
+        TORCH_CHECK(PyDict_Check(PyList_GET_ITEM(hooks, i)), "a list of dictionaries");
+        c.global_hooks.push_back(PyList_GET_ITEM(hooks, i));
     }
-    g_global_hooks.swap(hooks);
-    for (PyObject* h : hooks) Py_DECREF(h);
+    c.type = reinterpret_cast<PyTypeObject*>(type);
+    c.base = reinterpret_cast<PyTypeObject*>(base);
+    c.forward = forward;
+    c.call = call;
+    c.call_impl = call_impl;
+    for (PyObject* o : {type, forward, base, call, call_impl}) Py_INCREF(o);     // (for the life of the process)
+    for (PyObject* o : c.global_hooks) Py_INCREF(o);
+    g_module_class = std::move(c);
     Py_RETURN_NONE;
     END_HANDLE_TH_ERRORS
 }
@@ -618,7 +640,7 @@ PyMethodDef kMethods[] = {
     {"words_to", (PyCFunction)(void*)py_words_to, METH_FASTCALL, nullptr},
     {"permute_scale", (PyCFunction)(void*)py_permute_scale, METH_FASTCALL, nullptr},
     {"module_call", (PyCFunction)(void (*)(void))py_module_call, METH_FASTCALL, nullptr},
-    {"set_global_hooks", py_set_global_hooks, METH_O, nullptr},
+    {"set_module_class", py_set_module_class, METH_VARARGS, nullptr},
     {"set_scratch", py_set_scratch, METH_VARARGS, nullptr},
     {"set_thread_scratch", py_set_thread_scratch, METH_VARARGS, nullptr},
     {"set_callbacks", py_set_callbacks, METH_VARARGS, nullptr},

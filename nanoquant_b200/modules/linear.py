@@ -60,12 +60,9 @@ class NanoQuantLinear(nn.Module):
     # ------------------------------------------------------------------ forward
     def __call__(self, *args, **kwargs):
         # nn.Module's way from a call to `forward`, and from there to the launch, costs a third of a decode call's time on the host.
-        # It is taken for everything but a call that it would pass on unchanged and unseen: no hooks, no tracing, no compiler, no Python
-        # profiler or debugger, the forward below, and nn.Module's own way of calling (which tools replace to see every module's calls).
-        if (len(args) == 1 and not kwargs and self.__class__ is NanoQuantLinear and NanoQuantLinear.forward is _FORWARD
-                and nn.Module.__call__ is _CALL and NanoQuantLinear._call_impl is _CALL_IMPL
-                and not torch.compiler.is_compiling()):
-            y = _lib.ext().module_call(self.__dict__, args[0])
+        # `module_call` goes past it where nobody could tell: see there.
+        if len(args) == 1 and not kwargs and not torch.compiler.is_compiling():
+            y = _lib.ext().module_call(self, args[0])
             if y is not None:
                 return y
         return super().__call__(*args, **kwargs)
@@ -240,11 +237,16 @@ class NanoQuantLinear(nn.Module):
         return state
 
 
-def _stock(name):
-    """nn.Module's function `name`; something that nothing is when it has been replaced already."""
-    f = getattr(nn.Module, name, None)
-    return f if getattr(f, "__module__", "") == nn.Module.__module__ and not hasattr(f, "__wrapped__") else object()
+def module_class():
+    """What the native ``module_call`` compares with before it goes past ``nn.Module.__call__``.  A function of nn.Module that has been
+    replaced already is none of its own: every call then goes the long way, as in another torch without one of these."""
+    def own(name):
+        f = getattr(nn.Module, name, None)
+        return f if getattr(f, "__module__", "") == nn.Module.__module__ and not hasattr(f, "__wrapped__") else object()
+
+    hooks = [getattr(nn.modules.module, f"_global_{kind}_hooks", None) for kind in ("forward", "forward_pre", "backward", "backward_pre")]
+    return (NanoQuantLinear, _FORWARD, nn.Module, own("__call__"), own("_call_impl"),
+            hooks if all(isinstance(h, dict) for h in hooks) else [{"unknown": True}])
 
 
-# a call goes the long way when somebody has replaced one of these
-_FORWARD, _CALL, _CALL_IMPL = NanoQuantLinear.forward, _stock("__call__"), _stock("_call_impl")
+_FORWARD = NanoQuantLinear.forward

@@ -83,10 +83,8 @@ def connect_host_path(ext) -> None:
     implementations of the operators."""
     ext.set_callbacks(_lib.check, lambda idx, nbytes: scratch_for(torch.device("cuda", idx), nbytes),
                       _nanoquant_dyn_forward_cuda, _marlin_nanoquant_forward_cuda)
-    from torch.nn.modules import module as nn_module
-    kinds = ("_global_forward_hooks", "_global_forward_pre_hooks", "_global_backward_hooks", "_global_backward_pre_hooks")
-    hooks = [getattr(nn_module, kind, None) for kind in kinds]     # another torch, without one of them: no short way for module calls
-    ext.set_global_hooks(hooks if all(isinstance(h, dict) for h in hooks) else [{"unknown": True}])
+    from .modules import linear
+    ext.set_module_class(*linear.module_class())
     for idx, buf in _scratch.items():
         ext.set_scratch(idx, buf.data_ptr(), buf.numel())
 

@@ -166,7 +166,7 @@ def test_call_is_seen_by_whoever_watches_module_calls(tmp_path):
     m, _ = _module(256, 96, 200, torch.bfloat16, "gemv", False, seed=5)
     x = torch.randn(3, 256, device="cuda").to(torch.bfloat16)
     want, seen = m(x), []
-    assert linear._CALL is torch.nn.Module.__call__ and linear._CALL_IMPL is torch.nn.Module._call_impl   # (unwatched: the short way)
+    assert linear.module_class()[3:5] == (torch.nn.Module.__call__, torch.nn.Module._call_impl)      # (unwatched: the short way)
 
     def watched(f):
         def call(self, *args, **kwargs):
