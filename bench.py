@@ -265,14 +265,16 @@ def group_call(L, T, gemm_from=0):
 
 def group_kernels(L, shapes, T, gemm_from=0):
     """Kernels that one call of `group_call` launches for linears of `shapes` [(N, R, M)], in order: above the decode limit
-    one per stage (up to 16 tokens the batch kernel, 8 for large launches, as nq_batch.cu's batch_max_tokens; then one of the two
-    GEMMs, whose planners choose by a predicted time: named together); below it one launch of the decode kernel per four tokens, except that
-    linears with more than 3328 columns and a rank from 128 run four tokens as the two stages of the batch kernel."""
+    one per stage (the batch kernel or one of the two GEMMs: the library is asked); below it one launch of the decode kernel per four tokens,
+    except that linears with more than 3328 columns and a rank from 128 run four tokens as the two stages of the batch kernel."""
     if T >= (gemm_from or L.nq_gemv_max_tokens() + 1):
-        stages = [[(N, R) for (N, R, _) in shapes], [(R, M) for (_, R, M) in shapes]]
-        most = min(8 if b >= 8e6 or (b >= 4.5e6 and k >= 8192) else 16
-                   for b, k in ((sum(K * rows / 8 for K, rows in st), max(K for K, _ in st)) for st in stages))
-        return ["batch_stage_kernel" if T <= most else "wgemm_kernel, pgemm_kernel"] * 2
+        from nanoquant_b200 import _lib
+        arr = (_lib.LinearDesc * len(shapes))()
+        for d, (N, R, M) in zip(arr, shapes):
+            d.N, d.R, d.M = N, R, M
+        ids = (ctypes.c_int * 2)()
+        _lib.check(L.nq_gemm_group_kernels(arr, len(arr), T, ids), "nq_gemm_group_kernels")
+        return [_lib.GEMM_KERNELS[i] for i in ids]
     two = [N > 3328 and R >= 128 and N % 8 == 0 and R % 8 == 0 for (N, R, _) in shapes]
     if T < 4 or not any(two):
         return ["gemv_group_kernel"] * -(-T // 4)
@@ -282,7 +284,8 @@ def group_kernels(L, shapes, T, gemm_from=0):
 
 ARITHMETIC = {"gemv_group_kernel": "s8 mma / s32 accumulate on 16-bit fixed point; bf16 in/out",
               "batch_stage_kernel": "bf16 mma / f32 accumulate; bf16 in/out",
-              "wgemm_kernel, pgemm_kernel": "bf16 tcgen05 mma / f32 accumulate; bf16 in/out"}
+              "wgemm_kernel": "bf16 tcgen05 mma / f32 accumulate; bf16 in/out",
+              "pgemm_kernel": "bf16 tcgen05 mma / f32 accumulate; bf16 in/out"}
 
 
 class Step:

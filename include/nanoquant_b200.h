@@ -268,6 +268,11 @@ size_t nq_gemm_group_scratch_bytes(const nq_linear_desc* linears_host, int n_lin
 int nq_gemm_group_fwd(const nq_linear_desc* linears_host, int n_linears, int T, int dtype,
                       void* scratch, size_t scratch_bytes, nq_stream_t stream);
 
+/* Which kernels nq_gemm_group_fwd runs for such a group on the current device: kernels_host[0] its first stage, [1] its second.  Only the
+ * sizes N, R, M of the descriptors are read.  For tests and measurements, which name what they ran. */
+enum { NQ_KERNEL_BATCH = 0, NQ_KERNEL_WGEMM = 1, NQ_KERNEL_PGEMM = 2 };
+int nq_gemm_group_kernels(const nq_linear_desc* linears_host, int n_linears, int T, int* kernels_host);
+
 /* One stage: y[T, Nout] = s_out * (W . (s_in * x[T, K])) with W [Nout, K] in the
  * tile layout; s_in and s_out may be NULL.  `status_word` points at a zeroed
  * 16-byte device area (a scratch header works) whose third word receives a

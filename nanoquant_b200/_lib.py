@@ -18,6 +18,8 @@ NQ_F16, NQ_BF16 = 0, 1
 NQ_LSB_FIRST, NQ_HALF2 = 0, 1
 ORDER_ID = {"lsb_first": NQ_LSB_FIRST, "half2": NQ_HALF2}
 
+GEMM_KERNELS = ("batch_stage_kernel", "wgemm_kernel", "pgemm_kernel")     # NQ_KERNEL_*
+
 NQ_OK = 0
 NQ_ERR_NULL, NQ_ERR_SHAPE, NQ_ERR_DTYPE, NQ_ERR_ALIGN = -1, -2, -3, -4
 NQ_ERR_SCRATCH, NQ_ERR_CUDA, NQ_ERR_TIMEOUT, NQ_ERR_UNSUPPORTED, NQ_ERR_TOO_LARGE = -5, -6, -7, -8, -9
@@ -59,6 +61,7 @@ SIGNATURES = {
     "nq_gemm_fwd": (c_int, [c_void_p] * 8 + [c_size_t, c_int, c_int, c_int, c_int, c_int, c_void_p]),
     "nq_gemm_group_scratch_bytes": (c_size_t, [ctypes.POINTER(LinearDesc), c_int, c_int]),
     "nq_gemm_group_fwd": (c_int, [ctypes.POINTER(LinearDesc), c_int, c_int, c_int, c_void_p, c_size_t, c_void_p]),
+    "nq_gemm_group_kernels": (c_int, [ctypes.POINTER(LinearDesc), c_int, c_int, ctypes.POINTER(c_int)]),
     "nq_onebit_gemm_fwd": (c_int, [c_void_p] * 6 + [c_int, c_int, c_int, c_int, c_void_p]),
     "nq_allgather_state_bytes": (c_size_t, []),
     "nq_allgather_flags_bytes": (c_size_t, [c_int]),

@@ -140,6 +140,17 @@ int encode_activations(CUtensorMap* map, const StageJob& S, int bf16, int T, int
     return r == CUDA_SUCCESS ? NQ_OK : NQ_ERR_UNSUPPORTED;
 }
 
+// The kernel of a stage, with its plan.  (An intermediate in the GEMMs' column order is theirs.)
+static int pick_kernel(const StageJob* jobs, int n, int T, int order, WgemmPlan& w, PgemmPlan& p) {
+    if (order == 0 && T <= batch_max_tokens(jobs, n)) return NQ_KERNEL_BATCH;
+    p = plan_pgemm(jobs, n, T, order);
+    return plan_wgemm(jobs, n, T, order, w) && w.us <= p.us ? NQ_KERNEL_WGEMM : NQ_KERNEL_PGEMM;
+}
+// Both stages of a group by the batch kernel, which keeps the intermediate in its own order.
+static bool both_batch(const StageJob* s1, const StageJob* s2, int n, int T) {
+    return T <= batch_max_tokens(s1, n) && T <= batch_max_tokens(s2, n);
+}
+
 // One stage of up to four linears: out_j[T, Nout_j] = (a_j[T, K_j] . W_j^T) * post_j.
 static int launch_stage(const StageJob* jobs, int n, int T, StageTypes ty, int saturate, unsigned* status, cudaStream_t stream) {
     if (n < 1 || n > kMaxGemmJobs) return NQ_ERR_UNSUPPORTED;
@@ -148,11 +159,13 @@ static int launch_stage(const StageJob* jobs, int n, int T, StageTypes ty, int s
         if (!aligned16(S.a) || (S.lda % 8) != 0 || (S.K % 8) != 0) return NQ_ERR_ALIGN;   // TMA: 16-byte base and stride
         if (S.pre && !aligned16(S.pre)) return NQ_ERR_ALIGN;
     }
-    if (T <= batch_max_tokens(jobs, n) && ty.order == 0) return launch_batch_stage(jobs, n, T, ty, saturate, false, false, false, status, stream);
     WgemmPlan w;
-    const PgemmPlan p = plan_pgemm(jobs, n, T, ty.order);
-    if (plan_wgemm(jobs, n, T, ty.order, w) && w.us <= p.us) return launch_wgemm_stage(jobs, n, T, ty, saturate, w, status, stream);
-    return launch_pgemm_stage(jobs, n, T, ty, saturate, p, status, stream);
+    PgemmPlan p;
+    switch (pick_kernel(jobs, n, T, ty.order, w, p)) {
+        case NQ_KERNEL_BATCH: return launch_batch_stage(jobs, n, T, ty, saturate, false, false, false, status, stream);
+        case NQ_KERNEL_WGEMM: return launch_wgemm_stage(jobs, n, T, ty, saturate, w, status, stream);
+        default: return launch_pgemm_stage(jobs, n, T, ty, saturate, p, status, stream);
+    }
 }
 
 static int g_precise_intermediate = 0;   // see nq_gemm_set_precise_intermediate
@@ -232,8 +245,7 @@ int nq_gemm_group_fwd(const nq_linear_desc* d, int n_linears, int T, int dtype, 
         s1[j] = {L.x, L.ldx, L.v_tiles, L.s_in, L.s_mid, t, L.R, L.N, L.R, nullptr, nullptr, 0, row_exp};
         s2[j] = {t, L.R, L.u_tiles, nullptr, L.s_out, L.y, L.ldy, L.R, L.M, L.bias, L.residual, L.ldr, row_exp};
     }
-    // few tokens: both stages by the batch kernel, which keeps the intermediate in its own order
-    const bool batch = T <= batch_max_tokens(s1, n_linears) && T <= batch_max_tokens(s2, n_linears);
+    const bool batch = both_batch(s1, s2, n_linears, T);
     auto stages = [&](StageTypes ty1, StageTypes ty2) -> int {
         if (batch) {
             const int st = launch_batch_stage(s1, n_linears, T, ty1, 0, false, true, false, status, as_stream(stream));
@@ -283,6 +295,24 @@ int nq_gemm_group_fwd(const nq_linear_desc* d, int n_linears, int T, int dtype, 
         NQ_CUDA_TRY(e);
     }
     return stages(StageTypes{1, 1, 0, +1}, StageTypes{1, 0, 1, -1});
+}
+
+int nq_gemm_group_kernels(const nq_linear_desc* d, int n_linears, int T, int* kernels) {
+    if (!d || !kernels) return NQ_ERR_NULL;
+    if (n_linears <= 0 || n_linears > kMaxGemmJobs) return NQ_ERR_UNSUPPORTED;
+    if (T <= 0) return NQ_ERR_SHAPE;
+    StageJob s1[kMaxGemmJobs] = {}, s2[kMaxGemmJobs] = {};
+    for (int j = 0; j < n_linears; ++j) {
+        if (d[j].N <= 0 || d[j].R <= 0 || d[j].M <= 0 || d[j].N % 8 || d[j].R % 8) return NQ_ERR_SHAPE;
+        s1[j].K = d[j].N; s1[j].Nout = s2[j].K = d[j].R; s2[j].Nout = d[j].M;
+        s1[j].pre = d;      // (not read: a first stage has input scales)
+    }
+    WgemmPlan w;
+    PgemmPlan p;
+    const bool batch = both_batch(s1, s2, n_linears, T);
+    kernels[0] = batch ? (int)NQ_KERNEL_BATCH : pick_kernel(s1, n_linears, T, kOrderOut, w, p);
+    kernels[1] = batch ? (int)NQ_KERNEL_BATCH : pick_kernel(s2, n_linears, T, kOrderIn, w, p);
+    return NQ_OK;
 }
 
 int nq_gemm_fwd(const void* x, const void* s_in, const void* v_tiles, const void* s_mid, const void* u_tiles,
