@@ -273,6 +273,12 @@ int nq_gemm_group_fwd(const nq_linear_desc* linears_host, int n_linears, int T, 
 enum { NQ_KERNEL_BATCH = 0, NQ_KERNEL_WGEMM = 1, NQ_KERNEL_PGEMM = 2 };
 int nq_gemm_group_kernels(const nq_linear_desc* linears_host, int n_linears, int T, int* kernels_host);
 
+/* Attempts (of up to about 2 us each) that a wait inside the two GEMM kernels (17 tokens and more, and large launches from nine on) may
+ * spend before the launch gives up and sets the status word (NQ_ERR_TIMEOUT); its results are then void.  0 restores the default
+ * (2^21, seconds).  Host-side setting read at launch time; returns the previous value.  For failure-path tests and for callers that
+ * want a tighter bound. */
+unsigned nq_gemm_set_wait_limit(unsigned attempts);
+
 /* One stage: y[T, Nout] = s_out * (W . (s_in * x[T, K])) with W [Nout, K] in the
  * tile layout; s_in and s_out may be NULL.  `status_word` points at a zeroed
  * 16-byte device area (a scratch header works) whose third word receives a

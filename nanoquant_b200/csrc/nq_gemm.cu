@@ -168,6 +168,10 @@ static int launch_stage(const StageJob* jobs, int n, int T, StageTypes ty, int s
     }
 }
 
+constexpr unsigned kGemmWaitLimit = 1u << 21;      // seconds
+static unsigned g_gemm_wait_limit = kGemmWaitLimit;
+unsigned gemm_wait_limit() { return g_gemm_wait_limit; }
+
 static int g_precise_intermediate = 0;   // see nq_gemm_set_precise_intermediate
 
 }  // namespace nq
@@ -331,6 +335,12 @@ int nq_gemm_fwd(const void* x, const void* s_in, const void* v_tiles, const void
 int nq_gemm_set_precise_intermediate(int on) {
     const int old = g_precise_intermediate;
     g_precise_intermediate = on ? 1 : 0;
+    return old;
+}
+
+unsigned nq_gemm_set_wait_limit(unsigned attempts) {
+    const unsigned old = g_gemm_wait_limit;
+    g_gemm_wait_limit = attempts ? attempts : kGemmWaitLimit;
     return old;
 }
 

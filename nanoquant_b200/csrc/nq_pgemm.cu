@@ -63,13 +63,14 @@ struct alignas(16) PJob {
 };
 static_assert(sizeof(PJob) == 112, "seven 16-byte words");
 struct alignas(16) PHead {
-    unsigned* status;
+    unsigned* status;      // (this and the wait limit are read from the parameters, not from the copy)
     int njobs, tiles;
     int T;
     int ntok, stages, accs;   // tokens of a tile (a multiple of 16), pipeline stages of 64 columns, accumulators (1 or 2)
     int is_bf16, a_bf16, saturate, exp_sign;
     int order;                // kOrderOut, kOrderIn
     int off_out, off_pre;     // output staging; input scales of job j from off_pre + pre0 (pre0 < 0: read from global memory)
+    unsigned wait_limit;
 };
 struct alignas(64) PParams {
     CUtensorMap map_a[kMaxGemmJobs];     // activations [T, K], box 64 x half of a tile's tokens, 128-byte swizzle
@@ -83,17 +84,6 @@ static_assert(kPParamWords * 16 <= kPBarOff && kPBOff % 1024 == 0, "shared memor
 
 enum : int { kPOutFp16, kPOutBf16, kPOutBf16Saturated };
 
-// Bounded wait for a barrier that the other CTA signals as well (a whole warp).
-__device__ __forceinline__ bool pair_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag, unsigned* status) {
-    if (__all_sync(0xffffffffu, mbar_try_cluster(bar, parity))) return true;
-    for (unsigned i = 0; i < kMbarWaitLimit; ++i) {
-        if (__all_sync(0xffffffffu, mbar_try_cluster(bar, parity))) return true;
-        if (__any_sync(0xffffffffu, *abort_flag != 0)) return false;
-    }
-    *abort_flag = 1;
-    if ((threadIdx.x & 31) == 0) atomicExch(status, (unsigned)(-NQ_ERR_TIMEOUT));
-    return false;
-}
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {   // `bar`: an address of cluster_map
     asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }
@@ -191,7 +181,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPThreads, 1) pgemm_
             const CUtensorMap* map = &Pc.map_a[j];
             const int m0 = mt * ntok + rank * (ntok >> 1), nst = (jobs[j].K + 127) >> 7;
             for (int st = 0; st < nst; ++st) {
-                ok = mbar_wait_warp(bar_free(s), ph ^ 1, abort_flag, P.status);
+                ok = mbar_wait_warp(bar_free(s), ph ^ 1, abort_flag, Pc.head.status, Pc.head.wait_limit);
                 if (!ok) break;
                 if (elect_one()) {
                     if (rank == 0) mbar_expect_tx(bar_ready(s), 2u * stage_bytes);
@@ -213,9 +203,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPThreads, 1) pgemm_
             for (int t = first; t < tiles && ok; t += pairs) {
                 const int nst = (jobs[job_of(t)].K + 127) >> 7;
                 const uint32_t d = tmem_base + (uint32_t)(a * ntok);
-                ok = pair_wait_warp(bar_acc_empty(a), aph ^ 1, abort_flag, P.status);
+                ok = mbar_wait_warp<true>(bar_acc_empty(a), aph ^ 1, abort_flag, Pc.head.status, Pc.head.wait_limit);
                 for (int st = 0; st < nst && ok; ++st) {
-                    ok = pair_wait_warp(bar_ready(s), ph, abort_flag, P.status);
+                    ok = mbar_wait_warp<true>(bar_ready(s), ph, abort_flag, Pc.head.status, Pc.head.wait_limit);
                     if (!ok) break;
                     tc_fence_after();
                     if (elect_one()) {
@@ -286,7 +276,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPThreads, 1) pgemm_
         seek();
         uint4 w1 = fetch(), w2 = fetch();
         unsigned base = 0;                 // steps before this tile
-        bool ok = mbar_wait_warp(bar_pre, 0, abort_flag, P.status);
+        bool ok = mbar_wait_warp(bar_pre, 0, abort_flag, Pc.head.status, Pc.head.wait_limit);
         for (int t = first; t < tiles && ok; t += pairs) {
             const PJob& J = jobs[job_of(t)];
             const int K = J.K, nst = (K + 127) >> 7, chunks = J.chunks;
@@ -327,7 +317,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPThreads, 1) pgemm_
                             expand_swapped(w, hf, one2, v);
                         }
                         if (hf == 0) {
-                            ok = mbar_wait_warp(bar_free(s), ph ^ 1, abort_flag, P.status);
+                            ok = mbar_wait_warp(bar_free(s), ph ^ 1, abort_flag, Pc.head.status, Pc.head.wait_limit);
                             tc_fence_after();
                         }
                         tmem_st_frag4(a_lane + (uint32_t)(64 * s + 32 * hf), v);
@@ -372,7 +362,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPThreads, 1) pgemm_
             const long long ld_out = J.ld_out;
             uint16_t* out = static_cast<uint16_t*>(J.out) + (size_t)(m0 + 32 * set + ld_tok) * ld_out + row_s;
             const bool whole = row_s + 8 <= Nout && ((reinterpret_cast<uintptr_t>(out) | (uintptr_t)(2 * ld_out)) & 15u) == 0;
-            ok = ok && mbar_wait_warp(bar_acc_full(a), aph, abort_flag, P.status);
+            ok = ok && mbar_wait_warp(bar_acc_full(a), aph, abort_flag, Pc.head.status, Pc.head.wait_limit);
             tc_fence_after();                         // (not ok: on all the same, the four warps pass the same barriers)
             const uint32_t d_lane = tmem_base + (uint32_t)(a * ntok) + ((uint32_t)(32 * ew) << 16);
             bool held = true;                         // the accumulator
@@ -540,7 +530,7 @@ int launch_pgemm_stage(const StageJob* jobs_in, int n, int T, StageTypes ty, int
     PHead& H = P.head;
     int stages = (kPTmemCols - accs * ntok) / 64;
     if (stages > kPMaxStages) stages = kPMaxStages;
-    H.njobs = n; H.status = status; H.T = T; H.ntok = ntok; H.stages = stages; H.accs = accs;
+    H.njobs = n; H.status = status; H.wait_limit = gemm_wait_limit(); H.T = T; H.ntok = ntok; H.stages = stages; H.accs = accs;
     H.is_bf16 = ty.io_bf16; H.a_bf16 = ty.a_bf16; H.saturate = saturate; H.exp_sign = ty.exp_sign; H.order = ty.order;
     H.off_out = kPBOff + stages * ntok * 128;
     H.off_pre = H.off_out + kPOutBytes;

@@ -7,27 +7,27 @@
 
 namespace nq {
 
-constexpr unsigned kMbarWaitLimit = 1u << 21;   // attempts of up to ~2 us each
-
-// Bounded wait on an mbarrier phase.  Returns false when the limit expired or another
-// thread of the CTA already gave up; the caller then leaves its loop.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag,
-                                          unsigned* status) {
-    if (mbar_try(bar, parity)) return true;   // the common case: already complete
-    for (unsigned i = 0; i < kMbarWaitLimit; ++i) {
-        if (mbar_try(bar, parity)) return true;
-        if (*abort_flag) return false;
-    }
-    *abort_flag = 1;
-    atomicExch(status, (unsigned)(-NQ_ERR_TIMEOUT));
-    return false;
+// mbar_try for a barrier that other CTAs of the cluster signal.
+__device__ __forceinline__ bool mbar_try_cluster(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2, %3;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok) : "r"(bar), "r"(parity), "r"(2000u) : "memory");
+    return ok != 0;
 }
-
-// The same for a whole warp: every lane returns the same.
-__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag, unsigned* status) {
-    if (__all_sync(0xffffffffu, mbar_try(bar, parity))) return true;
-    for (unsigned i = 0; i < kMbarWaitLimit; ++i) {
-        if (__all_sync(0xffffffffu, mbar_try(bar, parity))) return true;
+// Bounded wait of a whole warp on an mbarrier phase; every lane returns the same.  False when `limit` more attempts (of some 2 us each)
+// after the first were in vain, which sets the status word, or when another warp of the CTA has already given up; the caller then leaves
+// its loop.  `status` and `limit` are taken from the kernel's parameters (__grid_constant__): as constants they occupy no registers.  Read from
+// the descriptors' copy in shared memory both GEMMs spilled 8 to 16 bytes (128 tokens module by module 135 -> 133 us without, 517 tokens 186 -> 183).
+// CLUSTER: a barrier that other CTAs of the cluster signal.
+template <bool CLUSTER = false>
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag, unsigned* status, unsigned limit) {
+    auto done = [&]() { return __all_sync(0xffffffffu, CLUSTER ? mbar_try_cluster(bar, parity) : mbar_try(bar, parity)); };
+    if (done()) return true;   // the common case: already complete
+    for (unsigned i = 0; i < limit; ++i) {
+        if (done()) return true;
         if (__any_sync(0xffffffffu, *abort_flag != 0)) return false;
     }
     *abort_flag = 1;
@@ -68,16 +68,6 @@ __device__ __forceinline__ uint32_t cluster_map(uint32_t local, uint32_t rank) {
 __device__ __forceinline__ void cluster_store4_tx(uint32_t addr, uint32_t bar, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
     asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1,%2,%3,%4}, [%5];"
                  ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d), "r"(bar) : "memory");
-}
-// mbar_try for a barrier that other CTAs of the cluster signal.
-__device__ __forceinline__ bool mbar_try_cluster(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2, %3;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok) : "r"(bar), "r"(parity), "r"(2000u) : "memory");
-    return ok != 0;
 }
 
 // ---------------------------------------------------------------------------

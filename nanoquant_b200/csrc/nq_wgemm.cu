@@ -64,7 +64,7 @@ struct alignas(16) WJob {
 };
 static_assert(sizeof(WJob) == 96, "six 16-byte words");
 struct alignas(16) WHead {
-    unsigned* status;
+    unsigned* status;      // (this and the wait limit are read from the parameters, not from the copy)
     int njobs;
     int T;
     int ntok, stages;      // tokens of a tile (a multiple of 16), pipeline stages of 128 columns
@@ -72,6 +72,7 @@ struct alignas(16) WHead {
     int order;             // kOrderOut, kOrderIn
     int csplit, owned;
     int off_recv, off_pre;
+    unsigned wait_limit;
 };
 struct alignas(64) WParams {
     CUtensorMap map_a[kMaxGemmJobs];     // activations [T, K], box 64 x tokens of a tile, 128-byte swizzle
@@ -190,7 +191,7 @@ __global__ void __launch_bounds__(kWThreads, 2) wgemm_kernel(const __grid_consta
         int s = 0;
         uint32_t ph = 0;
         for (int ks = 0; ks < nks; ++ks) {
-            if (!mbar_wait_warp(bar_free(s), ph ^ 1, abort_flag, P.status)) break;
+            if (!mbar_wait_warp(bar_free(s), ph ^ 1, abort_flag, Pc.head.status, Pc.head.wait_limit)) break;
             if (elect_one()) {
                 const uint32_t dst = b_base + (uint32_t)s * stage_bytes;
                 mbar_expect_tx(bar_ready(s), stage_bytes);
@@ -206,7 +207,7 @@ __global__ void __launch_bounds__(kWThreads, 2) wgemm_kernel(const __grid_consta
         uint32_t ph = 0;
         bool good = true;
         for (int ks = 0; ks < nks; ++ks) {
-            good = mbar_wait_warp(bar_ready(s), ph, abort_flag, P.status);
+            good = mbar_wait_warp(bar_ready(s), ph, abort_flag, Pc.head.status, Pc.head.wait_limit);
             if (!good) break;
             tc_fence_after();
             if (elect_one()) {
@@ -260,7 +261,7 @@ __global__ void __launch_bounds__(kWThreads, 2) wgemm_kernel(const __grid_consta
         const uint2* s_pre = reinterpret_cast<const uint2*>(smem + P.off_pre) + q;
         const int K_left = J.K - 256 * c_begin;
         const uint32_t a_lane = tmem_a + ((uint32_t)(32 * (warp & 3)) << 16);
-        if (pre && nks > 0) ok = mbar_wait_warp(bar_pre, 0, abort_flag, P.status);
+        if (pre && nks > 0) ok = mbar_wait_warp(bar_pre, 0, abort_flag, Pc.head.status, Pc.head.wait_limit);
         int s = grp;
         uint32_t ph = 0;
         const int pre_shift = grp ? 0 : 4;
@@ -293,7 +294,7 @@ __global__ void __launch_bounds__(kWThreads, 2) wgemm_kernel(const __grid_consta
                     if (in_order) expand_columns(w, hf, pn, v);
                     else expand_swapped(w, hf, one2, v);
                     if (hf == 0 && rr == 0) {
-                        ok = mbar_wait_warp(bar_free(s), ph ^ 1, abort_flag, P.status);
+                        ok = mbar_wait_warp(bar_free(s), ph ^ 1, abort_flag, Pc.head.status, Pc.head.wait_limit);
                         tc_fence_after();
                     }
                     tmem_st_frag4(a_lane + ((uint32_t)(16 * rr) << 16) + (uint32_t)(64 * s + 32 * hf), v);
@@ -313,7 +314,7 @@ __global__ void __launch_bounds__(kWThreads, 2) wgemm_kernel(const __grid_consta
             s_post[tu] = J.post ? as_float(raw_post) : 1.f;
             s_bias[tu] = J.bias ? as_float(raw_bias) : 0.f;
         }
-        if (ok) ok = mbar_wait_warp(bar_accum, 0, abort_flag, P.status);
+        if (ok) ok = mbar_wait_warp(bar_accum, 0, abort_flag, Pc.head.status, Pc.head.wait_limit);
         tc_fence_after();
     }
     // ---------------------------------------------------------------- exchange of the partial sums
@@ -367,7 +368,8 @@ __global__ void __launch_bounds__(kWThreads, 2) wgemm_kernel(const __grid_consta
                     for (int e = 0; e < 8; ++e) r[e] = 0.f;
                 }
                 if (csplit > 1 && b == crank) {
-                    for (unsigned i = 0; i < kMbarWaitLimit && !mbar_try_cluster(bar_recv, 0); ++i) {}
+                    ok = mbar_wait_warp<true>(bar_recv, 0, abort_flag, Pc.head.status, Pc.head.wait_limit);
+                    if (!ok) break;      // (all 256 threads still pass the barrier below)
                 }
                 for (int rk = 0; rk < csplit - 1; ++rk) {
                     const unsigned char* src = smem + P.off_recv + (rk * owned + idx) * 8192 + rgl * 1024 + lane * 16;
@@ -556,7 +558,7 @@ int launch_wgemm_stage(const StageJob* jobs, int n, int T, StageTypes ty, int sa
     WParams P;
     memset(&P, 0, sizeof(P));
     WHead& H = P.head;
-    H.njobs = n; H.status = status; H.T = T; H.ntok = pl.ntok; H.stages = pl.stages; H.csplit = pl.csplit;
+    H.njobs = n; H.status = status; H.wait_limit = gemm_wait_limit(); H.T = T; H.ntok = pl.ntok; H.stages = pl.stages; H.csplit = pl.csplit;
     H.owned = pl.owned; H.off_recv = pl.off_recv; H.off_pre = pl.off_pre;
     H.is_bf16 = ty.io_bf16; H.a_bf16 = ty.a_bf16; H.saturate = saturate; H.exp_sign = ty.exp_sign; H.order = ty.order;
     int tiles = 0;

@@ -4,7 +4,7 @@ next call after re-zeroing works."""
 import pytest
 import torch
 
-from tests.util import assert_parity, exact_np, make_layer, tiles_on_gpu
+from tests.util import assert_parity, exact_np, gemm_kernels, make_group, make_layer, tiles_on_gpu
 
 pytestmark = pytest.mark.gpu
 
@@ -94,3 +94,52 @@ def test_allgather_wait_for_an_absent_peer_expires():
         assert torch.equal(buf[1024:1024 + 128].view(torch.float16), shard)
     finally:
         Lb.nq_allgather_set_wait_limit(old)
+
+
+@pytest.mark.parametrize("kernel,stage,T,shapes", [
+    # 32 steps of 128 columns in a first stage of 16 CTAs: the second stage's CTAs, resident from the start, wait for it
+    ("wgemm_kernel", 1, 128, [(32768, 256, 4096)]),
+    # K split over two CTAs in the second stage: the second CTA of the linear of rank 256 has no columns, and owns the tokens from 16 on,
+    # for which it waits in vain (the first one gave up behind the first stage)
+    ("wgemm_kernel", 1, 32, [(32768, 512, 128), (32768, 256, 128)]),
+    # the epilogue of a pair waits for a tile's main loop
+    ("pgemm_kernel", 0, 2048, [(4096, 2048, 256)]),
+])
+def test_gemm_wait_that_runs_out(kernel, stage, T, shapes):
+    # With a limit of one attempt (some us) after the first, waits that are satisfied a little later run out.  The launch ends all the same,
+    # drains what is in flight, gives its tensor memory back and reports; the next one on a zeroed scratch is right.
+    from nanoquant_b200 import _lib
+    Lb = _lib.lib()
+    dtype = torch.float16
+    layers = make_group(shapes, T, dtype, seed=T)
+    keep, descs, ys = [], [], []
+    for L in layers:
+        vt, ut = tiles_on_gpu(L["V"]), tiles_on_gpu(L["U"])
+        keep += [vt, ut]
+        ys.append(torch.empty(T, L["M"], dtype=dtype, device="cuda"))
+        descs.append(_lib.LinearDesc(L["x"].data_ptr(), L["s_pre"].data_ptr(), vt.data_ptr(), L["s_mid"].data_ptr(), ut.data_ptr(),
+                                     L["s_post"].data_ptr(), ys[-1].data_ptr(), L["N"], L["R"], L["M"], L["N"], L["M"]))
+    arr = (_lib.LinearDesc * len(descs))(*descs)
+    st = torch.cuda.current_stream().cuda_stream
+    scratch = torch.zeros(Lb.nq_gemm_group_scratch_bytes(arr, len(arr), T), dtype=torch.uint8, device="cuda")
+    run = lambda: _lib.check(Lb.nq_gemm_group_fwd(arr, len(arr), T, _lib.NQ_F16, scratch.data_ptr(), scratch.numel(), st), "nq_gemm_group_fwd")
+    status = lambda: Lb.nq_scratch_status(scratch.data_ptr(), st)
+    assert gemm_kernels(shapes, T)[stage] == kernel
+    run()
+    assert status() == 0
+    old = Lb.nq_gemm_set_wait_limit(1)
+    try:
+        ys[-1].fill_(7)
+        run()
+        assert status() == _lib.NQ_ERR_TIMEOUT
+        if len(ys) > 1:                               # no CTA of this linear had all it needs: none stored anything
+            assert (ys[-1] == 7).all()
+    finally:
+        assert Lb.nq_gemm_set_wait_limit(old) == 1
+    run()
+    assert status() == _lib.NQ_ERR_TIMEOUT            # stays until the scratch is zeroed
+    scratch.zero_()
+    run()
+    assert status() == 0
+    for L, y in zip(layers, ys):
+        assert_parity(exact_np(y), L["y64"], dtype, what=f"{L['N']} columns")

@@ -91,3 +91,15 @@ def assert_parity(y, y64, dtype, rel=2e-3, what=""):
     worst = float(excess.max())
     assert worst <= 0, (f"{what}: element exceeds {rel:g}*max|y64| + half ulp by {worst:.3e} "
                         f"(max-normalised error {oc.rel_err(y, y64):.3e})")
+
+
+def gemm_kernels(shapes, T):
+    """The kernels that a launch group of linears `shapes` [(N, R, M)] takes at T tokens (above the decode limit), one per stage."""
+    import ctypes
+    from nanoquant_b200 import _lib
+    arr = (_lib.LinearDesc * len(shapes))()
+    for d, (N, R, M) in zip(arr, shapes):
+        d.N, d.R, d.M = N, R, M
+    ids = (ctypes.c_int * 2)()
+    _lib.check(_lib.lib().nq_gemm_group_kernels(arr, len(arr), T, ids), "nq_gemm_group_kernels")
+    return [_lib.GEMM_KERNELS[i] for i in ids]
