@@ -6,7 +6,7 @@ import pytest
 import torch
 
 from tests import test_batch_edges_gpu as edges
-from tests.util import make_group, tiles_on_gpu
+from tests.util import gemm_kernels, make_group, tiles_on_gpu
 
 pytestmark = pytest.mark.gpu
 
@@ -37,3 +37,26 @@ def test_runs_give_the_same_bits(T):
     run = lambda: ops.group_forward([L["x"]], tens, T, torch.bfloat16, torch.device("cuda", 0))[0].clone()
     first = run()
     assert all(torch.equal(run(), first) for _ in range(5))
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("T", [9, 12, 16])
+@pytest.mark.parametrize("shapes,below", [
+    # 4.5 MB of packed factors in a first stage with 8192 columns
+    ([(8192, 4400, 264), (8192, 40, 100)], [(8192, 4352, 264), (8192, 32, 100)]),
+    # 8 MB in a second stage
+    ([(264, 40, 100), (264, 1024, 62504)], [(264, 40, 100), (264, 1024, 62440)]),
+])
+def test_large_launches_of_nine_to_sixteen_tokens(shapes, below, T, dtype):
+    # launches above the lines of the rule in nq_batch.cu go to the GEMMs, in tiles of 16 tokens; the ones just below stay
+    batch = 2 * ["batch_stage_kernel"]
+    assert gemm_kernels(shapes, 8) == batch and gemm_kernels(below, T) == batch
+    assert gemm_kernels(shapes, T) == 2 * ["wgemm_kernel"]
+    edges.test_batch_tile_edges(shapes, T, dtype)
+
+
+def test_input_scales_beyond_shared_memory():
+    # pairs keep the input scales of all linears of a launch in shared memory; those of the last two here are read from global memory
+    shapes = 4 * [(16392, 1032, 64)]
+    assert gemm_kernels(shapes, 513)[0] == "pgemm_kernel"
+    edges.test_batch_tile_edges(shapes, 513, torch.bfloat16)
