@@ -540,29 +540,16 @@ int launch_batch_stage(const StageJob* jobs, int n, int tokens, StageTypes ty, i
     P.stage_off = (P.part_off + (int)part_used + 15) / 16 * 16;
     const size_t smem = P.stage_off + stage_bytes;
     if (smem > (size_t)limit) return NQ_ERR_UNSUPPORTED;
-    static bool pdl_ok = true;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(cta);
     cfg.blockDim = dim3(kBatchThreads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = pdl_ok ? 1 : 0;
+    cudaLaunchAttribute attr[1];
     void* args[] = {&P};
     const int rows = most_rows == 1 ? 1 : most_rows == 2 ? 2 : 4;
     const void* fn = split ? split_kernel(ty.a_bf16, rows, frag_in) : batch_kernel(ty.a_bf16, nt, rows, frag_in);
-    cudaError_t e = cudaLaunchKernelExC(&cfg, fn, args);
-    if (e != cudaSuccess && pdl_ok) {
-        (void)cudaGetLastError();
-        pdl_ok = false;
-        cfg.numAttrs = 0;
-        e = cudaLaunchKernelExC(&cfg, fn, args);
-    }
-    NQ_CUDA_TRY(e);
-    return NQ_OK;
+    return launch_dependent(cfg, attr, 0, fn, args);
 }
 
 }  // namespace nq

@@ -117,27 +117,13 @@ int nq_allgather_push(const void* shard, size_t shard_bytes, void* const* rank_b
     size_t ctas = (P.n16 + (size_t)kPushThreads * 4 - 1) / ((size_t)kPushThreads * 4);   // four words per thread
     const size_t cap = (size_t)sm_count();
     ctas = ctas < 1 ? 1 : (ctas > cap ? cap : ctas);
-    // programmatic stream serialization: see the kernel; plain launches from then on if the driver refuses it once
-    static bool pdl_ok = true;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)ctas);
     cfg.blockDim = dim3(kPushThreads);
     cfg.stream = as_stream(stream);
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = pdl_ok ? 1 : 0;
+    cudaLaunchAttribute attr[1];
     void* args[] = {&P};
-    cudaError_t e = cudaLaunchKernelExC(&cfg, (const void*)allgather_push_kernel, args);
-    if (e != cudaSuccess && pdl_ok) {
-        (void)cudaGetLastError();
-        pdl_ok = false;
-        cfg.numAttrs = 0;
-        e = cudaLaunchKernelExC(&cfg, (const void*)allgather_push_kernel, args);
-    }
-    NQ_CUDA_TRY(e);
-    return NQ_OK;
+    return launch_dependent(cfg, attr, 0, (const void*)allgather_push_kernel, args);   // (see the kernel)
 }
 
 unsigned nq_allgather_set_wait_limit(unsigned polls) {

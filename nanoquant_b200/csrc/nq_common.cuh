@@ -33,6 +33,10 @@ inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 
 
 inline cudaStream_t as_stream(nq_stream_t s) { return reinterpret_cast<cudaStream_t>(s); }
 
+// Launches `fn` with programmatic stream serialization, so that its prologue overlaps the previous kernel's tail, and the `n` attributes in
+// `attrs` (which has room for one more).  If the driver refuses that attribute, plain launches from then on.
+int launch_dependent(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attrs, int n, const void* fn, void** args);
+
 // Number of SMs of the current device (cached per device).
 int sm_count();
 

@@ -1,4 +1,5 @@
 // Library-wide pieces of the C ABI: status strings, CUDA error text, device info.
+#include <atomic>
 #include <cstdio>
 #include <cstring>
 
@@ -25,6 +26,23 @@ int sm_count() {
         cached[dev] = n;
     }
     return cached[dev];
+}
+
+int launch_dependent(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attrs, int n, const void* fn, void** args) {
+    static std::atomic<bool> refused{false};
+    attrs[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attrs[n].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attrs;
+    cfg.numAttrs = refused ? n : n + 1;
+    cudaError_t e = cudaLaunchKernelExC(&cfg, fn, args);
+    if (e != cudaSuccess && cfg.numAttrs == (unsigned)n + 1) {
+        (void)cudaGetLastError();
+        cfg.numAttrs = n;
+        e = cudaLaunchKernelExC(&cfg, fn, args);
+        if (e == cudaSuccess) refused = true;      // (an error of another kind says nothing about the attribute)
+    }
+    NQ_CUDA_TRY(e);
+    return NQ_OK;
 }
 
 }  // namespace nq

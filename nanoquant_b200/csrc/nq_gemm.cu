@@ -278,25 +278,14 @@ int nq_gemm_group_fwd(const nq_linear_desc* d, int n_linears, int T, int dtype, 
             B.job[j] = {static_cast<const uint16_t*>(L.x), L.ldx, static_cast<const uint16_t*>(L.s_in),
                         static_cast<const uint16_t*>(L.s_mid), const_cast<int*>(s1[j].row_exp), L.N, L.R};
         }
-        static bool pdl_ok = true;
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3((unsigned)((T + 7) / 8), (unsigned)n_linears);
         cfg.blockDim = dim3(256);
         cfg.stream = as_stream(stream);
-        cudaLaunchAttribute attr;
-        attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr.val.programmaticStreamSerializationAllowed = 1;
-        cfg.attrs = &attr;
-        cfg.numAttrs = pdl_ok ? 1 : 0;
+        cudaLaunchAttribute attr[1];
         void* args[] = {&B};
-        cudaError_t e = cudaLaunchKernelExC(&cfg, (const void*)row_bound_kernel, args);
-        if (e != cudaSuccess && pdl_ok) {
-            (void)cudaGetLastError();
-            pdl_ok = false;
-            cfg.numAttrs = 0;
-            e = cudaLaunchKernelExC(&cfg, (const void*)row_bound_kernel, args);
-        }
-        NQ_CUDA_TRY(e);
+        const int st = launch_dependent(cfg, attr, 0, (const void*)row_bound_kernel, args);
+        if (st != NQ_OK) return st;
     }
     return stages(StageTypes{1, 1, 0, +1}, StageTypes{1, 0, 1, -1});
 }

@@ -998,28 +998,14 @@ static int launch_decode(const nq_linear_desc* d, int n_linears, int t_first, in
         const size_t smem_bytes = P.part_off + part_used;
         if (smem_bytes > (size_t)smem_limit) return NQ_ERR_UNSUPPORTED;
         void* args[] = {&P};
-        // Programmatic stream serialization, so that this kernel's prologue overlaps the previous kernel's tail.  If the
-        // driver refuses the attribute once, plain launches are used from then on.
-        static bool pdl_ok = true;
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(grid);
         cfg.blockDim = dim3(kGemvThreads);
         cfg.dynamicSmemBytes = smem_bytes;
         cfg.stream = as_stream(stream);
-        cudaLaunchAttribute attr;
-        attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr.val.programmaticStreamSerializationAllowed = 1;
-        cfg.attrs = &attr;
-        cfg.numAttrs = pdl_ok ? 1 : 0;
-        const void* fn = gemv_kernel(dtype, tn);
-        cudaError_t e = cudaLaunchKernelExC(&cfg, fn, args);
-        if (e != cudaSuccess && pdl_ok) {
-            (void)cudaGetLastError();
-            pdl_ok = false;
-            cfg.numAttrs = 0;
-            e = cudaLaunchKernelExC(&cfg, fn, args);
-        }
-        NQ_CUDA_TRY(e);
+        cudaLaunchAttribute attr[1];
+        const int st = launch_dependent(cfg, attr, 0, gemv_kernel(dtype, tn), args);
+        if (st != NQ_OK) return st;
     }
     return NQ_OK;
 }

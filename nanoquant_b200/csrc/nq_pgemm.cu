@@ -565,23 +565,9 @@ int launch_pgemm_stage(const StageJob* jobs_in, int n, int T, StageTypes ty, int
     cfg.blockDim = dim3(kPThreads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = &attr;
+    cudaLaunchAttribute attr[1];
     void* args[] = {&P};
-    const void* fn = p_kernel(!ty.out_bf16 ? kPOutFp16 : saturate ? kPOutBf16Saturated : kPOutBf16);
-    static bool pdl_ok = true;
-    cfg.numAttrs = pdl_ok ? 1 : 0;
-    cudaError_t e = cudaLaunchKernelExC(&cfg, fn, args);
-    if (e != cudaSuccess && pdl_ok) {
-        (void)cudaGetLastError();
-        pdl_ok = false;
-        cfg.numAttrs = 0;
-        e = cudaLaunchKernelExC(&cfg, fn, args);
-    }
-    NQ_CUDA_TRY(e);
-    return NQ_OK;
+    return launch_dependent(cfg, attr, 0, p_kernel(!ty.out_bf16 ? kPOutFp16 : saturate ? kPOutBf16Saturated : kPOutBf16), args);
 }
 
 }  // namespace nq

@@ -590,22 +590,8 @@ int launch_wgemm_stage(const StageJob* jobs, int n, int T, StageTypes ty, int sa
         attrs[na].val.clusterDim.x = 1; attrs[na].val.clusterDim.y = 1; attrs[na].val.clusterDim.z = (unsigned)pl.csplit;
         ++na;
     }
-    attrs[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attrs[na].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attrs;
     void* args[] = {&P};
-    const void* fn = w_kernel(!ty.out_bf16 ? kWOutFp16 : saturate ? kWOutBf16Saturated : kWOutBf16);
-    static bool pdl_ok = true;
-    cfg.numAttrs = pdl_ok ? na + 1 : na;
-    cudaError_t e = cudaLaunchKernelExC(&cfg, fn, args);
-    if (e != cudaSuccess && pdl_ok) {
-        (void)cudaGetLastError();
-        pdl_ok = false;
-        cfg.numAttrs = na;
-        e = cudaLaunchKernelExC(&cfg, fn, args);
-    }
-    NQ_CUDA_TRY(e);
-    return NQ_OK;
+    return launch_dependent(cfg, attrs, na, w_kernel(!ty.out_bf16 ? kWOutFp16 : saturate ? kWOutBf16Saturated : kWOutBf16), args);
 }
 
 }  // namespace nq
