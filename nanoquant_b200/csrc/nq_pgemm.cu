@@ -82,8 +82,6 @@ constexpr int kPParamWords = (int)(sizeof(PJob) * kMaxGemmJobs + sizeof(PHead)) 
 constexpr int kPBarOff = 640, kPBOff = 1024, kPOutBytes = 4 * 32 * 256;
 static_assert(kPParamWords * 16 <= kPBarOff && kPBOff % 1024 == 0, "shared memory map");
 
-enum : int { kPOutFp16, kPOutBf16, kPOutBf16Saturated };
-
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {   // `bar`: an address of cluster_map
     asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }
@@ -352,9 +350,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPThreads, 1) pgemm_
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 const int row = n0 + 32 * ew + 8 * i + row_g;
-                auto as_float = [&](uint16_t h) { return P.is_bf16 ? __uint_as_float((uint32_t)h << 16) : __half2float(__ushort_as_half(h)); };
-                sc[i] = J.post && row < Nout ? as_float(__ldg(static_cast<const unsigned short*>(J.post) + row)) : 1.f;
-                bi[i] = J.bias && row < Nout ? as_float(__ldg(static_cast<const unsigned short*>(J.bias) + row)) : 0.f;
+                sc[i] = J.post && row < Nout ? io_float(__ldg(static_cast<const unsigned short*>(J.post) + row), P.is_bf16) : 1.f;
+                bi[i] = J.bias && row < Nout ? io_float(__ldg(static_cast<const unsigned short*>(J.bias) + row), P.is_bf16) : 0.f;
             }
             const uint16_t* resid = static_cast<const uint16_t*>(J.resid);
             const int* row_exp = J.row_exp;
@@ -397,8 +394,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPThreads, 1) pgemm_
                             const int tok = m0 + tb + 16 * (k >> 3) + 8 * ((k >> 2) & 1) + 2 * q + (k & 1);
                             const int row = n0 + 32 * ew + 16 * rr + 8 * ((k >> 1) & 1) + g;
                             if (tok < P.T && row < Nout) {
-                                const uint16_t x = resid[(size_t)tok * J.ld_res + row];
-                                r[k] += P.is_bf16 ? __uint_as_float((uint32_t)x << 16) : __half2float(__ushort_as_half(x));
+                                r[k] += io_float(resid[(size_t)tok * J.ld_res + row], P.is_bf16);
                             }
                         }
                     }
@@ -406,20 +402,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPThreads, 1) pgemm_
                     for (int h = 0; h < 2; ++h) {
                         uint32_t pk[4];
 #pragma unroll
-                        for (int i = 0; i < 4; ++i) {
-                            float o0 = r[8 * h + 2 * i], o1 = r[8 * h + 2 * i + 1];
-                            if (OUT == kPOutBf16Saturated) asm("cvt.rn.satfinite.bf16x2.f32 %0, %1, %2;" : "=r"(pk[i]) : "f"(o1), "f"(o0));
-                            else if (OUT == kPOutBf16) asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(pk[i]) : "f"(o1), "f"(o0));
-                            else {
-                                if (P.saturate) { o0 = clamp_or_nan(o0, 64504.0f); o1 = clamp_or_nan(o1, 64504.0f); }
-                                const __half2 h2 = __floats2half2_rn(o0, o1);
-                                pk[i] = *reinterpret_cast<const uint32_t*>(&h2);
-                            }
-                        }
+                        for (int i = 0; i < 4; ++i) pk[i] = pack_outputs<OUT>(r[8 * h + 2 * i], r[8 * h + 2 * i + 1], P.saturate);
                         const int tl = 16 * h + st_tok;
                         const uint32_t addr = stage + (uint32_t)(tl * 256 + (((st_unit + 2 * rr) ^ (tl & 7)) << 4));
-                        asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1,%2,%3,%4};"
-                                     ::"r"(addr), "r"(pk[0]), "r"(pk[1]), "r"(pk[2]), "r"(pk[3]) : "memory");
+                        stmatrix_trans(addr, pk);
                     }
                 }
                 asm volatile("bar.sync %0, 128;" ::"r"(3 + set) : "memory");     // (buffers alternate: one barrier per 32 tokens)
@@ -435,14 +421,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPThreads, 1) pgemm_
 #pragma unroll
                     for (int i = 0; i < 4; ++i, dst += 8 * ld_out) {
                         if (tb + 8 * i + ld_tok < live) {
-                            if (whole) {
-                                *reinterpret_cast<uint4*>(dst) = v[i];
-                            } else {
-                                const uint32_t vw[4] = {v[i].x, v[i].y, v[i].z, v[i].w};
-#pragma unroll
-                                for (int e = 0; e < 8; ++e)
-                                    if (row_s + e < Nout) dst[e] = (uint16_t)(vw[e >> 1] >> (16 * (e & 1)));
-                            }
+                            store_rows(dst, v[i], Nout - row_s, whole);
                         }
                     }
                 }
@@ -473,8 +452,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPThreads, 1) pgemm_
 }
 
 static const void* p_kernel(int out) {
-    return out == kPOutFp16 ? (const void*)pgemm_kernel<kPOutFp16> : out == kPOutBf16 ? (const void*)pgemm_kernel<kPOutBf16>
-                                                                                     : (const void*)pgemm_kernel<kPOutBf16Saturated>;
+    return out == kOutFp16 ? (const void*)pgemm_kernel<kOutFp16> : out == kOutBf16 ? (const void*)pgemm_kernel<kOutBf16>
+                                                                                     : (const void*)pgemm_kernel<kOutBf16Saturated>;
 }
 
 constexpr int kPSmemMost = 226 * 1024;
@@ -567,7 +546,7 @@ int launch_pgemm_stage(const StageJob* jobs_in, int n, int T, StageTypes ty, int
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
     void* args[] = {&P};
-    return launch_dependent(cfg, attr, 0, p_kernel(!ty.out_bf16 ? kPOutFp16 : saturate ? kPOutBf16Saturated : kPOutBf16), args);
+    return launch_dependent(cfg, attr, 0, p_kernel(out_kind(ty, saturate)), args);
 }
 
 }  // namespace nq

@@ -4,6 +4,7 @@
 #include <cuda.h>
 
 #include "nq_common.cuh"
+#include "nq_stage.h"
 
 namespace nq {
 
@@ -115,5 +116,44 @@ __device__ __forceinline__ void expand_swapped(const uint4& w, int hf, uint32_t 
 }
 // 0 2 1 3 4 6 5 7
 __device__ __forceinline__ int swap_middle(int g) { return (g & 4) | ((g & 1) << 1) | ((g >> 1) & 1); }
+
+// ---------------------------------------------------------------------------
+// outputs
+// ---------------------------------------------------------------------------
+enum : int { kOutFp16, kOutBf16, kOutBf16Saturated };      // kinds of a stage's output, a template argument of the kernels
+inline int out_kind(const StageTypes& ty, int saturate) { return !ty.out_bf16 ? kOutFp16 : saturate ? kOutBf16Saturated : kOutBf16; }
+
+__device__ __forceinline__ float io_float(uint16_t h, int is_bf16) {
+    return is_bf16 ? __uint_as_float((uint32_t)h << 16) : __half2float(__ushort_as_half(h));
+}
+// Two outputs, the first in the lower half.
+template <int OUT>
+__device__ __forceinline__ uint32_t pack_outputs(float o0, float o1, int saturate) {
+    uint32_t r;
+    if (OUT == kOutBf16Saturated) asm("cvt.rn.satfinite.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(o1), "f"(o0));
+    else if (OUT == kOutBf16) asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(o1), "f"(o0));
+    else {
+        if (saturate) { o0 = clamp_or_nan(o0, 64504.0f); o1 = clamp_or_nan(o1, 64504.0f); }
+        const __half2 h2 = __floats2half2_rn(o0, o1);
+        r = *reinterpret_cast<const uint32_t*>(&h2);
+    }
+    return r;
+}
+// Four 8 x 8 matrices, transposed: accumulator fragments (rows across the lanes) -> rows of one token side by side.
+__device__ __forceinline__ void stmatrix_trans(uint32_t addr, const uint32_t (&v)[4]) {
+    asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1,%2,%3,%4};"
+                 ::"r"(addr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]) : "memory");
+}
+// Eight rows of a token, of which `left` exist; `whole`: all do, at a 16-byte boundary.
+__device__ __forceinline__ void store_rows(uint16_t* dst, const uint4& v, int left, bool whole) {
+    if (whole) {
+        *reinterpret_cast<uint4*>(dst) = v;
+    } else {
+        const uint32_t vw[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int e = 0; e < 8; ++e)
+            if (e < left) dst[e] = (uint16_t)(vw[e >> 1] >> (16 * (e & 1)));
+    }
+}
 
 }  // namespace nq

@@ -84,8 +84,6 @@ constexpr int kWParamWords = (int)(sizeof(WJob) * kMaxGemmJobs + sizeof(WHead)) 
 constexpr int kWBarOff = 512, kWScaleOff = 1024, kWBOff = 2048;
 static_assert(kWParamWords * 16 <= kWBarOff, "shared memory map");
 
-enum : int { kWOutFp16, kWOutBf16, kWOutBf16Saturated };
-
 __device__ __forceinline__ void umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
@@ -308,11 +306,8 @@ __global__ void __launch_bounds__(kWThreads, 2) wgemm_kernel(const __grid_consta
             if (s >= stages) { s -= stages; ph ^= 1; }
         }
         if (tu < kWRows) {
-            auto as_float = [&](uint16_t raw) {
-                return P.is_bf16 ? __uint_as_float((uint32_t)raw << 16) : __half2float(__ushort_as_half(raw));
-            };
-            s_post[tu] = J.post ? as_float(raw_post) : 1.f;
-            s_bias[tu] = J.bias ? as_float(raw_bias) : 0.f;
+            s_post[tu] = J.post ? io_float(raw_post, P.is_bf16) : 1.f;
+            s_bias[tu] = J.bias ? io_float(raw_bias, P.is_bf16) : 0.f;
         }
         if (ok) ok = mbar_wait_warp(bar_accum, 0, abort_flag, Pc.head.status, Pc.head.wait_limit);
         tc_fence_after();
@@ -394,25 +389,18 @@ __global__ void __launch_bounds__(kWThreads, 2) wgemm_kernel(const __grid_consta
                     if (resid) {
                         const int tok = t0 + 8 * (i >> 2) + 2 * q + (i & 1), row = n0 + r0 + ((i & 2) ? 8 : 0);
                         if (tok < P.T && row < J.Nout) {
-                            const uint16_t h = resid[(size_t)tok * J.ld_res + row];
-                            add += P.is_bf16 ? __uint_as_float((uint32_t)h << 16) : __half2float(__ushort_as_half(h));
+                            add += io_float(resid[(size_t)tok * J.ld_res + row], P.is_bf16);
                         }
                     }
                     o[i] = r[i] * (((i & 2) ? sc1 : sc0) * ts[e]) + add;
-                    if (OUT == kWOutFp16 && P.saturate) o[i] = clamp_or_nan(o[i], 64504.0f);
                 }
                 uint32_t pk[4];
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    if (OUT == kWOutBf16Saturated) asm("cvt.rn.satfinite.bf16x2.f32 %0, %1, %2;" : "=r"(pk[i]) : "f"(o[2 * i + 1]), "f"(o[2 * i]));
-                    else if (OUT == kWOutBf16) asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(pk[i]) : "f"(o[2 * i + 1]), "f"(o[2 * i]));
-                    else { const __half2 h2 = __floats2half2_rn(o[2 * i], o[2 * i + 1]); pk[i] = *reinterpret_cast<const uint32_t*>(&h2); }
-                }
+                for (int i = 0; i < 4; ++i) pk[i] = pack_outputs<OUT>(o[2 * i], o[2 * i + 1], P.saturate);
                 // matrix i of the transposing store: tokens 8 (i >> 1) .., rows 8 (i & 1) ..
                 const int mi = lane >> 3, tl = 16 * idx + 8 * (mi >> 1) + (lane & 7), unit = 2 * rgl + (mi & 1);
                 const uint32_t addr = b_base + (uint32_t)(tl * 256 + ((unit ^ (tl & 7)) << 4));
-                asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1,%2,%3,%4};"
-                             ::"r"(addr), "r"(pk[0]), "r"(pk[1]), "r"(pk[2]), "r"(pk[3]) : "memory");
+                stmatrix_trans(addr, pk);
             }
         }
         asm volatile("bar.sync 2, 256;" ::: "memory");
@@ -427,14 +415,7 @@ __global__ void __launch_bounds__(kWThreads, 2) wgemm_kernel(const __grid_consta
                     if (tok >= P.T) break;
                     const uint4 v = *reinterpret_cast<const uint4*>(smem + kWBOff + tl * 256 + ((unit ^ (tl & 7)) << 4));
                     uint16_t* dst = out + (size_t)tok * J.ld_out;
-                    if (row + 8 <= J.Nout && (reinterpret_cast<uintptr_t>(dst) & 15u) == 0) {
-                        *reinterpret_cast<uint4*>(dst) = v;
-                    } else {
-                        const uint32_t vw[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-                        for (int e = 0; e < 8; ++e)
-                            if (row + e < J.Nout) dst[e] = (uint16_t)(vw[e >> 1] >> (16 * (e & 1)));
-                    }
+                    store_rows(dst, v, J.Nout - row, row + 8 <= J.Nout && (reinterpret_cast<uintptr_t>(dst) & 15u) == 0);
                 }
             }
         }
@@ -452,8 +433,8 @@ __global__ void __launch_bounds__(kWThreads, 2) wgemm_kernel(const __grid_consta
 }
 
 static const void* w_kernel(int out) {
-    return out == kWOutFp16 ? (const void*)wgemm_kernel<kWOutFp16> : out == kWOutBf16 ? (const void*)wgemm_kernel<kWOutBf16>
-                                                                                     : (const void*)wgemm_kernel<kWOutBf16Saturated>;
+    return out == kOutFp16 ? (const void*)wgemm_kernel<kOutFp16> : out == kOutBf16 ? (const void*)wgemm_kernel<kOutBf16>
+                                                                                     : (const void*)wgemm_kernel<kOutBf16Saturated>;
 }
 
 constexpr int kWSmemMost = 112 * 1024;   // two CTAs per SM
@@ -506,7 +487,7 @@ static int w_capacity(int s) {
         cfg.attrs = &attr;
         cfg.numAttrs = 1;
         int clusters = 0;
-        if (w_attributes() != NQ_OK || cudaOccupancyMaxActiveClusters(&clusters, w_kernel(kWOutFp16), &cfg) != cudaSuccess || clusters <= 0) {
+        if (w_attributes() != NQ_OK || cudaOccupancyMaxActiveClusters(&clusters, w_kernel(kOutFp16), &cfg) != cudaSuccess || clusters <= 0) {
             (void)cudaGetLastError();
             clusters = 0;
         }
@@ -591,7 +572,7 @@ int launch_wgemm_stage(const StageJob* jobs, int n, int T, StageTypes ty, int sa
         ++na;
     }
     void* args[] = {&P};
-    return launch_dependent(cfg, attrs, na, w_kernel(!ty.out_bf16 ? kWOutFp16 : saturate ? kWOutBf16Saturated : kWOutBf16), args);
+    return launch_dependent(cfg, attrs, na, w_kernel(out_kind(ty, saturate)), args);
 }
 
 }  // namespace nq
