@@ -424,11 +424,22 @@ static int batch_smem_limit(int* out) {
 }
 
 // From nine tokens on the second column group doubles the matrix instructions, and every CTA stages the whole input of a first stage:
-// launches with much of both are faster through nq_wgemm.cu.  Both stages of a group, 16 tokens, here and there, us:
-//   1.6 MB of packed factors (4096 -> 4096)  8.3 / 9.9      8.3 MB (8192 -> 8192)        16.8 / 20.5     29 MB (28672 -> 8192)      68.6 / 46.0
-//   5.0 MB (12288 -> 4096)                  16.2 / 16.1     10.0 MB (gate/up of 4096)    19.4 / 18.8     58 MB (gate/up of 8192)    88.5 / 73.7
-//   5.8 MB (q/k/v of 5120)                  16.6 / 15.1     10.3 MB (q/k/v of 8192)      24.9 / 21.3
-// Where the two are close (gate/up of 4096) a layer is faster through one kernel: eight layers 432 us, with gate/up there 448.
+// launches with much of both are faster through nq_wgemm.cu and nq_pgemm.cu.  The rule looks at each stage's packed factors, and either stage
+// decides for both.  Groups in a graph, bf16, 16 tokens: MB of the two stages, here / there in us; * marks what the rule sends there.
+//               q/k/v                        o                          gate/up                       down
+//   2048 cols   0.4 + 0.2   7.2 /  8.0      0.2 + 0.2   7.1 /  7.7      0.6 +  1.8   9.0 /  9.6       0.9 + 0.3   9.7 /  9.5
+//   4096        1.4 + 1.0  10.0 / 10.6      0.8 + 0.8   8.4 /  9.7      2.5 +  7.5  19.2 / 17.6       3.7 + 1.2  16.2 / 16.0
+//   5120        2.3 + 1.5  14.0 / 13.3      1.3 + 1.3  10.8 / 11.3      3.9 + 11.7  31.0 / 22.3 *     5.8 + 1.9  21.8 / 20.4 *
+//   6144        3.3 + 2.2  17.0 / 15.0      1.9 + 1.9  14.8 / 12.6      5.6 + 16.8  37.7 / 27.2 *     8.4 + 2.8  34.3 / 21.9 *
+//   8192        5.9 + 4.0  25.8 / 21.3 *    3.3 + 3.3  17.0 / 16.5     10.4 + 36.2  73.0 / 55.8 *    18.1 + 5.2  66.0 / 36.7 *
+// (0.8 bits per weight, inner width 3 times the columns, 28672 at 8192.)  A layer of all four, us, all here / all there / by the rule:
+//   9 tokens    2048  31.3 / 34.3 / 31.3    4096  51.5 / 52.9 / 51.5    5120  75.6 / 65.3 / 67.3    6144   90.4 / 75.4 / 79.8
+//               8192 157.7 / 126.8 / 129.1  4096 at 1.5 bits  63.7 / 66.5 / 65.4    5120 at 1.2 bits  95.8 / 80.8 / 89.6
+//   16 tokens   2048  31.9 / 34.4 / 31.9    4096  53.4 / 52.9 / 53.5    5120  76.3 / 65.4 / 67.4    6144  102.8 / 75.3 / 81.1
+//               8192 180.3 / 126.8 / 129.6  4096 at 1.5 bits  70.4 / 66.5 / 67.3    5120 at 1.2 bits  96.6 / 80.9 / 89.2
+// Changing kernels inside a layer costs what a group of 4096 columns gains, so the lines (8 MB; 4.5 MB with 8192 columns) leave such layers in
+// one kernel: they are within 3 % of the better one.  From 5120 columns on they are on the safe side: all of a layer through the GEMMs would be
+// 2 to 11 % faster still.  (A line at 4.5 MB for any K changes no layer from 5120 columns on, and loses 2 to 4 % at 4096.)
 int batch_max_tokens(const StageJob* jobs, int n) {
     double bytes = 0;                       // of this stage
     int most_k = 0;
