@@ -439,7 +439,7 @@ static int batch_smem_limit(int* out) {
 //               8192 180.3 / 126.8 / 129.6  4096 at 1.5 bits  70.4 / 66.5 / 67.3    5120 at 1.2 bits  96.6 / 80.9 / 89.2
 // Changing kernels inside a layer costs what a group of 4096 columns gains, so the lines (8 MB; 4.5 MB with 8192 columns) leave such layers in
 // one kernel: they are within 3 % of the better one.  From 5120 columns on they are on the safe side: all of a layer through the GEMMs would be
-// 2 to 11 % faster still.  (A line at 4.5 MB for any K changes no layer from 5120 columns on, and loses 2 to 4 % at 4096.)
+// 1 to 11 % faster still.  (A line at 4.5 MB for any K changes no layer from 5120 columns on, and loses 2 to 4 % at 4096.)
 int batch_max_tokens(const StageJob* jobs, int n) {
     double bytes = 0;                       // of this stage
     int most_k = 0;
