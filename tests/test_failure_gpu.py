@@ -97,17 +97,17 @@ def test_allgather_wait_for_an_absent_peer_expires():
 
 
 @pytest.mark.parametrize("kernel,stage,T,shapes", [
-    # 32 steps of 128 columns in a first stage of 16 CTAs: the second stage's CTAs, resident from the start, wait for it
-    ("wgemm_kernel", 1, 128, [(32768, 256, 4096)]),
+    # a first stage of 98304 columns, 45 us: the second stage's CTAs, resident from the start, wait for it
+    ("wgemm_kernel", 1, 128, [(98304, 256, 4096)]),
     # K split over two CTAs in the second stage: the second CTA of the linear of rank 256 has no columns, and owns the tokens from 16 on,
     # for which it waits in vain (the first one gave up behind the first stage)
-    ("wgemm_kernel", 1, 32, [(32768, 512, 128), (32768, 256, 128)]),
-    # the epilogue of a pair waits for a tile's main loop
+    ("wgemm_kernel", 1, 32, [(98304, 512, 128), (98304, 256, 128)]),
+    # the epilogue of a pair waits for a tile's main loop, 17 us
     ("pgemm_kernel", 0, 2048, [(4096, 2048, 256)]),
 ])
 def test_gemm_wait_that_runs_out(kernel, stage, T, shapes):
-    # With a limit of one attempt (some us) after the first, waits that are satisfied a little later run out.  The launch ends all the same,
-    # drains what is in flight, gives its tensor memory back and reports; the next one on a zeroed scratch is right.
+    # With a limit of one attempt after the first (10 us in all), these waits run out; with 8 (4 for the last) they always did, too.
+    # The launch ends all the same, drains what is in flight, gives its tensor memory back and reports; the next one on a zeroed scratch is right.
     from nanoquant_b200 import _lib
     Lb = _lib.lib()
     dtype = torch.float16
