@@ -243,8 +243,8 @@ __global__ void __launch_bounds__(kBatchThreads, 1) batch_stage_kernel(const __g
                     if (r < nr) {
                         const uint32_t w0 = h ? w[r].z : w[r].x, w1 = h ? w[r].w : w[r].y;   // rows g, g + 8
                         const uint32_t u0 = w0 * pw[7 - j], u1 = w1 * pw[7 - j];
-                        const uint32_t a0 = ((u0 * p256) & 0x80008000u) ^ se, a2 = (u0 & 0x80008000u) ^ so;
-                        const uint32_t a1 = ((u1 * p256) & 0x80008000u) ^ se, a3 = (u1 & 0x80008000u) ^ so;
+                        const uint32_t a0 = and_xor(u0 * p256, 0x80008000u, se), a2 = and_xor(u0, 0x80008000u, so);
+                        const uint32_t a1 = and_xor(u1 * p256, 0x80008000u, se), a3 = and_xor(u1, 0x80008000u, so);
 #pragma unroll
                         for (int nt = 0; nt < NT; ++nt) mma_16816<BF16>(acc[r][nt], a0, a1, a2, a3, be[nt], bo[nt]);
                     }

@@ -127,6 +127,19 @@ __device__ __forceinline__ float min_or_nan(float a, float b) {
 __device__ __forceinline__ float clamp_or_nan(float v, float lim) { return min_or_nan(max_or_nan(v, -lim), lim); }
 
 // ---------------------------------------------------------------------------
+// sign bits
+// ---------------------------------------------------------------------------
+// (a & m) ^ x as ONE LOP3.  Written as an expression it compiled to two of them (instruction counters: 9 ALU operations per 16 x 16 fragment
+// of signs instead of 5), on the half-rate pipe that bounds the expansion of sign bits.  A fragment, shifts and MMA included, takes
+// 21.3 -> 16.1 clk of a scheduler (16 warps, registers only); eight Qwen3-8B layers in a graph, four tokens 340.0 -> 326.1 us, sixteen
+// 434.6 -> 428.8 (the GEMMs, whose expansion waits for other things, are level).
+__device__ __forceinline__ uint32_t and_xor(uint32_t a, uint32_t m, uint32_t x) {
+    uint32_t r;
+    asm("lop3.b32 %0, %1, %2, %3, 0x6A;" : "=r"(r) : "r"(a), "r"(m), "r"(x));   // 0x6A = (0xF0 & 0xCC) ^ 0xAA
+    return r;
+}
+
+// ---------------------------------------------------------------------------
 // mbarriers and bulk copies
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }

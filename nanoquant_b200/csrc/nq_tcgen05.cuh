@@ -95,10 +95,10 @@ __device__ __forceinline__ void expand_columns(const uint4& w, int hf, const uin
     for (int i = 0; i < 4; ++i) {
         const int sh = 3 - (2 * hf + (i >> 1));
         const uint32_t u0 = ((i & 1) ? w.z : w.x) << sh, u1 = ((i & 1) ? w.w : w.y) << sh;
-        v[4 * i + 0] = (spread_signs(u0, 0x9988u) & 0x80008000u) ^ pn[i].x;
-        v[4 * i + 1] = (spread_signs(u0, 0xBBAAu) & 0x80008000u) ^ pn[i].y;
-        v[4 * i + 2] = (spread_signs(u1, 0x9988u) & 0x80008000u) ^ pn[i].x;
-        v[4 * i + 3] = (spread_signs(u1, 0xBBAAu) & 0x80008000u) ^ pn[i].y;
+        v[4 * i + 0] = and_xor(spread_signs(u0, 0x9988u), 0x80008000u, pn[i].x);
+        v[4 * i + 1] = and_xor(spread_signs(u0, 0xBBAAu), 0x80008000u, pn[i].y);
+        v[4 * i + 2] = and_xor(spread_signs(u1, 0x9988u), 0x80008000u, pn[i].x);
+        v[4 * i + 3] = and_xor(spread_signs(u1, 0xBBAAu), 0x80008000u, pn[i].y);
     }
 }
 // The same for +-1 and columns whose middle two of every four are swapped (kOrderIn): the bits of a pair are 16 apart, one ALU
@@ -108,10 +108,10 @@ __device__ __forceinline__ void expand_swapped(const uint4& w, int hf, uint32_t 
     for (int i = 0; i < 4; ++i) {
         const int sh = 3 - (2 * hf + (i >> 1));
         const uint32_t w0 = (i & 1) ? w.z : w.x, w1 = (i & 1) ? w.w : w.y;
-        v[4 * i + 0] = ((w0 << (sh + 8)) & 0x80008000u) ^ one2;
-        v[4 * i + 1] = ((w0 << sh) & 0x80008000u) ^ one2;
-        v[4 * i + 2] = ((w1 << (sh + 8)) & 0x80008000u) ^ one2;
-        v[4 * i + 3] = ((w1 << sh) & 0x80008000u) ^ one2;
+        v[4 * i + 0] = and_xor(w0 << (sh + 8), 0x80008000u, one2);
+        v[4 * i + 1] = and_xor(w0 << sh, 0x80008000u, one2);
+        v[4 * i + 2] = and_xor(w1 << (sh + 8), 0x80008000u, one2);
+        v[4 * i + 3] = and_xor(w1 << sh, 0x80008000u, one2);
     }
 }
 // 0 2 1 3 4 6 5 7
