@@ -8,25 +8,29 @@
 //
 //  * Weights: a CTA's row groups are contiguous in the tile layout; ONE thread fetches them as bulk copies before the
 //    dependency wait, all of them where they fit.
-//  * mma.sync m16n8k16 (16 rows x 8 tokens).  The bits of columns {4q, 4q+2} and {4q+1, 4q+3} of a 16-column block are
-//    16 apart in the lane's word, so a shift and ONE LOP3 ((word & 0x80008000) ^ {s, s'}) make an A register +-s: the
+//  * mma.sync m16n8k16 (16 rows x 8 tokens).  A shift and ONE LOP3 ((word & 0x80008000) ^ {s, s'}) make an A register +-s: the
 //    product x * (+-s_in) is exact.  The columns of a block may be permuted as long as A and B agree, so the B fragment
-//    of a token is its four consecutive columns 4q..4q+3.
+//    of a token is its four consecutive columns 4q..4q+3, as they lie in memory: a PRMT per word and chunk brings the bits of neighbouring
+//    columns, 8 apart in the tile layout, to 16 apart (two PRMTs per fragment of activations and of scales did before).
 //  * B fragments.  The intermediate is stored in fragment order (see fragment_index): a warp's load of one is 256
-//    contiguous bytes.  Activations come in rows: every warp stages its own columns through shared memory with 16-byte
-//    copies, 192 of them in flight.  (Fragments loaded from rows touch eight lines each.)
+//    contiguous bytes, and what a warp needs of a chunk is loaded at once.  Activations come in rows: every warp stages its own columns through
+//    shared memory with 16-byte copies, a chunk (half of one for two column groups) at a time: the 16 blocks of it are then ONE
+//    piece of code without a wait in between.  (Fragments loaded from rows touch eight lines each.)
+//  * A launch is a chain, and the warps of an SM are few: what counts is the length of a warp's path.  Pieces of 64 columns with a wait,
+//    a copy and 4 dependent MMAs each took 300 ns, whatever was in flight; a chunk with two accumulators in turn 900 ns for its 16 blocks.
+//    Output scales and bias come by bulk copy beside the weights, the input scales are prefetched to L2.  Eight Qwen3-8B layers in
+//    a graph, 4 / 8 / 12 / 16 tokens: 326 / 336 / 423 / 430 us -> 305 / 311 / 390 / 400; Llama-3.2-1B 238 / 233 / 279 / 289 -> 226 / 207 / 249 / 258.
 //  * Two barriers; no K split over CTAs, no counters, no slabs.
 //
 // Splitting K over the CTAs of a cluster (partial sums exchanged through distributed shared memory) and staging the whole
 // input by bulk copies before the loop both measured slower than this at every size.
 // It ends at 16 tokens (8 for large launches, see batch_max_tokens): 17 tokens took three column groups, eight Qwen3-8B layers 625 us, 473 through nq_wgemm.cu.
 //
-// What bounds it (counters of single launches at 16 tokens, cold): no throughput limit is near.  DRAM 3 to 6 % of its peak,
-// L2 4 to 16, tensor pipe 12 to 19.  The two stages of a group with little work take 8.8 us together, two launches of a fixed
-// chain (dependency, weights' arrival, a loop of a few steps, two barriers, output).  In first stages the 16 warps issue in
-// 56 to 60 % of the active cycles: copies, shifts and LOP3 around the MMAs; down's reads 56 MB through L2, since every CTA
-// stages the whole input.  Gate/up's second stage waits for the fragments of t (long scoreboard, 3.1 warps per issue, is its
-// largest stall) with four warps per scheduler to hide that.
+// What bounds it: the two stages of a group with little work are two launches of a fixed chain.  Stamps of o (4096 columns, 4 tokens; us after the last CTA
+// of the launch before): dependency 0.64, activations on their way 1.1, weights there 1.2, activations 1.5, products 2.5, outputs 3.1.  In launches
+// with much work the half-rate ALU pipe (a shift and a LOP3 per two weights, 16 clk of a scheduler per 16 x 16 weights, 12 with no shift)
+// beside 9 clk per MMA; gate/up's second stage 5 us of 9.  Two CTAs per SM (64 registers, or 256 threads), so that the next launch has its
+// weights before this one ends, lost 10 to 50 %: every phase is then longer.  The next stage's weights brought to L2 by this one: 1 to 4 % slower.
 #include <cstddef>
 #include <cstring>
 #include <type_traits>
@@ -39,16 +43,17 @@ namespace nq {
 
 constexpr int kBatchThreads = 512;
 constexpr int kBatchWarps = kBatchThreads / 32;
-// 16-column blocks of the intermediate whose B fragments a warp loads together
-constexpr int blocks_in_flight(int nt, int rows) { return nt == 1 || rows < 4 ? 8 : 4; }
 constexpr int tokens_groups(int T) { return T <= 8 ? 1 : 2; }
 constexpr int kMostRows = 4;             // row groups of a pass
-constexpr int kPieces = 3;               // pieces of 64 columns a warp has in flight
-constexpr int kPieceStride = 128 + 32;   // bytes of a staged row: 32 mod 128, so the eight tokens of a fragment fall on
-                                         // different banks
+// 16-column blocks that a warp stages together, and fragments of the intermediate it loads together
+constexpr int step_blocks(int nt) { return nt == 1 ? 16 : 8; }
+constexpr int blocks_in_flight(int nt, int rows) { return nt == 1 && rows < 4 ? 16 : nt == 1 || rows < 4 ? 8 : 4; }
+constexpr int kMostSteps = 2;            // steps in flight
 constexpr int kBatchSlots = 8;           // weight blocks in flight
 constexpr int kBatchMaxCtas = 256;
-constexpr size_t kOffParams = 64, kFixedBytes = 1024;
+constexpr size_t kOffParams = 128, kFixedBytes = 1024;
+constexpr int kMostBlock = 32;           // row groups of a block
+constexpr size_t kMostRowBytes = 8192;   // output scales of a CTA in shared memory
 constexpr unsigned kWeightWaitLimit = 1u << 20;   // attempts of up to ~2 us each
 
 struct alignas(16) BatchJob {
@@ -64,7 +69,8 @@ struct alignas(16) BatchJob {
     int rows, K, chunks;
     int cta0, g_q, g_r;      // first CTA of the range; row groups per CTA, one more for its first g_r CTAs
     int gb;                  // row groups per block
-    uint16_t wk, wr;         // chunk slices x row slices of a CTA's work, one warp each
+    uint8_t wk, wr;          // chunk slices x row slices of a CTA's work, one warp each
+    uint16_t bulk;           // output scales and bias come by bulk copy beside the weights
     int wk_magic, wr_magic;  // ceil(2^16 / .)
 };
 static_assert(sizeof(BatchJob) == 128, "128 bytes");
@@ -73,7 +79,9 @@ struct alignas(16) BatchParams {
     unsigned* status;
     int T, io_bf16, out_bf16, saturate, exp_sign;   // T: columns of partial sums (tokens, or 8 for a split input)
     int slots, slot_bytes, part_off;
-    int stage_off, frag_out;      // activation staging buffers; output in fragment order
+    int stage_off, steps, frag_out;      // activation staging buffers, their number per warp; output in fragment order
+    int post_off, bias_off;       // output scales and bias of the CTA's rows
+    int t_magic;                  // ceil(2^16 / tokens of the output)
     uint8_t cta_job[kBatchMaxCtas];
 };
 constexpr int kBatchWords = (int)offsetof(BatchParams, cta_job) / 16;
@@ -91,9 +99,14 @@ __device__ __forceinline__ void mma_16816(float (&d)[4], uint32_t a0, uint32_t a
 __device__ __forceinline__ float float_of(uint16_t h, int bf16) {
     return bf16 ? __uint_as_float((uint32_t)h << 16) : __half2float(__ushort_as_half(h));
 }
-// {a.lo, b.lo} and {a.hi, b.hi} of four consecutive 16-bit values: columns {0, 2} and {1, 3}
-__device__ __forceinline__ uint32_t even_columns(uint2 v) { return __byte_perm(v.x, v.y, 0x5410); }
-__device__ __forceinline__ uint32_t odd_columns(uint2 v) { return __byte_perm(v.x, v.y, 0x7632); }
+// The bits of columns {0, 1} and {2, 3} of every four, 8 apart in a word, 16 apart: bytes {0, 1} and {2, 3} to bytes 1 and 3.
+__device__ __forceinline__ uint32_t spread01(uint32_t w) { return __byte_perm(w, 0u, 0x1404); }
+__device__ __forceinline__ uint32_t spread23(uint32_t w) { return __byte_perm(w, 0u, 0x3424); }
+__device__ __forceinline__ uint2 lds8(uint32_t addr) {
+    uint2 v;
+    asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(addr) : "memory");
+    return v;
+}
 
 // Fragment order of an intermediate [T, K]: per chunk, 16-column block (32 j + 16 h) and group of eight tokens, the 8
 // bytes {columns 4q, 4q+2, 4q+1, 4q+3} of lane 4g + q (token g of the group).  Element index; the layout has
@@ -112,10 +125,14 @@ __device__ __forceinline__ void copy16_or_zero(uint32_t dst, const void* src, bo
 // kSplitTokens).
 template <bool BF16, int NT, int ROWS, bool FRAG, bool SPLIT>
 __global__ void __launch_bounds__(kBatchThreads, 1) batch_stage_kernel(const __grid_constant__ BatchParams Pc) {
-    constexpr int kRows = ROWS, kB = blocks_in_flight(NT, ROWS);
+    constexpr int kRows = ROWS, kB = blocks_in_flight(NT, ROWS), kStep = step_blocks(NT), kStepRow = kStep * 32;
+    constexpr uint32_t one2 = BF16 ? 0x3F803F80u : 0x3C003C00u;
+    // Accumulators of a fragment's blocks in turn: MMAs on one of them wait for each other.  (Of a split intermediate it must not depend on
+    // ROWS, which may differ between a linear alone and in a group.)
+    constexpr int kChains = SPLIT || NT * ROWS < 4 ? 2 : 1;
     extern __shared__ __align__(128) unsigned char smem[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, q = lane & 3;
-    const uint32_t bars = smem_u32(smem);
+    const uint32_t bars = smem_u32(smem);       // weight slots, then the constants
     // the parameter bank is read here and nowhere else, in one round trip (see nq_gemv.cu)
     const unsigned my_job = Pc.cta_job[blockIdx.x];
     {
@@ -129,17 +146,17 @@ __global__ void __launch_bounds__(kBatchThreads, 1) batch_stage_kernel(const __g
                 reinterpret_cast<uint4*>(smem + kOffParams)[min(warp + i * kBatchWarps, kBatchWords - 1)] = w[i];
         }
     }
-    if (tid >= kBatchThreads - kBatchSlots) {
-        mbar_init(bars + 8 * (tid - (kBatchThreads - kBatchSlots)), 1);
+    constexpr int kLoader = kBatchThreads - 32;
+    if (tid >= kLoader && tid <= kLoader + kBatchSlots) {
+        mbar_init(bars + 8 * (tid - kLoader), 1);
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
     __syncthreads();
     const BatchParams& P = *reinterpret_cast<const BatchParams*>(smem + kOffParams);
     const BatchJob& jb = P.job[my_job];
     unsigned char* weights = smem + kFixedBytes;
-    float* part = reinterpret_cast<float*>(smem + P.part_off);        // [chunk slice][token][row of the block]
     // (a constant where it is one: eight Qwen3-8B layers of four tokens 347.4 -> 338.9 us, two of 8192 columns 273 -> 267.5)
-    const int T = SPLIT ? (FRAG ? 2 * kSplitTokens : kSplitTokens) : P.T, slots = P.slots, slot_bytes = P.slot_bytes, chunks = jb.chunks, gb = jb.gb, rows = jb.rows;
+    const int T = SPLIT ? (FRAG ? 2 * kSplitTokens : kSplitTokens) : P.T, slots = P.slots, slot_bytes = P.slot_bytes, chunks = jb.chunks, gb = jb.gb, rows = jb.rows, K = jb.K;
     int first, groups;
     {
         const int c = (int)blockIdx.x - jb.cta0;
@@ -156,41 +173,56 @@ __global__ void __launch_bounds__(kBatchThreads, 1) batch_stage_kernel(const __g
         l_g += nb;
         l_slot = l_slot + 1 == slots ? 0 : l_slot + 1;
     };
-    const bool loader = tid == kBatchThreads - kBatchSlots;
+    const bool loader = tid == kLoader;
+    const uint32_t const_bar = bars + 8 * kBatchSlots;
     if (loader) {
 #pragma unroll 1
         for (int s = 0; s < slots; ++s) load_block();
+        if (!FRAG && jb.pre) asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(jb.pre), "r"(2 * K) : "memory");
+        const bool bulk = jb.bulk;
+        const uint32_t row_bytes = bulk ? 2u * min(groups * 16, rows - first * 16) : 0u;
+        mbar_expect_tx(const_bar, row_bytes * ((jb.post ? 1u : 0u) + (jb.bias ? 1u : 0u)));
+        if (bulk && jb.post) bulk_load(smem_u32(smem + P.post_off), static_cast<const uint16_t*>(jb.post) + first * 16, row_bytes, const_bar);
+        if (bulk && jb.bias) bulk_load(smem_u32(smem + P.bias_off), static_cast<const uint16_t*>(jb.bias) + first * 16, row_bytes, const_bar);
     }
     // this warp: chunks [c0, c1), row slice rw
     const int wk = jb.wk, wr = jb.wr;
     const int rw = (warp * jb.wk_magic) >> 16, kw = warp - rw * wk;
     const int c0 = (kw * chunks * jb.wk_magic) >> 16, c1 = ((kw + 1) * chunks * jb.wk_magic) >> 16;
-    const int wr_magic = jb.wr_magic, K = jb.K, tok_stride = gb * 16 + 4;   // 4 mod 16: an accumulator's 32 stores fall on 32 banks
-    const uint16_t* const pre = static_cast<const uint16_t*>(jb.pre);
-    const uint16_t* const a_in = static_cast<const uint16_t*>(jb.a);
+    const int wr_magic = jb.wr_magic, tok_stride = gb * 16 + 4;   // 4 mod 16: an accumulator's 32 stores fall on 32 banks
+    float* part = reinterpret_cast<float*>(smem + P.part_off);        // [chunk slice][token][row of the block]
+    // Staging: steps of kStep * 16 columns, T rows and the input scales.  The 32-byte blocks of four are swapped by the token (t & 3), so
+    // that the tokens of a fragment fall on different banks.  A lane copies column 8 (lane % kLanes) of the rows lane / kLanes + i * kPer.
+    constexpr int kLanes = kStep * 2, kPer = 32 / kLanes;      // lanes of a row, rows of a copy
+    const int step_bytes = (T + 1) * kStepRow, n_steps = P.steps;
+    const uint32_t stage = smem_u32(smem) + P.stage_off + warp * n_steps * step_bytes;
+    const int x_lane = (lane % kLanes) * 8;
+    const uint16_t* const x_src = static_cast<const uint16_t*>(jb.a) + x_lane;
+    const uint16_t* const pre_src = static_cast<const uint16_t*>(jb.pre) + x_lane;
     const long long lda = jb.lda;
-    // staging: buffers of T + 1 rows (the scales last) of 64 columns, one piece each
-    const int piece_bytes = (T + 1) * kPieceStride;
-    unsigned char* const stage = smem + P.stage_off + warp * kPieces * piece_bytes;
-    int a_row[NT];
+    const bool scaled = !FRAG && jb.pre;
+    int s_in = 0, s_out = 0;             // next buffer to fill, to read (bytes)
+    // the step from column `col` on
+    auto stage_step = [&](int col) {
+        if (col < c1 * 256) {
+            const bool there = col + x_lane < K;          // K is a multiple of 8
+            const int off = there ? col : -x_lane;
+            const uint32_t row0 = stage + s_in + (lane / kLanes) * kStepRow;
+            const uint16_t* src = x_src + off + (lane / kLanes) * lda;
 #pragma unroll
-    for (int nt = 0; nt < NT; ++nt) a_row[nt] = min(8 * nt + g, T - 1) * kPieceStride + 8 * q;   // tokens beyond T: not stored
-    int s_in = 0, s_out = 0;             // next buffer to fill, to read
-    // piece `pc` (columns 64 pc ..): eight lanes per row
-    auto stage_piece = [&](int pc) {
-        if (pc < 4 * c1) {
-            const int col = pc * 64 + (lane & 7) * 8, t0 = lane >> 3;
-            const bool there = col < K;          // K is a multiple of 8
-            const uint32_t dst = smem_u32(stage + s_in * piece_bytes) + (uint32_t)(t0 * kPieceStride + (lane & 7) * 16);
-            const uint16_t* src = a_in + (there ? col : 0);
-#pragma unroll
-            for (int t = 0; t < 8 * NT; t += 4)
-                if (t + t0 < T) copy16_or_zero(dst + (uint32_t)(t * kPieceStride), src + (t + t0) * lda, there);
-            if (pre && lane < 8) copy16_or_zero(dst + (uint32_t)(T * kPieceStride), pre + (there ? col : 0), there);
-            s_in = s_in + 1 == kPieces ? 0 : s_in + 1;
+            for (int t = 0; t < (SPLIT ? kSplitTokens : 8 * NT); t += kPer) {
+                const int tok = t + lane / kLanes;
+                if (SPLIT || tok < T) copy16_or_zero(row0 + t * kStepRow + ((x_lane * 2) ^ ((tok & 3) * 32)), src, there);
+                src += kPer * lda;
+            }
+            if (scaled && lane < kLanes) copy16_or_zero(stage + s_in + T * kStepRow + x_lane * 2, pre_src + off, there);
+            s_in = s_in + step_bytes == n_steps * step_bytes ? 0 : s_in + step_bytes;
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
+    // of a fragment: token g (+ 8), columns 4 q.. ; tokens beyond T: not stored
+    const uint32_t t_row[2] = {(uint32_t)(min(g, T - 1) * kStepRow + 8 * q), (uint32_t)((NT == 2 ? min(8 + g, T - 1) : 0) * kStepRow + 8 * q)};
+    const uint32_t t_swap[2] = {(uint32_t)(min(g, T - 1) & 3) * 32, (uint32_t)(NT == 2 ? min(8 + g, T - 1) & 3 : 0) * 32};
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
@@ -200,103 +232,112 @@ __global__ void __launch_bounds__(kBatchThreads, 1) batch_stage_kernel(const __g
     for (int blk = 0; blk < groups; blk += gb) {
         const int nb = min(gb, groups - blk);
         const int r0 = (rw * nb * wr_magic) >> 16, r1 = rw < wr ? ((rw + 1) * nb * wr_magic) >> 16 : r0;
-        // quotient by the rows of a block: exact below 2^22 / rows, and there are at most 16 times as many outputs as rows, 512 of them
-        const unsigned nb16_magic = ((1u << 22) + nb * 16 - 1) / (nb * 16);
-        // output scale and bias of row `tid` of the block (asm: a plain 16-bit load is widened, that is waited for, at once)
         const int row0 = (first + blk) * 16;
-        uint16_t post_raw = 0, bias_raw = 0;
-        if (tid < nb * 16 && row0 + tid < rows) {
-            if (jb.post) asm volatile("ld.global.nc.u16 %0, [%1];" : "=h"(post_raw) : "l"(static_cast<const uint16_t*>(jb.post) + row0 + tid));
-            if (jb.bias) asm volatile("ld.global.nc.u16 %0, [%1];" : "=h"(bias_raw) : "l"(static_cast<const uint16_t*>(jb.bias) + row0 + tid));
-        }
 #pragma unroll 1
         for (int rb = r0; rb < r1; rb += kRows) {
             const int nr = min(kRows, r1 - rb);
-            float acc[kRows][NT][4];
+            float acc[kChains][kRows][NT][4];
 #pragma unroll
-            for (int r = 0; r < kRows; ++r)
+            for (int k = 0; k < kChains; ++k)
 #pragma unroll
-                for (int nt = 0; nt < NT; ++nt)
+                for (int r = 0; r < kRows; ++r)
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) acc[r][nt][i] = 0.f;
-            if (!FRAG && c0 < c1) {
+                    for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) acc[k][r][nt][i] = 0.f;
+            if (!FRAG) {
 #pragma unroll 1
-                for (int i = 0; i < kPieces; ++i) stage_piece(4 * c0 + i);
+                for (int i = 0; i < n_steps; ++i) stage_step(c0 * 256 + i * (kStep * 16));
             }
-            if (rb == r0) {
+            auto wait_weights = [&]() {
 #pragma unroll 1
-                for (unsigned spins = 0; !mbar_try(bars + 8 * slot, parity); ++spins)
+                for (unsigned spins = 0; !(mbar_try(bars + 8 * slot, parity) && mbar_try(const_bar, 0)); ++spins)
                     if (spins >= kWeightWaitLimit) { atomicExch(P.status, (unsigned)(-NQ_ERR_TIMEOUT)); break; }
-            }
-            const uint32_t one2 = BF16 ? 0x3F803F80u : 0x3C003C00u;
-            // Shifts as products with powers of two the compiler cannot see: multiplications do not wait for the half-rate pipe of the LOP3s
-            // (16 tokens, eight layers: Llama-3.2-1B 315 -> 293 us, Qwen3-8B 438 -> 432, two of 8192 columns 393 -> 399; four and eight: level).
-            uint32_t pw[8], p256;
-            asm volatile("mov.u32 %0, %1;" : "=r"(p256) : "r"(256u));
-#pragma unroll
-            for (int i = 0; i < 8; ++i) asm volatile("mov.u32 %0, %1;" : "=r"(pw[i]) : "r"(1u << i));
-            // block b of a chunk (columns 32 j + 16 h + ..) against all row groups
-            auto block = [&](const uint4 (&w)[kRows], int b, uint32_t se, uint32_t so, const uint32_t (&be)[NT], const uint32_t (&bo)[NT]) {
-                const int j = b >> 1, h = b & 1;
-#pragma unroll
-                for (int r = 0; r < kRows; ++r)
-                    if (r < nr) {
-                        const uint32_t w0 = h ? w[r].z : w[r].x, w1 = h ? w[r].w : w[r].y;   // rows g, g + 8
-                        const uint32_t u0 = w0 * pw[7 - j], u1 = w1 * pw[7 - j];
-                        const uint32_t a0 = and_xor(u0 * p256, 0x80008000u, se), a2 = and_xor(u0, 0x80008000u, so);
-                        const uint32_t a1 = and_xor(u1 * p256, 0x80008000u, se), a3 = and_xor(u1, 0x80008000u, so);
-#pragma unroll
-                        for (int nt = 0; nt < NT; ++nt) mma_16816<BF16>(acc[r][nt], a0, a1, a2, a3, be[nt], bo[nt]);
-                    }
             };
+            if (!FRAG && rb == r0) wait_weights();
+            const unsigned char* wp = weights + slot * slot_bytes + (rb * chunks + c0) * 512 + lane * 16;
+            const int w_row = chunks * 512;
 #pragma unroll 1
-            for (int c = c0; c < c1; ++c) {
-                uint4 w[kRows];
-#pragma unroll
-                for (int r = 0; r < kRows; ++r)
-                    w[r] = *reinterpret_cast<const uint4*>(weights + slot * slot_bytes + ((rb + min(r, nr - 1)) * chunks + c) * 512 + lane * 16);
+            for (int c = c0; c < c1; ++c, wp += 512) {
                 if (FRAG) {
-                    const uint2* src = reinterpret_cast<const uint2*>(a_in) + (size_t)c * (16 * NT * 32) + lane;
+                    // neighbouring columns of a fragment are {0, 2} and {1, 3}: a word's bits are 16 apart as they are
+                    const uint2* src = static_cast<const uint2*>(jb.a) + (size_t)c * (16 * NT * 32) + lane;
+                    const bool full = c * 256 + 256 <= K;
+                    uint4 w[kRows];
 #pragma unroll
                     for (int b0 = 0; b0 < 16; b0 += kB) {
                         uint2 x[kB][NT];
+                        if (full) {
 #pragma unroll
-                        for (int b = 0; b < kB; ++b) {
-                            const bool in = c * 256 + (b0 + b) * 16 + 4 * q < K;
+                            for (int b = 0; b < kB; ++b)
 #pragma unroll
-                            for (int nt = 0; nt < NT; ++nt) x[b][nt] = in ? src[((b0 + b) * NT + nt) * 32] : make_uint2(0u, 0u);
+                                for (int nt = 0; nt < NT; ++nt) x[b][nt] = src[((b0 + b) * NT + nt) * 32];
+                        } else {
+#pragma unroll
+                            for (int b = 0; b < kB; ++b) {
+                                const bool in = c * 256 + (b0 + b) * 16 + 4 * q < K;
+#pragma unroll
+                                for (int nt = 0; nt < NT; ++nt) x[b][nt] = in ? src[((b0 + b) * NT + nt) * 32] : make_uint2(0u, 0u);
+                            }
+                        }
+                        if (b0 == 0) {
+                            if (c == c0 && rb == r0) wait_weights();
+#pragma unroll
+                            for (int r = 0; r < kRows; ++r) w[r] = *reinterpret_cast<const uint4*>(wp + min(r, nr - 1) * w_row);
                         }
 #pragma unroll
-                        for (int b = 0; b < kB; ++b) {
-                            uint32_t be[NT], bo[NT];
+                        for (int b = 0; b < kB; ++b)
 #pragma unroll
-                            for (int nt = 0; nt < NT; ++nt) { be[nt] = x[b][nt].x; bo[nt] = x[b][nt].y; }
-                            block(w, b0 + b, one2, one2, be, bo);
-                        }
+                            for (int r = 0; r < kRows; ++r)
+                                if (r < nr) {
+                                    const int j = (b0 + b) >> 1;
+                                    const uint32_t u0 = ((b & 1) ? w[r].z : w[r].x) << (7 - j), u1 = ((b & 1) ? w[r].w : w[r].y) << (7 - j);
+                                    const uint32_t a0 = and_xor(u0 << 8, 0x80008000u, one2), a2 = and_xor(u0, 0x80008000u, one2);
+                                    const uint32_t a1 = and_xor(u1 << 8, 0x80008000u, one2), a3 = and_xor(u1, 0x80008000u, one2);
+#pragma unroll
+                                    for (int nt = 0; nt < NT; ++nt) mma_16816<BF16>(acc[b % kChains][r][nt], a0, a1, a2, a3, x[b][nt].x, x[b][nt].y);
+                                }
                     }
                 } else {
+                    // words with the bits of neighbouring columns 16 apart, rows g and g + 8, halves of 16 columns
+                    uint32_t p[kRows][8];
 #pragma unroll
-                    for (int pc = 0; pc < 4; ++pc) {
-                        asm volatile("cp.async.wait_group %0;" ::"n"(kPieces - 1) : "memory");
+                    for (int r = 0; r < kRows; ++r) {
+                        const uint4 w = *reinterpret_cast<const uint4*>(wp + min(r, nr - 1) * w_row);
+                        p[r][0] = spread01(w.x); p[r][1] = spread23(w.x); p[r][2] = spread01(w.y); p[r][3] = spread23(w.y);
+                        p[r][4] = spread01(w.z); p[r][5] = spread23(w.z); p[r][6] = spread01(w.w); p[r][7] = spread23(w.w);
+                    }
+#pragma unroll
+                    for (int s0 = 0; s0 < 16; s0 += kStep) {
+                        if (n_steps > 1) asm volatile("cp.async.wait_group %0;" ::"n"(kMostSteps - 1) : "memory");
+                        else asm volatile("cp.async.wait_group 0;" ::: "memory");
                         __syncwarp();
-                        const unsigned char* buf = stage + s_out * piece_bytes;
-                        s_out = s_out + 1 == kPieces ? 0 : s_out + 1;
+                        const uint32_t buf = stage + s_out, s_addr = buf + T * kStepRow + 8 * q;
+                        uint32_t x_addr[NT][4];
 #pragma unroll
-                        for (int b = 0; b < 4; ++b) {
-                            uint32_t se = one2, so = one2, be[NT], bo[NT];
-                            if (pre) {
-                                const uint2 sv = *reinterpret_cast<const uint2*>(buf + T * kPieceStride + 8 * q + b * 32);
-                                se = even_columns(sv); so = odd_columns(sv);
-                            }
+                        for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
-                            for (int nt = 0; nt < NT; ++nt) {
-                                const uint2 xv = *reinterpret_cast<const uint2*>(buf + a_row[nt] + b * 32);
-                                be[nt] = even_columns(xv); bo[nt] = odd_columns(xv);
-                            }
-                            block(w, 4 * pc + b, se, so, be, bo);
+                            for (int k = 0; k < 4; ++k) x_addr[nt][k] = buf + t_row[nt] + ((32 * k) ^ t_swap[nt]);
+                        s_out = s_out + step_bytes == n_steps * step_bytes ? 0 : s_out + step_bytes;
+#pragma unroll
+                        for (int b = 0; b < kStep; ++b) {
+                            const int j = (s0 + b) >> 1;
+                            const uint2 sv = scaled ? lds8(s_addr + b * 32) : make_uint2(one2, one2);
+                            uint2 xv[NT];
+#pragma unroll
+                            for (int nt = 0; nt < NT; ++nt) xv[nt] = lds8(x_addr[nt][b & 3] + (b >> 2) * 128);
+#pragma unroll
+                            for (int r = 0; r < kRows; ++r)
+                                if (r < nr) {
+                                    const uint32_t* v = p[r] + 4 * (b & 1);
+                                    const uint32_t a0 = and_xor(v[0] << (7 - j), 0x80008000u, sv.x), a2 = and_xor(v[1] << (7 - j), 0x80008000u, sv.y);
+                                    const uint32_t a1 = and_xor(v[2] << (7 - j), 0x80008000u, sv.x), a3 = and_xor(v[3] << (7 - j), 0x80008000u, sv.y);
+#pragma unroll
+                                    for (int nt = 0; nt < NT; ++nt) mma_16816<BF16>(acc[b % kChains][r][nt], a0, a1, a2, a3, xv[nt].x, xv[nt].y);
+                                }
                         }
                         __syncwarp();            // the buffer has been read
-                        stage_piece(4 * c + pc + kPieces);
+                        stage_step(c * 256 + s0 * 16 + n_steps * (kStep * 16));
                     }
                 }
             }
@@ -313,12 +354,10 @@ __global__ void __launch_bounds__(kBatchThreads, 1) batch_stage_kernel(const __g
                     for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
                         for (int i = 0; i < 4; ++i)
-                            if (8 * nt + 2 * q + (i & 1) < T) dst[(8 * nt + (i & 1)) * tok_stride + r * 16 + 8 * (i >> 1)] = acc[r][nt][i];
+                            if (8 * nt + 2 * q + (i & 1) < T) dst[(8 * nt + (i & 1)) * tok_stride + r * 16 + 8 * (i >> 1)] = kChains == 2 ? acc[0][r][nt][i] + acc[kChains - 1][r][nt][i] : acc[0][r][nt][i];
                 }
         }
         const int io_bf16 = P.io_bf16, out_bf16 = P.out_bf16;
-        float2* const scale = reinterpret_cast<float2*>(part + (size_t)wk * T * tok_stride);   // {output scale, bias} of a row
-        if (tid < nb * 16) scale[tid] = make_float2(jb.post ? float_of(post_raw, io_bf16) : 1.f, jb.bias ? float_of(bias_raw, io_bf16) : 0.f);
         __syncthreads();   // partial sums complete, this block's weights have been read
         if (++slot == slots) { slot = 0; parity ^= 1u; }
         if (loader) load_block();
@@ -331,8 +370,13 @@ __global__ void __launch_bounds__(kBatchThreads, 1) batch_stage_kernel(const __g
         const float lim = P.saturate || (SPLIT && !FRAG) ? (out_bf16 ? 3.3895313892515355e+38f : 64504.0f) : 3.4e38f;
         const uint16_t* const resid = static_cast<const uint16_t*>(jb.resid);
         const int* const row_exp = jb.row_exp;
-        const int kslice = T * tok_stride, frag_out = P.frag_out, nb16 = nb * 16;
-        const int sums = (SPLIT ? kSplitTokens : T) * nb16 * (kPair ? 2 : 1);
+        // output scale and bias of a row of the block, from the copies in shared memory or as they lie in memory
+        const bool bulk = jb.bulk;
+        auto row_value = [&](const void* global, int copy, int idx) {
+            return float_of(bulk ? reinterpret_cast<const uint16_t*>(smem + copy)[blk * 16 + idx] : static_cast<const uint16_t*>(global)[row0 + idx], io_bf16);
+        };
+        const int kslice = T * tok_stride, frag_out = P.frag_out, t_magic = P.t_magic, tokens = SPLIT ? kSplitTokens : T;
+        const int sums = tokens * nb * 16 * (kPair ? 2 : 1);
         auto emit = [&](auto many, int e0) {
             constexpr int U = decltype(many)::value;
             float v[U];
@@ -341,8 +385,9 @@ __global__ void __launch_bounds__(kBatchThreads, 1) batch_stage_kernel(const __g
 #pragma unroll
             for (int u = 0; u < U; ++u) {
                 const int e = min(e0 + u * kBatchThreads, sums - 1), o = kPair ? e >> 1 : e;
-                tok[u] = (int)((unsigned)o * nb16_magic >> 22);
-                idx[u] = o - tok[u] * nb16;
+                const int gt = o >> 4, gi = SPLIT ? gt / kSplitTokens : (gt * t_magic) >> 16;      // [row group][token][row]
+                tok[u] = gt - gi * tokens;
+                idx[u] = gi * 16 + (o & 15);
                 src[u] = part + (tok[u] + (kPair && (e & 1) ? kSplitTokens : 0)) * tok_stride + idx[u];
                 v[u] = 0.f;
             }
@@ -353,13 +398,13 @@ __global__ void __launch_bounds__(kBatchThreads, 1) batch_stage_kernel(const __g
 #pragma unroll
             for (int u = 0; u < U; ++u) {
                 if (kPair) v[u] += __shfl_xor_sync(0xffffffffu, v[u], 1);
-                const float2 sc = scale[idx[u]];
                 const int row = row0 + idx[u];
                 if (e0 + u * kBatchThreads >= sums || row >= rows || (kPair && (lane & 1))) continue;
                 const float rs = row_exp ? exp2f((float)(P.exp_sign * row_exp[tok[u]])) : 1.f;
-                float extra = sc.y;
+                const float sc = jb.post ? row_value(jb.post, P.post_off, idx[u]) : 1.f;
+                float extra = jb.bias ? row_value(jb.bias, P.bias_off, idx[u]) : 0.f;
                 if (resid) extra += float_of(resid[tok[u] * jb.ld_res + row], io_bf16);
-                const float exact = v[u] * (sc.x * rs) + extra, w = clamp_or_nan(exact, lim);
+                const float exact = v[u] * (sc * rs) + extra, w = clamp_or_nan(exact, lim);
                 uint16_t* const out = static_cast<uint16_t*>(jb.out);
                 if (SPLIT && !FRAG) {
                     const __nv_bfloat16 value = __float2bfloat16(w);
@@ -492,9 +537,8 @@ int launch_batch_stage(const StageJob* jobs, int n, int tokens, StageTypes ty, i
     if (grid > total) grid = total;
     if (grid < n) grid = n;
     deal_ctas(grid, n, groups, chunks, ncta);
-    const size_t stage_bytes = frag_in ? 0 : (size_t)kBatchWarps * kPieces * (T + 1) * kPieceStride;
-    const size_t room = limit - kFixedBytes - stage_bytes;      // weights and partial sums of a block
-    size_t slot_used = 0, part_used = 0;
+    const size_t step_bytes = frag_in ? 0 : (size_t)kBatchWarps * (T + 1) * step_blocks(nt) * 32;
+    size_t row_bytes = 0, slot_used = 0, part_used = 0;      // row_bytes: output scales of a CTA, and as much for the bias
     int cta = 0, most_blocks = 1, most_rows = 1;
     for (int i = 0; i < n; ++i) {
         const StageJob& S = jobs[i];
@@ -507,14 +551,23 @@ int launch_batch_stage(const StageJob* jobs, int n, int tokens, StageTypes ty, i
         j.cta0 = cta;
         j.g_q = groups[i] / ncta[i];
         j.g_r = groups[i] % ncta[i];
+        const size_t bytes = (size_t)(j.g_q + (j.g_r ? 1 : 0)) * 32;
+        j.bulk = (!S.post || aligned16(S.post)) && (!S.bias || aligned16(S.bias)) && S.Nout % 8 == 0 && bytes <= kMostRowBytes;
+        if (j.bulk && bytes > row_bytes) row_bytes = bytes;
         memset(P.cta_job + cta, i, (size_t)ncta[i]);
         cta += ncta[i];
     }
     // Row blocks, as equal as possible: each job's weights and partial sums fit the room together; where the largest of
     // both over the jobs do not, each of them gets half; and where one row group does not fit half, one row group per
     // block (64 KB of weights at the largest K, 21 KB of partial sums).
-    for (int attempt = 0; attempt < 3; ++attempt) {
+    // Two staged steps per warp where that leaves each job in one block.
+    int steps = kMostSteps;
+    for (int attempt = -1; attempt < 3; ++attempt) {
+        steps = attempt < 0 ? kMostSteps : 1;
+        const size_t taken = kFixedBytes + steps * step_bytes + 2 * row_bytes + 256;
+        const size_t room = limit > (int)taken ? limit - taken : 0;      // weights and partial sums of a block
         slot_used = part_used = 0;
+        int most_block = 1;
         most_blocks = most_rows = 1;
         for (int i = 0; i < n; ++i) {
             BatchJob& j = P.job[i];
@@ -526,11 +579,11 @@ int launch_batch_stage(const StageJob* jobs, int n, int tokens, StageTypes ty, i
                 // the sums of a split linear have to be the same alone and in a group: slices as for the linear alone
                 split_warps(split ? (groups[i] + sm_count() - 1) / sm_count() : j.gb, chunks[i], nt, wk, wr);
                 if (split) wr = kBatchWarps / wk < j.gb ? kBatchWarps / wk : j.gb;
-                j.wk = (uint16_t)wk; j.wr = (uint16_t)wr;
-                part = (size_t)j.wk * T * (j.gb * 16 + 4) * 4 + (size_t)j.gb * 16 * 8;
+                j.wk = (uint8_t)wk; j.wr = (uint8_t)wr;
+                part = (size_t)j.wk * T * (j.gb * 16 + 4) * 4;
                 slot = (size_t)j.gb * chunks[i] * 512;
-                const bool fits = attempt == 0 ? part + slot <= room : part <= room / 2 && slot <= room / 2;
-                if (j.gb == 1 || (fits && j.gb <= kBatchThreads / 16)) break;
+                const bool fits = attempt <= 0 ? part + slot <= room : part <= room / 2 && slot <= room / 2;
+                if (j.gb == 1 || attempt < 0 || (fits && j.gb <= kMostBlock)) break;
             }
             part_used = part > part_used ? part : part_used;
             slot_used = slot > slot_used ? slot : slot_used;
@@ -538,18 +591,25 @@ int launch_batch_stage(const StageJob* jobs, int n, int tokens, StageTypes ty, i
             j.wr_magic = (65536 + j.wr - 1) / j.wr;
             const int blocks = (most + j.gb - 1) / j.gb, per_warp = (j.gb + j.wr - 1) / j.wr;
             most_blocks = blocks > most_blocks ? blocks : most_blocks;
+            most_block = j.gb > most_block ? j.gb : most_block;
             most_rows = per_warp > most_rows ? per_warp : most_rows;
         }
-        if (part_used + slot_used <= room) break;
+        if (part_used + slot_used <= room && (attempt >= 0 || most_block <= kMostBlock)) break;
     }
+    const size_t rest = kFixedBytes + steps * step_bytes + 2 * row_bytes + 256;
     int slots = most_blocks < kBatchSlots ? most_blocks : kBatchSlots;
-    while (slots > 1 && part_used + slots * slot_used > room) --slots;
+    while (slots > 1 && part_used + slots * slot_used + rest > (size_t)limit) --slots;
     P.slots = slots;
     P.slot_bytes = (int)slot_used;
     P.frag_out = frag_out;
+    P.steps = steps;
     P.part_off = (int)(kFixedBytes + slots * slot_used);
-    P.stage_off = (P.part_off + (int)part_used + 15) / 16 * 16;
-    const size_t smem = P.stage_off + stage_bytes;
+    P.post_off = (P.part_off + (int)part_used + 15) / 16 * 16;
+    P.bias_off = P.post_off + (int)row_bytes;
+    P.stage_off = (P.bias_off + (int)row_bytes + 127) / 128 * 128;
+    const int tokens_out = split ? kSplitTokens : T;
+    P.t_magic = (65536 + tokens_out - 1) / tokens_out;
+    const size_t smem = P.stage_off + steps * step_bytes;
     if (smem > (size_t)limit) return NQ_ERR_UNSUPPORTED;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(cta);
