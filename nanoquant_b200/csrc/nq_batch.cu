@@ -33,7 +33,6 @@
 // weights before this one ends, lost 10 to 50 %: every phase is then longer.  The next stage's weights brought to L2 by this one: 1 to 4 % slower.
 #include <cstddef>
 #include <cstring>
-#include <type_traits>
 
 #include "nq_common.cuh"
 #include "nq_plan.h"
@@ -70,7 +69,7 @@ struct alignas(16) BatchJob {
     int cta0, g_q, g_r;      // first CTA of the range; row groups per CTA, one more for its first g_r CTAs
     int gb;                  // row groups per block
     uint8_t wk, wr;          // chunk slices x row slices of a CTA's work, one warp each
-    uint16_t bulk;           // output scales and bias come by bulk copy beside the weights
+    uint8_t bulk, whole;     // output scales and bias come by bulk copy beside the weights; two neighbouring outputs are one 4-byte store
     int wk_magic, wr_magic;  // ceil(2^16 / .)
 };
 static_assert(sizeof(BatchJob) == 128, "128 bytes");
@@ -361,9 +360,11 @@ __global__ void __launch_bounds__(kBatchThreads, 1) batch_stage_kernel(const __g
         __syncthreads();   // partial sums complete, this block's weights have been read
         if (++slot == slots) { slot = 0; parity ^= 1u; }
         if (loader) load_block();
-        // Outputs, [token][row of the block] dealt to all threads, three at a time where there are more: the sums over the chunk slices are
-        // chains of shared-memory loads.  Of a split intermediate two neighbouring lanes sum value and remainder.  (A warp per token left
-        // 12 of 16 warps idle at four tokens: eight Qwen3-8B layers 356 -> 346 us, Llama-3.2-1B 264 -> 244, two of 8192 columns 289 -> 269.)
+        // Outputs.  Up to 512 of them are dealt to the threads one by one; of a split intermediate two neighbouring lanes sum value and
+        // remainder.  Larger blocks by two rows (two apart where they are neighbours in the next stage's fragments) of every tok_step-th
+        // token, with their scales converted once: the outputs of gate/up's second stage took 1.8 us of 9, now 1.  Eight Qwen3-8B layers, 4 / 8 / 12 /
+        // 16 tokens: 305 / 311 / 390 / 400 us -> 296 / 307 / 377 / 388; two of 8192 columns, 4 tokens, 192.8 -> 188.8.  (All blocks that way: one more
+        // dependent step where there are few outputs, Llama-3.2-1B 226 -> 229 and, eight tokens, 207 -> 213.)
         // An intermediate that is not a pair becomes infinite beyond its type's range, as in the GEMM; the value of a pair
         // stays finite, and it is the remainder that an infinity goes to.  NaN passes every clamp.
         constexpr bool kPair = SPLIT && FRAG;
@@ -377,49 +378,78 @@ __global__ void __launch_bounds__(kBatchThreads, 1) batch_stage_kernel(const __g
         };
         const int kslice = T * tok_stride, frag_out = P.frag_out, t_magic = P.t_magic, tokens = SPLIT ? kSplitTokens : T;
         const int sums = tokens * nb * 16 * (kPair ? 2 : 1);
-        auto emit = [&](auto many, int e0) {
-            constexpr int U = decltype(many)::value;
-            float v[U];
-            const float* src[U];
-            int tok[U], idx[U];
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                const int e = min(e0 + u * kBatchThreads, sums - 1), o = kPair ? e >> 1 : e;
+        if (sums <= kBatchThreads) {
+            if ((tid & ~31) < sums) {
+                const int e = min(tid, sums - 1), o = kPair ? e >> 1 : e;
                 const int gt = o >> 4, gi = SPLIT ? gt / kSplitTokens : (gt * t_magic) >> 16;      // [row group][token][row]
-                tok[u] = gt - gi * tokens;
-                idx[u] = gi * 16 + (o & 15);
-                src[u] = part + (tok[u] + (kPair && (e & 1) ? kSplitTokens : 0)) * tok_stride + idx[u];
-                v[u] = 0.f;
-            }
+                const int tok = gt - gi * tokens, idx = gi * 16 + (o & 15), row = row0 + idx;
+                const float* src = part + (tok + (kPair && (e & 1) ? kSplitTokens : 0)) * tok_stride + idx;
+                float v = 0.f;
 #pragma unroll 4
-            for (int k = 0; k < wk; ++k)
-#pragma unroll
-                for (int u = 0; u < U; ++u) { v[u] += *src[u]; src[u] += kslice; }
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                if (kPair) v[u] += __shfl_xor_sync(0xffffffffu, v[u], 1);
-                const int row = row0 + idx[u];
-                if (e0 + u * kBatchThreads >= sums || row >= rows || (kPair && (lane & 1))) continue;
-                const float rs = row_exp ? exp2f((float)(P.exp_sign * row_exp[tok[u]])) : 1.f;
-                const float sc = jb.post ? row_value(jb.post, P.post_off, idx[u]) : 1.f;
-                float extra = jb.bias ? row_value(jb.bias, P.bias_off, idx[u]) : 0.f;
-                if (resid) extra += float_of(resid[tok[u] * jb.ld_res + row], io_bf16);
-                const float exact = v[u] * (sc * rs) + extra, w = clamp_or_nan(exact, lim);
-                uint16_t* const out = static_cast<uint16_t*>(jb.out);
-                if (SPLIT && !FRAG) {
-                    const __nv_bfloat16 value = __float2bfloat16(w);
-                    out[fragment_index<1>(tok[u], row)] = __bfloat16_as_ushort(value);
-                    out[fragment_index<1>(kSplitTokens + tok[u], row)] = __bfloat16_as_ushort(__float2bfloat16(exact - __bfloat162float(value)));
-                } else {
-                    out[frag_out ? fragment_index<NT>(tok[u], row) : tok[u] * jb.ld_out + row] = out_bf16 ? __bfloat16_as_ushort(__float2bfloat16(w)) : __half_as_ushort(__float2half(w));
+                for (int k = 0; k < wk; ++k, src += kslice) v += *src;
+                if (kPair) v += __shfl_xor_sync(0xffffffffu, v, 1);
+                if (tid < sums && row < rows && !(kPair && (lane & 1))) {
+                    const float rs = row_exp ? exp2f((float)(P.exp_sign * row_exp[tok])) : 1.f;
+                    const float sc = jb.post ? row_value(jb.post, P.post_off, idx) : 1.f;
+                    float extra = jb.bias ? row_value(jb.bias, P.bias_off, idx) : 0.f;
+                    if (resid) extra += float_of(resid[tok * jb.ld_res + row], io_bf16);
+                    const float exact = v * (sc * rs) + extra, w = clamp_or_nan(exact, lim);
+                    uint16_t* const out = static_cast<uint16_t*>(jb.out);
+                    if (SPLIT && !FRAG) {
+                        const __nv_bfloat16 value = __float2bfloat16(w);
+                        out[fragment_index<1>(tok, row)] = __bfloat16_as_ushort(value);
+                        out[fragment_index<1>(kSplitTokens + tok, row)] = __bfloat16_as_ushort(__float2bfloat16(exact - __bfloat162float(value)));
+                    } else {
+                        out[frag_out ? fragment_index<NT>(tok, row) : tok * jb.ld_out + row] = out_bf16 ? __bfloat16_as_ushort(__float2bfloat16(w)) : __half_as_ushort(__float2half(w));
+                    }
                 }
             }
-        };
-        if (sums <= kBatchThreads) {
-            if ((tid & ~31) < sums) emit(std::integral_constant<int, 1>{}, tid);
         } else {
+            const int pair_bits = 3 + (nb > 1) + (nb > 2) + (nb > 4) + (nb > 8) + (nb > 16);
+            const int pair = tid & ((1 << pair_bits) - 1), tok_step = kBatchThreads >> pair_bits;
+            const bool frag = !FRAG && frag_out;
+            const int apart = frag ? 2 : 1, idx = frag ? 4 * (pair >> 1) + (pair & 1) : 2 * pair, row = row0 + idx;
+            if (idx < nb * 16 && row < rows) {
+                const bool both = row + apart < rows;
+                float sc0 = 1.f, sc1 = 1.f, bi0 = 0.f, bi1 = 0.f;
+                if (jb.post) { sc0 = row_value(jb.post, P.post_off, idx); if (both) sc1 = row_value(jb.post, P.post_off, idx + apart); }
+                if (jb.bias) { bi0 = row_value(jb.bias, P.bias_off, idx); if (both) bi1 = row_value(jb.bias, P.bias_off, idx + apart); }
+                uint16_t* const out = static_cast<uint16_t*>(jb.out);
+                const float* src = part + (tid >> pair_bits) * tok_stride + idx;
 #pragma unroll 1
-            for (int e0 = tid; (e0 & ~31) < sums; e0 += 3 * kBatchThreads) emit(std::integral_constant<int, 3>{}, e0);
+                for (int tok = tid >> pair_bits; tok < tokens; tok += tok_step, src += tok_step * tok_stride) {
+                    float x0 = bi0, x1 = bi1, v0 = 0.f, v1 = 0.f, r0 = 0.f, r1 = 0.f, s0 = sc0, s1 = sc1;
+                    if (resid) {
+                        const uint16_t* const r = resid + tok * jb.ld_res + row;
+                        x0 += float_of(r[0], io_bf16);
+                        if (both) x1 += float_of(r[1], io_bf16);
+                    }
+                    const float* from = src;
+#pragma unroll 4
+                    for (int k = 0; k < wk; ++k, from += kslice) {
+                        v0 += from[0]; v1 += from[apart];
+                        if (kPair) { r0 += from[kSplitTokens * tok_stride]; r1 += from[kSplitTokens * tok_stride + apart]; }
+                    }
+                    if (kPair) { v0 += r0; v1 += r1; }      // (the same order of sums as above: a linear's bits do not depend on the block)
+                    if (row_exp) { const float rs = exp2f((float)(P.exp_sign * row_exp[tok])); s0 *= rs; s1 *= rs; }
+                    const float e0 = v0 * s0 + x0, e1 = v1 * s1 + x1, w0 = clamp_or_nan(e0, lim), w1 = clamp_or_nan(e1, lim);
+                    if (SPLIT && !FRAG) {
+                        const __nv_bfloat162 value = __floats2bfloat162_rn(w0, w1);
+                        *reinterpret_cast<__nv_bfloat162*>(out + fragment_index<1>(tok, row)) = value;
+                        *reinterpret_cast<__nv_bfloat162*>(out + fragment_index<1>(kSplitTokens + tok, row)) = __floats2bfloat162_rn(e0 - __low2float(value), e1 - __high2float(value));
+                        continue;
+                    }
+                    uint32_t o;
+                    if (out_bf16) { const __nv_bfloat162 h = __floats2bfloat162_rn(w0, w1); o = *reinterpret_cast<const uint32_t*>(&h); }
+                    else { const __half2 h = __floats2half2_rn(w0, w1); o = *reinterpret_cast<const uint32_t*>(&h); }
+                    uint16_t* const dst = out + (frag ? fragment_index<NT>(tok, row) : tok * jb.ld_out + row);
+                    if (both && jb.whole) *reinterpret_cast<uint32_t*>(dst) = o;
+                    else {
+                        dst[0] = (uint16_t)o;
+                        if (both) dst[1] = (uint16_t)(o >> 16);
+                    }
+                }
+            }
         }
         if (blk + gb < groups) __syncthreads();   // the partial sums have been read
     }
@@ -554,6 +584,7 @@ int launch_batch_stage(const StageJob* jobs, int n, int tokens, StageTypes ty, i
         const size_t bytes = (size_t)(j.g_q + (j.g_r ? 1 : 0)) * 32;
         j.bulk = (!S.post || aligned16(S.post)) && (!S.bias || aligned16(S.bias)) && S.Nout % 8 == 0 && bytes <= kMostRowBytes;
         if (j.bulk && bytes > row_bytes) row_bytes = bytes;
+        j.whole = frag_out || (reinterpret_cast<uintptr_t>(S.out) % 4 == 0 && S.ld_out % 2 == 0);
         memset(P.cta_job + cta, i, (size_t)ncta[i]);
         cta += ncta[i];
     }
