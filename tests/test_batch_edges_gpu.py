@@ -53,3 +53,25 @@ def test_batch_tile_edges(shapes, T, dtype):
         y = exact_np(ys[i])
         worst = float((np.abs(y - want) - bound(layers[i], y, want, dtype)).max())
         assert worst <= 0, f"linear {i} of {shapes}, {T} tokens: {worst:.3e} beyond the bound"
+
+
+@pytest.mark.parametrize("shape,T", [
+    ((264, 5016, 9999), 5), ((264, 5016, 9999), 16),      # blocks of up to and beyond 512 outputs, an odd last row, rows at odd addresses
+    ((264, 5016, 10000), 16),                             # pairs of outputs as one store
+    ((8, 8, 700000), 5),                                  # more rows of a CTA than it keeps scales of
+    ((28680, 2376, 48), 8),                               # one staged step per warp
+])
+@pytest.mark.parametrize("shifted", [False, True])        # output scales and bias at an address that a bulk copy does not take
+def test_batch_blocks_of_outputs(shape, T, shifted):
+    from nanoquant_b200 import ops
+    dtype = torch.bfloat16
+    L = make_group([shape], T, dtype, seed=T)[0]
+    scale = float(abs(L["y64"]).max())
+    g = torch.Generator(device="cuda").manual_seed(T)
+    bias = (torch.randn(L["M"], generator=g, device="cuda") * scale).to(dtype)
+    resid = (torch.randn(T, L["M"], generator=g, device="cuda") * scale).to(dtype)
+    move = lambda v: torch.cat([v[:1], v])[1:] if shifted else v
+    tens = (L["s_pre"], tiles_on_gpu(L["V"]), L["s_mid"], tiles_on_gpu(L["U"]), move(L["s_post"]), L["R"])
+    y = exact_np(ops.group_forward([L["x"]], [tens], T, dtype, torch.device("cuda", 0), [move(bias)], [resid])[0])
+    want = L["y64"] + exact_np(bias) + exact_np(resid)
+    assert float((np.abs(y - want) - bound(L, y, want, dtype)).max()) <= 0

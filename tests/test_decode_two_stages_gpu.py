@@ -73,3 +73,14 @@ def test_group_equals_linears_alone(shapes, dtype):
         assert torch.equal(group[7][i][:4], group[4][i])         # four tokens at a time, the rest by the decode kernel
         # up to three tokens: the same bits however many ride along
         assert torch.equal(group[1][i], group[3][i][:1]) and torch.equal(group[2][i], group[3][i][:2])
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_group_equals_linears_alone_in_larger_blocks(dtype):
+    """A CTA has 2 and 6 row groups of these linears alone, 7 of either in the group: outputs dealt one by one and by pairs of rows."""
+    layers = make_group([(4096, 264, 4736), (4096, 264, 12288)], 4, dtype, seed=5)
+    tiles = [(tiles_on_gpu(L["V"]), tiles_on_gpu(L["U"])) for L in layers]
+    group = call(layers, tiles, 4, dtype)
+    for i, L in enumerate(layers):
+        assert torch.equal(group[i], call([L], tiles[i:i + 1], 4, dtype)[0])
+        assert_parity(exact_np(group[i]), L["y64"], dtype, rel=1e-4, what=f"linear {i}")
