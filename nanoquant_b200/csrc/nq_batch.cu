@@ -53,7 +53,7 @@ constexpr int kBatchMaxCtas = 256;
 constexpr size_t kOffParams = 128, kFixedBytes = 1024;
 constexpr int kMostBlock = 32;           // row groups of a block
 constexpr size_t kMostRowBytes = 8192;   // output scales of a CTA in shared memory
-constexpr unsigned kWeightWaitLimit = 1u << 20;   // attempts of up to ~2 us each
+constexpr unsigned kWeightWaitLimit = 1u << 20;   // attempts of some 4 us each
 
 struct alignas(16) BatchJob {
     const uint4* tiles;

@@ -69,7 +69,7 @@ constexpr size_t kFixedBytes = kOffMeta + (size_t)kMaxTok * kMaxChunks * 8;
 static_assert(8 * kMaxSlots <= kOffParams && kFixedBytes % 128 == 0, "shared memory map");
 constexpr size_t kPartBytes = 32 << 10;    // partial sums of a row block
 constexpr size_t kSlotBytes = 64 << 10;    // weights of a row block
-constexpr unsigned kWeightWaitLimit = 1u << 20;   // attempts of up to ~2 us each
+constexpr unsigned kWeightWaitLimit = 1u << 20;   // attempts of some 4 us each
 constexpr unsigned kPollBackoffNs = 20;    // pause between two polls of the tagged intermediate (100: 0.4 to 0.9 % slower, 300: more)
 constexpr unsigned kHelpAfter = 256;       // polls (about 0.1 ms) before a CTA helps; 1/16 of the limit where that is less,
                                            // never with a limit below 16
