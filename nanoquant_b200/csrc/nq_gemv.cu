@@ -139,18 +139,26 @@ __device__ __forceinline__ void quantise_unit(float (&p)[8], unsigned char* xq_c
     for (int e = 0; e < 8; ++e) m = max_or_nan(m, fabsf(p[e]));
     m = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(m)));   // as bits: a NaN is above infinity
     float unit = m * (1.0f / (128.f * kQMax));
-    if (!(m > 1e-31f && m <= 3.4028235e38f)) {
-        const bool tiny = m > 0.f && m <= 1e-31f;       // the reciprocal would overflow: the same integers from p * 2^64
+    if (!(m > 1e-31f && m < 1e37f)) {
+        // Beyond what the approximate reciprocal takes: the same integers from p * 2^64 or p * 2^-64.
+        const float f = m > 0.f && m <= 1e-31f ? 1.8446744e19f : m >= 1e37f && m <= 3.4028235e38f ? 5.4210109e-20f : 0.f;
         // All zero, or not finite.  A value that is not finite makes the unit a NaN, and with it every sum over this
         // chunk and every output of this token, as the same sums in floating point would be (an infinity meets another of
         // the opposite sign); left in, its bits would spill into the bytes of neighbouring columns.
-        if (!tiny && m != 0.f) unit = __uint_as_float(0x7FFFFFFFu);
-        m = tiny ? m * 1.8446744e19f : 1.f;
+        if (f == 0.f && m != 0.f) unit = __uint_as_float(0x7FFFFFFFu);
+        m = f != 0.f ? m * f : 1.f;
 #pragma unroll
-        for (int e = 0; e < 8; ++e) p[e] = tiny ? p[e] * 1.8446744e19f : 0.f;
+        for (int e = 0; e < 8; ++e) p[e] = f != 0.f ? p[e] * f : 0.f;
     }
+    // The approximate reciprocal is some (1 + d) / m with |d| <= 2^-23.  The integers may be of any unit, as long as it is the one that they
+    // are multiplied by again: the unit takes the factor 1 - d = 2 - m * inv.  (The rounded reciprocal is a sequence of dependent
+    // instructions and a branch: eight layers, one / two / three tokens, Qwen3-8B 208 / 246 / 322 -> 206 / 240 / 319 us,
+    // Llama-3.2-1B 159 / 182 / 231 -> 156 / 179 / 229.)
+    float inv;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(inv) : "f"(m));
+    unit *= fmaf(-m, inv, 2.f);
     // times 2^(7-j), negative for j = 7 (the A operand of class 7 is -128)
-    const float inv_j = kQMax * __frcp_rn(m) * __uint_as_float(j == 7 ? 0xBF800000u : (uint32_t)(127 + 7 - j) << 23);
+    const float inv_j = kQMax * inv * __uint_as_float(j == 7 ? 0xBF800000u : (uint32_t)(127 + 7 - j) << 23);
     // 1.5 * 2^23 + v rounds v to an integer Z in the low mantissa bits (|v| < 2^22).  With 0x8080 added, bytes 0 and 1
     // of the sum are the two low signed bytes of Z with their top bits flipped, and bits 16..22 are the high byte + 64.
     uint32_t z[8], zsum = 0;

@@ -102,3 +102,19 @@ def test_the_largest_finite_maximum_stays_in_range():
     _, _, (b0, b1, b2) = unit_of(p)
     z = 65536 * b2 + 256 * b1 + b0
     assert np.abs(z).max() < 2 ** 22 and np.abs(A * z).max() <= 128 * Q_MAX * (1 + 2.0 ** -20)
+
+
+def test_a_unit_that_takes_the_error_of_the_reciprocal():
+    # an approximate reciprocal (1 + d) / m, |d| <= 2^-23, and the unit times 2 - m * inv (fused): half an integer stays half an integer
+    for seed in range(1, 40):
+        p = products(seed)
+        m = np.float32(np.abs(p).max())
+        for steps in (-1, 0, 1):
+            inv = np.float32(1) / m
+            inv = np.nextafter(inv, np.float32(np.inf if steps > 0 else 0)) if steps else inv
+            scale = (np.float32(Q_MAX) * inv * np.where(J == 7, np.float32(-1), np.float32(2.0) ** (7 - J)).astype(np.float32))
+            z = np.rint(p.astype(np.float64) * scale.astype(np.float64))
+            assert np.abs(z).max() < 2 ** 22
+            factor = np.float32(2.0 - np.float64(m) * np.float64(inv))
+            unit = m * np.float32(1.0 / (128 * Q_MAX)) * factor
+            assert np.abs(A * z * np.float64(unit) - p).max() <= np.abs(p).max() * (64 / (128 * Q_MAX) + 2.0 ** -21)

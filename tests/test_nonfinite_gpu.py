@@ -60,6 +60,21 @@ def test_decode_kernel_small_activations(T, exponent):
     assert_parity(exact_np(y) * 2.0 ** -exponent, want, torch.bfloat16, rel=1e-4, what=f"2^{exponent}")
 
 
+@pytest.mark.parametrize("exponent", [60, 119, 121, 122, 123])
+@pytest.mark.parametrize("T", [1, 2, 3, 4])
+def test_decode_kernel_large_activations(T, exponent):
+    # maxima on both sides of 1e37, from where on their approximate reciprocal would be subnormal
+    N, R, M = 40, 136, 520
+    L = make_layer(N, R, M, T, torch.bfloat16, seed=5)
+    L["s_pre"] = torch.ones_like(L["s_pre"])
+    L["s_mid"] = torch.full_like(L["s_mid"], 2.0 ** -100)
+    from oracle import nanoquant_oracle as oc
+    x = L["x"] * 2.0 ** exponent
+    assert torch.isfinite(x).all() and (exponent < 123 or x.abs().max() > 1e37)
+    want = oc.forward_fp64(exact_np(x), L["V"], L["U"], exact_np(L["s_pre"]), exact_np(L["s_mid"]), exact_np(L["s_post"]))
+    assert_parity(exact_np(gemv(L, x)), want, torch.bfloat16, rel=1e-4, what=f"2^{exponent}")
+
+
 def dispatched(L, x, resid=None, precise=False):
     """A launch group of one, as the module calls it."""
     from nanoquant_b200 import ops
