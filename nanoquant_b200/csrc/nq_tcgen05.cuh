@@ -82,23 +82,21 @@ __device__ __forceinline__ void tmem_st_frag4(uint32_t taddr, const uint32_t (&v
                  "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
                  : "memory");
 }
-// Selector nibble 8 + b: the sign of byte b in every bit.
-__device__ __forceinline__ uint32_t spread_signs(uint32_t u, uint32_t sel) {
-    uint32_t r;
-    asm("prmt.b32 %0, %1, 0, %2;" : "=r"(r) : "r"(u), "r"(sel));
-    return r;
-}
+// Bytes {0, 1} and {2, 3} of a word to bytes 1 and 3: bits of neighbouring columns, 8 apart, are then 16 apart.
+__device__ __forceinline__ uint32_t spread_bytes(uint32_t w, int pair) { return __byte_perm(w, 0u, pair ? 0x3424 : 0x1404); }
 // 64 columns of 16 rows: `w` with the bits of column class j at 8 b + j + 4 - (j & 4), half `hf` of the 128 columns -> the words of
-// tcgen05.st 16x256b.x4, +-pn.  Two ALU operations per two weights.
+// tcgen05.st 16x256b.x4, +-pn.  Two ALU operations per two weights, and a PRMT per two words for all eight classes.  (A PRMT that spreads sign bits
+// per two weights beside half a shift before: two layers of 64 / 128 / 256 / 517 tokens, Qwen3-8B 133.6 / 164.2 / 223.0 / 335.8 -> 130.2 /
+// 160.3 / 217.4 / 329.4 us, Llama-2-7B 145.3 / 204.0 / 260.2 / 390.8 -> 143.6 / 197.2 / 253.0 / 387.9.  Shifts as products, beside the ALU pipe: level.)
 __device__ __forceinline__ void expand_columns(const uint4& w, int hf, const uint2 (&pn)[4], uint32_t (&v)[16]) {
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         const int sh = 3 - (2 * hf + (i >> 1));
-        const uint32_t u0 = ((i & 1) ? w.z : w.x) << sh, u1 = ((i & 1) ? w.w : w.y) << sh;
-        v[4 * i + 0] = and_xor(spread_signs(u0, 0x9988u), 0x80008000u, pn[i].x);
-        v[4 * i + 1] = and_xor(spread_signs(u0, 0xBBAAu), 0x80008000u, pn[i].y);
-        v[4 * i + 2] = and_xor(spread_signs(u1, 0x9988u), 0x80008000u, pn[i].x);
-        v[4 * i + 3] = and_xor(spread_signs(u1, 0xBBAAu), 0x80008000u, pn[i].y);
+        const uint32_t w0 = (i & 1) ? w.z : w.x, w1 = (i & 1) ? w.w : w.y;
+        v[4 * i + 0] = and_xor(spread_bytes(w0, 0) << sh, 0x80008000u, pn[i].x);
+        v[4 * i + 1] = and_xor(spread_bytes(w0, 1) << sh, 0x80008000u, pn[i].y);
+        v[4 * i + 2] = and_xor(spread_bytes(w1, 0) << sh, 0x80008000u, pn[i].x);
+        v[4 * i + 3] = and_xor(spread_bytes(w1, 1) << sh, 0x80008000u, pn[i].y);
     }
 }
 // The same for +-1 and columns whose middle two of every four are swapped (kOrderIn): the bits of a pair are 16 apart, one ALU

@@ -10,7 +10,7 @@
 //               exchange and the epilogue
 //
 //  * No expanded weight passes through shared memory.  tcgen05.st 16x256b gives lane 4g + q the columns 4q..4q+3 of rows g and
-//    g + 8 of a 16-column block, which are the bits that this lane holds in the tile layout: a shift, a PRMT that spreads
+//    g + 8 of a 16-column block, which are the bits that this lane holds in the tile layout: a PRMT that spreads
 //    sign bits and one LOP3 per two weights.  Written to shared memory and read back by the MMA, as the operand of a 128 x 128
 //    tile of the first GEMM here was, they made it shared-memory bound (485 cycles per 64 columns for 256 of MMA).
 //  * Tokens are columns, so 33 tokens pay for 48 and not for 128.
