@@ -47,6 +47,8 @@ constexpr int kMostRows = 4;             // row groups of a pass
 // 16-column blocks that a warp stages together, and fragments of the intermediate it loads together
 constexpr int step_blocks(int nt) { return nt == 1 ? 16 : 8; }
 constexpr int blocks_in_flight(int nt, int rows) { return nt == 1 && rows < 4 ? 16 : nt == 1 || rows < 4 ? 8 : 4; }
+// staged fragments a warp holds for its row groups in turn
+constexpr int fragments_held(int nt, int rows) { return nt * rows >= 8 ? 2 : 4; }
 constexpr int kMostSteps = 2;            // steps in flight
 constexpr int kBatchSlots = 8;           // weight blocks in flight
 constexpr int kBatchMaxCtas = 256;
@@ -124,7 +126,7 @@ __device__ __forceinline__ void copy16_or_zero(uint32_t dst, const void* src, bo
 // kSplitTokens).
 template <bool BF16, int NT, int ROWS, bool FRAG, bool SPLIT>
 __global__ void __launch_bounds__(kBatchThreads, 1) batch_stage_kernel(const __grid_constant__ BatchParams Pc) {
-    constexpr int kRows = ROWS, kB = blocks_in_flight(NT, ROWS), kStep = step_blocks(NT), kStepRow = kStep * 32;
+    constexpr int kRows = ROWS, kB = blocks_in_flight(NT, ROWS), kStep = step_blocks(NT), kStepRow = kStep * 32, kQ = fragments_held(NT, ROWS);
     constexpr uint32_t one2 = BF16 ? 0x3F803F80u : 0x3C003C00u;
     // Accumulators of a fragment's blocks in turn: MMAs on one of them wait for each other.  (Of a split intermediate it must not depend on
     // ROWS, which may differ between a linear alone and in a group.)
@@ -262,6 +264,9 @@ __global__ void __launch_bounds__(kBatchThreads, 1) batch_stage_kernel(const __g
                     // neighbouring columns of a fragment are {0, 2} and {1, 3}: a word's bits are 16 apart as they are
                     const uint2* src = static_cast<const uint2*>(jb.a) + (size_t)c * (16 * NT * 32) + lane;
                     const bool full = c * 256 + 256 <= K;
+                    // (Several fragments per row group in both kinds of stages: with the row groups inside, whether one exists was a branch around
+                    // every MMA.  Eight Qwen3-8B layers, 4 / 8 / 12 / 16 tokens: 296 / 306 / 376 / 387 -> 267 / 278 / 364 / 373 us; two of 8192
+                    // columns, 4 and 8 tokens, 189 / 209 -> 162 / 179.)
                     uint4 w[kRows];
 #pragma unroll
                     for (int b0 = 0; b0 < 16; b0 += kB) {
@@ -285,10 +290,10 @@ __global__ void __launch_bounds__(kBatchThreads, 1) batch_stage_kernel(const __g
                             for (int r = 0; r < kRows; ++r) w[r] = *reinterpret_cast<const uint4*>(wp + min(r, nr - 1) * w_row);
                         }
 #pragma unroll
-                        for (int b = 0; b < kB; ++b)
+                        for (int r = 0; r < kRows; ++r)
+                            if (r < nr)
 #pragma unroll
-                            for (int r = 0; r < kRows; ++r)
-                                if (r < nr) {
+                                for (int b = 0; b < kB; ++b) {
                                     const int j = (b0 + b) >> 1;
                                     const uint32_t u0 = ((b & 1) ? w[r].z : w[r].x) << (7 - j), u1 = ((b & 1) ? w[r].w : w[r].y) << (7 - j);
                                     const uint32_t a0 = and_xor(u0 << 8, 0x80008000u, one2), a2 = and_xor(u0, 0x80008000u, one2);
@@ -319,21 +324,26 @@ __global__ void __launch_bounds__(kBatchThreads, 1) batch_stage_kernel(const __g
                             for (int k = 0; k < 4; ++k) x_addr[nt][k] = buf + t_row[nt] + ((32 * k) ^ t_swap[nt]);
                         s_out = s_out + step_bytes == n_steps * step_bytes ? 0 : s_out + step_bytes;
 #pragma unroll
-                        for (int b = 0; b < kStep; ++b) {
-                            const int j = (s0 + b) >> 1;
-                            const uint2 sv = scaled ? lds8(s_addr + b * 32) : make_uint2(one2, one2);
-                            uint2 xv[NT];
+                        for (int q0 = 0; q0 < kStep; q0 += kQ) {
+                            uint2 sv[kQ], xv[kQ][NT];
 #pragma unroll
-                            for (int nt = 0; nt < NT; ++nt) xv[nt] = lds8(x_addr[nt][b & 3] + (b >> 2) * 128);
+                            for (int b = 0; b < kQ; ++b) {
+                                sv[b] = scaled ? lds8(s_addr + (q0 + b) * 32) : make_uint2(one2, one2);
+#pragma unroll
+                                for (int nt = 0; nt < NT; ++nt) xv[b][nt] = lds8(x_addr[nt][(q0 + b) & 3] + ((q0 + b) >> 2) * 128);
+                            }
 #pragma unroll
                             for (int r = 0; r < kRows; ++r)
-                                if (r < nr) {
-                                    const uint32_t* v = p[r] + 4 * (b & 1);
-                                    const uint32_t a0 = and_xor(v[0] << (7 - j), 0x80008000u, sv.x), a2 = and_xor(v[1] << (7 - j), 0x80008000u, sv.y);
-                                    const uint32_t a1 = and_xor(v[2] << (7 - j), 0x80008000u, sv.x), a3 = and_xor(v[3] << (7 - j), 0x80008000u, sv.y);
+                                if (r < nr)
 #pragma unroll
-                                    for (int nt = 0; nt < NT; ++nt) mma_16816<BF16>(acc[b % kChains][r][nt], a0, a1, a2, a3, xv[nt].x, xv[nt].y);
-                                }
+                                    for (int b = 0; b < kQ; ++b) {
+                                        const int j = (s0 + q0 + b) >> 1;
+                                        const uint32_t* v = p[r] + 4 * ((q0 + b) & 1);
+                                        const uint32_t a0 = and_xor(v[0] << (7 - j), 0x80008000u, sv[b].x), a2 = and_xor(v[1] << (7 - j), 0x80008000u, sv[b].y);
+                                        const uint32_t a1 = and_xor(v[2] << (7 - j), 0x80008000u, sv[b].x), a3 = and_xor(v[3] << (7 - j), 0x80008000u, sv[b].y);
+#pragma unroll
+                                        for (int nt = 0; nt < NT; ++nt) mma_16816<BF16>(acc[(q0 + b) % kChains][r][nt], a0, a1, a2, a3, xv[b][nt].x, xv[b][nt].y);
+                                    }
                         }
                         __syncwarp();            // the buffer has been read
                         stage_step(c * 256 + s0 * 16 + n_steps * (kStep * 16));
