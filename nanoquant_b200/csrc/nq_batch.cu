@@ -33,6 +33,7 @@
 // weights before this one ends, lost 10 to 50 %: every phase is then longer.  The next stage's weights brought to L2 by this one: 1 to 4 % slower.
 #include <cstddef>
 #include <cstring>
+#include <type_traits>
 
 #include "nq_common.cuh"
 #include "nq_plan.h"
@@ -424,40 +425,71 @@ __global__ void __launch_bounds__(kBatchThreads, 1) batch_stage_kernel(const __g
                 float sc0 = 1.f, sc1 = 1.f, bi0 = 0.f, bi1 = 0.f;
                 if (jb.post) { sc0 = row_value(jb.post, P.post_off, idx); if (both) sc1 = row_value(jb.post, P.post_off, idx + apart); }
                 if (jb.bias) { bi0 = row_value(jb.bias, P.bias_off, idx); if (both) bi1 = row_value(jb.bias, P.bias_off, idx + apart); }
-                uint16_t* const out = static_cast<uint16_t*>(jb.out);
-                const float* src = part + (tid >> pair_bits) * tok_stride + idx;
-#pragma unroll 1
-                for (int tok = tid >> pair_bits; tok < tokens; tok += tok_step, src += tok_step * tok_stride) {
-                    float x0 = bi0, x1 = bi1, v0 = 0.f, v1 = 0.f, r0 = 0.f, r1 = 0.f, s0 = sc0, s1 = sc1;
-                    if (resid) {
-                        const uint16_t* const r = resid + tok * jb.ld_res + row;
-                        x0 += float_of(r[0], io_bf16);
-                        if (both) x1 += float_of(r[1], io_bf16);
-                    }
-                    const float* from = src;
+                uint16_t* const out = static_cast<uint16_t*>(jb.out) + (frag ? 0 : row);
+                const long long ld_out = jb.ld_out, ld_res = jb.ld_res;
+                const bool pairs = both && jb.whole;
+                const int exp_sign = P.exp_sign;
+                // Two tokens at a time where a thread has more than one: the sums are chains of shared-memory loads (sixteen tokens 373 -> 368 us, six
+                // layers of 3072 columns 258 -> 253).
+                auto take = [&](auto many, int tok0) {
+                    constexpr int U = decltype(many)::value;
+                    float v0[U], v1[U], r0[U], r1[U];
+                    const float* from = part + tok0 * tok_stride + idx;
+                    const int next = tok0 + tok_step < tokens ? tok_step * tok_stride : 0;      // (a second token that does not exist: the first again)
+#pragma unroll
+                    for (int u = 0; u < U; ++u) v0[u] = v1[u] = r0[u] = r1[u] = 0.f;
 #pragma unroll 4
                     for (int k = 0; k < wk; ++k, from += kslice) {
-                        v0 += from[0]; v1 += from[apart];
-                        if (kPair) { r0 += from[kSplitTokens * tok_stride]; r1 += from[kSplitTokens * tok_stride + apart]; }
+#pragma unroll
+                        for (int u = 0; u < U; ++u) {
+                            const float* f = from + (u ? next : 0);
+                            if (FRAG) {       // (neighbouring rows)
+                                const float2 a = *reinterpret_cast<const float2*>(f);
+                                v0[u] += a.x; v1[u] += a.y;
+                                if (kPair) {
+                                    const float2 r = *reinterpret_cast<const float2*>(f + kSplitTokens * tok_stride);
+                                    r0[u] += r.x; r1[u] += r.y;
+                                }
+                            } else {
+                                v0[u] += f[0]; v1[u] += f[apart];
+                            }
+                        }
                     }
-                    if (kPair) { v0 += r0; v1 += r1; }      // (the same order of sums as above: a linear's bits do not depend on the block)
-                    if (row_exp) { const float rs = exp2f((float)(P.exp_sign * row_exp[tok])); s0 *= rs; s1 *= rs; }
-                    const float e0 = v0 * s0 + x0, e1 = v1 * s1 + x1, w0 = clamp_or_nan(e0, lim), w1 = clamp_or_nan(e1, lim);
-                    if (SPLIT && !FRAG) {
-                        const __nv_bfloat162 value = __floats2bfloat162_rn(w0, w1);
-                        *reinterpret_cast<__nv_bfloat162*>(out + fragment_index<1>(tok, row)) = value;
-                        *reinterpret_cast<__nv_bfloat162*>(out + fragment_index<1>(kSplitTokens + tok, row)) = __floats2bfloat162_rn(e0 - __low2float(value), e1 - __high2float(value));
-                        continue;
+#pragma unroll
+                    for (int u = 0; u < U; ++u) {
+                        const int tok = tok0 + u * tok_step;
+                        if (u && next == 0) break;
+                        if (kPair) { v0[u] += r0[u]; v1[u] += r1[u]; }      // (the same order of sums as above: a linear's bits do not depend on the block)
+                        float x0 = bi0, x1 = bi1, s0 = sc0, s1 = sc1;
+                        if (resid) {
+                            const uint16_t* const r = resid + tok * ld_res + row;
+                            x0 += float_of(r[0], io_bf16);
+                            if (both) x1 += float_of(r[1], io_bf16);
+                        }
+                        if (row_exp) { const float rs = exp2f((float)(exp_sign * row_exp[tok])); s0 *= rs; s1 *= rs; }
+                        const float e0 = v0[u] * s0 + x0, e1 = v1[u] * s1 + x1, w0 = clamp_or_nan(e0, lim), w1 = clamp_or_nan(e1, lim);
+                        if (SPLIT && !FRAG) {
+                            const __nv_bfloat162 value = __floats2bfloat162_rn(w0, w1);
+                            *reinterpret_cast<__nv_bfloat162*>(out + fragment_index<1>(tok, row)) = value;
+                            *reinterpret_cast<__nv_bfloat162*>(out + fragment_index<1>(kSplitTokens + tok, row)) = __floats2bfloat162_rn(e0 - __low2float(value), e1 - __high2float(value));
+                            continue;
+                        }
+                        uint32_t o;
+                        if (out_bf16) { const __nv_bfloat162 h = __floats2bfloat162_rn(w0, w1); o = *reinterpret_cast<const uint32_t*>(&h); }
+                        else { const __half2 h = __floats2half2_rn(w0, w1); o = *reinterpret_cast<const uint32_t*>(&h); }
+                        uint16_t* const dst = out + (frag ? fragment_index<NT>(tok, row) : tok * ld_out);
+                        if (pairs) *reinterpret_cast<uint32_t*>(dst) = o;
+                        else {
+                            dst[0] = (uint16_t)o;
+                            if (both) dst[1] = (uint16_t)(o >> 16);
+                        }
                     }
-                    uint32_t o;
-                    if (out_bf16) { const __nv_bfloat162 h = __floats2bfloat162_rn(w0, w1); o = *reinterpret_cast<const uint32_t*>(&h); }
-                    else { const __half2 h = __floats2half2_rn(w0, w1); o = *reinterpret_cast<const uint32_t*>(&h); }
-                    uint16_t* const dst = out + (frag ? fragment_index<NT>(tok, row) : tok * jb.ld_out + row);
-                    if (both && jb.whole) *reinterpret_cast<uint32_t*>(dst) = o;
-                    else {
-                        dst[0] = (uint16_t)o;
-                        if (both) dst[1] = (uint16_t)(o >> 16);
-                    }
+                };
+                if (tokens <= tok_step) {
+                    if ((tid >> pair_bits) < tokens) take(std::integral_constant<int, 1>{}, tid >> pair_bits);
+                } else {
+#pragma unroll 1
+                    for (int tok = tid >> pair_bits; tok < tokens; tok += 2 * tok_step) take(std::integral_constant<int, 2>{}, tok);
                 }
             }
         }
