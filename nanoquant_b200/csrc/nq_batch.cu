@@ -17,7 +17,7 @@
 //    shared memory with 16-byte copies, a chunk (half of one for two column groups) at a time: the 16 blocks of it are then ONE
 //    piece of code without a wait in between.  (Fragments loaded from rows touch eight lines each.)
 //  * A launch is a chain, and the warps of an SM are few: what counts is the length of a warp's path.  Pieces of 64 columns with a wait,
-//    a copy and 4 dependent MMAs each took 300 ns, whatever was in flight; a chunk with two accumulators in turn 900 ns for its 16 blocks.
+//    a copy and 4 dependent MMAs each took 300 ns, whatever was in flight; a chunk with two accumulators in turn 700 to 900 ns for its 16 blocks.
 //    Output scales and bias come by bulk copy beside the weights, the input scales are prefetched to L2.  Eight Qwen3-8B layers in
 //    a graph, 4 / 8 / 12 / 16 tokens: 326 / 336 / 423 / 430 us -> 305 / 311 / 390 / 400; Llama-3.2-1B 238 / 233 / 279 / 289 -> 226 / 207 / 249 / 258.
 //  * Two barriers; no K split over CTAs, no counters, no slabs.
@@ -27,9 +27,9 @@
 // It ends at 16 tokens (8 for large launches, see batch_max_tokens): 17 tokens took three column groups, eight Qwen3-8B layers 625 us, 473 through nq_wgemm.cu.
 //
 // What bounds it: the two stages of a group with little work are two launches of a fixed chain.  Stamps of o (4096 columns, 4 tokens; us after the last CTA
-// of the launch before): dependency 0.64, activations on their way 1.1, weights there 1.2, activations 1.5, products 2.5, outputs 3.1.  In launches
+// of the launch before): dependency 0.7, activations on their way 1.2, weights there 1.3, activations 1.55, products 2.4, outputs 3.0.  In launches
 // with much work the half-rate ALU pipe (a shift and a LOP3 per two weights, 16 clk of a scheduler per 16 x 16 weights, 12 with no shift)
-// beside 9 clk per MMA; gate/up's second stage 5 us of 9.  Two CTAs per SM (64 registers, or 256 threads), so that the next launch has its
+// beside 9 clk per MMA; gate/up's second stage 4.1 us of 7.4.  Two CTAs per SM (64 registers, or 256 threads), so that the next launch has its
 // weights before this one ends, lost 10 to 50 %: every phase is then longer.  The next stage's weights brought to L2 by this one: 1 to 4 % slower.
 #include <cstddef>
 #include <cstring>
@@ -544,19 +544,19 @@ static int batch_smem_limit(int* out) {
 // launches with much of both are faster through nq_wgemm.cu and nq_pgemm.cu.  The rule looks at each stage's packed factors, and either stage
 // decides for both.  Groups in a graph, bf16, 16 tokens: MB of the two stages, here / there in us; * marks what the rule sends there.
 //               q/k/v                        o                          gate/up                       down
-//   2048 cols   0.4 + 0.2   7.2 /  8.0      0.2 + 0.2   7.1 /  7.7      0.6 +  1.8   9.0 /  9.6       0.9 + 0.3   9.7 /  9.5
-//   4096        1.4 + 1.0  10.0 / 10.6      0.8 + 0.8   8.4 /  9.7      2.5 +  7.5  19.2 / 17.6       3.7 + 1.2  16.2 / 16.0
-//   5120        2.3 + 1.5  14.0 / 13.3      1.3 + 1.3  10.8 / 11.3      3.9 + 11.7  31.0 / 22.3 *     5.8 + 1.9  21.8 / 20.4 *
-//   6144        3.3 + 2.2  17.0 / 15.0      1.9 + 1.9  14.8 / 12.6      5.6 + 16.8  37.7 / 27.2 *     8.4 + 2.8  34.3 / 21.9 *
-//   8192        5.9 + 4.0  25.8 / 21.3 *    3.3 + 3.3  17.0 / 16.5     10.4 + 36.2  73.0 / 55.8 *    18.1 + 5.2  66.0 / 36.7 *
+//   2048 cols   0.4 + 0.2   6.2 /  8.0      0.2 + 0.2   6.0 /  7.9      0.6 +  1.8   7.7 /  9.4       0.9 + 0.3   7.8 /  9.4
+//   4096        1.4 + 1.0   8.8 / 10.3      0.8 + 0.8   7.3 /  9.6      2.5 +  7.5  16.4 / 16.9       3.7 + 1.2  14.4 / 15.1
+//   5120        2.3 + 1.5  11.5 / 12.2      1.3 + 1.3   8.8 / 10.9      3.9 + 11.7  22.8 / 21.5 *     5.8 + 1.9  18.0 / 19.1 *
+//   6144        3.3 + 2.2  12.4 / 13.3      1.9 + 1.9  11.9 / 12.2      5.6 + 16.8  28.5 / 26.1 *     8.4 + 2.8  21.0 / 20.6 *
+//   8192        5.9 + 4.0  14.2 / 17.7 *    3.3 + 3.3  13.9 / 15.6     10.4 + 36.2  58.2 / 52.8 *    18.1 + 5.2  45.7 / 33.3 *
 // (0.8 bits per weight, inner width 3 times the columns, 28672 at 8192.)  A layer of all four, us, all here / all there / by the rule:
-//   9 tokens    2048  31.3 / 34.3 / 31.3    4096  51.5 / 52.9 / 51.5    5120  75.6 / 65.3 / 67.3    6144   90.4 / 75.4 / 79.8
-//               8192 157.7 / 126.8 / 129.1  4096 at 1.5 bits  63.7 / 66.5 / 65.4    5120 at 1.2 bits  95.8 / 80.8 / 89.6
-//   16 tokens   2048  31.9 / 34.4 / 31.9    4096  53.4 / 52.9 / 53.5    5120  76.3 / 65.4 / 67.4    6144  102.8 / 75.3 / 81.1
-//               8192 180.3 / 126.8 / 129.6  4096 at 1.5 bits  70.4 / 66.5 / 67.3    5120 at 1.2 bits  96.6 / 80.9 / 89.2
-// Changing kernels inside a layer costs what a group of 4096 columns gains, so the lines (8 MB; 4.5 MB with 8192 columns) leave such layers in
-// one kernel: they are within 3 % of the better one.  From 5120 columns on they are on the safe side: all of a layer through the GEMMs would be
-// 1 to 11 % faster still.  (A line at 4.5 MB for any K changes no layer from 5120 columns on, and loses 2 to 4 % at 4096.)
+//   9 tokens    2048  26.3 / 34.5 / 26.2    4096  44.2 / 51.2 / 44.2    5120  59.1 / 62.8 / 60.8    6144   72.3 / 73.0 / 70.9
+//               8192 126.5 / 117.9 / 117.5  4096 at 1.5 bits  55.7 / 65.2 / 61.7    5120 at 1.2 bits  74.1 / 76.9 / 77.7
+//   16 tokens   2048  26.6 / 34.4 / 26.8    4096  46.1 / 51.3 / 46.2    5120  61.4 / 62.8 / 61.7    6144   74.9 / 72.9 / 71.9
+//               8192 132.1 / 118.1 / 117.9  4096 at 1.5 bits  60.1 / 65.4 / 62.8    5120 at 1.2 bits  77.9 / 77.1 / 78.7
+// The lines (8 MB; 4.5 MB with 8192 columns) were drawn for an earlier main loop, 15 % slower.  They leave layers in one kernel or send there what
+// still belongs there, within 3 % of the better one, except nine tokens of 4096 columns at 1.5 bits (11 %) and of 5120 at 1.2 (5 %): lines at 16 MB, and
+// 8 MB with 8192 columns, would be better now (tests/test_gemm_edges_gpu.py holds the present ones).
 int batch_max_tokens(const StageJob* jobs, int n) {
     double bytes = 0;                       // of this stage
     int most_k = 0;
