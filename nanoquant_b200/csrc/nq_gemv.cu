@@ -807,15 +807,13 @@ static size_t intermediate_bytes(int R) { return round_up((size_t)kMaxTok * (siz
 // linears of a group share, so that a group is not torn apart.  The line: input of 14 chunks and more (above 3328
 // columns).  us at four tokens, 0.8 bits per weight, one launch -> two:
 //                                    2048 columns       3072              3584              4096              8192
-//   q/k/v, in a graph                6.6 -> 5.9        8.5 -> 6.5        9.2 -> 7.2       10.1 -> 7.9       17.4 -> 17.3
-//   gate/up, in a graph              9.3 -> 7.6       11.5 -> 11.2      13.9 -> 13.8      15.4 -> 16.4      39.5 -> 48.3
-//   square linear alone, in a graph  6.7 -> 6.1        8.4 -> 6.2        9.0 -> 6.5        9.5 -> 6.6       15.7 -> 13.2
-//   square linear called eagerly     6.8 -> 8.5        8.5 -> 8.6        9.4 -> 9.1        9.8 -> 8.9       15.9 -> 13.5
-//   its quarter (k) called eagerly   6.3 -> 8.4        6.6 -> 8.5        7.1 -> 8.4        7.2 -> 8.6       11.0 -> 8.7
-// A graph gains from 2048 columns on, but a call in a stream is bound by the host there, which pays 2.3 us for the second
-// launch; from 3584 on the seven linears of a layer gain called one by one as well, though not the smallest of them.  Groups
-// of more than some 9 MB of factors lose (gate/up at 8192 columns), because the batch kernel computes all eight columns:
-// that is the price of a rule that does not see the group.
+//   q/k/v, in a graph                6.2 -> 4.8        7.8 -> 5.2        8.8 -> 6.2        8.8 -> 6.5       14.9 -> 12.1
+//   gate/up, in a graph              7.9 -> 6.0       10.1 -> 8.0       12.4 -> 9.3       13.8 -> 11.1      40.5 -> 36.5
+//   square linear alone, in a graph  6.0 -> 4.7        7.2 -> 5.1        8.0 -> 5.4        8.3 -> 5.7       13.8 -> 9.6
+//   square linear called eagerly     5.8 -> 7.7        7.0 -> 7.9        7.9 -> 7.8        8.1 -> 7.9       13.7 -> 9.7
+//   its quarter (k) called eagerly   5.3 -> 7.5        6.1 -> 7.7        6.5 -> 7.6        6.6 -> 7.7        9.6 -> 7.7
+// A graph gains from 2048 columns on, but a call in a stream is bound by the host there, which pays 2 us for the second
+// launch; from 3584 on the seven linears of a layer gain called one by one as well, though not the smallest of them.
 constexpr int kTwoStageChunks = 14;
 static bool takes_two_stages(const nq_linear_desc& L) {
     return (L.N + 255) / 256 >= kTwoStageChunks && L.N % 8 == 0 && L.R % 8 == 0 && L.ldx % 8 == 0 && aligned16(L.x) &&
