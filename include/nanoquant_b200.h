@@ -251,7 +251,13 @@ int nq_gemm_set_precise_intermediate(int on);
  * once by the caller; a device-side wait that gives up sets its status word (nq_scratch_status).
  * Consecutive launches overlap through programmatic dependent launch: a
  * kernel loads activations and stores results only after the previous kernel
- * of the stream has completed.
+ * of the stream has completed.  Tiles may be read before, and so may scales and
+ * bias in the two GEMMs (17 tokens and more, large launches from nine on) and
+ * with the precise intermediate; the decode and the batch kernel (up to 16
+ * tokens) read scales and bias behind the kernels before the call.  This matters
+ * only where a kernel releases its dependents early, as the linears and the
+ * all-gather here do (the packers and the head do not): it must not write what a
+ * later call may read before, unless a kernel that does not lies between.
  * replaces: marlin_nanoquant_cuda, src/nanoquant/kernel/cuda/gemm.cpp:112-122
  * (schema src/nanoquant/kernel/pybind.cpp:99-104) */
 int nq_gemm_fwd(const void* x, const void* s_in, const void* v_tiles, const void* s_mid,

@@ -18,7 +18,7 @@
 //    piece of code without a wait in between.  (Fragments loaded from rows touch eight lines each.)
 //  * A launch is a chain, and the warps of an SM are few: what counts is the length of a warp's path.  Pieces of 64 columns with a wait,
 //    a copy and 4 dependent MMAs each took 300 ns, whatever was in flight; a chunk with two accumulators in turn 700 to 900 ns for its 16 blocks.
-//    Output scales and bias come by bulk copy beside the weights, the input scales are prefetched to L2.  Eight Qwen3-8B layers in
+//    A second stage's output scales and bias come by bulk copy beside the weights, the input scales are prefetched to L2.  Eight Qwen3-8B layers in
 //    a graph, 4 / 8 / 12 / 16 tokens: 326 / 336 / 423 / 430 us -> 305 / 311 / 390 / 400; Llama-3.2-1B 238 / 233 / 279 / 289 -> 226 / 207 / 249 / 258.
 //  * Two barriers; no K split over CTAs, no counters, no slabs.
 //
@@ -72,7 +72,7 @@ struct alignas(16) BatchJob {
     int cta0, g_q, g_r;      // first CTA of the range; row groups per CTA, one more for its first g_r CTAs
     int gb;                  // row groups per block
     uint8_t wk, wr;          // chunk slices x row slices of a CTA's work, one warp each
-    uint8_t bulk, whole;     // output scales and bias come by bulk copy beside the weights; two neighbouring outputs are one 4-byte store
+    uint8_t bulk, whole;     // output scales and bias come by bulk copy beside the weights (second stages); two neighbouring outputs are one 4-byte store
     int wk_magic, wr_magic;  // ceil(2^16 / .)
 };
 static_assert(sizeof(BatchJob) == 128, "128 bytes");
@@ -177,15 +177,17 @@ __global__ void __launch_bounds__(kBatchThreads, 1) batch_stage_kernel(const __g
     };
     const bool loader = tid == kLoader;
     const uint32_t const_bar = bars + 8 * kBatchSlots;
+    const bool bulk = FRAG && jb.bulk;
     if (loader) {
 #pragma unroll 1
         for (int s = 0; s < slots; ++s) load_block();
         if (!FRAG && jb.pre) asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(jb.pre), "r"(2 * K) : "memory");
-        const bool bulk = jb.bulk;
-        const uint32_t row_bytes = bulk ? 2u * min(groups * 16, rows - first * 16) : 0u;
-        mbar_expect_tx(const_bar, row_bytes * ((jb.post ? 1u : 0u) + (jb.bias ? 1u : 0u)));
-        if (bulk && jb.post) bulk_load(smem_u32(smem + P.post_off), static_cast<const uint16_t*>(jb.post) + first * 16, row_bytes, const_bar);
-        if (bulk && jb.bias) bulk_load(smem_u32(smem + P.bias_off), static_cast<const uint16_t*>(jb.bias) + first * 16, row_bytes, const_bar);
+        if (bulk) {
+            const uint32_t row_bytes = 2u * min(groups * 16, rows - first * 16);
+            mbar_expect_tx(const_bar, row_bytes * ((jb.post ? 1u : 0u) + (jb.bias ? 1u : 0u)));
+            if (jb.post) bulk_load(smem_u32(smem + P.post_off), static_cast<const uint16_t*>(jb.post) + first * 16, row_bytes, const_bar);
+            if (jb.bias) bulk_load(smem_u32(smem + P.bias_off), static_cast<const uint16_t*>(jb.bias) + first * 16, row_bytes, const_bar);
+        }
     }
     // this warp: chunks [c0, c1), row slice rw
     const int wk = jb.wk, wr = jb.wr;
@@ -235,6 +237,15 @@ __global__ void __launch_bounds__(kBatchThreads, 1) batch_stage_kernel(const __g
         const int nb = min(gb, groups - blk);
         const int r0 = (rw * nb * wr_magic) >> 16, r1 = rw < wr ? ((rw + 1) * nb * wr_magic) >> 16 : r0;
         const int row0 = (first + blk) * 16;
+        // Output scale and bias of row `tid` of the block, of a first stage: into registers before the main loop (asm: a plain 16-bit load is
+        // widened, that is waited for, at once).  Not by bulk copy ahead of the dependency wait: a kernel before a first stage may have let it in
+        // early and still be writing them.  (The predecessor of a second stage is the first stage of the same call, which lets it in behind its own wait.)
+        // Two stages in a graph, 8 copies of 4096 -> 1024 -> 4096, 5 / 16 tokens: 5.30 / 6.95 us with that copy, 5.16 / 6.94 so.
+        uint16_t post_raw = 0, bias_raw = 0;
+        if (!FRAG && tid < nb * 16 && row0 + tid < rows) {
+            if (jb.post) asm volatile("ld.global.nc.u16 %0, [%1];" : "=h"(post_raw) : "l"(static_cast<const uint16_t*>(jb.post) + row0 + tid));
+            if (jb.bias) asm volatile("ld.global.nc.u16 %0, [%1];" : "=h"(bias_raw) : "l"(static_cast<const uint16_t*>(jb.bias) + row0 + tid));
+        }
 #pragma unroll 1
         for (int rb = r0; rb < r1; rb += kRows) {
             const int nr = min(kRows, r1 - rb);
@@ -253,7 +264,7 @@ __global__ void __launch_bounds__(kBatchThreads, 1) batch_stage_kernel(const __g
             }
             auto wait_weights = [&]() {
 #pragma unroll 1
-                for (unsigned spins = 0; !(mbar_try(bars + 8 * slot, parity) && mbar_try(const_bar, 0)); ++spins)
+                for (unsigned spins = 0; !(mbar_try(bars + 8 * slot, parity) && (!bulk || mbar_try(const_bar, 0))); ++spins)
                     if (spins >= kWeightWaitLimit) { atomicExch(P.status, (unsigned)(-NQ_ERR_TIMEOUT)); break; }
             };
             if (!FRAG && rb == r0) wait_weights();
@@ -368,6 +379,10 @@ __global__ void __launch_bounds__(kBatchThreads, 1) batch_stage_kernel(const __g
                 }
         }
         const int io_bf16 = P.io_bf16, out_bf16 = P.out_bf16;
+        if (!FRAG && tid < nb * 16) {
+            reinterpret_cast<uint16_t*>(smem + P.post_off)[tid] = post_raw;
+            reinterpret_cast<uint16_t*>(smem + P.bias_off)[tid] = bias_raw;
+        }
         __syncthreads();   // partial sums complete, this block's weights have been read
         if (++slot == slots) { slot = 0; parity ^= 1u; }
         if (loader) load_block();
@@ -383,9 +398,8 @@ __global__ void __launch_bounds__(kBatchThreads, 1) batch_stage_kernel(const __g
         const uint16_t* const resid = static_cast<const uint16_t*>(jb.resid);
         const int* const row_exp = jb.row_exp;
         // output scale and bias of a row of the block, from the copies in shared memory or as they lie in memory
-        const bool bulk = jb.bulk;
         auto row_value = [&](const void* global, int copy, int idx) {
-            return float_of(bulk ? reinterpret_cast<const uint16_t*>(smem + copy)[blk * 16 + idx] : static_cast<const uint16_t*>(global)[row0 + idx], io_bf16);
+            return float_of(!FRAG || bulk ? reinterpret_cast<const uint16_t*>(smem + copy)[(FRAG ? blk * 16 : 0) + idx] : static_cast<const uint16_t*>(global)[row0 + idx], io_bf16);
         };
         const int kslice = T * tok_stride, frag_out = P.frag_out, t_magic = P.t_magic, tokens = SPLIT ? kSplitTokens : T;
         const int sums = tokens * nb * 16 * (kPair ? 2 : 1);
@@ -625,7 +639,10 @@ int launch_batch_stage(const StageJob* jobs, int n, int tokens, StageTypes ty, i
         j.g_r = groups[i] % ncta[i];
         const size_t bytes = (size_t)(j.g_q + (j.g_r ? 1 : 0)) * 32;
         j.bulk = (!S.post || aligned16(S.post)) && (!S.bias || aligned16(S.bias)) && S.Nout % 8 == 0 && bytes <= kMostRowBytes;
-        if (j.bulk && bytes > row_bytes) row_bytes = bytes;
+        if (!frag_in || j.bulk) {       // (of a first stage: of a block)
+            const size_t kept = frag_in || bytes < 32 * kMostBlock ? bytes : 32 * kMostBlock;
+            if (kept > row_bytes) row_bytes = kept;
+        }
         j.whole = frag_out || (reinterpret_cast<uintptr_t>(S.out) % 4 == 0 && S.ld_out % 2 == 0);
         memset(P.cta_job + cta, i, (size_t)ncta[i]);
         cta += ncta[i];

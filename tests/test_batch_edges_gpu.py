@@ -61,7 +61,7 @@ def test_batch_tile_edges(shapes, T, dtype):
     ((8, 8, 700000), 5),                                  # more rows of a CTA than it keeps scales of
     ((28680, 2376, 48), 8),                               # one staged step per warp
 ])
-@pytest.mark.parametrize("shifted", [False, True])        # output scales and bias at an address that a bulk copy does not take
+@pytest.mark.parametrize("shifted", [False, True])        # scales of both stages and bias at an address that a bulk copy does not take
 def test_batch_blocks_of_outputs(shape, T, shifted):
     from nanoquant_b200 import ops
     dtype = torch.bfloat16
@@ -71,7 +71,48 @@ def test_batch_blocks_of_outputs(shape, T, shifted):
     bias = (torch.randn(L["M"], generator=g, device="cuda") * scale).to(dtype)
     resid = (torch.randn(T, L["M"], generator=g, device="cuda") * scale).to(dtype)
     move = lambda v: torch.cat([v[:1], v])[1:] if shifted else v
-    tens = (L["s_pre"], tiles_on_gpu(L["V"]), L["s_mid"], tiles_on_gpu(L["U"]), move(L["s_post"]), L["R"])
+    tens = (L["s_pre"], tiles_on_gpu(L["V"]), move(L["s_mid"]), tiles_on_gpu(L["U"]), move(L["s_post"]), L["R"])
     y = exact_np(ops.group_forward([L["x"]], [tens], T, dtype, torch.device("cuda", 0), [move(bias)], [resid])[0])
     want = L["y64"] + exact_np(bias) + exact_np(resid)
     assert float((np.abs(y - want) - bound(L, y, want, dtype)).max()) <= 0
+
+
+@pytest.mark.parametrize("T,single", [(4, False), (8, False), (16, False), (16, True)])
+def test_output_scales_written_by_the_kernel_before(T, single):
+    """The output scales of a first stage are the result of the linear directly before it on the stream, which lets its successor in early."""
+    from nanoquant_b200 import _lib, ops
+    dtype, dev = torch.bfloat16, torch.device("cuda", 0)
+    # few CTAs, a long chunk loop; four tokens of more than 3328 columns take the batch kernel
+    A, B = make_group([(8192, 64, 1032), (4104, 1032, 264)], T, dtype, seed=T)
+    tiles = {id(L): (tiles_on_gpu(L["V"]), tiles_on_gpu(L["U"])) for L in (A, B)}
+    tens = lambda L, mid: (L["s_pre"], tiles[id(L)][0], mid, tiles[id(L)][1], L["s_post"], L["R"])
+    ops.reserve_scratch(dev, max(ops.group_scratch_bytes([(L["N"], L["R"], L["M"])], T) for L in (A, B)))
+    x = A["x"][:1].clone()
+    out, status = torch.empty(T, B["R"], dtype=dtype, device=dev), torch.zeros(64, dtype=torch.int32, device=dev)
+
+    def use(scales):
+        if not single:
+            return ops.group_forward([B["x"]], [tens(B, scales)], T, dtype, dev)[0]
+        _lib.check(_lib.lib().nq_onebit_gemm_fwd(B["x"].data_ptr(), tiles[id(B)][0].data_ptr(), B["s_pre"].data_ptr(), scales.data_ptr(), out.data_ptr(),
+                                                 status.data_ptr(), T, B["N"], B["R"], _lib.NQ_BF16, torch.cuda.current_stream().cuda_stream), "nq_onebit_gemm_fwd")
+        return out
+
+    def both():
+        scales = ops.group_forward([x], [tens(A, A["s_mid"])], 1, dtype, dev)[0].view(-1)
+        return scales, use(scales)
+
+    stream = torch.cuda.Stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(stream):
+        both()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            scales, y = both()
+    torch.cuda.current_stream().wait_stream(stream)
+    for i in range(8):
+        x.copy_(torch.randn_like(x))          # other scales in the same place
+        torch.cuda.synchronize()
+        graph.replay()
+        torch.cuda.synchronize()
+        got, now = y.clone(), scales.clone()
+        assert torch.equal(got, use(now)), f"replay {i}"
