@@ -237,12 +237,13 @@ __global__ void __launch_bounds__(kBatchThreads, 1) batch_stage_kernel(const __g
         const int nb = min(gb, groups - blk);
         const int r0 = (rw * nb * wr_magic) >> 16, r1 = rw < wr ? ((rw + 1) * nb * wr_magic) >> 16 : r0;
         const int row0 = (first + blk) * 16;
-        // Output scale and bias of row `tid` of the block, of a first stage: into registers before the main loop (asm: a plain 16-bit load is
-        // widened, that is waited for, at once).  Not by bulk copy ahead of the dependency wait: a kernel before a first stage may have let it in
-        // early and still be writing them.  (The predecessor of a second stage is the first stage of the same call, which lets it in behind its own wait.)
-        // Two stages in a graph, 8 copies of 4096 -> 1024 -> 4096, 5 / 16 tokens: 5.30 / 6.95 us with that copy, 5.16 / 6.94 so.
+        // Output scale and bias of row `tid` of the block, where they do not come by bulk copy: into registers before the main loop (asm: a plain
+        // 16-bit load is widened, that is waited for, at once).  Those of a first stage are not copied ahead of the dependency wait: a kernel
+        // before it may have let it in early and still be writing them.  (The predecessor of a second stage is the first stage of the same call, which lets it
+        // in behind its own wait.)  Two stages in a graph, 8 copies of 4096 -> 1024 -> 4096, 5 / 16 tokens: 5.30 / 6.95 us with that copy, 5.16 / 6.94 so; with
+        // 4099 outputs and a bias 5.55 / 7.26 when a second stage read them behind its last barrier, 5.25 / 6.95 so; 700000 outputs, 8 tokens, 39.1 -> 36.0.
         uint16_t post_raw = 0, bias_raw = 0;
-        if (!FRAG && tid < nb * 16 && row0 + tid < rows) {
+        if (!bulk && tid < nb * 16 && row0 + tid < rows) {
             if (jb.post) asm volatile("ld.global.nc.u16 %0, [%1];" : "=h"(post_raw) : "l"(static_cast<const uint16_t*>(jb.post) + row0 + tid));
             if (jb.bias) asm volatile("ld.global.nc.u16 %0, [%1];" : "=h"(bias_raw) : "l"(static_cast<const uint16_t*>(jb.bias) + row0 + tid));
         }
@@ -379,7 +380,7 @@ __global__ void __launch_bounds__(kBatchThreads, 1) batch_stage_kernel(const __g
                 }
         }
         const int io_bf16 = P.io_bf16, out_bf16 = P.out_bf16;
-        if (!FRAG && tid < nb * 16) {
+        if (!bulk && tid < nb * 16) {
             reinterpret_cast<uint16_t*>(smem + P.post_off)[tid] = post_raw;
             reinterpret_cast<uint16_t*>(smem + P.bias_off)[tid] = bias_raw;
         }
@@ -397,10 +398,8 @@ __global__ void __launch_bounds__(kBatchThreads, 1) batch_stage_kernel(const __g
         const float lim = P.saturate || (SPLIT && !FRAG) ? (out_bf16 ? 3.3895313892515355e+38f : 64504.0f) : 3.4e38f;
         const uint16_t* const resid = static_cast<const uint16_t*>(jb.resid);
         const int* const row_exp = jb.row_exp;
-        // output scale and bias of a row of the block, from the copies in shared memory or as they lie in memory
-        auto row_value = [&](const void* global, int copy, int idx) {
-            return float_of(!FRAG || bulk ? reinterpret_cast<const uint16_t*>(smem + copy)[(FRAG ? blk * 16 : 0) + idx] : static_cast<const uint16_t*>(global)[row0 + idx], io_bf16);
-        };
+        // output scale and bias of a row of the block
+        auto row_value = [&](int copy, int idx) { return float_of(reinterpret_cast<const uint16_t*>(smem + copy)[(bulk ? blk * 16 : 0) + idx], io_bf16); };
         const int kslice = T * tok_stride, frag_out = P.frag_out, t_magic = P.t_magic, tokens = SPLIT ? kSplitTokens : T;
         const int sums = tokens * nb * 16 * (kPair ? 2 : 1);
         if (sums <= kBatchThreads) {
@@ -415,8 +414,8 @@ __global__ void __launch_bounds__(kBatchThreads, 1) batch_stage_kernel(const __g
                 if (kPair) v += __shfl_xor_sync(0xffffffffu, v, 1);
                 if (tid < sums && row < rows && !(kPair && (lane & 1))) {
                     const float rs = row_exp ? exp2f((float)(P.exp_sign * row_exp[tok])) : 1.f;
-                    const float sc = jb.post ? row_value(jb.post, P.post_off, idx) : 1.f;
-                    float extra = jb.bias ? row_value(jb.bias, P.bias_off, idx) : 0.f;
+                    const float sc = jb.post ? row_value(P.post_off, idx) : 1.f;
+                    float extra = jb.bias ? row_value(P.bias_off, idx) : 0.f;
                     if (resid) extra += float_of(resid[tok * jb.ld_res + row], io_bf16);
                     const float exact = v * (sc * rs) + extra, w = clamp_or_nan(exact, lim);
                     uint16_t* const out = static_cast<uint16_t*>(jb.out);
@@ -437,8 +436,8 @@ __global__ void __launch_bounds__(kBatchThreads, 1) batch_stage_kernel(const __g
             if (idx < nb * 16 && row < rows) {
                 const bool both = row + apart < rows;
                 float sc0 = 1.f, sc1 = 1.f, bi0 = 0.f, bi1 = 0.f;
-                if (jb.post) { sc0 = row_value(jb.post, P.post_off, idx); if (both) sc1 = row_value(jb.post, P.post_off, idx + apart); }
-                if (jb.bias) { bi0 = row_value(jb.bias, P.bias_off, idx); if (both) bi1 = row_value(jb.bias, P.bias_off, idx + apart); }
+                if (jb.post) { sc0 = row_value(P.post_off, idx); if (both) sc1 = row_value(P.post_off, idx + apart); }
+                if (jb.bias) { bi0 = row_value(P.bias_off, idx); if (both) bi1 = row_value(P.bias_off, idx + apart); }
                 uint16_t* const out = static_cast<uint16_t*>(jb.out) + (frag ? 0 : row);
                 const long long ld_out = jb.ld_out, ld_res = jb.ld_res;
                 const bool pairs = both && jb.whole;
@@ -638,11 +637,9 @@ int launch_batch_stage(const StageJob* jobs, int n, int tokens, StageTypes ty, i
         j.g_q = groups[i] / ncta[i];
         j.g_r = groups[i] % ncta[i];
         const size_t bytes = (size_t)(j.g_q + (j.g_r ? 1 : 0)) * 32;
-        j.bulk = (!S.post || aligned16(S.post)) && (!S.bias || aligned16(S.bias)) && S.Nout % 8 == 0 && bytes <= kMostRowBytes;
-        if (!frag_in || j.bulk) {       // (of a first stage: of a block)
-            const size_t kept = frag_in || bytes < 32 * kMostBlock ? bytes : 32 * kMostBlock;
-            if (kept > row_bytes) row_bytes = kept;
-        }
+        j.bulk = frag_in && (!S.post || aligned16(S.post)) && (!S.bias || aligned16(S.bias)) && S.Nout % 8 == 0 && bytes <= kMostRowBytes;
+        const size_t kept = j.bulk || bytes < 32 * kMostBlock ? bytes : 32 * kMostBlock;      // of all rows of a CTA, or of a block
+        if (kept > row_bytes) row_bytes = kept;
         j.whole = frag_out || (reinterpret_cast<uintptr_t>(S.out) % 4 == 0 && S.ld_out % 2 == 0);
         memset(P.cta_job + cta, i, (size_t)ncta[i]);
         cta += ncta[i];
