@@ -116,3 +116,52 @@ def test_output_scales_written_by_the_kernel_before(T, single):
         torch.cuda.synchronize()
         got, now = y.clone(), scales.clone()
         assert torch.equal(got, use(now)), f"replay {i}"
+
+
+def with_epilogue(layers, T, dtype, seed):
+    """Biases and residuals of the size of the outputs, and what is expected with them."""
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    draw = lambda shape, L: (torch.randn(shape, generator=g, device="cuda") * float(abs(L["y64"]).max())).to(dtype)
+    biases, resid = [draw((L["M"],), L) for L in layers], [draw((T, L["M"]), L) for L in layers]
+    return biases, resid, [L["y64"] + exact_np(b) + exact_np(r) for L, b, r in zip(layers, biases, resid)]
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("shapes,T", [(2 * [(8192, 5056, 264)], 7), (2 * [(8192, 5056, 264)], 8), (4 * [(2048, 5056, 64)], 5), (4 * [(2048, 5056, 64)], 8)])
+def test_first_stage_of_more_than_512_outputs_per_block(shapes, T, dtype):
+    """Rows two apart of the fragment order are stored together, one column group.  gate/up of 8192 columns: five row groups per CTA and a token per thread;
+    the others nine and up to two, the second of which does not exist for all threads at five tokens."""
+    from nanoquant_b200 import ops
+    layers = make_group(shapes, T, dtype, seed=T)
+    tens = [(L["s_pre"], tiles_on_gpu(L["V"]), L["s_mid"], tiles_on_gpu(L["U"]), L["s_post"], L["R"]) for L in layers]
+    biases, resid, wants = with_epilogue(layers, T, dtype, T)
+    ys = ops.group_forward([L["x"] for L in layers], tens, T, dtype, torch.device("cuda", 0), biases, resid)
+    for L, y, want in zip(layers, ys, wants):
+        y = exact_np(y)
+        assert float((np.abs(y - want) - bound(L, y, want, dtype)).max()) <= 0
+
+
+@pytest.mark.parametrize("T", [9, 16])
+def test_precise_intermediate_in_large_blocks(T):
+    """Powers of two per token taken out of more than 512 outputs per block, with a residual that is the output itself."""
+    from nanoquant_b200 import ops
+    dtype = torch.bfloat16
+    L = make_group([(1032, 1000, 10001)], T, dtype, seed=T)[0]
+    tens = (L["s_pre"], tiles_on_gpu(L["V"]), L["s_mid"], tiles_on_gpu(L["U"]), L["s_post"], L["R"])
+    x = L["x"].clone()
+    x[1] *= 2.0 ** 20          # powers of two that differ between the tokens
+    x[T - 1] *= 2.0 ** -20
+    token = np.ones((T, 1))
+    token[1], token[T - 1] = 2.0 ** 20, 2.0 ** -20
+    g = torch.Generator(device="cuda").manual_seed(T)
+    bias = (torch.randn(L["M"], generator=g, device="cuda") * float(abs(L["y64"]).max())).to(dtype)
+    resid = (torch.randn(T, L["M"], generator=g, device="cuda") * torch.from_numpy(token * np.abs(L["y64"]).max()).float().cuda()).to(dtype)
+    want = L["y64"] * token + exact_np(bias) + exact_np(resid)
+    old = ops.set_precise_intermediate(True)
+    try:
+        y = exact_np(ops.group_forward([x], [tens], T, dtype, x.device, [bias], [resid], out=resid)[0])
+    finally:
+        ops.set_precise_intermediate(old)
+    # 1e-3 of a token's largest product, the bar of this mode, and half a unit of the output
+    half_ulp = 2.0 ** (np.floor(np.log2(np.maximum(np.maximum(np.abs(y), np.abs(want)), 2.0 ** -126))) - 8)
+    assert (np.abs(y - want) <= 1e-3 * token * np.abs(L["y64"]).max(axis=1, keepdims=True) + half_ulp).all()

@@ -84,3 +84,14 @@ def test_group_equals_linears_alone_in_larger_blocks(dtype):
     for i, L in enumerate(layers):
         assert torch.equal(group[i], call([L], tiles[i:i + 1], 4, dtype)[0])
         assert_parity(exact_np(group[i]), L["y64"], dtype, rel=1e-4, what=f"linear {i}")
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_group_equals_linears_alone_in_larger_blocks_of_the_first_stage(dtype):
+    """A CTA has three row groups of the first stage of these linears alone and nine in the group: value and remainder stored one by one and by pairs."""
+    layers = make_group(4 * [(4096, 5000, 64)], 4, dtype, seed=7)
+    tiles = [(tiles_on_gpu(L["V"]), tiles_on_gpu(L["U"])) for L in layers]
+    group = call(layers, tiles, 4, dtype)
+    for i, L in enumerate(layers):
+        assert torch.equal(group[i], call([L], tiles[i:i + 1], 4, dtype)[0])
+        assert_parity(exact_np(group[i]), L["y64"], dtype, rel=1e-4, what=f"linear {i}")
