@@ -140,7 +140,8 @@ __device__ __forceinline__ void quantise_unit(float (&p)[8], unsigned char* xq_c
     m = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(m)));   // as bits: a NaN is above infinity
     float unit = m * (1.0f / (128.f * kQMax));
     if (!(m > 1e-31f && m < 1e37f)) {
-        // Beyond what the approximate reciprocal takes: the same integers from p * 2^64 or p * 2^-64.
+        // Below 1e-31 the scale of the integers overflows; above 2^126 (8.5e37) the reciprocal is subnormal, which the approximate one flushes to zero
+        // (1e37 keeps a distance from it).  There the same integers come from p * 2^64 or p * 2^-64.
         const float f = m > 0.f && m <= 1e-31f ? 1.8446744e19f : m >= 1e37f && m <= 3.4028235e38f ? 5.4210109e-20f : 0.f;
         // All zero, or not finite.  A value that is not finite makes the unit a NaN, and with it every sum over this
         // chunk and every output of this token, as the same sums in floating point would be (an infinity meets another of

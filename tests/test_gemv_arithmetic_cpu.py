@@ -118,3 +118,35 @@ def test_a_unit_that_takes_the_error_of_the_reciprocal():
             factor = np.float32(2.0 - np.float64(m) * np.float64(inv))
             unit = m * np.float32(1.0 / (128 * Q_MAX)) * factor
             assert np.abs(A * z * np.float64(unit) - p).max() <= np.abs(p).max() * (64 / (128 * Q_MAX) + 2.0 ** -21)
+
+
+def test_the_unit_times_the_scale_of_the_integers_is_one():
+    # The reciprocal moved by up to 2^-17 of itself: the unit that takes 2 - m * inv makes up for it to five roundings of 2^-24 (unit's constant and product,
+    # scale, factor, their product); without the factor, or with the error's sign the other way, it does not.
+    def worst(factor_of):
+        most = 0.0
+        for seed in range(1, 40):
+            m = np.float32(np.abs(products(seed)).max())
+            for steps in (-64, -9, -1, 0, 1, 9, 64):
+                inv = np.float32(1) / m
+                inv = np.float32(inv + steps * np.spacing(inv))
+                factor = np.float32(factor_of(np.float64(m) * np.float64(inv)))
+                unit = np.float32(m * np.float32(1.0 / (128 * Q_MAX))) * factor
+                scale = np.float32(Q_MAX) * inv
+                most = max(most, abs(np.float64(unit) * np.float64(scale) * 128 - 1))
+        return most
+    five_roundings = 5 * 2.0 ** -24 + 2.0 ** -33       # (the square of the largest error beside them)
+    assert worst(lambda m_inv: 2.0 - m_inv) <= five_roundings
+    assert worst(lambda m_inv: 1.0) > 8 * five_roundings
+    assert worst(lambda m_inv: m_inv) > 16 * five_roundings
+
+
+def test_reciprocals_above_2_to_126_are_subnormal():
+    # flushed to zero by the approximate reciprocal; maxima from 1e37 on are scaled by 2^-64 first, with the same integers
+    tiny = np.finfo(np.float32).tiny
+    above = np.nextafter(np.float32(2.0 ** 126), np.float32(np.inf))
+    assert 0 < np.float32(1) / above < tiny <= np.float32(1) / np.float32(2.0 ** 126) and np.float32(1e37) < above
+    p = (products(3) / np.abs(products(3)).max()).astype(np.float32)
+    want, _ = words_of(p)
+    got, m = words_of((p * np.float32(2.0 ** 127)) * np.float32(2.0 ** -64))
+    assert np.array_equal(got, want) and m == np.float32(2.0 ** 63)

@@ -75,6 +75,25 @@ def test_decode_kernel_large_activations(T, exponent):
     assert_parity(exact_np(gemv(L, x)), want, torch.bfloat16, rel=1e-4, what=f"2^{exponent}")
 
 
+@pytest.mark.parametrize("largest", [8.4e37, 8.6e37, 1.5e38, 2.5e38])
+@pytest.mark.parametrize("T", [1, 2, 3, 4])
+def test_decode_kernel_reciprocal_below_normal_numbers(T, largest):
+    # Above 2^126 = 8.5e37 the reciprocal of a maximum is subnormal (flushed, all integers would be zero).  Three columns of a token, whose sum
+    # stays finite: each is at most half an integer, 1.5e-5 of the maximum, off, the intermediate the same again, which averages over the rank.
+    N, R, M = 40, 136, 520
+    L = make_layer(N, R, M, T, torch.bfloat16, seed=5)
+    L["s_pre"] = torch.ones_like(L["s_pre"])
+    L["s_mid"] = torch.full_like(L["s_mid"], 2.0 ** -100)
+    x = torch.zeros_like(L["x"])
+    for t in range(T):
+        for k, part in enumerate((1.0, -0.25, 0.0625)):
+            x[t, (7 * t + 11 * k) % N] = largest * part
+    assert torch.isfinite(x).all() and ((x.abs().amax(dim=1) > 2.0 ** 126) == (largest > 8.5e37)).all()
+    from oracle import nanoquant_oracle as oc
+    want = oc.forward_fp64(exact_np(x), L["V"], L["U"], exact_np(L["s_pre"]), exact_np(L["s_mid"]), exact_np(L["s_post"]))
+    assert_parity(exact_np(gemv(L, x)), want, torch.bfloat16, rel=1e-4, what=f"{largest}")
+
+
 def dispatched(L, x, resid=None, precise=False):
     """A launch group of one, as the module calls it."""
     from nanoquant_b200 import ops
