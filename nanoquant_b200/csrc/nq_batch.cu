@@ -101,9 +101,6 @@ __device__ __forceinline__ void mma_16816(float (&d)[4], uint32_t a0, uint32_t a
 __device__ __forceinline__ float float_of(uint16_t h, int bf16) {
     return bf16 ? __uint_as_float((uint32_t)h << 16) : __half2float(__ushort_as_half(h));
 }
-// The bits of columns {0, 1} and {2, 3} of every four, 8 apart in a word, 16 apart: bytes {0, 1} and {2, 3} to bytes 1 and 3.
-__device__ __forceinline__ uint32_t spread01(uint32_t w) { return __byte_perm(w, 0u, 0x1404); }
-__device__ __forceinline__ uint32_t spread23(uint32_t w) { return __byte_perm(w, 0u, 0x3424); }
 __device__ __forceinline__ uint2 lds8(uint32_t addr) {
     uint2 v;
     asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(addr) : "memory");
@@ -321,8 +318,8 @@ __global__ void __launch_bounds__(kBatchThreads, 1) batch_stage_kernel(const __g
 #pragma unroll
                     for (int r = 0; r < kRows; ++r) {
                         const uint4 w = *reinterpret_cast<const uint4*>(wp + min(r, nr - 1) * w_row);
-                        p[r][0] = spread01(w.x); p[r][1] = spread23(w.x); p[r][2] = spread01(w.y); p[r][3] = spread23(w.y);
-                        p[r][4] = spread01(w.z); p[r][5] = spread23(w.z); p[r][6] = spread01(w.w); p[r][7] = spread23(w.w);
+                        p[r][0] = spread_bytes(w.x, 0); p[r][1] = spread_bytes(w.x, 1); p[r][2] = spread_bytes(w.y, 0); p[r][3] = spread_bytes(w.y, 1);
+                        p[r][4] = spread_bytes(w.z, 0); p[r][5] = spread_bytes(w.z, 1); p[r][6] = spread_bytes(w.w, 0); p[r][7] = spread_bytes(w.w, 1);
                     }
 #pragma unroll
                     for (int s0 = 0; s0 < 16; s0 += kStep) {

@@ -138,6 +138,8 @@ __device__ __forceinline__ uint32_t and_xor(uint32_t a, uint32_t m, uint32_t x) 
     asm("lop3.b32 %0, %1, %2, %3, 0x6A;" : "=r"(r) : "r"(a), "r"(m), "r"(x));   // 0x6A = (0xF0 & 0xCC) ^ 0xAA
     return r;
 }
+// Bytes {0, 1} and {2, 3} of a word to bytes 1 and 3: bits of neighbouring columns, 8 apart, are then 16 apart.
+__device__ __forceinline__ uint32_t spread_bytes(uint32_t w, int pair) { return __byte_perm(w, 0u, pair ? 0x3424 : 0x1404); }
 
 // ---------------------------------------------------------------------------
 // mbarriers and bulk copies

@@ -82,8 +82,6 @@ __device__ __forceinline__ void tmem_st_frag4(uint32_t taddr, const uint32_t (&v
                  "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
                  : "memory");
 }
-// Bytes {0, 1} and {2, 3} of a word to bytes 1 and 3: bits of neighbouring columns, 8 apart, are then 16 apart.
-__device__ __forceinline__ uint32_t spread_bytes(uint32_t w, int pair) { return __byte_perm(w, 0u, pair ? 0x3424 : 0x1404); }
 // 64 columns of 16 rows: `w` with the bits of column class j at 8 b + j + 4 - (j & 4), half `hf` of the 128 columns -> the words of
 // tcgen05.st 16x256b.x4, +-pn.  Two ALU operations per two weights, and a PRMT per two words for all eight classes.  (A PRMT that spreads sign bits
 // per two weights beside half a shift before: two layers of 64 / 128 / 256 / 517 tokens, Qwen3-8B 133.6 / 164.2 / 223.0 / 335.8 -> 130.2 /
