@@ -279,7 +279,7 @@ int nq_gemm_group_fwd(const nq_linear_desc* linears_host, int n_linears, int T, 
 enum { NQ_KERNEL_BATCH = 0, NQ_KERNEL_WGEMM = 1, NQ_KERNEL_PGEMM = 2 };
 int nq_gemm_group_kernels(const nq_linear_desc* linears_host, int n_linears, int T, int* kernels_host);
 
-/* Attempts (of about 5 us each, after a first one) that a wait inside the two GEMM kernels (17 tokens and more, and large launches from nine on) may
+/* Attempts (of about 4 us each, after a first one) that a wait inside the two GEMM kernels (17 tokens and more, and large launches from nine on) may
  * spend before the launch gives up and sets the status word (NQ_ERR_TIMEOUT); its results are then void.  0 restores the default
  * (2^21, seconds).  Host-side setting read at launch time; returns the previous value.  For failure-path tests and for callers that
  * want a tighter bound. */

@@ -20,6 +20,7 @@
 //    a copy and 4 dependent MMAs each took 300 ns, whatever was in flight; a chunk with two accumulators in turn 700 to 900 ns for its 16 blocks.
 //    A second stage's output scales and bias come by bulk copy beside the weights, the input scales are prefetched to L2.  Eight Qwen3-8B layers in
 //    a graph, 4 / 8 / 12 / 16 tokens: 326 / 336 / 423 / 430 us -> 305 / 311 / 390 / 400; Llama-3.2-1B 238 / 233 / 279 / 289 -> 226 / 207 / 249 / 258.
+//    With the steps beside the code below: 264 / 273 / 362 / 369; Llama-3.2-1B 222 / 191 / 239 / 242.
 //  * Two barriers; no K split over CTAs, no counters, no slabs.
 //
 // Splitting K over the CTAs of a cluster (partial sums exchanged through distributed shared memory) and staging the whole
@@ -386,7 +387,7 @@ __global__ void __launch_bounds__(kBatchThreads, 1) batch_stage_kernel(const __g
         if (loader) load_block();
         // Outputs.  Up to 512 of them are dealt to the threads one by one; of a split intermediate two neighbouring lanes sum value and
         // remainder.  Larger blocks by two rows (two apart where they are neighbours in the next stage's fragments) of every tok_step-th
-        // token, with their scales converted once: the outputs of gate/up's second stage took 1.8 us of 9, now 1.  Eight Qwen3-8B layers, 4 / 8 / 12 /
+        // token, with their scales converted once: the outputs of gate/up's second stage took 1.8 us of 9, now 1.1.  Eight Qwen3-8B layers, 4 / 8 / 12 /
         // 16 tokens: 305 / 311 / 390 / 400 us -> 296 / 307 / 377 / 388; two of 8192 columns, 4 tokens, 192.8 -> 188.8.  (All blocks that way: one more
         // dependent step where there are few outputs, Llama-3.2-1B 226 -> 229 and, eight tokens, 207 -> 213.)
         // An intermediate that is not a pair becomes infinite beyond its type's range, as in the GEMM; the value of a pair
@@ -566,7 +567,8 @@ static int batch_smem_limit(int* out) {
 //               8192 132.1 / 118.1 / 117.9  4096 at 1.5 bits  60.1 / 65.4 / 62.8    5120 at 1.2 bits  77.9 / 77.1 / 78.7
 // The lines (8 MB; 4.5 MB with 8192 columns) were drawn for an earlier main loop, 15 % slower.  They leave layers in one kernel or send there what
 // still belongs there, within 3 % of the better one, except nine tokens of 4096 columns at 1.5 bits (11 %) and of 5120 at 1.2 (5 %): lines at 16 MB, and
-// 8 MB with 8192 columns, would be better now (tests/test_gemm_edges_gpu.py holds the present ones).
+// 8 MB with 8192 columns, would be better for those, but every line in MB is wrong somewhere in this table (down of 5120 columns, q/k/v of 8192): what
+// should decide is a predicted time, as between the two GEMMs.
 int batch_max_tokens(const StageJob* jobs, int n) {
     double bytes = 0;                       // of this stage
     int most_k = 0;

@@ -155,10 +155,10 @@ __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
-// One bounded attempt: the hardware suspends the thread until the phase completes or its own limit (4 us here) runs out, so
-// a waiting warp does not compete for issue slots.  (No time hint: with one of 2 us the limit was the same, but an attempt on a phase that
-// is already complete took 107 to 134 clk instead of 64 to 82.  Eight layers: one to sixteen tokens 0.2 to 0.6 % faster, two layers
-// through the GEMMs 0.5 to 1 %.)
+// One bounded attempt: the hardware suspends the thread until the phase completes or its own limit (7760 clk, 4 us; the cluster form in
+// nq_tcgen05.cuh has the same) runs out, so a waiting warp does not compete for issue slots.  (No time hint: with one of 2 us the limit was
+// 7850 clk, but an attempt on a phase that is already complete took 107 to 134 clk instead of 64 to 82.  Eight layers: one to sixteen tokens
+// 0.2 to 0.6 % faster, two layers through the GEMMs 0.5 to 1 %.)
 __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
     uint32_t ok;
     asm volatile(

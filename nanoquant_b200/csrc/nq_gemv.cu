@@ -906,10 +906,10 @@ static int launch_decode(const nq_linear_desc* d, int n_linears, int t_first, in
     // One CTA per SM, fewer for launches with less than 2.25 MB of packed factors: their row groups do not divide any finer by
     // 148, every CTA fetches the whole input and polls the whole intermediate, and the SMs left free let CTAs of the next launch in.  One
     // token, us per launch in a graph by CTAs (52 / 74 / 103 / 148):
-    //   0.4 MB (4096 -> 1024)  4.7 / 4.6 / 4.7 / 4.6      2.1 MB (8192 -> 2048)           6.3 / 6.1 / 5.9 / 5.9
-    //   0.7 MB (q/k/v of 2048) 4.7 / 4.6 / 4.7 / 4.8      2.4 MB (q/k/v of 4096)          6.3 / 5.8 / 5.5 / 5.4
-    //   1.7 MB (4096 -> 4096)  5.7 / 5.4 / 5.3 / 5.3      4.1 MB (gate/up of 2048)        8.8 / 6.8 / 6.5 / 5.9
-    //   1.8 MB (3072 -> 3072)  5.7 / 5.4 / 5.3 / 5.5      5.0 MB (12288 -> 4096)          9.6 / 9.3 / 7.5 / 7.3
+    //   0.4 MB (4096 -> 1024)  4.5 / 4.5 / 4.5 / 4.5      2.1 MB (8192 -> 2048)           6.0 / 5.8 / 5.7 / 5.7
+    //   0.7 MB (q/k/v of 2048) 4.5 / 4.4 / 4.5 / 4.5      2.4 MB (q/k/v of 4096)          6.1 / 5.7 / 5.2 / 5.2
+    //   1.7 MB (4096 -> 4096)  5.4 / 5.2 / 5.2 / 5.2      4.1 MB (gate/up of 2048)        8.6 / 6.5 / 6.3 / 5.7
+    //   1.8 MB (3072 -> 3072)  5.5 / 5.2 / 5.1 / 5.2      5.0 MB (12288 -> 4096)          9.3 / 8.9 / 7.2 / 7.0
     // (While the intermediate was polled in 16-byte loads the line was at 3 MB.  Eight layers, 3 MB and now, one / two / three tokens: 4096
     // columns 216.0 / 253.8 / 331.4 -> 215.3 / 252.2 / 328.9, 3072 columns 188.8 / 217.5 / 276.9 -> 187.4 / 215.2 / 273.0.)
     int grid = sm_count() < kMaxCtas ? sm_count() : kMaxCtas;

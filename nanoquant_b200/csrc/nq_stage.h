@@ -47,7 +47,7 @@ int launch_batch_stage(const StageJob* jobs, int n, int T, StageTypes ty, int sa
 // Tensor map of a stage's activations: boxes of 64 columns x `box_rows` tokens, 128-byte swizzle.
 int encode_activations(CUtensorMap* map, const StageJob& S, int bf16, int T, int box_rows);
 
-// Attempts (of some 5 us each) that a wait inside the GEMMs may spend before it gives up (nq_gemm_set_wait_limit).
+// Attempts (of some 4 us each) that a wait inside the GEMMs may spend before it gives up (nq_gemm_set_wait_limit).
 unsigned gemm_wait_limit();
 
 // GEMMs with the weights on the row side of the MMA; `us` is the predicted time of the launch.

@@ -18,7 +18,7 @@ __device__ __forceinline__ bool mbar_try_cluster(uint32_t bar, uint32_t parity) 
         : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
     return ok != 0;
 }
-// Bounded wait of a whole warp on an mbarrier phase; every lane returns the same.  False when `limit` more attempts (of some 5 us each)
+// Bounded wait of a whole warp on an mbarrier phase; every lane returns the same.  False when `limit` more attempts (of some 4 us each)
 // after the first were in vain, which sets the status word, or when another warp of the CTA has already given up; the caller then leaves
 // its loop.  `status` and `limit` are taken from the kernel's parameters (__grid_constant__): as constants they occupy no registers.  Read from
 // the descriptors' copy in shared memory both GEMMs spilled 8 to 16 bytes (128 tokens module by module 135 -> 133 us without, 517 tokens 186 -> 183).
